@@ -8,12 +8,17 @@ from __future__ import annotations
 
 import ctypes
 import functools
+import importlib.util
 import os
 from pathlib import Path
+from types import ModuleType
 
 LIBRARY_NAME = "libflashim_sm100.so"
 #: the in-tree build; ``FLASHIM_B200_LIBRARY`` names another build of the same sources (e.g. one with measurement probes)
 LIBRARY_PATH = Path(os.environ.get("FLASHIM_B200_LIBRARY") or Path(__file__).resolve().parent / "_lib" / LIBRARY_NAME)
+
+#: the native host path of the ops (a Python extension module, ``csrc/host.cpp``)
+HOST_PATH = Path(__file__).resolve().parent / "_lib" / "_fim_host.so"
 
 DTYPE_F32, DTYPE_BF16 = 0, 1
 ACT = {"none": 0, "relu": 1, "gelu": 2, "relu_early": 3}
@@ -106,8 +111,19 @@ def library() -> ctypes.CDLL:
     return lib
 
 
+@functools.cache
+def host() -> ModuleType:
+    """The extension module with one native call per op. Its ``bind`` has to run before the first call."""
+    if not HOST_PATH.is_file():
+        raise NativeLibraryMissing(f"{HOST_PATH} is missing: build it with `python -m flashim_b200.build_native`")
+    spec = importlib.util.spec_from_file_location("_fim_host", HOST_PATH)
+    module = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(module)
+    return module
+
+
 def available() -> bool:
-    return LIBRARY_PATH.is_file()
+    return LIBRARY_PATH.is_file() and HOST_PATH.is_file()
 
 
 def check(code: int, what: str) -> None:

@@ -10,8 +10,9 @@ FlashIM's own ``flashim.ops`` (see ``flashim_b200.integration``).
 from __future__ import annotations
 
 import ctypes
+import functools
 import os
-from collections import OrderedDict
+import warnings
 
 import torch
 from torch import Tensor
@@ -498,22 +499,21 @@ def _(value, input_bias, exponent):
 
 # ---- weight-scale layout cache (ops whose signature carries plain int8 exponents) ----------------------------------------
 
-_SWIZZLED: OrderedDict = OrderedDict()
-
 
 def swizzled_weight_scales(weight_exponent: Tensor) -> Tensor:
     """The 128x4-swizzled E8M0 bytes of ``weight_exponent`` ``[Cout, K/32]``, computed once per tensor (keyed on its
-    storage, shape and version; the source tensor is kept alive by the entry so the key cannot be reused)."""
-    key = (weight_exponent.data_ptr(), tuple(weight_exponent.shape), weight_exponent._version, weight_exponent.device)
-    hit = _SWIZZLED.get(key)
-    if hit is not None:
-        _SWIZZLED.move_to_end(key)
-        return hit[1]
-    packed = swizzle_scales(weight_exponent)
-    _SWIZZLED[key] = (weight_exponent, packed)
-    if len(_SWIZZLED) > 512:
-        _SWIZZLED.popitem(last=False)
-    return packed
+    storage, shape and version; the cache lives in ``csrc/host.cpp`` and holds 512 tensors)."""
+    packed = _host().swizzled_scales(weight_exponent)  # (None: a tensor the cache cannot key)
+    return swizzle_scales(weight_exponent) if packed is None else packed
+
+
+@functools.cache
+def _host():
+    """The native host path, bound to the kernel library and to this module's status word and containers."""
+    module = _native.host()
+    module.bind(str(_native.LIBRARY_PATH), lambda index: status_word(torch.device("cuda", index)), _native.check,
+                check_status if _CHECK_EVERY_CALL else None, swizzle_scales, QuantizedTensor, Int8Tensor)
+    return module
 
 
 # ---- eligibility ---------------------------------------------------------------------------------------------------------
@@ -561,6 +561,17 @@ def register(ops=None, device_spec=None, feature=None) -> None:
         requires.append(feature.SM100A_KERNELS)
     have = _native.available
     act_code = _native.ACT
+    # the registry of this package takes the native call of each op beside its predicate and implementation
+    native = None
+    if own and have():
+        try:
+            native = _host()
+        except ImportError as error:  # built against another torch: the Python path below serves every call meanwhile
+            warnings.warn(f"{_native.HOST_PATH} does not load ({error}): rebuild it with `python -m flashim_b200.build_native`")
+
+    def sm100(op, requires, when):
+        direct = {"direct": getattr(native, op.name)} if native is not None and hasattr(native, op.name) else {}
+        return op.register("sm100", device=spec, requires=requires, priority=3, when=when, **direct)
 
     def mxfp8_when(x, channel_exponent, weight, weight_exponent, bias, kh, kw, sh, sw, ph, pw, dh, dw, *, relu=False,
                    residual=None, out_exponent=None):
@@ -574,7 +585,7 @@ def register(ops=None, device_spec=None, feature=None) -> None:
             and _residual_ok(residual, weight.shape[0])
         )
 
-    @ops.mxfp8_conv2d.register("sm100", device=spec, requires=requires, priority=3, when=mxfp8_when)
+    @sm100(ops.mxfp8_conv2d, requires, mxfp8_when)
     def mxfp8_conv2d(x, channel_exponent, weight, weight_exponent, bias, kh, kw, sh, sw, ph, pw, dh, dw, *, relu=False,
                      residual=None, out_exponent=None):
         mode = _native.OUT_BF16 if out_exponent is None else _native.OUT_E4M3_STATIC
@@ -601,7 +612,7 @@ def register(ops=None, device_spec=None, feature=None) -> None:
         )
 
     if hasattr(ops, "mxfp8_conv2d_fused"):
-        @ops.mxfp8_conv2d_fused.register("sm100", device=spec, requires=requires, priority=3, when=fused_when)
+        @sm100(ops.mxfp8_conv2d_fused, requires, fused_when)
         def mxfp8_conv2d_fused(x, act_scale, weight, weight_scales, bias, kh, kw, sh, sw, ph, pw, dh, dw, *, act="none",
                                residual=None, out_exponent=None, dynamic_out=False, out_fp32=False):
             per_pixel = act_scale.dtype == torch.uint8
@@ -631,7 +642,7 @@ def register(ops=None, device_spec=None, feature=None) -> None:
                 and residual.dtype == torch.bfloat16 and residual.shape == x.shape
             )
 
-        @ops.mxfp8_gelu_mlp_residual.register("sm100", device=spec, requires=requires, priority=3, when=mlp_residual_when)
+        @sm100(ops.mxfp8_gelu_mlp_residual, requires, mlp_residual_when)
         def mxfp8_gelu_mlp_residual(x, x_scales, w1, w1_scales, b1, w2, w2_scales, b2, residual):
             return mxfp8_gelu_mlp_residual_launch(x, x_scales, w1, w1_scales, b1.contiguous(), w2, w2_scales, b2.contiguous(), residual)
 
@@ -649,7 +660,7 @@ def register(ops=None, device_spec=None, feature=None) -> None:
         )
 
     if hasattr(ops, "mxfp8_conv2d_bf16"):
-        @ops.mxfp8_conv2d_bf16.register("sm100", device=spec, requires=requires, priority=3, when=bf16_in_when)
+        @sm100(ops.mxfp8_conv2d_bf16, requires, bf16_in_when)
         def mxfp8_conv2d_bf16(x, act_exponent, weight, weight_scales, bias, *, act="none", residual=None, out_exponent=None,
                               dynamic_out=False, out_fp32=False):
             if out_fp32:
@@ -673,7 +684,7 @@ def register(ops=None, device_spec=None, feature=None) -> None:
             and _residual_ok(residual, weight.shape[0])
         )
 
-    @ops.int8_conv2d.register("sm100", device=spec, requires=requires, priority=3, when=int8_when)
+    @sm100(ops.int8_conv2d, requires, int8_when)
     def int8_conv2d(x, weight, a_scale, w_scale, bias, kh, kw, sh, sw, ph, pw, dh, dw, *, relu=False, residual=None,
                     out_scale=None):
         scale = None if out_scale is None else out_scale.to(device=x.device, dtype=torch.float32).reshape(1)
@@ -687,7 +698,7 @@ def register(ops=None, device_spec=None, feature=None) -> None:
             return (int8_when(x, weight, a_scale, w_scale, bias, kh, kw, sh, sw, ph, pw, dh, dw, relu=relu)
                     and _cuda(out_scale) and out_scale.numel() == 1 and weight.shape[0] % 8 == 0)
 
-        @ops.int8_conv2d_maxpool.register("sm100", device=spec, requires=requires, priority=3, when=pool_when)
+        @sm100(ops.int8_conv2d_maxpool, requires, pool_when)
         def int8_conv2d_maxpool(x, weight, a_scale, w_scale, bias, kh, kw, sh, sw, ph, pw, dh, dw, *, relu=False, out_scale):
             scale = out_scale.to(device=x.device, dtype=torch.float32).reshape(1)
             b, h, w, _ = x.shape
@@ -706,7 +717,7 @@ def register(ops=None, device_spec=None, feature=None) -> None:
                     and weight.is_contiguous()
                     and _conv_geometry_ok(x, weight.shape[0], weight.shape[1], kh, kw, sh, sw, ph, pw, dh, dw))
 
-        @ops.int8_conv2d_accumulators.register("sm100", device=spec, requires=requires, priority=3, when=acc_when)
+        @sm100(ops.int8_conv2d_accumulators, requires, acc_when)
         def int8_conv2d_accumulators(x, weight, kh, kw, sh, sw, ph, pw, dh, dw):
             return int8_conv2d_launch(x, weight, None, None, None, None, None, kh, kw, sh, sw, ph, pw, dh, dw, 0, _native.OUT_INT32)
 
@@ -723,7 +734,7 @@ def register(ops=None, device_spec=None, feature=None) -> None:
                 and (bias is None or (bias.dtype == torch.bfloat16 and bias.numel() == b_t.shape[1]))
             )
 
-        @ops.mxfp8_scaled_mm.register("sm100", device=spec, requires=requires, priority=3, when=scaled_mm_when)
+        @sm100(ops.mxfp8_scaled_mm, requires, scaled_mm_when)
         def mxfp8_scaled_mm(a, b_t, a_scale, b_scale, bias=None):
             m, k = a.shape
             out, _ = mxfp8_conv2d_launch(
@@ -744,7 +755,7 @@ def register(ops=None, device_spec=None, feature=None) -> None:
                                           and tuple(residual.shape) == (a.shape[0], weight.shape[0])))
             )
 
-        @ops.int8_linear.register("sm100", device=spec, requires=requires, priority=3, when=int8_linear_when)
+        @sm100(ops.int8_linear, requires, int8_linear_when)
         def int8_linear(a, weight, a_scale, w_scale, bias, *, relu=False, gelu=False, residual=None):
             # the linear's order is ReLU -> bf16 -> GELU -> residual (flashim/ops/gemm.py:87-98): its ReLU comes before the
             # residual, the conv's after it, hence the epilogue's own activation code
@@ -790,7 +801,7 @@ def register(ops=None, device_spec=None, feature=None) -> None:
         def linear_when(activation, bias, weight):
             return _quantized_ok(activation, weight) and _bias_exact_in_bf16(bias, weight.values.shape[0])
 
-        @ops.mxfp8_linear.register("sm100", device=spec, requires=requires, priority=3, when=linear_when)
+        @sm100(ops.mxfp8_linear, requires, linear_when)
         def mxfp8_linear(activation, bias, weight):
             values = activation.values.reshape(-1, activation.values.shape[-1])
             return _linear(values, activation.scale_exponent, bias, weight.values, weight.scale_exponent)
@@ -804,7 +815,7 @@ def register(ops=None, device_spec=None, feature=None) -> None:
                 and (input_bias is None or input_bias.numel() == value.shape[-1])
             )
 
-        @ops.gelu_quantize.register("sm100", device=spec, requires=dw_requires_early(feature), priority=3, when=gelu_quantize_when)
+        @sm100(ops.gelu_quantize, dw_requires_early(feature), gelu_quantize_when)
         def gelu_quantize(value, scale_exponent, approximate="none", *, input_bias=None):
             exponent = (scale_exponent if scale_exponent.dtype == torch.int8 else scale_exponent.to(torch.int8)).contiguous()
             bias = None if input_bias is None else input_bias.float().contiguous()
@@ -824,7 +835,7 @@ def register(ops=None, device_spec=None, feature=None) -> None:
                 and tuple(w2.scale_exponent.shape) == (w2.values.shape[0], hidden // 32) and w2.scale_exponent.dtype == torch.int8
             )
 
-        @ops.mxfp8_gelu_mlp.register("sm100", device=spec, requires=requires, priority=3, when=mlp_when)
+        @sm100(ops.mxfp8_gelu_mlp, requires, mlp_when)
         def mxfp8_gelu_mlp(x, w1, b1, hidden_exponent, w2):
             # three launches with the reference's rounding points: the first product rounds to bf16 before b1 is added,
             # GELU runs in fp32 on that sum, and the second product has no bias
@@ -840,7 +851,7 @@ def register(ops=None, device_spec=None, feature=None) -> None:
     def dw_when(value, weight, bias, *rest, **kw):
         return have() and _depthwise_ok(value, weight, bias)
 
-    @ops.depthwise5x5_relu_mxfp8.register("sm100", device=spec, requires=dw_requires, priority=3, when=dw_when)
+    @sm100(ops.depthwise5x5_relu_mxfp8, dw_requires, dw_when)
     def depthwise5x5_relu_mxfp8(value, weight, bias):
         q, scales = dw5x5_mxfp8(_nhwc(value), weight, bias, act_code["relu"], True)
         return q, scales.view(torch.float8_e8m0fnu)
@@ -848,7 +859,7 @@ def register(ops=None, device_spec=None, feature=None) -> None:
     def dw_int8_when(value, weight, bias, scale):
         return dw_when(value, weight, bias) and _cuda(scale) and scale.numel() == 1
 
-    @ops.depthwise5x5_relu_int8.register("sm100", device=spec, requires=dw_requires, priority=3, when=dw_int8_when)
+    @sm100(ops.depthwise5x5_relu_int8, dw_requires, dw_int8_when)
     def depthwise5x5_relu_int8(value, weight, bias, scale):
         return dw5x5_relu_int8(_nhwc(value), weight, bias, scale.float().reshape(1))
 
@@ -856,11 +867,11 @@ def register(ops=None, device_spec=None, feature=None) -> None:
         def dw_act_when(value, weight, bias, act="gelu"):
             return dw_when(value, weight, bias) and act in act_code
 
-        @ops.depthwise5x5_act.register("sm100", device=spec, requires=dw_requires, priority=3, when=dw_act_when)
+        @sm100(ops.depthwise5x5_act, dw_requires, dw_act_when)
         def depthwise5x5_act(value, weight, bias, act="gelu"):
             return dw5x5_bf16(_nhwc(value), weight, bias, act_code[act])
 
-        @ops.depthwise5x5_act_mxfp8.register("sm100", device=spec, requires=dw_requires, priority=3, when=dw_act_when)
+        @sm100(ops.depthwise5x5_act_mxfp8, dw_requires, dw_act_when)
         def depthwise5x5_act_mxfp8(value, weight, bias, act="gelu"):
             return dw5x5_mxfp8(_nhwc(value), weight, bias, act_code[act], True)
 
@@ -877,7 +888,7 @@ def register(ops=None, device_spec=None, feature=None) -> None:
                 and pw_bias.dtype == torch.bfloat16 and pw_bias.numel() == pw_weight.shape[0]
             )
 
-        @ops.depthwise5x5_relu_pointwise.register("sm100", device=spec, requires=requires, priority=3, when=dwpw_when)
+        @sm100(ops.depthwise5x5_relu_pointwise, requires, dwpw_when)
         def depthwise5x5_relu_pointwise(value, dw_weight, dw_bias, pw_weight, pw_bias):
             # two launches: the depthwise kernel writes its ReLU output once as bf16 (the rounding point of the reference),
             # the pointwise product is a bf16 tensor-core GEMM over the pixels with the bias in its epilogue
@@ -896,7 +907,7 @@ def register(ops=None, device_spec=None, feature=None) -> None:
                 and (pw_bias is None or (pw_bias.dtype == torch.bfloat16 and pw_bias.numel() == pw_weight.shape[0]))
             )
 
-        @ops.depthwise5x5_relu_pointwise_mxfp8.register("sm100", device=spec, requires=requires, priority=3, when=dwpw_mx_when)
+        @sm100(ops.depthwise5x5_relu_pointwise_mxfp8, requires, dwpw_mx_when)
         def depthwise5x5_relu_pointwise_mxfp8(value, dw_weight, dw_bias, pw_weight, pw_scale_swizzled, pw_scale_u8, pw_bias):
             # the producer's swizzled E8M0 tiles are what the GEMM's tensor-memory copies read: no re-layout in between
             b, c, h, w = value.shape
@@ -917,7 +928,7 @@ def register(ops=None, device_spec=None, feature=None) -> None:
                 and (pw_bias is None or (pw_bias.dtype == torch.bfloat16 and pw_bias.numel() == pw_weight.shape[0]))
             )
 
-        @ops.depthwise5x5_relu_pointwise_int8.register("sm100", device=spec, requires=requires, priority=3, when=dwpw_i8_when)
+        @sm100(ops.depthwise5x5_relu_pointwise_int8, requires, dwpw_i8_when)
         def depthwise5x5_relu_pointwise_int8(value, dw_weight, dw_bias, pw_weight, pw_wscale, pw_bias, scale):
             b, c, h, w = value.shape
             scale32 = scale.float().reshape(1)
@@ -939,7 +950,7 @@ def register(ops=None, device_spec=None, feature=None) -> None:
                 and (pair == 0 or f_a.shape[0] == 2 * pair)
             )
 
-        @ops.romav2_refiner_input.register("sm100", device=spec, requires=dw_requires, priority=3, when=input_when)
+        @sm100(ops.romav2_refiner_input, dw_requires, input_when)
         def romav2_refiner_input(f_a, f_b, warp, emb_weight, emb_bias, scale_factor, radius, pair=0):
             scale = scale_factor.detach().float().cpu().tolist() if isinstance(scale_factor, Tensor) else list(scale_factor)
             rows = romav2_refiner_input_launch(
@@ -958,7 +969,7 @@ def register(ops=None, device_spec=None, feature=None) -> None:
                 and prev_warp.dtype == torch.float32 and prev_confidence.dtype == torch.float32 and z.numel() > 0
             )
 
-        @ops.romav2_refiner_heads.register("sm100", device=spec, requires=dw_requires, priority=3, when=heads_when)
+        @sm100(ops.romav2_refiner_heads, dw_requires, heads_when)
         def romav2_refiner_heads(z, weight, bias, prev_warp, prev_confidence, refine_init):
             _, _, h, w = z.shape
             return romav2_refiner_heads_launch(
@@ -973,7 +984,7 @@ def register(ops=None, device_spec=None, feature=None) -> None:
             and tuple(scale_exponent.shape) == (padded_channels(value.shape[-1]) // 32,)
         )
 
-    @ops.quantize_mxfp8.register("sm100", device=spec, requires=dw_requires, priority=3, when=quantize_when)
+    @sm100(ops.quantize_mxfp8, dw_requires, quantize_when)
     def quantize_mxfp8(value, scale_exponent):
         exponent = (scale_exponent if scale_exponent.dtype == torch.int8 else scale_exponent.to(torch.int8)).contiguous()
         if _channels_first_view(value):
@@ -991,7 +1002,7 @@ def register(ops=None, device_spec=None, feature=None) -> None:
         return (have() and channel_scale is None and _cuda(value, scale) and value.dtype in _IN_DTYPES
                 and (row_major or channels_first) and scale.numel() == 1)
 
-    @ops.quantize_int8.register("sm100", device=spec, requires=dw_requires, priority=3, when=quantize_int8_when)
+    @sm100(ops.quantize_int8, dw_requires, quantize_int8_when)
     def quantize_int8(value, scale, *, channel_scale=None):
         scale32 = scale.to(device=value.device, dtype=torch.float32).reshape(())
         if _channels_first_view(value):
@@ -1003,7 +1014,7 @@ def register(ops=None, device_spec=None, feature=None) -> None:
             return (have() and _cuda(value) and value.dtype in _IN_DTYPES and value.is_contiguous()
                     and value.shape[-1] % 32 == 0)
 
-        @ops.quantize_mxfp8_dynamic.register("sm100", device=spec, requires=dw_requires, priority=3, when=dynamic_when)
+        @sm100(ops.quantize_mxfp8_dynamic, dw_requires, dynamic_when)
         def quantize_mxfp8_dynamic_impl(value):
             return quantize_mxfp8_dynamic(value, True)
 

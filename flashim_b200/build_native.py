@@ -1,4 +1,5 @@
-"""Build ``flashim_b200/_lib/libflashim_sm100.so`` from ``flashim_b200/csrc/*.cu`` with ``nvcc`` for sm_100a.
+"""Build ``flashim_b200/_lib/libflashim_sm100.so`` from ``flashim_b200/csrc/*.cu`` with ``nvcc`` for sm_100a, and the
+native host path of the ops, ``_lib/_fim_host.so``, from ``csrc/host.cpp`` with ``g++`` against the installed torch.
 
 ``python -m flashim_b200.build_native [--force]``. The arch flag must carry the ``a`` suffix: tcgen05 / tensor-memory
 instructions do not exist in the forward-compatible ``sm_100`` target. The build is atomic (temporary file + rename),
@@ -19,6 +20,8 @@ SOURCES = ("quantize.cu", "depthwise.cu", "conv.cu", "refiner_heads.cu", "refine
 HEADERS = ("common.cuh",)
 INCLUDE = PACKAGE.parent / "include"
 OUTPUT = PACKAGE / "_lib" / "libflashim_sm100.so"
+HOST_SOURCE = "host.cpp"
+HOST_OUTPUT = PACKAGE / "_lib" / "_fim_host.so"
 FLAGS = ("-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-std=c++17", "-lineinfo", "-shared", "-Xcompiler", "-fPIC")
 
 
@@ -63,5 +66,37 @@ def build(force: bool = False, verbose: bool = False, output: Path = OUTPUT, def
     return OUTPUT
 
 
+def build_host(force: bool = False) -> Path:
+    """Build the extension module of the host path (it holds no device code: a kernel change does not rebuild it)."""
+    import sysconfig
+
+    import torch
+    from torch.utils import cpp_extension
+
+    stamp = HOST_OUTPUT.with_suffix(".digest")
+    h = hashlib.sha256(f"{torch.__version__} {sys.version}".encode())
+    h.update((PACKAGE / "csrc" / HOST_SOURCE).read_bytes())
+    h.update((INCLUDE / "flashim_sm100.h").read_bytes())
+    digest = h.hexdigest()[:16]
+    if not force and HOST_OUTPUT.is_file() and stamp.is_file() and stamp.read_text().strip() == digest:
+        return HOST_OUTPUT
+    cuda = Path(nvcc_path() or "/usr/local/cuda/bin/nvcc").parents[1]
+    HOST_OUTPUT.parent.mkdir(parents=True, exist_ok=True)
+    temporary = HOST_OUTPUT.with_suffix(f".{os.getpid()}.tmp")
+    command = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
+               *(flag for path in cpp_extension.include_paths() for flag in ("-isystem", path)), "-isystem", str(cuda / "include"),
+               f"-I{sysconfig.get_paths()['include']}", f"-I{INCLUDE}", str(PACKAGE / "csrc" / HOST_SOURCE), "-o", str(temporary),
+               *(f"-L{path}" for path in cpp_extension.library_paths()), f"-L{cuda / 'lib64'}",
+               "-lc10", "-lc10_cuda", "-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-ltorch_python", "-lcudart", "-ldl"]
+    result = subprocess.run(command, capture_output=True, text=True, check=False)
+    if result.returncode != 0:
+        temporary.unlink(missing_ok=True)
+        raise RuntimeError(f"g++ failed:\n{result.stderr[-4000:]}")
+    temporary.replace(HOST_OUTPUT)
+    stamp.write_text(digest)
+    return HOST_OUTPUT
+
+
 if __name__ == "__main__":
+    print(build_host(force="--force" in sys.argv))
     print(build(force="--force" in sys.argv, verbose="-v" in sys.argv))

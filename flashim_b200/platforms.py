@@ -91,9 +91,23 @@ _DETECTORS: dict[str, Detector] = {"cuda": detect_cuda}
 _PLATFORMS: dict[tuple[str, int | None], Platform] = {}
 
 
+_ON_CHANGE: list[Callable[[], None]] = []
+
+
 def register_detector(device_type: str, detector: Detector) -> None:
     _DETECTORS[device_type] = detector
     _PLATFORMS.clear()
+    for notify in _ON_CHANGE:
+        notify()
+
+
+def detectors_replaced() -> bool:
+    """Whether CUDA devices are described by something other than :func:`detect_cuda`."""
+    return _DETECTORS.get("cuda") is not detect_cuda
+
+
+def on_detector_change(notify: Callable[[], None]) -> None:
+    _ON_CHANGE.append(notify)
 
 
 def default_device() -> torch.device:
