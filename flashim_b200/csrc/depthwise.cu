@@ -1,22 +1,50 @@
 // Depthwise 5x5 (pad 2, stride 1) + bias + activation on bf16 NHWC, with three epilogues: bf16, dynamic MXFP8,
-// static INT8. Arithmetic follows FlashIM's torch reference (flashim/ops/conv.py:30-61): bf16 inputs and weights,
-// fp32 FMA chain ordered (ky, kx) from zero, bias added last.
+// static INT8. Operands and roundings follow FlashIM's torch reference (flashim/ops/conv.py:30-61): bf16 inputs and
+// weights, exact products summed in fp32, bias added last in fp32.
 //
-// Layout of the work. A CTA works on strips of 64 channels x (COLS * WARPS) columns of one image, five output rows (a
-// unit) at a time; the persistent CTAs split the sequence of all units evenly. Input rows (with their 2-pixel halo,
-// zero-filled outside the image by TMA) arrive five at a time in a ring of shared-memory chunks. A lane owns one bf16x2
-// channel pair and COLS adjacent columns, keeps the 25 weight pairs and five rows of partial sums in registers as packed
-// fp32 pairs (fma.rn.f32x2: both channels in one issue slot), and finishes one output row per input row.
+// The sums run on the tensor cores (mma.sync m16n8k16, bf16 in, fp32 accumulators), one channel at a time:
+//   M: 16 blocks of 2 rows x 4 columns of output pixels, N: the 8 pixels of a block, K: the 6 x 8 input patch of a block
+//   (48 values, 3 K steps of two rows); B is the 5x5 kernel shifted to each of the 8 pixels (25 of its 48 rows non-zero).
+// On the fp32 pipe the 25 multiply-adds per element alone take longer than the tensor's way through HBM. As MMAs they are
+// a few percent of the tensor pipe; what the layout is chosen for is shared-memory bandwidth, the next bound:
+//   - A warp sweeps down its strip, 32 columns wide, 4 output rows per step. M is 8 blocks side by side x 2 blocks one below the
+//     other, so the two row pairs of the patch that a step shares with the step before, and the three that the two block
+//     rows share, stay in registers: a step loads four input rows for four output rows, each value once per column block
+//     that needs it (two), 16 bytes (8 channels) per lane and pixel.
+//   - K is ordered (row, column pair) with patch columns q and q + 4 in one register: lane l reads pixels l and l + 4 of a
+//     row, so the lanes of a shared-memory phase read neighbours, which the 64-byte TMA swizzle keeps free of conflicts.
+//   - N is ordered (column, row): a lane ends up with four pixels of one column, column l of the tile, for 8 channels.
+//   - A warp keeps to 8 channels, whose B fragments (48 registers) stay resident; four warps (a quad) cover the 32 channels
+//     of an MX block, exchange block maxima through shared memory and fill one output panel for a TMA store. Storing 8
+//     or 16 bytes per pixel from registers instead costs a shared-memory wavefront per lane.
 //
-// What bounds it is the fp32 pipe (25 FMAs per element, plus the polynomial of the GELU) and, next to it, the issue slots
-// of everything else. Two things keep the pipe fed: (1) every warp computes - there is no producer warp holding
-// registers; lane 0 of warp 0 issues the TMA copy four chunks ahead whenever it hands a chunk back - so that three CTAs
-// of four warps fit on an SM at 168 registers and the latency of one warp's shared-memory reads and shuffles hides
-// behind the FMAs of the others; (2) the epilogue is written for issue
-// slots: the five rows of a chunk are one straight-line block (accumulator slots, shared-memory offsets and weights are
-// all compile-time), barriers are touched once per chunk, a fresh accumulator starts with a multiply instead of being
-// zeroed, GELU is one MUFU and a Horner polynomial with immediate operands per value, and the MX block maximum over 16
-// lanes is a transposing butterfly.
+// Measured against the fp32-pipe kernel before it (B200, inputs in L2 where they fit):
+//   4x200x200x256: GELU -> bf16 68 -> 52 us, ReLU -> bf16 54 -> 41, GELU -> MXFP8 88 -> 69, ReLU -> INT8 87 -> 51
+//   8x400x400x128: GELU -> bf16 232 -> 163, ReLU -> bf16 183 -> 125 (80 % of the HBM copy rate), GELU -> MXFP8 303 -> 220,
+//   ReLU -> MXFP8 252 -> 174, ReLU -> INT8 299 -> 165
+// What bounds the GELU and quantising forms now is the arithmetic of their epilogues on twelve warps per SM (issue slots about
+// half busy); the care for equal results (below) is a quarter of the MXFP8 form's time.
+//
+// Precision: the tensor cores add the exact products into fp32 accumulators, as the fp32 chain of the reference does, but in
+// another order; the two differ by about one fp32 ulp of the largest partial sum. Outputs on which that could show are
+// noted in a list of the quad and summed again at its end in the reference's order (ky-major FMA chain, bias last): bf16
+// outputs below 2**-14 of the sums in their column, where bias and products cancel, and MXFP8 blocks with a value within
+// 2**-20 of a rounding boundary of E4M3 or a maximum within a few ulp of one of the exponent rule (with normal data one
+// output in 30000 and one block in 1000). INT8 codes have an absolute resolution far above the difference.
+//
+// Not-a-number and infinite inputs: a patch value outside an output's 5x5 window is multiplied by a zero of B, so they
+// spoil the outputs of their 6 x 8 patches instead of those of their 5x5 windows.
+//
+// Work: a strip is one (image, 32-column tile) over all rows, cut into steps of four output rows; a span is the part of a
+// range of steps inside one strip. The quads of all CTAs (three per CTA, one CTA per SM) form groups of one quad per
+// 32-channel tile, side by side on the SMs; the groups split the sequence of all steps evenly. The quads of a group thus read
+// the 64-byte parts of the same lines at about the same time, so DRAM delivers every line once (channel tile by channel
+// tile, 8x400x400x128 read twice its bytes: ReLU -> bf16 201 instead of 132 us), and a quad builds its B fragments once.
+// Each quad has a ring of input chunks of its own: 4 rows x 36 columns x 32 channels, zero-filled outside the image by TMA.
+// One named barrier per step orders all of it: behind it the step's chunk has been read by all four warps (and is
+// refilled), their maxima are visible, and the output panel is complete.
+#include <type_traits>
+
 #include "common.cuh"
 #include "flashim_sm100.h"
 #include "flashim_sm100_tune.h"
@@ -24,85 +52,49 @@
 namespace fim {
 namespace {
 
-#ifndef FIM_PROBE_BUILD
-#define FIM_PROBE_BUILD 0
-#endif
-
-// store only where `on` is non-zero, as a predicated instruction (no branch, the warp stays converged)
-__device__ __forceinline__ void store_if(uint32_t* at, uint32_t v, uint32_t on) {
-  asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %2, 0;\n\t@q st.global.b32 [%0], %1;\n\t}" ::"l"(at), "r"(v), "r"(on) : "memory");
-}
-__device__ __forceinline__ void store_if(uint16_t* at, uint16_t v, uint32_t on) {
-  asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %2, 0;\n\t@q st.global.b16 [%0], %1;\n\t}" ::"l"(at), "h"(v), "r"(on) : "memory");
-}
-
-// The 25 * COLS multiply-adds per output row and channel pair as mixed-precision FMAs (fp32 += bf16 * bf16, one per
-// channel, operands read from the halves of the packed words as they arrive from shared memory) instead of packed fp32
-// FMAs on unpacked values: the same bits (a bf16 product is exact in fp32), no unpacking, and the weights stay packed
-// (25 registers instead of 50). Measured per epilogue at 8x400x400x128: bf16 outputs 7-10 % faster (GELU 255 -> 238 us,
-// ReLU 205 -> 185), ReLU -> MXFP8 7 % faster, GELU -> MXFP8 unchanged at first (its long epilogue is short of issue slots,
-// and this form issues two instructions where the packed one issues one) and 8 % faster (329 -> 304 us) once the
-// registers the packed weights free hold the coefficient pairs of a packed GELU polynomial; ReLU -> INT8 4 % slower: it
-// keeps the packed fp32 form.
-#ifndef FIM_DW_MIXED_FMA
-#define FIM_DW_MIXED_FMA 1
-#endif
-__host__ __device__ constexpr bool mixed_fma_for(int mode, int min_ctas) {
-  // (four CTAs per SM leave 128 registers per thread: only the packed weights fit)
-  return FIM_DW_MIXED_FMA != 0 && (min_ctas >= 4 || mode != 2 /* every output but INT8 */);
-}
-
-// d = a * w + c per half of the packed bf16x2 words a and w, in fp32 (one rounding each)
-__device__ __forceinline__ void fma_bf16x2(uint32_t a, uint32_t w, float c0, float c1, float& d0, float& d1) {
-  asm("{\n\t.reg .b16 al, ah, wl, wh;\n\tmov.b32 {al, ah}, %2;\n\tmov.b32 {wl, wh}, %3;\n\t"
-      "fma.rn.f32.bf16 %0, al, wl, %4;\n\tfma.rn.f32.bf16 %1, ah, wh, %5;\n\t}"
-      : "=f"(d0), "=f"(d1)
-      : "r"(a), "r"(w), "f"(c0), "f"(c1));
-}
-
-constexpr int kChannels = 64;    // per CTA: one 128-byte line per pixel
-constexpr int kChunkRows = 5;    // input rows per ring chunk = accumulator slots
-// chunks in the ring: copies run up to 20 rows ahead (a chunk takes ~2 us to arrive); four CTAs per SM have room for four
-__host__ __device__ constexpr int ring_stages(int min_ctas) { return min_ctas >= 4 ? 4 : 5; }
+constexpr int kTileX = 32, kStepRows = 4, kTileC = 32, kQuads = 3;
+constexpr int kHaloX = kTileX + 4;
+constexpr uint32_t kPixelBytes = kTileC * 2, kRowBytes = kHaloX * kPixelBytes, kChunkBytes = kStepRows * kRowBytes;
+constexpr int kTaps = 25, kMaxStages = 6;
+constexpr float kCancelled = 16384.0f;  // an output below 1 / kCancelled of the sums it comes from is summed again (bf16)
+constexpr uint32_t kListEntries = 126, kListBytes = 1024;  // {count, -}, then {image row, column * 32 + channel} per entry
+constexpr uint32_t kWeightBytes = kTaps * kTileC * 2, kBiasBytes = kTileC * 8;
 
 enum { kOutBf16 = 0, kOutMx = 1, kOutInt8 = 2 };
 
+// shared memory of one quad: ring, two output panels (128 pixels x 32 channels), block maxima of two steps, list, B fragments,
+// weights, bias. The MXFP8 form holds its values across a barrier and has no registers left for the B fragments (48): it reads
+// them from shared memory, whose bandwidth it does not use up, at the price of a shorter ring. (Spilled to local memory, which
+// the shared memory leaves hardly any L1 for, they cost a third of the kernel's time.)
+__host__ __device__ constexpr uint32_t panel_bytes(int mode) { return mode == kOutBf16 ? 8192u : 4096u; }
+__host__ __device__ constexpr uint32_t exchange_bytes(int mode) { return mode == kOutMx ? 4096u : 0u; }
+__host__ __device__ constexpr int stages(int mode) { return mode == kOutMx ? 4 : kMaxStages; }
+__host__ __device__ constexpr uint32_t fragment_bytes(int mode) { return mode == kOutMx ? 4u * 12u * 512u : 0u; }
+__host__ __device__ constexpr uint32_t quad_bytes(int mode) {
+  return (stages(mode) * kChunkBytes + fragment_bytes(mode) + 2 * panel_bytes(mode) + exchange_bytes(mode) + kListBytes + kWeightBytes + kBiasBytes + 1023u) / 1024u * 1024u;
+}
+
 struct DwParams {
+  const uint16_t* value;   // bf16 NHWC
   const uint32_t* weight;  // bf16x2 words, [25][C/2]
   const float* bias;
-  void* out;
+  uint8_t* out;
   uint8_t* scales;
   const float* scale;  // INT8
   int batch, height, width, channels;
-  int tiles_x, channel_tiles;  // a strip = (image, 64-channel tile, column tile), all rows of the image
-  int strip_chunks, total_units;  // 5-row output chunks per strip; work units = strips * strip_chunks
-  int act, swizzled;
+  int tiles_x, channel_tiles;
+  int strip_steps, total_steps;  // four-row steps per strip; all steps of one channel tile
+  int groups, group_quads;       // quads of a group: min(channel tiles, quads of the grid), each takes every group_quads-th tile
+  int cta_quads;                 // quads in use per CTA
+  int swizzled, tma_out;         // tma_out: the output can be the target of TMA stores (16-byte aligned)
   int* status;
-  int debug;  // probe builds only: 1 = no FMAs, 2 = no epilogue, 4 = no loads and no waits for them
 };
 
-// GELU(x) = x * Phi(x) on an fp32 value. With p = Phi(-|x|) = 2**q(-|x|), q the degree-7 minimax polynomial of
-// log2 Phi on [-5.5, 0] (relative error of p below 4e-6; q keeps falling beyond -5.5, so p underflows to 0 for large |x|),
-// the value is max(x, 0) - |x| p for either sign. One MUFU; the Horner steps take their coefficients as immediates, so the
-// constants occupy no registers beside the 25 weight pairs. For x < -4.4 torch's own fp32 expression
-// x * 0.5 * (1 + erf(x / sqrt 2)) is dominated by the rounding of 1 + erf; this form stays accurate there.
-__device__ __forceinline__ float gelu_phi(float x) {
-  const float u = -fabsf(x);
-  float q = 1.793454771359393e-06f;
-  q = fmaf(q, u, 6.090417082305066e-05f);
-  q = fmaf(q, u, 0.000926029053516686f);
-  q = fmaf(q, u, 0.00849375780671835f);
-  q = fmaf(q, u, 0.053937844932079315f);
-  q = fmaf(q, u, -0.45848050713539124f);
-  q = fmaf(q, u, 1.1512467861175537f);
-  q = fmaf(q, u, -0.9999954700469971f);
-  float p;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(p) : "f"(q));
-  return fmaf(u, p, fmaxf(x, 0.0f));
-}
-
-// The same on a pair of values with packed FMAs (one issue slot per Horner step of both); the coefficient pairs then live
-// in registers, which only the kernels with packed weights have to spare.
+// GELU(x) = x * Phi(x) on a pair of fp32 values, one packed FMA per Horner step of both. With p = Phi(-|x|) =
+// 2**q(-|x|), q the degree-7 minimax polynomial of log2 Phi on [-5.5, 0] (relative error of p below 4e-6; q keeps falling
+// beyond -5.5, so p underflows to 0 for large |x|), the value is max(x, 0) - |x| p for either sign. One MUFU per value. For
+// x < -4.4 torch's own fp32 expression x * 0.5 * (1 + erf(x / sqrt 2)) is dominated by the rounding of 1 + erf; this form
+// stays accurate there.
 __device__ __forceinline__ uint64_t gelu_phi2(uint64_t x2) {
   float x0, x1;
   unpack2(x2, x0, x1);
@@ -115,369 +107,560 @@ __device__ __forceinline__ uint64_t gelu_phi2(uint64_t x2) {
   q = fma2(q, u, pack2(-0.45848050713539124f, -0.45848050713539124f));
   q = fma2(q, u, pack2(1.1512467861175537f, 1.1512467861175537f));
   q = fma2(q, u, pack2(-0.9999954700469971f, -0.9999954700469971f));
-  float q0, q1, p0, p1;
+  float q0, q1;
   unpack2(q, q0, q1);
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(p0) : "f"(q0));
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(p1) : "f"(q1));
-  return fma2(u, pack2(p0, p1), pack2(fmaxf(x0, 0.0f), fmaxf(x1, 0.0f)));
+  return fma2(u, pack2(ex2_approx(q0), ex2_approx(q1)), pack2(fmaxf(x0, 0.0f), fmaxf(x1, 0.0f)));
 }
 
-template <int ACT, bool PACKED_GELU = false>
+template <int ACT>
 __device__ __forceinline__ uint64_t activate2(uint64_t v) {
   if (ACT == kActNone) return v;
-  if (ACT == kActGelu && PACKED_GELU) return gelu_phi2(v);
+  if (ACT == kActGelu) return gelu_phi2(v);
   float lo, hi;
   unpack2(v, lo, hi);
-  if (ACT == kActGelu) return pack2(gelu_phi(lo), gelu_phi(hi));
   return pack2(fmaxf(lo, 0.0f), fmaxf(hi, 0.0f));
 }
 
-// Finish one output row of this lane: bias, activation and the epilogue of MODE for the lane's COLS pixels.
-// `out_row` points at this lane's channel pair of pixel (row, x0) in units of output pairs; `pixel0` is that pixel's
-// index in the batch; `cols_ok` has bit j set when column x0 + j exists (0 for a lane without channels).
-template <int MODE, int ACT, int COLS, bool PACKED_GELU = false>
-__device__ __forceinline__ void emit_row(const DwParams& p, const uint64_t (&acc)[COLS], uint64_t bias2, void* out_row,
-                                         size_t pixel0, int c, uint32_t cols_ok, const Int8Quantizer& int8, int lane) {
-  const size_t pair_stride = static_cast<size_t>(p.channels >> 1);
-  uint64_t v[COLS];
-#pragma unroll
-  for (int j = 0; j < COLS; ++j) v[j] = activate2<ACT, PACKED_GELU>(add2(acc[j], bias2));
-  if (MODE == kOutBf16) {
-    uint32_t* out = static_cast<uint32_t*>(out_row);
-#pragma unroll
-    for (int j = 0; j < COLS; ++j) {
-      float lo, hi;
-      unpack2(v[j], lo, hi);
-      store_if(out + j * pair_stride, pack_bf16(lo, hi), cols_ok & (1u << j));
-    }
-  } else if (MODE == kOutMx) {
-    // amax of each pixel over the 16 lanes of its 32-channel block by a transposing butterfly: every exchange halves the
-    // pixels a lane keeps until it holds one, whose maximum the remaining exchanges complete. With four pixels lane l
-    // ends up with pixel ((l & 1) << 1) | ((l >> 1) & 1), with two pixels with pixel l & 1. The lane computes that
-    // pixel's exponent; the first lanes of each half-warp store the scale bytes; 2**-e goes back with one shuffle per pixel.
-    float m[COLS];
-#pragma unroll
-    for (int j = 0; j < COLS; ++j) {
-      float lo, hi;
-      unpack2(v[j], lo, hi);
-      m[j] = fmaxf(fabsf(lo), fabsf(hi));
-    }
-    int mine;  // the pixel this lane holds after the butterfly
-    if (COLS == 4) {
-      const bool odd = lane & 1;  // even lanes keep pixels 0, 1 and odd lanes pixels 2, 3
-      const float s0 = __shfl_xor_sync(0xffffffffu, odd ? m[0] : m[2], 1);
-      const float s1 = __shfl_xor_sync(0xffffffffu, odd ? m[1] : m[3], 1);
-      m[0] = fmaxf(odd ? m[2] : m[0], s0);
-      m[1] = fmaxf(odd ? m[3] : m[1], s1);
-      const bool up = lane & 2;  // then bit 1 of the lane picks the second of the pair
-      const float s2 = __shfl_xor_sync(0xffffffffu, up ? m[0] : m[1], 2);
-      m[0] = fmaxf(up ? m[1] : m[0], s2);
-      mine = ((lane & 1) << 1) | ((lane >> 1) & 1);
-    } else {
-      const bool odd = lane & 1;  // even lanes keep pixel 0, odd lanes pixel 1
-      const float s0 = __shfl_xor_sync(0xffffffffu, odd ? m[0] : m[1], 1);
-      m[0] = fmaxf(odd ? m[1] : m[0], s0);
-      m[0] = fmaxf(m[0], __shfl_xor_sync(0xffffffffu, m[0], 2));
-      mine = lane & 1;
-    }
-    m[0] = fmaxf(m[0], __shfl_xor_sync(0xffffffffu, m[0], 4));
-    m[0] = fmaxf(m[0], __shfl_xor_sync(0xffffffffu, m[0], 8));
-    const int e = e8m0_exponent_bits(__float_as_uint(m[0]));
-    const float inv_mine = exp2_int(-e);
-    {
-      // the owner lanes (the first COLS of each half-warp) store their pixel's scale byte; the address is computed by all
-      // lanes and only the store is predicated, which keeps the warp converged
-      const size_t pixel = pixel0 + mine;
-      const int groups = p.channels >> 5;
-      const int g = c >> 5;
-      const size_t at = p.swizzled ? swizzled_scale_offset(pixel, g, (groups + 3) >> 2) : pixel * groups + g;
-      const uint32_t owner = ((lane & 15) < COLS && ((cols_ok >> mine) & 1u)) ? 1u : 0u;
-      asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %2, 0;\n\t@q st.global.u8 [%0], %1;\n\t}" ::"l"(p.scales + at),
-                   "r"(static_cast<uint32_t>(e + 127)), "r"(owner)
-                   : "memory");
-    }
-    const int half = lane & 16;
-    uint16_t* out = static_cast<uint16_t*>(out_row);
-#pragma unroll
-    for (int j = 0; j < COLS; ++j) {
-      const int holder = COLS == 4 ? (((j >> 1) & 1) | ((j & 1) << 1)) : j;  // a lane of this half-warp that holds pixel j
-      const float inv = __shfl_sync(0xffffffffu, inv_mine, half | holder);
-      float lo, hi;
-      unpack2(mul2(v[j], pack2(inv, inv)), lo, hi);
-      store_if(out + j * pair_stride, e4m3x2(lo, hi), cols_ok & (1u << j));
-    }
+__device__ __forceinline__ void lds128(uint32_t addr, uint32_t (&v)[4]) {
+  asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]) : "r"(addr));
+}
+
+// d += a b, or d = a b for the first K step
+template <bool FIRST>
+__device__ __forceinline__ void mma_16x8x16(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+  if (FIRST) {
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%10, %10, %10, %10};"
+        : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(0.0f));
   } else {
-    uint16_t* out = static_cast<uint16_t*>(out_row);
-#pragma unroll
-    for (int j = 0; j < COLS; ++j) {
-      float lo, hi;
-      unpack2(v[j], lo, hi);
-      const uint32_t rounded = pack_bf16(lo, hi);  // one packed conversion instead of two scalar ones
-      const uint16_t codes = static_cast<uint16_t>(int8_pack2(int8, bf16_lo(rounded), bf16_hi(rounded)));
-      store_if(out + j * pair_stride, codes, cols_ok & (1u << j));
-    }
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+        : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
   }
 }
 
-__device__ __forceinline__ uint32_t lds32(uint32_t addr) {
-  uint32_t v;
-  asm volatile("ld.shared.b32 %0, [%1];" : "=r"(v) : "r"(addr));
-  return v;
+// Two image rows of the patch for 8 channels, as A operands: [channel][row], patch columns q and q + 4 in one register.
+// `at`: the lane's pixel in the upper row, its 16-byte piece chosen by the swizzle; in the odd row and four columns on, the
+// swizzle phase differs in one bit.
+struct RowPair {
+  uint32_t a[8][2];
+};
+__device__ __forceinline__ void load_pair(uint32_t at, RowPair& p) {
+  uint32_t v[4][4];
+  lds128(at, v[0]);
+  lds128((at ^ 32u) + 4 * kPixelBytes, v[1]);
+  lds128((at ^ 32u) + kRowBytes, v[2]);
+  lds128(at + kRowBytes + 4 * kPixelBytes, v[3]);
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    p.a[2 * j][0] = __byte_perm(v[0][j], v[1][j], 0x5410);
+    p.a[2 * j + 1][0] = __byte_perm(v[0][j], v[1][j], 0x7632);
+    p.a[2 * j][1] = __byte_perm(v[2][j], v[3][j], 0x5410);
+    p.a[2 * j + 1][1] = __byte_perm(v[2][j], v[3][j], 0x7632);
+  }
 }
 
-// Where the copies of a CTA stand: the chunk sequence of its unit range [u, u_end), span by span.
-struct CopyCursor {
-  int u, u_end;       // next unit that starts a span
-  int g, len;         // next chunk of the current span (0 .. len) and the span's length in units
-  int k0, tx, ct, b;  // the span's first unit within its strip and the strip's coordinates
-};
+// One K step for the 8 channels: the upper blocks (M rows 0-7) see row pair `upper` of the patch, the blocks below them the
+// next pair.
+template <bool FIRST>
+__device__ __forceinline__ void multiply_step_shared(const RowPair& upper, const RowPair& lower, uint32_t fragments, float (&acc)[8][4]) {
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    uint32_t b[4];
+    lds128(fragments + j * 512, b);
+    mma_16x8x16<FIRST>(acc[2 * j], upper.a[2 * j][0], lower.a[2 * j][0], upper.a[2 * j][1], lower.a[2 * j][1], b[0], b[1]);
+    mma_16x8x16<FIRST>(acc[2 * j + 1], upper.a[2 * j + 1][0], lower.a[2 * j + 1][0], upper.a[2 * j + 1][1], lower.a[2 * j + 1][1], b[2], b[3]);
+  }
+}
+template <bool FIRST>
+__device__ __forceinline__ void multiply_step(const RowPair& upper, const RowPair& lower, const uint32_t (&b)[8][2], float (&acc)[8][4]) {
+#pragma unroll
+  for (int c = 0; c < 8; ++c) mma_16x8x16<FIRST>(acc[c], upper.a[c][0], lower.a[c][0], upper.a[c][1], lower.a[c][1], b[c][0], b[c][1]);
+}
 
-// Thread layout: WARPS compute warps; warp w owns columns COLS * w .. COLS * w + COLS - 1 of the tile. Lane 0 of warp 0
-// also issues the copies.
-template <int MODE, int ACT, int COLS, int WARPS, int MIN_CTAS, bool PROBE>
-__global__ void __launch_bounds__(32 * WARPS, MIN_CTAS) dw5x5_kernel(const __grid_constant__ CUtensorMap in_map, const DwParams p) {
-  constexpr bool kMixedFma = mixed_fma_for(MODE, MIN_CTAS);
-  constexpr int kStages = ring_stages(MIN_CTAS);
-  constexpr int kTileCols = WARPS * COLS;
-  constexpr uint32_t kRowBytes = (kTileCols + 4) * kChannels * 2;
-  constexpr uint32_t kChunkBytes = kChunkRows * kRowBytes;
-  extern __shared__ __align__(128) uint8_t smem_raw[];
-  __shared__ __align__(8) uint64_t full_bar[kStages];
-  __shared__ __align__(8) uint64_t empty_bar[kStages];
+// The pre-activation value of one output as the reference sums it: an fp32 FMA chain over the taps, ky-major, bias last.
+// `image`: the channel's first pixel, `weights`: the shared-memory address of its first tap. Five loads are in flight at a
+// time; unrolling all 25 is slower, since the code runs once and is fetched as it runs.
+__device__ __noinline__ float chain_sum(const uint16_t* image, int height, int width, int channels, uint32_t weights, float bias, int y, int x) {
+  float sum = 0.0f;
+#pragma unroll 1
+  for (int ky = 0; ky < 5; ++ky) {
+    const int iy = y + ky - 2;
+    const bool row_in = static_cast<unsigned>(iy) < static_cast<unsigned>(height);
+    const uint16_t* row = image + static_cast<ptrdiff_t>(row_in ? iy : y) * width * channels;
+    uint16_t v[5];
+#pragma unroll
+    for (int kx = 0; kx < 5; ++kx) {
+      const int ix = x + kx - 2;
+      const bool in = row_in && static_cast<unsigned>(ix) < static_cast<unsigned>(width);
+      v[kx] = __ldg(row + static_cast<ptrdiff_t>(in ? ix : x) * channels);
+      v[kx] = in ? v[kx] : static_cast<uint16_t>(0);
+    }
+#pragma unroll
+    for (int kx = 0; kx < 5; ++kx) {
+      uint16_t w;
+      asm volatile("ld.shared.u16 %0, [%1];" : "=h"(w) : "r"(weights + (ky * 5 + kx) * (kTileC * 2)));
+      sum = fmaf(bf16_lo(v[kx]), bf16_lo(w), sum);
+    }
+  }
+  return sum + bias;
+}
+
+// Notes an output (or the block it lies in) in the quad's list. A full list drops it: the output keeps its tensor-core sum.
+__device__ __forceinline__ void note(uint32_t list, uint32_t row, uint32_t x, uint32_t channel) {
+  uint32_t at;
+  asm volatile("atom.shared.add.u32 %0, [%1], 1;" : "=r"(at) : "r"(list) : "memory");
+  if (at < kListEntries) asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(list + 8 + at * 8), "r"(row), "r"(x * 32 + channel) : "memory");
+}
+
+// min(|a|, |b|, |c|)
+__device__ __forceinline__ float min_abs(float a, float b, float c) {
+  float r;
+  asm("min.abs.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+}
+// max(|m|, |a|, |b|)
+__device__ __forceinline__ float max_abs(float m, float a, float b) {
+  float r;
+  asm("max.abs.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(m), "f"(a), "f"(b));
+  return r;
+}
+
+// E8M0 bytes and the factors 2**-e of four block maxima: e = E - 8 + (mantissa > 1.75), one carry away from the exponent field,
+// unless one of them lies in the window where the reference's rule departs from that or is not finite. Returns a bit per
+// maximum that lies in that window or within 8 ulp of it (one block in 150000).
+__device__ __forceinline__ uint32_t block_scales(const float (&amax)[4], uint32_t (&bytes)[4], float (&inv)[4]) {
+  uint32_t unsure = 0;
+  bool rare = false;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const uint32_t bits = __float_as_uint(amax[i]);
+    bytes[i] = static_cast<uint32_t>(max(static_cast<int>((bits + 0x1FFFFFu) >> 23) - 8, 0));
+    inv[i] = __uint_as_float((254u - bytes[i]) << 23);
+    rare |= ((bits & 0x7FFFFFu) - 0x5FFFF8u) < 57u || bits >= 0x7F800000u;
+  }
+  if (rare) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      if (((__float_as_uint(amax[i]) & 0x7FFFFFu) - 0x5FFFF8u) < 57u) unsure |= 1u << i;
+      const int e = e8m0_exponent(amax[i]);
+      bytes[i] = static_cast<uint32_t>(e + 127);
+      inv[i] = exp2_int(-e);
+    }
+  }
+  return unsure;
+}
+
+// Where the steps of a quad start in the image.
+struct Position {
+  int k0, tx, b;
+};
+__device__ __forceinline__ Position position_of(const DwParams& p, int step) {
+  Position at;
+  int t = step / p.strip_steps;
+  at.k0 = step - t * p.strip_steps;
+  at.tx = t % p.tiles_x;
+  at.b = t / p.tiles_x;
+  return at;
+}
+
+template <int MODE, int ACT>
+__global__ void __launch_bounds__(128 * kQuads, 1)
+dw5x5_kernel(const __grid_constant__ CUtensorMap in_map, const __grid_constant__ CUtensorMap out_map, const DwParams p) {
+  extern __shared__ uint8_t smem_raw[];
+  constexpr int kStages = stages(MODE);
+  __shared__ __align__(8) uint64_t full_bar[kQuads * kStages];
   __shared__ int abort_flag;
 
   // (the warp index through a shuffle: uniform to the compiler, and so is everything derived from it)
   const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
-
-  // Persistent CTAs over work units of five output rows. A strip is one (image, channel tile, column tile) over all rows;
-  // the units of all strips form one sequence, of which this CTA owns the contiguous range [u_begin, u_end): an equal
-  // share to within one unit, cut into spans where it crosses a strip. A span of `len` units reads len + 1 input chunks
-  // (its rows plus the halo above and below), so the chunk ring flows on from span to span without draining.
-  const int u_begin = static_cast<int>(static_cast<long long>(blockIdx.x) * p.total_units / gridDim.x);
-  const int u_end = static_cast<int>(static_cast<long long>(blockIdx.x + 1) * p.total_units / gridDim.x);
-  const bool loads = !(PROBE && (p.debug & 4));
-
-  const uint32_t smem0 = smem_u32(smem_raw), full0 = smem_u32(&full_bar[0]), empty0 = smem_u32(&empty_bar[0]);
+  const int quad = warp >> 2, piece = warp & 3;  // piece: which 8 of the 32 channels
+  const uint32_t ring = ((smem_u32(smem_raw) + 1023u) & ~1023u) + quad * quad_bytes(MODE);
+  const uint32_t panels = ring + kStages * kChunkBytes, exchange = panels + 2 * panel_bytes(MODE);
+  const uint32_t list = exchange + exchange_bytes(MODE), fragments = list + kListBytes + piece * (12 * 512) + lane * 16;
+  const uint32_t weights_at = list + kListBytes + fragment_bytes(MODE), bias_at = weights_at + kWeightBytes;
+  const uint32_t full0 = smem_u32(&full_bar[quad * kStages]);
 
   if (threadIdx.x == 0) {
     abort_flag = 0;
-    for (int s = 0; s < kStages; ++s) {
-      mbar_init(&full_bar[s], 1);
-      mbar_init(&empty_bar[s], WARPS);
-    }
+    for (int s = 0; s < kQuads * kStages; ++s) mbar_init(&full_bar[s], 1);
     mbar_fence_init();
     fence_async_proxy();
     tma_prefetch_desc(&in_map);
+    tma_prefetch_desc(&out_map);
   }
   __syncthreads();
-  if (u_end <= u_begin) return;
 
-  // ---- copies: issued by one lane of warp 0 (the cursor lives in every lane of that warp, uniformly) ----
-  CopyCursor cur;
-  cur.u = u_begin, cur.u_end = u_end, cur.g = 1, cur.len = 0, cur.k0 = 0, cur.tx = 0, cur.ct = 0, cur.b = 0;
-  uint32_t copy_stage = 0;
-  // Issue the next chunk of the sequence into ring stage `copy_stage`; false when the sequence has ended.
-  auto issue_copy = [&]() -> bool {
-    if (cur.g > cur.len) {  // the span is complete: open the next one
-      if (cur.u >= cur.u_end) return false;
-      const int strip = cur.u / p.strip_chunks;
-      cur.k0 = cur.u - strip * p.strip_chunks;
-      cur.len = min(p.strip_chunks - cur.k0, cur.u_end - cur.u);
-      cur.u += cur.len;
-      int t = strip;
-      cur.tx = t % p.tiles_x; t /= p.tiles_x;
-      cur.ct = t % p.channel_tiles;
-      cur.b = t / p.channel_tiles;
-      cur.g = 0;
-    }
-    if (elect_one()) {  // one lane, known to the compiler as one: the copy's operands stay in uniform registers
-      mbar_expect_tx_addr(full0 + 8 * copy_stage, kChunkBytes);
-      tma_load_4d_addr(smem0 + copy_stage * kChunkBytes, &in_map, full0 + 8 * copy_stage, cur.ct * kChannels,
-                       cur.tx * kTileCols - 2, (cur.k0 + cur.g) * kChunkRows - 2, cur.b);
-    }
-    ++cur.g;
-    if (++copy_stage == kStages) copy_stage = 0;
-    return true;
-  };
-  bool copies_left = loads;
-  if (warp == 0) {
-    // the ring starts with all stages but one in flight; from then on every chunk handed back is answered by one copy
-    for (int i = 0; i < kStages - 1 && copies_left; ++i) copies_left = issue_copy();
-  }
+  const int worker = blockIdx.x * p.cta_quads + quad, group = worker / p.group_quads, member = worker % p.group_quads;
+  const bool idle = quad >= p.cta_quads || group >= p.groups;
+  const int s_begin = idle ? 0 : static_cast<int>(static_cast<long long>(group) * p.total_steps / p.groups);
+  const int s_end = idle ? 0 : static_cast<int>(static_cast<long long>(group + 1) * p.total_steps / p.groups);
+  const uint32_t quad_barrier = 1 + quad;
 
-  // ---- compute ----
-  const Int8Quantizer int8_scale = make_int8_quantizer(MODE == kOutInt8 ? __ldg(p.scale) : 1.0f);
-  const uint32_t lane_smem = smem0 + (warp * COLS * (kChannels / 2) + lane) * 4;
-  constexpr int kOutBytes = MODE == kOutBf16 ? 4 : 2;  // per channel pair
-  const size_t pair_stride = static_cast<size_t>(p.channels >> 1);
-  const size_t row_pairs = static_cast<size_t>(p.width) * pair_stride;
-
-  // per-span state
-  uint64_t wreg[kMixedFma ? 1 : 25];   // unpacked weight pairs (packed-fp32 form)
-  uint32_t wpack[kMixedFma ? 25 : 1];  // bf16x2 weight words (mixed-precision form)
-  uint64_t bias2 = 0ull;
-  int c = 0, last_ct = -1, y_base = 0, y_end = 0, y_out = 0;
-  uint32_t cols_ok = 0;
-  size_t pixel0 = 0;
-  uint8_t* out_row = nullptr;
-#pragma unroll
-  for (int k = 0; k < (kMixedFma ? 1 : 25); ++k) wreg[k] = 0ull;
-#pragma unroll
-  for (int k = 0; k < (kMixedFma ? 25 : 1); ++k) wpack[k] = 0u;
-  uint64_t acc[kMixedFma ? 1 : kChunkRows][COLS];
-  float facc[kMixedFma ? kChunkRows : 1][COLS][2];
-#pragma unroll
-  for (int s = 0; s < (kMixedFma ? 1 : kChunkRows); ++s)
-#pragma unroll
-    for (int j = 0; j < COLS; ++j) acc[s][j] = 0ull;  // a slot is read for real only after its first multiply
-#pragma unroll
-  for (int s = 0; s < (kMixedFma ? kChunkRows : 1); ++s)
-#pragma unroll
-    for (int j = 0; j < COLS; ++j) facc[s][j][0] = facc[s][j][1] = 0.0f;
-
-  uint32_t s = 0, phase = 0, taken = 0;  // ring position of the chunk in use; chunks handed back so far
-  uint32_t raw[COLS + 4];  // bf16x2 words of the input row about to be used
-  bool ok = !loads || mbar_wait_addr(full0, 0, &abort_flag, p.status, kStatusWaitRows);
-  bool alive = __all_sync(0xffffffffu, ok);
-  if (alive) {
-#pragma unroll
-    for (int j = 0; j < COLS + 4; ++j) raw[j] = lds32(lane_smem + j * (kChannels * 2));
-  }
-  for (int u = u_begin; u < u_end && alive;) {
-    const int strip = u / p.strip_chunks, k0 = u - strip * p.strip_chunks;
-    const int len = min(p.strip_chunks - k0, u_end - u);
-    u += len;
-    {
-      int t = strip;
-      const int tx = t % p.tiles_x; t /= p.tiles_x;
-      const int ct = t % p.channel_tiles;
-      const int b = t / p.channel_tiles;
-      c = ct * kChannels + 2 * lane;
-      const bool lane_active = c < p.channels;
-      if (ct != last_ct) {  // uniform: a new channel tile brings new weights and bias
-        last_ct = ct;
-#pragma unroll
-        for (int k = 0; k < 25; ++k) {
-          const uint32_t word = lane_active ? __ldg(p.weight + ((static_cast<size_t>(k) * p.channels + c) >> 1)) : 0u;
-          if (kMixedFma) {
-            wpack[k] = word;
-          } else {
-            wreg[k] = bf16x2_to_f32x2(word);
-          }
+  // ---- copies: issued by one lane of the quad's first warp ----
+  int copy_ct = member, copy_step = s_begin, copy_g = 0, copy_len = -1;  // next span's start; chunk and length of the span under way
+  Position copy_at = {};
+  uint32_t issued = 0, issue_slot = 0;
+  auto issue_until = [&](uint32_t target) {
+    while (issued < target) {
+      if (copy_g > copy_len) {
+        if (copy_step >= s_end) {  // the range once more for the quad's next channel tile
+          copy_ct += p.group_quads, copy_step = s_begin;
         }
-        bias2 = lane_active ? pack2(__ldg(p.bias + c), __ldg(p.bias + c + 1)) : pack2(0.f, 0.f);
+        if (copy_ct >= p.channel_tiles || copy_step >= s_end) return;
+        copy_at = position_of(p, copy_step);
+        copy_len = min(p.strip_steps - copy_at.k0, s_end - copy_step);
+        copy_step += copy_len;
+        copy_g = 0;
       }
-      const int x0 = tx * kTileCols + warp * COLS;
-      cols_ok = 0;
-#pragma unroll
-      for (int j = 0; j < COLS; ++j) cols_ok |= (lane_active && x0 + j < p.width) ? (1u << j) : 0u;
-      y_base = k0 * kChunkRows;
-      y_end = min(y_base + len * kChunkRows, p.height);
-      y_out = y_base - 4;  // where the span's first input row would "finish": four rows above the span
-      pixel0 = (static_cast<size_t>(b) * p.height + y_base) * p.width + x0;  // of output row y_base, advanced per emitted row
-      out_row = static_cast<uint8_t*>(p.out) + (pixel0 * pair_stride + (c >> 1)) * kOutBytes;
+      if (elect_one()) {
+        mbar_expect_tx_addr(full0 + 8 * issue_slot, kChunkBytes);
+        tma_load_4d_addr(ring + issue_slot * kChunkBytes, &in_map, full0 + 8 * issue_slot, copy_ct * kTileC, copy_at.tx * kTileX - 2,
+                         (copy_at.k0 + copy_g) * kStepRows - 2, copy_at.b);
+      }
+      ++copy_g;
+      ++issued;
+      if (++issue_slot == kStages) issue_slot = 0;
     }
-    for (int g = 0; g <= len && alive; ++g) {
-      const bool more = g < len || u < u_end;  // another chunk follows, in this span or the next
-      const uint32_t chunk = lane_smem + s * kChunkBytes;
-      const uint32_t s_next = s + 1 == kStages ? 0u : s + 1;
-      const uint32_t phase_next = s + 1 == kStages ? phase ^ 1u : phase;
+  };
+  if (piece == 0) issue_until(kStages);
+
+  const Int8Quantizer int8 = make_int8_quantizer(MODE == kOutInt8 ? __ldg(p.scale) : 1.0f);
+  constexpr int kOutBytes = MODE == kOutBf16 ? 2 : 1;
+  const uint32_t turn = static_cast<uint32_t>(piece ^ ((lane >> 1) & 3)) << 4;  // the 16-byte piece under the swizzle
+  const uint32_t lane_at = ring + lane * kPixelBytes + turn;
+
+  uint32_t taken = 0, slot = 0, parity = 0, flip = 0;  // chunks taken so far, the next one's ring position; panel in use
+  bool alive = true;
+  auto take_chunk = [&]() -> uint32_t {  // the lane's address in the next chunk, once it has arrived
+    if (alive) alive = mbar_wait_warp(full0 + 8 * slot, parity, &abort_flag, p.status, kStatusWaitRows);
+    const uint32_t at = lane_at + slot * kChunkBytes;
+    ++taken;
+    if (++slot == kStages) slot = 0, parity ^= 1u;
+    return at;
+  };
+  // MX panels are filled behind the step's barrier and stored behind the next one
+  int stored_x = 0, stored_y = 0, stored_c = 0, stored_b = -1;
+  auto store_panel = [&](uint32_t panel, int c, int x, int y, int b) {
+    if (elect_one()) {
+      tma_store_4d(&out_map, panel, c, x, y, b);
+      bulk_commit();
+    }
+  };
+
+  for (int ct = member; ct < p.channel_tiles && s_begin < s_end; ct += p.group_quads) {
+    const int c0 = ct * kTileC;
+    uint32_t bfrag[3][8][2];
+    {  // weights through shared memory into the B fragments
+      if (ct != member) named_barrier(quad_barrier, 128);  // every warp has read those of the tile before
+      for (int i = threadIdx.x & 127; i < kTaps * (kTileC / 2); i += 128) {
+        const uint32_t word = __ldg(p.weight + ((static_cast<size_t>(i >> 4) * p.channels + c0) >> 1) + (i & 15));
+        asm volatile("st.shared.b32 [%0], %1;" ::"r"(weights_at + i * 4), "r"(word) : "memory");
+      }
+      if (piece == 0) {
+        if (lane == 0) asm volatile("st.shared.b32 [%0], 0;" ::"r"(list) : "memory");
+        const float bias = __ldg(p.bias + c0 + lane);
+        asm volatile("st.shared.v2.f32 [%0], {%1, %1};" ::"r"(bias_at + lane * 8), "f"(bias) : "memory");
+      }
+      named_barrier(quad_barrier, 128);
+      // B[k][n] = w[row - dy][column - dx] for patch position k = (row, column) and output pixel n = (dx, dy), else 0; this
+      // lane holds columns q and q + 4 of pixel n
+      const int q = lane & 3, dx = lane >> 3, dy = (lane >> 2) & 1;
+      const bool lo_in = q >= dx, hi_in = q <= dx;
 #pragma unroll
-      for (int ph = 0; ph < kChunkRows; ++ph) {
-        uint64_t in[kMixedFma ? 1 : COLS + 4];
-        uint32_t row[kMixedFma ? COLS + 4 : 1];  // this row's packed words, while `raw` takes the next row
+      for (int st = 0; st < 3; ++st) {
 #pragma unroll
-        for (int j = 0; j < COLS + 4; ++j) {
-          if (kMixedFma) {
-            row[j] = raw[j];
-          } else {
-            in[j] = bf16x2_to_f32x2(raw[j]);
+        for (int h = 0; h < 2; ++h) {
+          const int ky = 2 * st + h - dy;
+          const bool in = ky >= 0 && ky < 5;
+          uint32_t lo[4] = {}, hi[4] = {};  // 8 channels of the two taps
+          const uint32_t tap = weights_at + (ky * 5 + q - dx) * (kTileC * 2) + piece * 16;
+          if (in && lo_in) lds128(tap, lo);
+          if (in && hi_in) lds128(tap + 4 * kTileC * 2, hi);
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            bfrag[st][2 * j][h] = __byte_perm(lo[j], hi[j], 0x5410);
+            bfrag[st][2 * j + 1][h] = __byte_perm(lo[j], hi[j], 0x7632);
           }
         }
-        // fetch the next input row while this one is in the FMAs
-        if (ph + 1 < kChunkRows) {
+        if (MODE == kOutMx) {
 #pragma unroll
-          for (int j = 0; j < COLS + 4; ++j) raw[j] = lds32(chunk + (ph + 1) * kRowBytes + j * (kChannels * 2));
-        } else {
-          // every word of this chunk is in registers: hand it back, then take the first row of the next chunk (which
-          // may already belong to the next tile)
-          __syncwarp();
-          if (lane == 0 && loads) mbar_arrive_addr(empty0 + 8 * s);
-          if (warp == 0 && copies_left) {
-            // One copy per chunk handed back, into the stage handed back one chunk ago: the other warps have had a whole
-            // chunk's time to release it, so this wait rarely spins. Stage (taken - 1) mod kStages has then been released
-            // (taken - 1) / kStages + 1 times; the first kStages - 1 copies went out before the loop.
-            bool free_stage = true;
-            if (taken >= 1) {
-              const uint32_t round = (taken - 1) / kStages;
-              // (the warp agrees on the outcome: the copy below is issued through elect.sync, which every lane must reach)
-              free_stage = __all_sync(0xffffffffu, mbar_wait_addr(empty0 + 8 * copy_stage, round & 1u, &abort_flag, p.status, kStatusWaitRows));
+          for (int j = 0; j < 4; ++j) {
+            asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(fragments + (st * 4 + j) * 512), "r"(bfrag[st][2 * j][0]),
+                         "r"(bfrag[st][2 * j][1]), "r"(bfrag[st][2 * j + 1][0]), "r"(bfrag[st][2 * j + 1][1])
+                         : "memory");  // (each lane reads back only what it wrote)
+          }
+        }
+      }
+    }
+
+    for (int s = s_begin; s < s_end;) {
+      const Position at = position_of(p, s);
+      const int len = min(p.strip_steps - at.k0, s_end - s);
+      s += len;
+      const int x0 = at.tx * kTileX, x = x0 + lane;
+      // (rows of the scale matrix fit 32 bits: one more would be 256 GB of input)
+      const uint32_t scale_row = (static_cast<uint32_t>(at.b) * p.height + piece) * p.width + x;
+      const uint32_t scale_tile_bytes = ((p.channels >> 5) + 3) / 4 * 512, scale_at = (ct >> 2) * 512 + (ct & 3);
+      RowPair r0, r1;  // the two row pairs above the ones a step brings
+      {
+        const uint32_t from = take_chunk();
+        load_pair(from, r0);
+        load_pair(from + 2 * kRowBytes, r1);
+      }
+      for (int k = 0; k < len; ++k) {
+        const int y = (at.k0 + k) * kStepRows;
+        const uint32_t from = take_chunk();
+        const uint32_t panel = panels + flip * panel_bytes(MODE);
+        float acc[8][4];
+        {
+          RowPair r2;
+          const auto multiply = [&](auto first, const RowPair& upper, const RowPair& lower, int st) {
+            if constexpr (MODE == kOutMx) {
+              multiply_step_shared<decltype(first)::value>(upper, lower, fragments + st * (4 * 512), acc);
+            } else {
+              multiply_step<decltype(first)::value>(upper, lower, bfrag[st], acc);
             }
-            copies_left = free_stage && issue_copy();
-          }
-          ++taken;
-          if (more) {
-            ok = !loads || mbar_wait_addr(full0 + 8 * s_next, phase_next, &abort_flag, p.status, kStatusWaitRows);
-            alive = __all_sync(0xffffffffu, ok);
+          };
+          multiply(std::true_type{}, r0, r1, 0);
+          load_pair(from, r2);
+          multiply(std::false_type{}, r1, r2, 1);
+          r0 = r2;
+          load_pair(from + 2 * kRowBytes, r1);
+          multiply(std::false_type{}, r0, r1, 2);
+        }
+        // bias and activation: v[channel][0 / 1] = rows (0, 1) / (2, 3) of the lane's column
+        uint64_t v[8][2];
+        float margin = 0.0f;
 #pragma unroll
-            for (int j = 0; j < COLS + 4; ++j) raw[j] = lds32(lane_smem + s_next * kChunkBytes + j * (kChannels * 2));
+        for (int c = 0; c < 8; c += 2) {
+          uint64_t bias[2];
+          asm volatile("ld.shared.v2.b64 {%0, %1}, [%2];" : "=l"(bias[0]), "=l"(bias[1]) : "r"(bias_at + (piece * 8 + c) * 8));
+          float slack[2];
+#pragma unroll
+          for (int d = 0; d < 2; ++d) {
+            const float(&a)[4] = acc[c + d];
+            v[c + d][0] = add2(pack2(a[0], a[1]), bias[d]);
+            v[c + d][1] = add2(pack2(a[2], a[3]), bias[d]);
+            if (MODE == kOutBf16) {
+              float b, unused, f[4];
+              unpack2(bias[d], b, unused);
+              unpack2(v[c + d][0], f[0], f[1]);
+              unpack2(v[c + d][1], f[2], f[3]);
+              const float size = max_abs(max_abs(a[0], a[1], a[2]), a[3], b);
+              slack[d] = fmaf(min_abs(min_abs(f[0], f[1], f[2]), f[3], f[3]), kCancelled, -size);
+            }
+          }
+          if (MODE == kOutBf16) margin = fminf(fminf(margin, slack[0]), slack[1]);
+        }
+        if (MODE == kOutBf16 && margin < 0.0f) {
+          uint32_t cancelled = 0;  // bit 4 c + i
+#pragma unroll
+          for (int c = 0; c < 8; ++c) {
+            float f[4];
+            unpack2(v[c][0], f[0], f[1]);
+            unpack2(v[c][1], f[2], f[3]);
+            // (the bias is part of the size as the difference of sum and product part)
+            const float size = max_abs(max_abs(acc[c][0], acc[c][1], acc[c][2]), acc[c][3], f[0] - acc[c][0]) * (1.001f / kCancelled);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) cancelled |= fabsf(f[i]) <= size ? 1u << (4 * c + i) : 0u;
+          }
+#pragma unroll 1
+          for (; cancelled != 0; cancelled &= cancelled - 1) {
+            const int bit = __ffs(cancelled) - 1, row = y + (bit & 3);
+            if (x < p.width && row < p.height) note(list, at.b * p.height + row, x, piece * 8 + (bit >> 2));
           }
         }
-        if (!(PROBE && (p.debug & 1))) {
-          // 25 * COLS packed FMAs: input row r = 5 g + ph feeds tap row ky of the output row in slot (ph - ky) mod 5. Tap
-          // column outermost, so neighbouring instructions belong to 5 * COLS different accumulators and nothing waits on
-          // the FMA latency. Tap row 0 opens a new output row: its first term is a plain product (0 + a*b == a*b).
 #pragma unroll
-          for (int kx = 0; kx < 5; ++kx) {
+        for (int c = 0; c < 8; ++c) v[c][0] = activate2<ACT>(v[c][0]), v[c][1] = activate2<ACT>(v[c][1]);
+        float inv[4];
+        uint32_t unsure = 0;  // MX: bit i for a pixel whose block is to be summed again
+        if (MODE == kOutMx) {
+          float amax[4] = {0.0f, 0.0f, 0.0f, 0.0f};
 #pragma unroll
-            for (int ky = 0; ky < 5; ++ky) {
-              const int slot = (ph - ky + 5) % 5;
+          for (int c = 0; c < 8; c += 2) {
 #pragma unroll
-              for (int j = 0; j < COLS; ++j) {
-                if (kMixedFma) {
-                  // (a new output row starts from -0: the sum then keeps the sign of a zero first product, like a plain multiply)
-                  const bool first = ky == 0 && kx == 0;
-                  fma_bf16x2(row[j + kx], wpack[ky * 5 + kx], first ? -0.0f : facc[slot][j][0], first ? -0.0f : facc[slot][j][1],
-                             facc[slot][j][0], facc[slot][j][1]);
-                } else {
-                  acc[slot][j] = (ky == 0 && kx == 0) ? mul2(in[j], wreg[0]) : fma2(in[j + kx], wreg[ky * 5 + kx], acc[slot][j]);
-                }
+            for (int h = 0; h < 2; ++h) {
+              float lo0, hi0, lo1, hi1;
+              unpack2(v[c][h], lo0, hi0);
+              unpack2(v[c + 1][h], lo1, hi1);
+              amax[2 * h] = max_abs(amax[2 * h], lo0, lo1), amax[2 * h + 1] = max_abs(amax[2 * h + 1], hi0, hi1);
+            }
+          }
+          const uint32_t mine = exchange + flip * 2048 + lane * 16;
+          asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(mine + piece * 512), "f"(amax[0]), "f"(amax[1]), "f"(amax[2]), "f"(amax[3])
+                       : "memory");
+          if (piece == 0 && elect_one()) bulk_wait_read<0>();  // the store of the panel before the last
+          named_barrier(quad_barrier, 128);
+          if (piece == 0) {
+            if (stored_b >= 0) store_panel(panels + (flip ^ 1u) * panel_bytes(MODE), stored_c, stored_x, stored_y, stored_b);
+            if (alive) issue_until(taken + kStages);
+          }
+          stored_c = c0, stored_x = x0, stored_y = y, stored_b = p.tma_out ? at.b : -1;
+          float theirs[3][4];
+#pragma unroll
+          for (int other = 1; other < 4; ++other) {
+            float(&t)[4] = theirs[other - 1];
+            asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(t[0]), "=f"(t[1]), "=f"(t[2]), "=f"(t[3]) : "r"(mine + (piece ^ other) * 512));
+          }
+#pragma unroll
+          for (int i = 0; i < 4; ++i) amax[i] = fmaxf(max_abs(amax[i], theirs[0][i], theirs[1][i]), theirs[2][i]);
+          uint32_t bytes[4];
+          unsure = block_scales(amax, bytes, inv);
+          if (alive && x < p.width && y + piece < p.height) {  // each warp stores the scales of one row
+            const uint32_t byte = piece == 0 ? bytes[0] : piece == 1 ? bytes[1] : piece == 2 ? bytes[2] : bytes[3];
+            const uint32_t row = scale_row + y * p.width, groups = p.channels >> 5;
+            p.scales[p.swizzled ? static_cast<uint64_t>(row >> 7) * scale_tile_bytes + (row & 31) * 16 + ((row & 127) >> 5) * 4 + scale_at
+                                : static_cast<uint64_t>(row) * groups + ct] = static_cast<uint8_t>(byte);
+          }
+        }
+        // the lane's 8 channels of each of its four pixels, as they are stored
+        constexpr int kWords = 2 * kOutBytes;
+        uint32_t words[4][kWords];
+        const auto values_of = [&](int c, int i, float (&f)[4]) {  // channels c .. c + 3 of pixel i
+#pragma unroll
+          for (int d = 0; d < 4; ++d) {
+            float lo, hi;
+            unpack2(v[c + d][i >> 1], lo, hi);
+            f[d] = i & 1 ? hi : lo;
+          }
+        };
+        if (MODE == kOutMx) {
+          // Codes of the values pushed up and down by 2**-20: where they agree, they are the code, and no other order of
+          // summation gives another one.
+          constexpr float kUp = 1.0f + 0x1p-20f, kDown = 1.0f - 0x1p-20f;
+          const uint64_t up[2] = {pack2(inv[0] * kUp, inv[1] * kUp), pack2(inv[2] * kUp, inv[3] * kUp)};
+          const uint64_t down[2] = {pack2(inv[0] * kDown, inv[1] * kDown), pack2(inv[2] * kDown, inv[3] * kDown)};
+          uint32_t differ[4] = {0, 0, 0, 0};
+#pragma unroll
+          for (int c = 0; c < 8; c += 4) {
+            float f[4][4], g[4][4];
+#pragma unroll
+            for (int d = 0; d < 4; ++d) {
+#pragma unroll
+              for (int h = 0; h < 2; ++h) {
+                unpack2(mul2(v[c + d][h], up[h]), f[d][2 * h], f[d][2 * h + 1]);
+                unpack2(mul2(v[c + d][h], down[h]), g[d][2 * h], g[d][2 * h + 1]);
+              }
+            }
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              words[i][c / 4] = e4m3x4(f[0][i], f[1][i], f[2][i], f[3][i]);
+              differ[i] |= words[i][c / 4] ^ e4m3x4(g[0][i], g[1][i], g[2][i], g[3][i]);
+            }
+          }
+          if (((differ[0] | differ[1]) | (differ[2] | differ[3])) != 0 || unsure != 0) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              if (differ[i] != 0) {
+                float f[4], g[4];
+                values_of(0, i, f);
+                values_of(4, i, g);
+                words[i][0] = e4m3x4(f[0] * inv[i], f[1] * inv[i], f[2] * inv[i], f[3] * inv[i]);
+                words[i][1] = e4m3x4(g[0] * inv[i], g[1] * inv[i], g[2] * inv[i], g[3] * inv[i]);
+                unsure |= 1u << i;
+              }
+            }
+#pragma unroll 1
+            for (; unsure != 0; unsure &= unsure - 1) {
+              const int row = y + __ffs(unsure) - 1;
+              if (x < p.width && row < p.height) note(list, at.b * p.height + row, x, 0);
+            }
+          }
+        } else {
+#pragma unroll
+          for (int c = 0; c < 8; c += 4) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              float f[4];
+              values_of(c, i, f);
+              const uint32_t w0 = pack_bf16(f[0], f[1]), w1 = pack_bf16(f[2], f[3]);
+              if (MODE == kOutBf16) {
+                words[i][c / 2] = w0;
+                words[i][(c / 2 + 1) % kWords] = w1;
+              } else {
+                words[i][c / 4] = int8_pack4(int8, bf16_lo(w0), bf16_hi(w0), bf16_lo(w1), bf16_hi(w1));
               }
             }
           }
-        } else {
+        }
+        if (p.tma_out) {
 #pragma unroll
-          for (int j = 0; j < COLS; ++j) {  // keep the loads alive
-            if (kMixedFma) {
-              facc[(ph + 1) % 5][j][0] = __uint_as_float(row[j]), facc[(ph + 1) % 5][j][1] = __uint_as_float(row[j + 4]);
+          for (int i = 0; i < 4; ++i) {
+            const uint32_t pixel = i * kTileX + lane;
+            if (MODE == kOutBf16) {
+              asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(panel + pixel * 64 + turn), "r"(words[i][0]), "r"(words[i][1]),
+                           "r"(words[i][2 % kWords]), "r"(words[i][3 % kWords])
+                           : "memory");
             } else {
-              acc[(ph + 1) % 5][j] = in[j] ^ in[j + 4];
+              asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(panel + pixel * 32 + (((piece >> 1) ^ ((lane >> 2) & 1)) << 4) + (piece & 1) * 8),
+                           "r"(words[i][0]), "r"(words[i][1])
+                           : "memory");
+            }
+          }
+          fence_async_proxy();
+        } else if (alive) {
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            if (x < p.width && y + i < p.height) {
+              uint32_t* to = reinterpret_cast<uint32_t*>(
+                  p.out + (((static_cast<size_t>(at.b) * p.height + y + i) * p.width + x) * p.channels + c0 + piece * 8) * kOutBytes);
+#pragma unroll
+              for (int j = 0; j < kWords; ++j) to[j] = words[i][j];
             }
           }
         }
-        // The output row in slot (ph + 1) mod 5 has now received all five input rows: finish it (bias, activation, stores)
-        // straight from its accumulators. Nothing branches here: a row outside the span has an empty store mask, so the
-        // compiler is free to overlap this epilogue with the FMAs of the next input row.
-        {
-          const bool valid = y_out >= y_base && y_out < y_end;
-          if (!(PROBE && (p.debug & 2))) {
-            if (kMixedFma) {
-              uint64_t done[COLS];
-#pragma unroll
-              for (int j = 0; j < COLS; ++j) done[j] = pack2(facc[(ph + 1) % 5][j][0], facc[(ph + 1) % 5][j][1]);
-              emit_row<MODE, ACT, COLS, true>(p, done, bias2, out_row, pixel0, c, valid ? cols_ok : 0u, int8_scale, lane);
-            } else {
-              emit_row<MODE, ACT, COLS>(p, acc[(ph + 1) % 5], bias2, out_row, pixel0, c, valid ? cols_ok : 0u, int8_scale, lane);
-            }
+        if (MODE != kOutMx) {
+          if (piece == 0 && elect_one()) bulk_wait_read<0>();  // the store of the other panel
+          named_barrier(quad_barrier, 128);
+          if (piece == 0) {
+            if (p.tma_out && alive) store_panel(panel, c0 * kOutBytes, x0, y, at.b);
+            if (alive) issue_until(taken + kStages);
           }
-          pixel0 += valid ? static_cast<size_t>(p.width) : 0;
-          out_row += valid ? row_pairs * kOutBytes : 0;
         }
-        ++y_out;
+        flip ^= 1u;
       }
-      s = s_next, phase = phase_next;
+    }
+    if (MODE == kOutMx) {  // the last panel
+      named_barrier(quad_barrier, 128);
+      if (piece == 0 && stored_b >= 0 && alive) store_panel(panels + (flip ^ 1u) * panel_bytes(MODE), stored_c, stored_x, stored_y, stored_b);
+      stored_b = -1;
+    }
+    if (MODE != kOutInt8) {
+      // the outputs in the list once more, after the stores of their panels have completed
+      named_barrier(quad_barrier, 128);
+      uint32_t count;
+      asm volatile("ld.shared.b32 %0, [%1];" : "=r"(count) : "r"(list));
+      count = min(count, kListEntries);
+      if (count != 0) {
+        if (piece == 0 && elect_one()) bulk_wait_all();
+        named_barrier(quad_barrier, 128);
+      }
+      if (!alive) count = 0;
+#pragma unroll 1
+      for (uint32_t i = MODE == kOutMx ? piece : threadIdx.x & 127; i < count; i += MODE == kOutMx ? 4 : 128) {
+        uint32_t row, place;
+        asm volatile("ld.shared.v2.b32 {%0, %1}, [%2];" : "=r"(row), "=r"(place) : "r"(list + 8 + i * 8));
+        const int c = MODE == kOutMx ? lane : place & 31, px = place >> 5, b = row / p.height, y = row - b * p.height;
+        float bias;
+        asm volatile("ld.shared.f32 %0, [%1];" : "=f"(bias) : "r"(bias_at + c * 8));
+        const float sum = chain_sum(p.value + static_cast<size_t>(b) * p.height * p.width * p.channels + c0 + c, p.height, p.width, p.channels,
+                                    weights_at + c * 2, bias, y, px);
+        float out, unused;
+        unpack2(activate2<ACT>(pack2(sum, sum)), out, unused);
+        const size_t pixel = static_cast<size_t>(row) * p.width + px, to = pixel * p.channels + c0 + c;
+        if (MODE == kOutBf16) {
+          reinterpret_cast<uint16_t*>(p.out)[to] = static_cast<uint16_t>(pack_bf16(out, 0.0f));
+        } else {  // a warp per block
+          const int e = e8m0_exponent(__uint_as_float(redux_max(__float_as_uint(fabsf(out)), 0xffffffffu)));
+          p.out[to] = static_cast<uint8_t>(e4m3x2(out * exp2_int(-e), 0.0f));
+          const int groups = p.channels >> 5;
+          if (lane == 0) p.scales[p.swizzled ? swizzled_scale_offset(pixel, ct, (groups + 3) >> 2) : pixel * groups + ct] = static_cast<uint8_t>(e + 127);
+        }
+      }
     }
   }
+  if (piece == 0 && elect_one()) bulk_wait_read<0>();
   if (abort_flag) {
     // a wait ran out: give copies that are still in flight time to land before the shared memory is released
     const uint64_t t0 = global_timer_ns();
@@ -485,70 +668,23 @@ __global__ void __launch_bounds__(32 * WARPS, MIN_CTAS) dw5x5_kernel(const __gri
   }
 }
 
-int g_dw_variant = 0;
-int g_dw_probe = 0;
+int g_dw_max_ctas = 0;
 
-// Thread layouts that are compiled in: columns per lane, warps per CTA and the CTAs an SM is meant to hold (which caps
-// the registers). Tiles are COLS * WARPS columns wide.
-struct Variant {
-  int cols, warps, ctas_per_sm;
-};
-constexpr Variant kVariants[] = {
-    {4, 4, 3},  // 1: 16 columns, 12 warps per SM at 168 registers
-    {4, 5, 2},  // 2: 20 columns, 10 warps per SM
-    {2, 8, 2},  // 3: 16 columns, 16 warps per SM at 128 registers (two columns per lane)
-    {4, 4, 4},  // 4: 16 columns, 16 warps per SM at 128 registers (mixed-precision FMAs, packed weights, four-chunk ring)
-};
-constexpr int kVariantCount = sizeof(kVariants) / sizeof(kVariants[0]);
-
-int pick_variant(int width) {
-  if (g_dw_variant >= 1 && g_dw_variant <= kVariantCount) return g_dw_variant - 1;
-  // Measured on 100- to 400-pixel-wide images with every epilogue: four columns per lane on three CTAs of four warps is the
-  // fastest layout throughout. Two columns per lane hold sixteen warps on an SM but spend more instructions per element
-  // (dw -> MXFP8 on 8 x 400 x 400 x 128: 463 us against 369 us); 20-column tiles fit 100 and 200 columns exactly yet lose
-  // more to the fifth warp doubling up on one scheduler. Four CTAs per SM (128 registers with the packed weights of the
-  // mixed-precision form) measured 2-8 % slower than three: more warps do not buy the FMA pipe any time.
-  (void)width;
-  return 0;
-}
-
-template <int MODE, int COLS, int WARPS, int MIN_CTAS>
-cudaError_t launch_kernel(const CUtensorMap& map, const DwParams& p, int act, unsigned grid, cudaStream_t s) {
-  constexpr unsigned kBlock = WARPS * 32;
-  constexpr size_t kSmem = static_cast<size_t>(ring_stages(MIN_CTAS)) * kChunkRows * (WARPS * COLS + 4) * kChannels * 2;
-  // every instantiation gets the opt-in limit once per device (some chunk rings exceed the 48 KB default)
-  static bool configured[kMaxDevices] = {};
+template <int MODE>
+int launch_kernel(const CUtensorMap& in_map, const CUtensorMap& out_map, const DwParams& p, int act, unsigned grid, cudaStream_t s) {
+  constexpr size_t kSmem = 1024 + kQuads * quad_bytes(MODE);
+  static_assert(kSmem <= 227 * 1024, "shared memory of one CTA");
+  auto kernel = act == kActGelu ? dw5x5_kernel<MODE, kActGelu> : act == kActRelu ? dw5x5_kernel<MODE, kActRelu> : dw5x5_kernel<MODE, kActNone>;
+  // every instantiation gets the opt-in limit once per device
+  static bool configured[3][kMaxDevices] = {};
   const int device = current_device();
-  if (device < 0 || device >= kMaxDevices || !configured[device]) {
-    cudaError_t e = cudaSuccess;
-    auto set = [&](auto kernel) {
-      if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kSmem));
-    };
-    set(dw5x5_kernel<MODE, kActNone, COLS, WARPS, MIN_CTAS, false>);
-    set(dw5x5_kernel<MODE, kActRelu, COLS, WARPS, MIN_CTAS, false>);
-    set(dw5x5_kernel<MODE, kActGelu, COLS, WARPS, MIN_CTAS, false>);
-#if FIM_PROBE_BUILD
-    set(dw5x5_kernel<MODE, kActRelu, COLS, WARPS, MIN_CTAS, true>);
-    set(dw5x5_kernel<MODE, kActGelu, COLS, WARPS, MIN_CTAS, true>);
-#endif
-    if (e != cudaSuccess) return e;
-    if (device >= 0 && device < kMaxDevices) configured[device] = true;
+  if (device < 0 || device >= kMaxDevices || !configured[act][device]) {
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kSmem));
+    if (e != cudaSuccess) return static_cast<int>(e);
+    if (device >= 0 && device < kMaxDevices) configured[act][device] = true;
   }
-#if FIM_PROBE_BUILD
-  if (g_dw_probe != 0) {  // measurement hooks: a separate instantiation, so the production kernel carries no flag tests
-    if (act == kActGelu) dw5x5_kernel<MODE, kActGelu, COLS, WARPS, MIN_CTAS, true><<<grid, kBlock, kSmem, s>>>(map, p);
-    else dw5x5_kernel<MODE, kActRelu, COLS, WARPS, MIN_CTAS, true><<<grid, kBlock, kSmem, s>>>(map, p);
-    return cudaGetLastError();
-  }
-#endif
-  if (act == kActGelu) {
-    dw5x5_kernel<MODE, kActGelu, COLS, WARPS, MIN_CTAS, false><<<grid, kBlock, kSmem, s>>>(map, p);
-  } else if (act == kActRelu) {
-    dw5x5_kernel<MODE, kActRelu, COLS, WARPS, MIN_CTAS, false><<<grid, kBlock, kSmem, s>>>(map, p);
-  } else {
-    dw5x5_kernel<MODE, kActNone, COLS, WARPS, MIN_CTAS, false><<<grid, kBlock, kSmem, s>>>(map, p);
-  }
-  return cudaGetLastError();
+  kernel<<<grid, 128 * kQuads, kSmem, s>>>(in_map, out_map, p);
+  return static_cast<int>(cudaGetLastError());
 }
 
 template <int MODE>
@@ -562,47 +698,54 @@ int launch(const void* value, const void* weight, const float* bias, void* out, 
       (reinterpret_cast<uintptr_t>(out) & 3u)) {
     return kBadLayout;
   }
-  const Variant variant = kVariants[pick_variant(width)];
-  const int tile_cols = variant.cols * variant.warps;
   DwParams p;
+  p.value = static_cast<const uint16_t*>(value);
   p.weight = static_cast<const uint32_t*>(weight);
   p.bias = bias;
-  p.out = out;
+  p.out = static_cast<uint8_t*>(out);
   p.scales = static_cast<uint8_t*>(scales);
   p.scale = scale;
   p.batch = batch, p.height = height, p.width = width, p.channels = channels;
-  p.tiles_x = ceil_div(width, tile_cols);
-  p.channel_tiles = ceil_div(channels, kChannels);
-  p.strip_chunks = ceil_div(height, kChunkRows);
-  p.act = act, p.swizzled = swizzled, p.status = status, p.debug = g_dw_probe;
-  const long long units = static_cast<long long>(p.tiles_x) * p.channel_tiles * batch * p.strip_chunks;
-  if (units > 0x7fffffffLL) return kUnsupported;
-  p.total_units = static_cast<int>(units);
+  p.tiles_x = ceil_div(width, kTileX);
+  p.channel_tiles = channels / kTileC;
+  p.strip_steps = ceil_div(height, kStepRows);
+  p.swizzled = swizzled, p.status = status;
+  p.tma_out = (reinterpret_cast<uintptr_t>(out) & 15u) == 0;
+  const long long steps = static_cast<long long>(p.tiles_x) * batch * p.strip_steps;
+  if (steps > 0x3fffffffLL || steps * p.channel_tiles > 0x3fffffffffLL) return kUnsupported;
+  p.total_steps = static_cast<int>(steps);
 
-  CUtensorMap map;
-  const uint64_t dims[4] = {static_cast<uint64_t>(channels), static_cast<uint64_t>(width), static_cast<uint64_t>(height),
-                            static_cast<uint64_t>(batch)};
-  const uint64_t strides[3] = {static_cast<uint64_t>(channels) * 2, static_cast<uint64_t>(width) * channels * 2,
-                               static_cast<uint64_t>(height) * width * channels * 2};
-  const uint32_t box[4] = {kChannels, static_cast<uint32_t>(tile_cols + 4), kChunkRows, 1};
-  // a CTA reads 128 bytes (64 channels) of every pixel: with more channels than that, fetching 256-byte granules into L2
-  // would drag in the neighbouring channel tile, which another CTA reads much later
-  const int rc = make_tensor_map(&map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, value, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_NONE,
-                                 channels > kChannels ? CU_TENSOR_MAP_L2_PROMOTION_L2_128B : CU_TENSOR_MAP_L2_PROMOTION_L2_256B);
-  if (rc != kOk) return rc;
-
-  // persistent CTAs, as many as the SMs hold; a small problem gets fewer, each with at least four units so the halo chunk
-  // stays cheap
-  const long long resident = static_cast<long long>(sm_count()) * variant.ctas_per_sm;
-  const long long want = (units + 3) / 4;
-  const unsigned grid = static_cast<unsigned>(want < resident ? want : resident);
-  cudaStream_t s = static_cast<cudaStream_t>(stream);
-  cudaError_t e;
-  if (variant.cols == 2) e = launch_kernel<MODE, 2, 8, 2>(map, p, act, grid, s);
-  else if (variant.warps == 4 && variant.ctas_per_sm == 4) e = launch_kernel<MODE, 4, 4, 4>(map, p, act, grid, s);
-  else if (variant.warps == 4) e = launch_kernel<MODE, 4, 4, 3>(map, p, act, grid, s);
-  else e = launch_kernel<MODE, 4, 5, 2>(map, p, act, grid, s);
-  return static_cast<int>(e);
+  CUtensorMap in_map, out_map;
+  {
+    const uint64_t dims[4] = {static_cast<uint64_t>(channels), static_cast<uint64_t>(width), static_cast<uint64_t>(height),
+                              static_cast<uint64_t>(batch)};
+    const uint64_t row = static_cast<uint64_t>(channels) * 2;
+    const uint64_t strides[3] = {row, width * row, static_cast<uint64_t>(height) * width * row};
+    const uint32_t box[4] = {kTileC, kHaloX, kStepRows, 1};
+    const int rc = make_tensor_map(&in_map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, value, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_64B,
+                                   CU_TENSOR_MAP_L2_PROMOTION_L2_128B);
+    if (rc != kOk) return rc;
+  }
+  out_map = in_map;
+  if (p.tma_out) {
+    const int elem = MODE == kOutBf16 ? 2 : 1;
+    const uint64_t row = static_cast<uint64_t>(channels) * elem;  // (in bytes, whatever the element)
+    const uint64_t dims[4] = {row, static_cast<uint64_t>(width), static_cast<uint64_t>(height), static_cast<uint64_t>(batch)};
+    const uint64_t strides[3] = {row, width * row, static_cast<uint64_t>(height) * width * row};
+    const uint32_t box[4] = {static_cast<uint32_t>(kTileC * elem), kTileX, kStepRows, 1};
+    const int rc = make_tensor_map(&out_map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 4, out, dims, strides, box,
+                                   MODE == kOutBf16 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B);
+    if (rc != kOk) return rc;
+  }
+  // one persistent CTA per SM with three quads; a small problem spreads over as many SMs as it has work for
+  const int sms = g_dw_max_ctas > 0 && g_dw_max_ctas < sm_count() ? g_dw_max_ctas : sm_count();
+  p.group_quads = p.channel_tiles < sms * kQuads ? p.channel_tiles : sms * kQuads;
+  const long long most_groups = sms * kQuads / p.group_quads;
+  p.groups = static_cast<int>(steps < most_groups ? steps : most_groups);
+  const int quads = p.groups * p.group_quads;
+  p.cta_quads = ceil_div(quads, sms);
+  const unsigned grid = static_cast<unsigned>(ceil_div(quads, p.cta_quads));
+  return launch_kernel<MODE>(in_map, out_map, p, act, grid, static_cast<cudaStream_t>(stream));
 }
 
 }  // namespace
@@ -628,8 +771,8 @@ extern "C" int fim_dw5x5_relu_int8(const void* value, const void* weight, const 
 }
 
 extern "C" void fim_dw_tune(int variant, int probe_flags) {
-  g_dw_variant = variant;
-  g_dw_probe = probe_flags;
+  g_dw_max_ctas = variant;
+  (void)probe_flags;
 }
 
 extern "C" int fim_abi_version(void) { return FIM_ABI_VERSION; }
