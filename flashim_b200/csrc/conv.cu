@@ -36,6 +36,7 @@ constexpr int kTileM = 128;
 constexpr uint32_t kTmemColumns = 512;
 constexpr int kMaxStages = 12;  // a short K loop is bound by the latency of a stage's round trip: more stages in flight
 constexpr int kSmemLimit = 226 * 1024;
+constexpr int kMaxWeightSteps = 32;  // patch kernels: K steps (tap, channel chunk) whose weights have a barrier of their own
 
 // Division of a tile index by a run-time constant without the integer-division sequence (some forty instructions, which a
 // warp that owns 32 columns of a tile would pay several times per tile): q = floor(x * floor(2**32 / d) / 2**32) is the
@@ -93,6 +94,7 @@ struct ConvParams {
   int convert_static;        // bf16 activations: 1 = quantise with act_exponent, 0 = per pixel and 32 channels on the fly
   int warp_panels;           // flat 1x1 convs: every epilogue warp stages and stores its own 32 rows (no barrier between warps)
   int pool;                  // INT8, bf16 output: the 2x2 max pool of the output also leaves the epilogue, as INT8 codes (out_scale)
+  uint32_t patch_bytes, patch_pitch, patch_rows;  // kPatch: one channel chunk's patch (rounded up to 1 KB), one patch row, its rows
   int debug;  // probe builds only (FIM_PROBE_BUILD): 1 = no activation loads, 2 = no weight loads, 4 = no output stores, 8 = no scale copies
 };
 
@@ -109,6 +111,7 @@ struct SharedControl {
   uint64_t tmem_full[2];
   uint64_t tmem_empty[2];
   uint64_t weights_ready;          // resident weights: their one-time copies have landed
+  uint64_t weights_step[kMaxWeightSteps];  // kPatch: the same per K step (the first one's counts the scale tiles too)
   uint64_t raw_full[kRawStages];   // bf16 landing ring of a converting layer
   uint64_t raw_empty[kRawStages];
   uint32_t tmem_base;
@@ -187,6 +190,18 @@ __device__ __forceinline__ uint32_t idesc_bf16(int block_n, int block_m = kTileM
 constexpr uint32_t kPoolPanelBytes = 1024;  // 32 pooled pixels x 32 INT8 channels
 constexpr int kEpiGelu = 1, kEpiDynamic = 2, kEpiResidual = 4, kEpiLean = 8, kEpiFixed = 16, kEpiStatic = 32, kEpiPool = 64;
 
+// kPatch (with any of the epilogues above): a spatial conv whose whole weight matrix stays in shared memory and whose
+// activations arrive as one halo patch per tile instead of one shifted tile per tap. A tile is 8 columns x 16 rows of output
+// pixels; its patch of (8 + halo) x (16 + halo) pixels lies in the swizzled layout TMA gives it, and a tap's A operand is
+// that patch read from a shifted start address: eight pixels of a row are one 8-row group of the K-major layout, and the
+// groups are one patch row apart (the descriptor's stride). The swizzle is a function of the shared-memory address, so a
+// shifted start needs no other layout. Per tile that is one copy and one barrier round instead of one per tap and channel
+// chunk, 1.4 activation bytes per input byte instead of 9 (3x3), and no scale copies: all weight scales stay in tensor memory.
+//   MXFP8 3x3 + bias + GELU + static requantisation, N = 4: 800x800x64 363 -> 232 us, 400x400x128 117 -> 96 (with a plain
+//   bf16 output 107 -> 77); INT8 3x3 + bias: 4x201x199x128 31 -> 22, 4x400x400x64 84 -> 54.
+constexpr int kPatch = 128;
+constexpr int kPatchTileW = 8, kPatchTileH = 16;
+
 struct EpilogueSwitches {
   int act, out_mode;
   uint32_t out_elem, panels;  // bytes per output element; output panels per group
@@ -199,7 +214,7 @@ __device__ __forceinline__ EpilogueSwitches epilogue_switches(const ConvParams& 
     sw.act = (EPI & kEpiGelu) ? kActGelu : kActNone;
     sw.out_mode = (EPI & kEpiStatic) ? FIM_OUT_E4M3_STATIC : ((EPI & kEpiDynamic) ? FIM_OUT_E4M3_DYNAMIC : FIM_OUT_BF16);
     sw.out_elem = sw.out_mode == FIM_OUT_BF16 ? 2u : 1u;
-    sw.panels = 2u;
+    sw.panels = (EPI & kPatch) != 0 ? static_cast<uint32_t>(p.panels_per_half) : 2u;
     sw.has_bias = true;
     sw.has_residual = (EPI & kEpiResidual) != 0;
   } else {
@@ -443,7 +458,9 @@ conv_kernel(const __grid_constant__ CUtensorMap act_map, const __grid_constant__
   static_assert(!PAIR || BN == 256 || (BN == 128 && FMT == kFmtMx), "CTA pairs are built for 256-wide tiles (and 128-wide block-scaled ones)");
   static_assert(!CONVERT || (FMT == kFmtMx && !PAIR && BK == 128), "the converter feeds flat block-scaled layers");
   constexpr int kBlockThreads = CONVERT ? kConvertThreads : kThreads;
-  static_assert((EPI & kEpiPool) == 0 || (FMT == kFmtI8 && EPI == kEpiPool), "the pooled output belongs to the INT8 conv's general epilogue");
+  constexpr bool PATCH = (EPI & kPatch) != 0;
+  static_assert(!PATCH || (!PAIR && !CONVERT && BN <= 128), "patches serve single CTAs with resident weights");
+  static_assert((EPI & kEpiPool) == 0 || (FMT == kFmtI8 && (EPI & ~kPatch) == kEpiPool), "the pooled output belongs to the INT8 conv's general epilogue");
   static_assert((EPI & kEpiLean) == 0 || (FMT == kFmtMx && !PAIR && BN >= 128), "the short epilogues serve flat block-scaled layers");
   constexpr bool INT8 = FMT == kFmtI8;
   constexpr bool SCALED = FMT == kFmtMx;  // operands carry E8M0 block scales
@@ -476,12 +493,16 @@ conv_kernel(const __grid_constant__ CUtensorMap act_map, const __grid_constant__
   const uint32_t panel_bytes = 4096u * p.out_elem;
   const uint32_t smem_gelu = base;  // kGeluTable first, when the epilogue applies GELU: within 64 KB of the window's start
   const uint32_t smem_a = base + (p.act == kActGelu ? kGeluSmemBytes : 0u);
-  const uint32_t smem_b = smem_a + p.stages * kABytes;
+  const uint32_t a_stage = PATCH ? p.patch_bytes * static_cast<uint32_t>(p.k_chunks) : kABytes;
+  const uint32_t smem_b = smem_a + p.stages * a_stage;
   const uint32_t smem_out = smem_b + static_cast<uint32_t>(p.b_slots) * kBBytes;
   const uint32_t smem_pool = smem_out + kPanelGroups * p.panels_per_half * panel_bytes;  // pooled panels: two of 1 KB per group
-  const uint32_t smem_sfb = smem_pool + (p.pool ? kPanelGroups * 2u * kPoolPanelBytes : 0u);
-  const uint32_t smem_sfa = smem_sfb + static_cast<uint32_t>(p.b_slots) * kScaleTilesB * 512;
-  const uint32_t smem_sfa_static = smem_sfa + p.stages * 512;
+  const uint32_t smem_scales = smem_pool + (p.pool ? kPanelGroups * 2u * kPoolPanelBytes : 0u);
+  // (kPatch: the weight scale tiles pass through the output panels on their way to tensor memory; no panel is written before
+  // the first accumulator, and that comes after these copies)
+  const uint32_t smem_sfb = PATCH ? smem_out : smem_scales;
+  const uint32_t smem_sfa = PATCH ? smem_scales : smem_sfb + static_cast<uint32_t>(p.b_slots) * kScaleTilesB * 512;
+  const uint32_t smem_sfa_static = PATCH ? smem_scales : smem_sfa + p.stages * 512;
   const uint32_t smem_bias = smem_sfa_static + ((p.cin + 127) / 128) * 512;  // fp32, tiles_n * BN entries
   const uint32_t smem_raw = (smem_bias + static_cast<uint32_t>(p.tiles_n * BN) * 4u + 1023u) & ~1023u;  // CONVERT: bf16 landing ring
 
@@ -502,6 +523,9 @@ conv_kernel(const __grid_constant__ CUtensorMap act_map, const __grid_constant__
       mbar_init(&ctl.empty[s], 1);
     }
     mbar_init(&ctl.weights_ready, 1);
+    if (PATCH) {
+      for (int i = 0; i < taps * p.k_chunks; ++i) mbar_init(&ctl.weights_step[i], 1);
+    }
     if (CONVERT) {
       for (int s = 0; s < kRawStages; ++s) {
         mbar_init(&ctl.raw_full[s], 1);
@@ -590,6 +614,35 @@ conv_kernel(const __grid_constant__ CUtensorMap act_map, const __grid_constant__
       bool alive = true;
       int last_n0 = -1;
       const bool resident_b = in_register(static_cast<uint32_t>(p.weights_resident)) != 0;
+      if constexpr (PATCH) {
+        // one patch per tile; behind the first one the weights, K step by K step, which the first tile's MMAs wait for singly
+        const int k_total = kh * kw * k_chunks;
+        const uint32_t chunk_bytes = in_register(p.patch_pitch * p.patch_rows), chunk_at = in_register(p.patch_bytes);
+        bool first = true;
+        for (int tile = worker; tile < p.total_tiles; tile += workers) {
+          int m, n0, width, tx, ty, b;
+          decode_tile<BN>(p, tile, m, n0, width);
+          divmod(m, p.div_tiles_x, m, tx);
+          divmod(m, p.div_tiles_y, b, ty);
+          const int x0 = tx * kPatchTileW - p.pad_w, y0 = ty * kPatchTileH - p.pad_h;
+          if (!loop_wait(empty0 + 8 * s, phase ^ 1, kStatusWaitEmpty)) break;
+          mbar_expect_tx_addr(full0 + 8 * s, chunk_bytes * static_cast<uint32_t>(k_chunks));
+          for (int j = 0; j < k_chunks; ++j) {
+            tma_load_4d_addr(smem_a + s * a_stage + j * chunk_at, &act_map, full0 + 8 * s, j * BK, x0, y0, b);
+          }
+          if (++s == stages) s = 0, phase ^= 1;
+          if (first) {
+            first = false;
+            const uint32_t step0 = smem_u32(&ctl.weights_step[0]);
+            const int scale_tiles = SCALED ? (k_total * kKSteps + 3) / 4 : 0;
+            for (int ki = 0; ki < k_total; ++ki) {
+              mbar_expect_tx_addr(step0 + 8 * ki, kBBytes + (ki == 0 ? scale_tiles * 512u : 0u));
+              if (ki == 0 && SCALED) bulk_load_addr(smem_sfb, p.weight_scales, scale_tiles * 512u, step0);
+              tma_load_2d_addr(smem_b + ki * kBBytes, &weight_map, step0 + 8 * ki, ki * BK, 0);
+            }
+          }
+        }
+      } else {
       if (resident_b && worker < p.total_tiles && (kLaneLoop || elect_one())) {
         // A layer with one output-channel tile whose weights fit beside the activation ring: every K step's weight tile
         // and scale tiles are copied once and stay; the loop below then moves activations only.
@@ -723,6 +776,7 @@ conv_kernel(const __grid_constant__ CUtensorMap act_map, const __grid_constant__
           }
         }
       }
+      }
     }
   } else if (warp == 1) {
     // ===== MMA issuer (of a pair: the leader CTA's) =====
@@ -753,6 +807,73 @@ conv_kernel(const __grid_constant__ CUtensorMap act_map, const __grid_constant__
       uint32_t s = 0, phase = 0, tile_it = 0;
       bool alive = true;
       int last_n0 = -1;
+      if constexpr (PATCH) {
+        const int taps_w = static_cast<int>(in_register(static_cast<uint32_t>(p.kw)));
+        const uint32_t pitch = in_register(p.patch_pitch), chunk_at = in_register(p.patch_bytes);
+        const uint32_t step_x = in_register(static_cast<uint32_t>(p.dil_w) * BK), step_y = in_register(static_cast<uint32_t>(p.dil_h) * p.patch_pitch);
+        const uint32_t step0 = smem_u32(&ctl.weights_step[0]);
+        // eight pixels of a patch row per 8-row group, groups one patch row apart
+        const uint64_t patch_desc0 = (a_desc0 & ~(0x3FFFull << 32)) | (static_cast<uint64_t>(pitch >> 4) << 32);
+        const uint32_t idesc = INT8 ? idesc_i8(BN) : idesc_mxf8(BN);
+        bool first = true;
+        for (int tile = worker; tile < p.total_tiles; tile += workers, ++tile_it) {
+          const uint32_t acc = kAccStages == 2 ? (tile_it & 1u) : 0u;
+          const uint32_t acc_phase = kAccStages == 2 ? ((tile_it >> 1) & 1u) : (tile_it & 1u);
+          if (!loop_wait(tempty0 + 8 * acc, acc_phase ^ 1, kStatusWaitTmemEmpty)) break;
+          if (!loop_wait(full0 + 8 * s, phase, kStatusWaitFull)) break;
+          tc_fence_after();
+          const uint32_t d_tmem = tmem + acc * BN;
+          uint64_t row_desc = patch_desc0 + static_cast<uint64_t>((s * a_stage) >> 4), tap_desc = row_desc, b_desc = b_desc0;
+          uint32_t kb = 0;  // 32-channel block along the weight's K axis
+          int tap_x = 0, j = 0;
+          uint32_t chunk = 0;
+          for (int ki = 0; ki < k_iters; ++ki) {
+            if (first) {
+              if (!loop_wait(step0 + 8 * ki, 0, kStatusWaitFull)) {
+                alive = false;
+                break;
+              }
+              tc_fence_after();
+              if (ki == 0 && copy_scales) {
+                for (int t = 0; t < (k_iters * kKSteps + 3) / 4; ++t) {
+                  tc_copy_scales(sfb_resident_base + kSfbColumns * t, sfb_desc0 + static_cast<uint64_t>((t * 512) >> 4));
+                }
+              }
+            }
+            const uint64_t a_desc = tap_desc + (chunk >> 4);
+            const uint32_t kb_a = static_cast<uint32_t>(j) * kKSteps;
+            const uint32_t scaled0 = idesc | ((kb_a & 3u) << 29) | ((kb & 3u) << 4);
+            const uint32_t sfa_tmem = sfa_base + 4 * (kb_a >> 2), sfb_tmem = sfb_resident_base + kSfbColumns * (kb >> 2);
+#pragma unroll
+            for (int k = 0; k < kKSteps; ++k) {
+              const uint32_t accumulate = k > 0 ? 1u : (ki > 0 ? 1u : 0u);
+              if (INT8) {
+                tc_mma_i8(d_tmem, a_desc + 2 * k, b_desc + 2 * k, idesc, accumulate);
+              } else {
+                tc_mma_mxf8(d_tmem, a_desc + 2 * k, b_desc + 2 * k, scaled0 + static_cast<uint32_t>(k) * ((1u << 29) | (1u << 4)), sfa_tmem,
+                            sfb_tmem, accumulate);
+              }
+            }
+            b_desc += kBBytes >> 4;
+            kb += kKSteps;
+            chunk += chunk_at;
+            if (++j == k_chunks) {
+              j = 0, chunk = 0;
+              tap_desc += step_x >> 4;
+              if (++tap_x == taps_w) {
+                tap_x = 0;
+                row_desc += step_y >> 4;
+                tap_desc = row_desc;
+              }
+            }
+          }
+          if (!alive) break;
+          first = false;
+          tc_commit(&ctl.empty[s]);
+          tc_commit(&ctl.tmem_full[acc]);
+          if (++s == stages) s = 0, phase ^= 1;
+        }
+      } else {
       const bool resident_b = in_register(static_cast<uint32_t>(p.weights_resident)) != 0;
       if (resident_b && worker < p.total_tiles) alive = loop_wait(smem_u32(&ctl.weights_ready), 0, kStatusWaitFull);
 #if FIM_PROBE_BUILD
@@ -883,6 +1004,7 @@ conv_kernel(const __grid_constant__ CUtensorMap act_map, const __grid_constant__
                double(c_wait) / double(c_rounds), double(c_issue) / double(c_rounds), double(c_tile) / double(tile_it), tile_it, clock64() - c_start);
       }
 #endif
+      }
     }
   } else if (CONVERT && warp >= 2 + 16) {
     // ===== converter: bf16 landing tile -> E4M3 K-major stage (+ the stage's activation-scale tile) =====
@@ -1769,6 +1891,8 @@ struct Plan {
   bool flat;
   bool pair;  // clusters of two CTAs driving one cta_group::2 instruction stream
   bool convert = false;    // bf16 activations, quantised on chip
+  bool patch = false;      // one halo patch of activations per tile (kPatch)
+  int patch_w = 0, patch_h = 0, patch_bytes = 0;
   bool resident_b = false; // the whole weight matrix stays in shared memory (one output-channel tile, small K)
   int fixed_epilogue = 0;  // kEpiLean | switches when one of the compile-time epilogues serves this call, else 0
   int out_h, out_w;
@@ -1890,6 +2014,31 @@ int make_plan(const FimConvGeometry& g, int fmt, bool per_pixel, bool allow_flat
       pl.smem = static_cast<size_t>(fixed) + all_b + static_cast<size_t>(pl.stages) * a_stage;
     }
   }
+  // Patches instead of one activation tile per tap: a spatial conv (stride 1) with one output-channel tile of at most 128
+  // columns whose weights fit in shared memory beside two patches. Its tiles are 8 x 16 whatever the image; the padded
+  // pixels that costs at the edges (14 % at 100 x 100) are less than the copies it saves at any size measured.
+  if (g.kh * g.kw > 1 && g.stride_h == 1 && g.stride_w == 1 && fmt != kFmtBf16 && !per_pixel && !convert && bn <= 128 && pl.tiles_n == 1 &&
+      !(g_debug_flags & 2048) && k_iters <= kMaxWeightSteps) {
+    const int pw = kPatchTileW + g.dil_w * (g.kw - 1), ph = kPatchTileH + g.dil_h * (g.kh - 1);
+    const int chunk = (pw * ph * pl.block_k + 1023) / 1024 * 1024, chunks = g.cin / pl.block_k;
+    const int scale_tiles = scaled ? (k_iters * (pl.block_k / 32) + 3) / 4 : 0;
+    const long long tx = ceil_div(out_w, kPatchTileW), ty = ceil_div(out_h, kPatchTileH), tiles = tx * ty * g.batch;
+    for (int panels = pl.panels_per_half; panels >= 1 && !pl.patch; --panels) {
+      const int room = kSmemLimit - (1024 + epilogue_groups * panels * 4096 * out_elem + ((g.cin + 127) / 128) * 512 + bias_bytes + gelu_bytes +
+                                     pool_bytes) - k_iters * bn * pl.block_k;
+      const int fit = room / (chunks * chunk);
+      if (fit < 2 || pw > 256 || ph > 256 || tiles > 0x3fffffffLL || scale_tiles * 512 > epilogue_groups * panels * 4096 * out_elem) continue;
+      if (acc_stages(bn) * bn + 4 * 6 + 4 * ((g.cin + 127) / 128) + 4 * scale_tiles > 512) continue;  // tensor memory
+      pl.patch = true, pl.pair = false, pl.resident_b = true;
+      pl.panels_per_half = panels;
+      pl.stages = fit < 6 ? fit : 6;
+      pl.tile_w = kPatchTileW, pl.tile_h = kPatchTileH;
+      pl.patch_w = pw, pl.patch_h = ph, pl.patch_bytes = chunk;
+      pl.tiles_x = static_cast<int>(tx), pl.tiles_y = static_cast<int>(ty);
+      pl.total_tiles = static_cast<int>(tiles);
+      pl.smem = static_cast<size_t>(kSmemLimit - room) + static_cast<size_t>(pl.stages) * chunks * chunk;
+    }
+  }
   const int device_sms = sm_count();
   const int sms = g_max_ctas > 0 && g_max_ctas < device_sms ? g_max_ctas : device_sms;
   pl.ctas = pl.total_tiles < sms ? pl.total_tiles : sms;
@@ -1969,8 +2118,27 @@ int launch_conv(const ConvMaps& maps, const ConvParams& p, const Plan& pl, cudaS
   return static_cast<int>(cudaGetLastError());
 }
 
+// The patch kernels of one format and tile width, by K step and epilogue.
+template <int FMT, int BN, int EPI>
+int launch_patch(const ConvMaps& maps, const ConvParams& p, const Plan& pl, cudaStream_t stream) {
+  if (pl.block_k == 128) return launch_conv<FMT, BN, 128, false, kPatch | EPI>(maps, p, pl, stream);
+  if (pl.block_k == 64) return launch_conv<FMT, BN, 64, false, kPatch | EPI>(maps, p, pl, stream);
+  if constexpr ((EPI & kEpiPool) == 0) return launch_conv<FMT, BN, 32, false, kPatch | EPI>(maps, p, pl, stream);
+  return kUnsupported;
+}
+
 template <int FMT, int BN>
 int launch_conv_k(const ConvMaps& maps, const ConvParams& p, const Plan& pl, cudaStream_t stream) {
+  if constexpr (FMT != kFmtBf16 && BN <= 128) {
+    if (pl.patch) {
+      if constexpr (FMT == kFmtMx) {
+        if (pl.fixed_epilogue == (kEpiFixed | kEpiGelu | kEpiStatic)) return launch_patch<FMT, BN, kEpiFixed | kEpiGelu | kEpiStatic>(maps, p, pl, stream);
+      } else {
+        if (pl.fixed_epilogue == kEpiPool) return launch_patch<FMT, BN, kEpiPool>(maps, p, pl, stream);
+      }
+      return launch_patch<FMT, BN, 0>(maps, p, pl, stream);
+    }
+  }
   // the general epilogue with its switches fixed at compile time, for the layers measured most: a block-scaled conv with
   // bias, GELU and static requantisation at each tile width's usual K step, and the INT8 conv with bias and bf16 output
   constexpr int kGeluStatic = kEpiFixed | kEpiGelu | kEpiStatic;
@@ -2094,7 +2262,7 @@ int run_conv(int fmt, const void* x, const int8_t* act_exponent, const void* act
   }
   const int rc = make_plan(*g, fmt, per_pixel, allow_flat, out_elem, ep->act == FIM_ACT_GELU, &pl, convert, pool);
   if (rc != kOk) return rc;
-  if (pool && (pl.out_h < 2 || pl.out_w < 2 || pl.panels_per_half != 2)) return kUnsupported;  // no whole window: nothing to pool
+  if (pool && (pl.out_h < 2 || pl.out_w < 2 || (pl.panels_per_half != 2 && !pl.patch))) return kUnsupported;  // no whole window: nothing to pool
 
   const Schedule sc = make_schedule(*g, pl, fmt != kFmtMx, per_pixel);
   ConvParams p;
@@ -2130,6 +2298,8 @@ int run_conv(int fmt, const void* x, const int8_t* act_exponent, const void* act
   p.out_scales = static_cast<uint8_t*>(ep->out_scales);
   p.out_scale = ep->out_scale;
   p.pool = pool ? 1 : 0;
+  p.patch_bytes = static_cast<uint32_t>(pl.patch_bytes), p.patch_pitch = static_cast<uint32_t>(pl.patch_w * pl.block_k);
+  p.patch_rows = static_cast<uint32_t>(pl.patch_h);
   p.status = status;
   p.debug = g_debug_flags;
   p.poll_backoff_ns = (g_debug_flags & 32) ? 0u : 200u;
@@ -2162,8 +2332,8 @@ int run_conv(int fmt, const void* x, const int8_t* act_exponent, const void* act
     const uint64_t strides[3] = {static_cast<uint64_t>(g->cin), static_cast<uint64_t>(in_w) * g->cin,
                                  static_cast<uint64_t>(in_h) * in_w * g->cin};
     // a strided conv reads every stride-th pixel of a box stride times as wide: the copy lands densely in shared memory
-    const uint32_t box[4] = {static_cast<uint32_t>(pl.block_k), static_cast<uint32_t>(pl.tile_w * g->stride_w),
-                             static_cast<uint32_t>(pl.tile_h * g->stride_h), 1};
+    const uint32_t box[4] = {static_cast<uint32_t>(pl.block_k), static_cast<uint32_t>(pl.patch ? pl.patch_w : pl.tile_w * g->stride_w),
+                             static_cast<uint32_t>(pl.patch ? pl.patch_h : pl.tile_h * g->stride_h), 1};
     const uint32_t steps[4] = {1, static_cast<uint32_t>(g->stride_w), static_cast<uint32_t>(g->stride_h), 1};
     const int rcm = make_tensor_map(&act_map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 4, x, dims, strides, box, swizzle_for_bytes(pl.block_k),
                                     CU_TENSOR_MAP_L2_PROMOTION_L2_256B, steps);
@@ -2214,7 +2384,7 @@ int run_conv(int fmt, const void* x, const int8_t* act_exponent, const void* act
       pl.fixed_epilogue = kEpiLean | kEpiGelu | kEpiDynamic;
     }
   }
-  if (pl.fixed_epilogue == 0 && p.bias != nullptr && p.residual == nullptr && pl.panels_per_half == 2 && !(g_debug_flags & 1024)) {
+  if (pl.fixed_epilogue == 0 && p.bias != nullptr && p.residual == nullptr && (pl.panels_per_half == 2 || pl.patch) && !(g_debug_flags & 1024)) {
     if (fmt == kFmtMx && p.act == kActGelu && p.out_mode == FIM_OUT_E4M3_STATIC) pl.fixed_epilogue = kEpiFixed | kEpiGelu | kEpiStatic;
     if (fmt == kFmtI8 && p.act == kActNone && p.out_mode == FIM_OUT_BF16 && !pool) pl.fixed_epilogue = kEpiFixed;
   }
