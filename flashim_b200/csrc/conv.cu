@@ -197,7 +197,7 @@ constexpr int kEpiGelu = 1, kEpiDynamic = 2, kEpiResidual = 4, kEpiLean = 8, kEp
 // groups are one patch row apart (the descriptor's stride). The swizzle is a function of the shared-memory address, so a
 // shifted start needs no other layout. Per tile that is one copy and one barrier round instead of one per tap and channel
 // chunk, 1.4 activation bytes per input byte instead of 9 (3x3), and no scale copies: all weight scales stay in tensor memory.
-//   MXFP8 3x3 + bias + GELU + static requantisation, N = 4: 800x800x64 363 -> 232 us, 400x400x128 117 -> 96 (with a plain
+//   MXFP8 3x3 + bias + GELU + static requantisation, N = 4: 800x800x64 363 -> 176 us, 400x400x128 117 -> 96 (with a plain
 //   bf16 output 107 -> 77); INT8 3x3 + bias: 4x201x199x128 31 -> 22, 4x400x400x64 84 -> 54.
 constexpr int kPatch = 128;
 constexpr int kPatchTileW = 8, kPatchTileH = 16;
@@ -812,27 +812,50 @@ conv_kernel(const __grid_constant__ CUtensorMap act_map, const __grid_constant__
         const uint32_t pitch = in_register(p.patch_pitch), chunk_at = in_register(p.patch_bytes);
         const uint32_t step_x = in_register(static_cast<uint32_t>(p.dil_w) * BK), step_y = in_register(static_cast<uint32_t>(p.dil_h) * p.patch_pitch);
         const uint32_t step0 = smem_u32(&ctl.weights_step[0]);
-        // eight pixels of a patch row per 8-row group, groups one patch row apart
+        // eight pixels of a patch row per 8-row group, groups one patch row apart. Only the low words of the descriptors
+        // (the addresses) change from step to step.
         const uint64_t patch_desc0 = (a_desc0 & ~(0x3FFFull << 32)) | (static_cast<uint64_t>(pitch >> 4) << 32);
-        const uint32_t idesc = INT8 ? idesc_i8(BN) : idesc_mxf8(BN);
-        bool first = true;
-        for (int tile = worker; tile < p.total_tiles; tile += workers, ++tile_it) {
-          const uint32_t acc = kAccStages == 2 ? (tile_it & 1u) : 0u;
+        const uint32_t a_low0 = in_register(static_cast<uint32_t>(patch_desc0)), a_high = in_register(static_cast<uint32_t>(patch_desc0 >> 32));
+        const uint32_t b_low0 = in_register(static_cast<uint32_t>(b_desc0)), b_high = in_register(static_cast<uint32_t>(b_desc0 >> 32));
+        const auto desc = [](uint32_t low, uint32_t high) { return static_cast<uint64_t>(high) << 32 | low; };
+        const uint32_t idesc = in_register(INT8 ? idesc_i8(BN) : idesc_mxf8(BN));
+        // the MMAs of one K step (a tap's channel chunk): A from the patch at `a_low`, block `kb` along the weight's K axis
+        const auto multiply = [&](uint32_t d_tmem, uint32_t a_low, uint32_t b_low, uint32_t kb, uint32_t kb_a, uint32_t accumulate) {
+          const uint32_t scaled0 = idesc + (((kb_a & 3u) << 29) | ((kb & 3u) << 4));
+          const uint32_t sfa_tmem = sfa_base + 4 * (kb_a >> 2), sfb_tmem = sfb_resident_base + kSfbColumns * (kb >> 2);
+#pragma unroll
+          for (int k = 0; k < kKSteps; ++k) {
+            const uint64_t a = desc(a_low + 2 * k, a_high), b = desc(b_low + 2 * k, b_high);
+            if (INT8) {
+              tc_mma_i8(d_tmem, a, b, idesc, k > 0 ? 1u : accumulate);
+            } else {
+              tc_mma_mxf8(d_tmem, a, b, scaled0 + static_cast<uint32_t>(k) * ((1u << 29) | (1u << 4)), sfa_tmem, sfb_tmem, k > 0 ? 1u : accumulate);
+            }
+          }
+        };
+        const auto tile_begin = [&](uint32_t& acc) -> bool {
+          acc = kAccStages == 2 ? (tile_it & 1u) : 0u;
           const uint32_t acc_phase = kAccStages == 2 ? ((tile_it >> 1) & 1u) : (tile_it & 1u);
-          if (!loop_wait(tempty0 + 8 * acc, acc_phase ^ 1, kStatusWaitTmemEmpty)) break;
-          if (!loop_wait(full0 + 8 * s, phase, kStatusWaitFull)) break;
+          if (!loop_wait(tempty0 + 8 * acc, acc_phase ^ 1, kStatusWaitTmemEmpty)) return false;
+          if (!loop_wait(full0 + 8 * s, phase, kStatusWaitFull)) return false;
           tc_fence_after();
-          const uint32_t d_tmem = tmem + acc * BN;
-          uint64_t row_desc = patch_desc0 + static_cast<uint64_t>((s * a_stage) >> 4), tap_desc = row_desc, b_desc = b_desc0;
-          uint32_t kb = 0;  // 32-channel block along the weight's K axis
+          return true;
+        };
+        const auto tile_end = [&](uint32_t acc) {
+          tc_commit(&ctl.empty[s]);
+          tc_commit(&ctl.tmem_full[acc]);
+          if (++s == stages) s = 0, phase ^= 1;
+          ++tile_it;
+        };
+        // any number of taps and channel chunks; the first tile of a CTA waits for the weights of each K step
+        const auto general_tile = [&](bool first) -> bool {
+          uint32_t acc;
+          if (!tile_begin(acc)) return false;
+          uint32_t row_low = a_low0 + ((s * a_stage) >> 4), tap_low = row_low, b_low = b_low0, kb = 0, chunk = 0;
           int tap_x = 0, j = 0;
-          uint32_t chunk = 0;
           for (int ki = 0; ki < k_iters; ++ki) {
             if (first) {
-              if (!loop_wait(step0 + 8 * ki, 0, kStatusWaitFull)) {
-                alive = false;
-                break;
-              }
+              if (!loop_wait(step0 + 8 * ki, 0, kStatusWaitFull)) return false;
               tc_fence_after();
               if (ki == 0 && copy_scales) {
                 for (int t = 0; t < (k_iters * kKSteps + 3) / 4; ++t) {
@@ -840,38 +863,45 @@ conv_kernel(const __grid_constant__ CUtensorMap act_map, const __grid_constant__
                 }
               }
             }
-            const uint64_t a_desc = tap_desc + (chunk >> 4);
-            const uint32_t kb_a = static_cast<uint32_t>(j) * kKSteps;
-            const uint32_t scaled0 = idesc | ((kb_a & 3u) << 29) | ((kb & 3u) << 4);
-            const uint32_t sfa_tmem = sfa_base + 4 * (kb_a >> 2), sfb_tmem = sfb_resident_base + kSfbColumns * (kb >> 2);
-#pragma unroll
-            for (int k = 0; k < kKSteps; ++k) {
-              const uint32_t accumulate = k > 0 ? 1u : (ki > 0 ? 1u : 0u);
-              if (INT8) {
-                tc_mma_i8(d_tmem, a_desc + 2 * k, b_desc + 2 * k, idesc, accumulate);
-              } else {
-                tc_mma_mxf8(d_tmem, a_desc + 2 * k, b_desc + 2 * k, scaled0 + static_cast<uint32_t>(k) * ((1u << 29) | (1u << 4)), sfa_tmem,
-                            sfb_tmem, accumulate);
-              }
-            }
-            b_desc += kBBytes >> 4;
+            multiply(tmem + acc * BN, tap_low + (chunk >> 4), b_low, kb, static_cast<uint32_t>(j) * kKSteps, ki > 0 ? 1u : 0u);
+            b_low += kBBytes >> 4;
             kb += kKSteps;
             chunk += chunk_at;
             if (++j == k_chunks) {
               j = 0, chunk = 0;
-              tap_desc += step_x >> 4;
+              tap_low += step_x >> 4;
               if (++tap_x == taps_w) {
                 tap_x = 0;
-                row_desc += step_y >> 4;
-                tap_desc = row_desc;
+                row_low += step_y >> 4;
+                tap_low = row_low;
               }
             }
           }
-          if (!alive) break;
-          first = false;
-          tc_commit(&ctl.empty[s]);
-          tc_commit(&ctl.tmem_full[acc]);
-          if (++s == stages) s = 0, phase ^= 1;
+          tile_end(acc);
+          return true;
+        };
+        int tile = worker;
+        if (tile < p.total_tiles && general_tile(true)) {
+          tile += workers;
+          if (taps == 9 && taps_w == 3 && k_chunks == 1) {
+            // 3x3 with one channel chunk, unrolled: every offset along K is an immediate, so the issuing lane spends its time
+            // on the MMAs (the general loop takes about 150 cycles for each)
+            for (; tile < p.total_tiles; tile += workers) {
+              uint32_t acc;
+              if (!tile_begin(acc)) break;
+              const uint32_t a_low = a_low0 + ((s * a_stage) >> 4), d_tmem = tmem + acc * BN;
+#pragma unroll
+              for (int tap = 0; tap < 9; ++tap) {
+                multiply(d_tmem, a_low + tap / 3 * (step_y >> 4) + tap % 3 * (step_x >> 4), b_low0 + tap * (kBBytes >> 4), tap * kKSteps, 0,
+                         tap > 0 ? 1u : 0u);
+              }
+              tile_end(acc);
+            }
+          } else {
+            for (; tile < p.total_tiles; tile += workers) {
+              if (!general_tile(false)) break;
+            }
+          }
         }
       } else {
       const bool resident_b = in_register(static_cast<uint32_t>(p.weights_resident)) != 0;
@@ -2018,7 +2048,7 @@ int make_plan(const FimConvGeometry& g, int fmt, bool per_pixel, bool allow_flat
   // columns whose weights fit in shared memory beside two patches. Its tiles are 8 x 16 whatever the image; the padded
   // pixels that costs at the edges (14 % at 100 x 100) are less than the copies it saves at any size measured.
   if (g.kh * g.kw > 1 && g.stride_h == 1 && g.stride_w == 1 && fmt != kFmtBf16 && !per_pixel && !convert && bn <= 128 && pl.tiles_n == 1 &&
-      !(g_debug_flags & 2048) && k_iters <= kMaxWeightSteps) {
+      !(g_debug_flags & (2048 | 16384)) && k_iters <= kMaxWeightSteps) {
     const int pw = kPatchTileW + g.dil_w * (g.kw - 1), ph = kPatchTileH + g.dil_h * (g.kh - 1);
     const int chunk = (pw * ph * pl.block_k + 1023) / 1024 * 1024, chunks = g.cin / pl.block_k;
     const int scale_tiles = scaled ? (k_iters * (pl.block_k / 32) + 3) / 4 : 0;

@@ -22,7 +22,8 @@ extern "C" {
  *   512  makes the four warps of an epilogue group of a 1x1 conv share one output panel and one store (as the spatial
  *        convs do) instead of one per warp;
  *  1024  sends every call through the general epilogue instead of the ones whose switches are fixed at compile time;
- *  2048  streams the weights of a layer through the stage ring even where they are kept in shared memory by default;
+ *  2048  streams the weights of a layer (and the activations tap by tap, instead of one halo patch per tile) through the
+ *        stage ring even where they are kept in shared memory by default;
  *  4096  keeps them resident for every tile width where they fit (by default only 64-wide tiles do);
  * 16384  runs 128-wide block-scaled tiles as CTA pairs whatever the size of the layer.
  * A library built with -DFIM_PROBE_BUILD=1 (never shipped) also honours bits 1, 2, 4, 8 (skip activation loads / weight
