@@ -17,6 +17,7 @@
 //
 // Rounding points follow FlashIM's torch reference: flashim/ops/conv.py:174-206,309-342 and flashim/ops/gemm.py:58-98.
 #include <cstdio>
+#include <cstring>
 
 #include "common.cuh"
 #include "flashim_sm100.h"
@@ -2115,6 +2116,48 @@ Schedule make_schedule(const FimConvGeometry& g, const Plan& pl, bool int8, bool
   return sc;
 }
 
+// The plan and schedule of a call, kept for the calls that repeat it: working them out (the tile shape search above all) takes
+// longer than the launch. One small table per thread, so that no lock is needed; an entry is one comparison of its key.
+struct PlanKey {
+  FimConvGeometry geometry;
+  int fmt, per_pixel, allow_flat, out_elem, gelu, convert, pool, forced_n, max_ctas, flags, device;
+};
+struct PlanEntry {
+  PlanKey key;
+  int code = 1;  // kOk once filled (errors are not kept)
+  Plan plan;
+  Schedule schedule;
+};
+constexpr unsigned kPlanEntries = 64;
+
+int plan_for(const FimConvGeometry& g, int fmt, bool per_pixel, bool allow_flat, int out_elem, bool gelu, bool convert, bool pool, Plan* plan,
+             Schedule* schedule) {
+  static thread_local PlanEntry table[kPlanEntries];
+  PlanKey key;
+  key.geometry = g;
+  key.fmt = fmt, key.per_pixel = per_pixel, key.allow_flat = allow_flat, key.out_elem = out_elem, key.gelu = gelu, key.convert = convert;
+  key.pool = pool, key.forced_n = g_forced_block_n, key.max_ctas = g_max_ctas, key.flags = g_debug_flags, key.device = current_device();
+  unsigned h = 2166136261u;
+  const unsigned char* bytes = reinterpret_cast<const unsigned char*>(&key);
+  for (size_t i = 0; i < sizeof(key); i += 4) {
+    unsigned word;
+    memcpy(&word, bytes + i, 4);
+    h = (h ^ word) * 16777619u;
+  }
+  PlanEntry& entry = table[(h ^ (h >> 16)) % kPlanEntries];
+  if (entry.code != kOk || memcmp(&entry.key, &key, sizeof(key)) != 0) {
+    entry.code = 1;
+    const int rc = make_plan(g, fmt, per_pixel, allow_flat, out_elem, gelu, &entry.plan, convert, pool);
+    if (rc != kOk) return rc;
+    entry.schedule = make_schedule(g, entry.plan, fmt != kFmtMx, per_pixel);
+    entry.key = key;
+    entry.code = kOk;
+  }
+  *plan = entry.plan;
+  *schedule = entry.schedule;
+  return kOk;
+}
+
 struct ConvMaps {
   CUtensorMap act, weight, out, sfb, sfa, out_warp;
 };
@@ -2280,21 +2323,17 @@ int run_conv(int fmt, const void* x, const int8_t* act_exponent, const void* act
   // a 1x1 conv is a plain GEMM over flattened pixels when the residual (if any) is dense NHWC
   bool allow_flat = !pool;  // pooling windows need the tile to be a patch of the image
   Plan pl;
-  if (allow_flat) {
-    Plan probe;
-    const int rc0 = make_plan(*g, fmt, per_pixel, true, out_elem, ep->act == FIM_ACT_GELU, &probe, convert);
-    if (rc0 != kOk) return rc0;
-    if (probe.flat && ep->residual != nullptr) {
-      const long long c = ep->res_stride[3], xs = ep->res_stride[2], ys = ep->res_stride[1], bs = ep->res_stride[0];
-      const bool dense = c == 1 && ys == xs * probe.out_w && bs == ys * probe.out_h;
-      if (!dense) allow_flat = false;
-    }
+  Schedule sc;
+  const bool gelu = ep->act == FIM_ACT_GELU;
+  int rc = plan_for(*g, fmt, per_pixel, allow_flat, out_elem, gelu, convert, pool, &pl, &sc);
+  if (rc == kOk && allow_flat && pl.flat && ep->residual != nullptr) {
+    const long long c = ep->res_stride[3], xs = ep->res_stride[2], ys = ep->res_stride[1], bs = ep->res_stride[0];
+    const bool dense = c == 1 && ys == xs * pl.out_w && bs == ys * pl.out_h;
+    if (!dense) rc = plan_for(*g, fmt, per_pixel, false, out_elem, gelu, convert, pool, &pl, &sc);
   }
-  const int rc = make_plan(*g, fmt, per_pixel, allow_flat, out_elem, ep->act == FIM_ACT_GELU, &pl, convert, pool);
   if (rc != kOk) return rc;
   if (pool && (pl.out_h < 2 || pl.out_w < 2 || (pl.panels_per_half != 2 && !pl.patch))) return kUnsupported;  // no whole window: nothing to pool
 
-  const Schedule sc = make_schedule(*g, pl, fmt != kFmtMx, per_pixel);
   ConvParams p;
   p.cin = g->cin, p.cout = g->cout;
   p.out_h = pl.out_h, p.out_w = pl.out_w;

@@ -86,7 +86,8 @@ struct DwParams {
   int strip_steps, total_steps;  // four-row steps per strip; all steps of one channel tile
   int groups, group_quads;       // quads of a group: min(channel tiles, quads of the grid), each takes every group_quads-th tile
   int cta_quads;                 // quads in use per CTA
-  int swizzled, tma_out;         // tma_out: the output can be the target of TMA stores (16-byte aligned)
+  int swizzled;                  // 0: plain scales; else 1 + the padding groups behind the last one of a row
+  int tma_out;                   // tma_out: the output can be the target of TMA stores (16-byte aligned)
   int* status;
 };
 
@@ -292,6 +293,16 @@ dw5x5_kernel(const __grid_constant__ CUtensorMap in_map, const __grid_constant__
   __syncthreads();
 
   const int worker = blockIdx.x * p.cta_quads + quad, group = worker / p.group_quads, member = worker % p.group_quads;
+  if (MODE == kOutMx && p.swizzled && blockIdx.x == gridDim.x - 1) {
+    // the padding rows of the last scale tiles (the swizzled layout is zero there, and the caller's buffer need not be)
+    const uint32_t rows = static_cast<uint32_t>(p.batch) * p.height * p.width, tiles = ((p.channels >> 5) + 3) / 4;
+    const uint32_t pad_rows = (128u - rows % 128u) % 128u;
+    for (uint32_t i = threadIdx.x; i < pad_rows * tiles; i += 128 * kQuads) {
+      const uint32_t row = rows + i / tiles;
+      uint8_t* to = p.scales + (static_cast<uint64_t>(row >> 7) * tiles + i % tiles) * 512 + (row & 31) * 16 + ((row & 127) >> 5) * 4;
+      to[0] = to[1] = to[2] = to[3] = 0;
+    }
+  }
   const bool idle = quad >= p.cta_quads || group >= p.groups;
   const int s_begin = idle ? 0 : static_cast<int>(static_cast<long long>(group) * p.total_steps / p.groups);
   const int s_end = idle ? 0 : static_cast<int>(static_cast<long long>(group + 1) * p.total_steps / p.groups);
@@ -510,8 +521,12 @@ dw5x5_kernel(const __grid_constant__ CUtensorMap in_map, const __grid_constant__
           if (alive && x < p.width && y + piece < p.height) {  // each warp stores the scales of one row
             const uint32_t byte = piece == 0 ? bytes[0] : piece == 1 ? bytes[1] : piece == 2 ? bytes[2] : bytes[3];
             const uint32_t row = scale_row + y * p.width, groups = p.channels >> 5;
-            p.scales[p.swizzled ? static_cast<uint64_t>(row >> 7) * scale_tile_bytes + (row & 31) * 16 + ((row & 127) >> 5) * 4 + scale_at
-                                : static_cast<uint64_t>(row) * groups + ct] = static_cast<uint8_t>(byte);
+            uint8_t* to = p.scales + (p.swizzled ? static_cast<uint64_t>(row >> 7) * scale_tile_bytes + (row & 31) * 16 + ((row & 127) >> 5) * 4 + scale_at
+                                                 : static_cast<uint64_t>(row) * groups + ct);
+            *to = static_cast<uint8_t>(byte);
+            if (ct + 1 == p.channel_tiles) {  // the padding groups of a swizzled row
+              for (int pad = 1; pad < p.swizzled; ++pad) to[pad] = 0;
+            }
           }
         }
         // the lane's 8 channels of each of its four pixels, as they are stored
@@ -709,7 +724,7 @@ int launch(const void* value, const void* weight, const float* bias, void* out, 
   p.tiles_x = ceil_div(width, kTileX);
   p.channel_tiles = channels / kTileC;
   p.strip_steps = ceil_div(height, kStepRows);
-  p.swizzled = swizzled, p.status = status;
+  p.swizzled = swizzled ? 1 + (4 - p.channel_tiles % 4) % 4 : 0, p.status = status;
   p.tma_out = (reinterpret_cast<uintptr_t>(out) & 15u) == 0;
   const long long steps = static_cast<long long>(p.tiles_x) * batch * p.strip_steps;
   if (steps > 0x3fffffffLL || steps * p.channel_tiles > 0x3fffffffffLL) return kUnsupported;

@@ -802,7 +802,7 @@ void depthwise_mx_launch(const Tensor& v, const Tensor& w, const Tensor& b, int 
                          const Call& call, const char* what) {
   const int64_t c = v.size(1), rows = v.size(0) * v.size(2) * v.size(3);
   out = call.empty({rows, c}, kE4M3);
-  scales = call.scales(rows, c / 32, scale_dtype);
+  scales = call.empty({swizzled_bytes(rows, c / 32)}, scale_dtype);  // (the kernel writes the padding too)
   call.launch(what, [&] {
     return abi.fim_dw5x5_mxfp8(v.data_ptr(), w.data_ptr(), static_cast<const float*>(b.data_ptr()), out.data_ptr(), scales.data_ptr(), 1,
                                v.size(0), v.size(2), v.size(3), c, act, call.status, call.stream);

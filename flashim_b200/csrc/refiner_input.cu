@@ -134,6 +134,133 @@ __global__ void __launch_bounds__(32 * kInputWarps) refiner_input_kernel(const I
   }
 }
 
+// The same rows for P = 32 NF features (the widths RoMaV2 uses), arranged for latency and for whole sectors: f_a stays in
+// registers, the patch pixels of several steps are in flight together, the eight partial sums a group of lanes gathers in
+// eight steps are added by one transposing butterfly (7 shuffles instead of 24, each sum over the same pairs of lanes as
+// above; the division by sqrt(P) comes last, once per value), the radius is a constant of the code, and the eight rows of a block, which are contiguous in the output, go through shared memory and
+// leave as 16-byte words instead of single bf16 values. The kernel above waits for one pair of loads per four patch pixels.
+// Refiner input + heads of both directions of a pair, 96x72x64, radius 3: 45 -> 23 us; 200x200x128, radius 2: 225 -> 164.
+template <int NF, int R>
+__global__ void __launch_bounds__(32 * kInputWarps, 3) refiner_input_wide_kernel(const InputParams p) {
+  constexpr int P = 32 * NF, kAhead = NF >= 4 ? 2 : 8 / NF;  // patch pixels in flight per group of eight lanes
+  extern __shared__ __align__(16) __nv_bfloat16 tile[];      // kInputWarps output rows
+  __shared__ float dots[kInputWarps][kInputMaxPatch];
+  const int warp_id = threadIdx.x >> 5, lane = threadIdx.x & 31, group = lane >> 3, sub = lane & 7;
+  constexpr int side = 2 * R + 2, window = 2 * R + 1, K = window * window;
+  const int E = p.embedding, C = 2 * P + E + K;
+  const unsigned pixels = static_cast<unsigned>(p.batch) * p.height * p.width;  // (the host refuses more than 2**31)
+  __nv_bfloat16* row = tile + warp_id * C;
+  float* dot = dots[warp_id];
+  for (unsigned first = blockIdx.x * kInputWarps; first < pixels; first += gridDim.x * kInputWarps) {
+    const unsigned flat = first + warp_id;
+    if (flat < pixels) {
+      const int x = static_cast<int>(flat % static_cast<unsigned>(p.width));
+      const int y = static_cast<int>((flat / static_cast<unsigned>(p.width)) % static_cast<unsigned>(p.height));
+      const int b = static_cast<int>(flat / (static_cast<unsigned>(p.width) * static_cast<unsigned>(p.height)));
+      const int b_other = p.pair > 0 ? (b + p.batch - p.pair) % p.batch : b;
+      const float* other = p.f_b + static_cast<long long>(b_other) * p.height * p.width * P;
+      const float2 at = __ldg(reinterpret_cast<const float2*>(p.warp) + flat);
+      float4 a[NF];  // channels 4 sub + 32 i, in every group
+#pragma unroll
+      for (int i = 0; i < NF; ++i) a[i] = __ldg(reinterpret_cast<const float4*>(p.f_a + static_cast<long long>(flat) * P + 32 * i) + sub);
+      const float ix = ((at.x + 1.0f) * p.width - 1.0f) * 0.5f, iy = ((at.y + 1.0f) * p.height - 1.0f) * 0.5f;
+      const float fx0 = floorf(ix), fy0 = floorf(iy);
+      const float tx = ix - fx0, ty = iy - fy0;
+      const float w_nw = (1.0f - tx) * (1.0f - ty), w_ne = tx * (1.0f - ty), w_sw = (1.0f - tx) * ty, w_se = tx * ty;
+      const int x0 = static_cast<int>(fminf(fmaxf(fx0, -16.0f), static_cast<float>(p.width) + 16.0f));
+      const int y0 = static_cast<int>(fminf(fmaxf(fy0, -16.0f), static_cast<float>(p.height) + 16.0f));
+      const bool finite = fabsf(ix) < 1e9f && fabsf(iy) < 1e9f;
+      const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+      // f_b at the warp: a lane per four channels; the corners are patch pixels too
+      if (lane < P / 4) {
+        const bool north = finite && y0 >= 0 && y0 < p.height, south = finite && y0 + 1 >= 0 && y0 + 1 < p.height;
+        const bool west = x0 >= 0 && x0 < p.width, east = x0 + 1 >= 0 && x0 + 1 < p.width;
+        const float* base = other + (static_cast<long long>(y0) * p.width + x0) * P + 4 * lane;
+        const long long down = static_cast<long long>(p.width) * P;
+        const float4 nw = north && west ? __ldg(reinterpret_cast<const float4*>(base)) : zero;
+        const float4 ne = north && east ? __ldg(reinterpret_cast<const float4*>(base + P)) : zero;
+        const float4 sw = south && west ? __ldg(reinterpret_cast<const float4*>(base + down)) : zero;
+        const float4 se = south && east ? __ldg(reinterpret_cast<const float4*>(base + down + P)) : zero;
+        __nv_bfloat16* to = row + P + 4 * lane;
+        store_bf16(to, nw.x * w_nw + ne.x * w_ne + sw.x * w_sw + se.x * w_se);
+        store_bf16(to + 1, nw.y * w_nw + ne.y * w_ne + sw.y * w_sw + se.y * w_se);
+        store_bf16(to + 2, nw.z * w_nw + ne.z * w_ne + sw.z * w_sw + se.z * w_se);
+        store_bf16(to + 3, nw.w * w_nw + ne.w * w_ne + sw.w * w_sw + se.w * w_se);
+      }
+      if (group == 0) {
+#pragma unroll
+        for (int i = 0; i < NF; ++i) {
+          __nv_bfloat16* to = row + 32 * i + 4 * sub;
+          store_bf16(to, a[i].x), store_bf16(to + 1, a[i].y), store_bf16(to + 2, a[i].z), store_bf16(to + 3, a[i].w);
+        }
+      }
+      // dot products with the patch pixels, a group of eight lanes per pixel, eight pixels of a group per butterfly
+#pragma unroll
+      for (int base = 0; base < side * side; base += 32) {
+        float sum[8];
+#pragma unroll
+        for (int ahead = 0; ahead < 8; ahead += kAhead) {
+          float4 v[kAhead][NF];
+#pragma unroll
+          for (int q = 0; q < kAhead; ++q) {
+            const int pos = base + 4 * (ahead + q) + group;
+            const int yy = y0 - R + pos / side, xx = x0 - R + pos % side;
+            const bool in = base + 4 * (ahead + q) < side * side && finite && pos < side * side &&
+                            static_cast<unsigned>(yy) < static_cast<unsigned>(p.height) && static_cast<unsigned>(xx) < static_cast<unsigned>(p.width);
+            const float* src = other + static_cast<long long>(yy * p.width + xx) * P;  // (below 2**31 pixels)
+#pragma unroll
+            for (int i = 0; i < NF; ++i) v[q][i] = in ? __ldg(reinterpret_cast<const float4*>(src + 32 * i) + sub) : zero;
+          }
+#pragma unroll
+          for (int q = 0; q < kAhead; ++q) {
+            float t = 0.0f;
+#pragma unroll
+            for (int i = 0; i < NF; ++i) {
+              t = fmaf(a[i].x, v[q][i].x, t), t = fmaf(a[i].y, v[q][i].y, t), t = fmaf(a[i].z, v[q][i].z, t), t = fmaf(a[i].w, v[q][i].w, t);
+            }
+            sum[ahead + q] = t;
+          }
+        }
+        float half[4], quarter[2];
+        const bool odd = sub & 1, second = sub & 2, fourth = sub & 4;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) half[i] = (odd ? sum[2 * i + 1] : sum[2 * i]) + __shfl_xor_sync(0xffffffffu, odd ? sum[2 * i] : sum[2 * i + 1], 1);
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          quarter[i] = (second ? half[2 * i + 1] : half[2 * i]) + __shfl_xor_sync(0xffffffffu, second ? half[2 * i] : half[2 * i + 1], 2);
+        }
+        const float total = (fourth ? quarter[1] : quarter[0]) + __shfl_xor_sync(0xffffffffu, fourth ? quarter[0] : quarter[1], 4);
+        const int pos = base + 4 * sub + group;  // the lane's own step
+        if (pos < side * side) dot[pos] = total / p.root_features;
+      }
+      {
+        const float dx = p.scale_x * (at.x - (-1.0f + (2.0f * x + 1.0f) / p.width));
+        const float dy = p.scale_y * (at.y - (-1.0f + (2.0f * y + 1.0f) / p.height));
+        for (int e = lane; e < E; e += 32) {
+          const float2 weight = __ldg(reinterpret_cast<const float2*>(p.emb_weight) + e);
+          store_bf16(row + 2 * P + e, fmaf(weight.y, dy, weight.x * dx) + __ldg(p.emb_bias + e));
+        }
+      }
+      __syncwarp();
+      for (int k = lane; k < K; k += 32) {
+        const int at_patch = (k / window) * side + k % window;
+        const float v = dot[at_patch] * w_nw + dot[at_patch + 1] * w_ne + dot[at_patch + side] * w_sw + dot[at_patch + side + 1] * w_se;
+        store_bf16(row + 2 * P + E + k, v);
+      }
+    }
+    __syncthreads();
+    {
+      // eight rows of C values are C 16-byte words; `first` is a multiple of eight, so the block's rows start on one
+      const unsigned rows = min(static_cast<unsigned>(kInputWarps), pixels - first);
+      const unsigned words = rows * C / 8;
+      uint4* to = reinterpret_cast<uint4*>(p.out + static_cast<size_t>(first) * C);
+      for (unsigned i = threadIdx.x; i < words; i += 32 * kInputWarps) to[i] = reinterpret_cast<const uint4*>(tile)[i];
+      for (unsigned i = words * 8 + threadIdx.x; i < rows * C; i += 32 * kInputWarps) p.out[static_cast<size_t>(first) * C + i] = tile[i];
+    }
+    __syncthreads();
+  }
+}
+
 // Without a correlation window (radius < 0, RoMaV2's full-resolution refiner with 12 features) a pixel is little work:
 // eight lanes share one, so a warp handles four pixels at a time.
 __global__ void __launch_bounds__(256) refiner_input_plain_kernel(const InputParams p) {
@@ -213,6 +340,18 @@ extern "C" int fim_romav2_refiner_input(const float* f_a, const float* f_b, cons
     return static_cast<int>(cudaGetLastError());
   }
   const long long blocks = (pixels + kInputWarps - 1) / kInputWarps;
+  const size_t row_bytes = (2 * static_cast<size_t>(features) + embedding + (2 * radius + 1) * (2 * radius + 1)) * 2;
+  if ((features == 32 || features == 64 || features == 128) && kInputWarps * row_bytes <= 32 * 1024 && !misaligned(out, 16)) {
+    using Kernel = void (*)(InputParams);
+    static constexpr Kernel kKernels[3][4] = {
+        {refiner_input_wide_kernel<1, 0>, refiner_input_wide_kernel<1, 1>, refiner_input_wide_kernel<1, 2>, refiner_input_wide_kernel<1, 3>},
+        {refiner_input_wide_kernel<2, 0>, refiner_input_wide_kernel<2, 1>, refiner_input_wide_kernel<2, 2>, refiner_input_wide_kernel<2, 3>},
+        {refiner_input_wide_kernel<4, 0>, refiner_input_wide_kernel<4, 1>, refiner_input_wide_kernel<4, 2>, refiner_input_wide_kernel<4, 3>}};
+    const Kernel kernel = kKernels[features == 32 ? 0 : features == 64 ? 1 : 2][radius];
+    const unsigned grid = static_cast<unsigned>(blocks < 148LL * 32 ? blocks : 148LL * 32);
+    kernel<<<grid, 32 * kInputWarps, kInputWarps * row_bytes, static_cast<cudaStream_t>(stream)>>>(p);
+    return static_cast<int>(cudaGetLastError());
+  }
   const unsigned grid = static_cast<unsigned>(blocks < 148LL * 16 ? blocks : 148LL * 16);
   refiner_input_kernel<<<grid, 32 * kInputWarps, 0, static_cast<cudaStream_t>(stream)>>>(p);
   return static_cast<int>(cudaGetLastError());

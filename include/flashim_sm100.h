@@ -143,7 +143,8 @@ int fim_dw5x5_bf16(const void* value, const void* weight, const float* bias, voi
                    int channels, int act, int* status, void* stream);
 
 /* Depthwise + bias + act, the fp32 result quantised per (pixel, 32 channels) to MXFP8 without an intermediate bf16
- * rounding: E4M3 [B*H*W, C] and E8M0 bytes (swizzled != 0: 128x4 swizzled layout; else [B*H*W, C/32]).
+ * rounding: E4M3 [B*H*W, C] and E8M0 bytes (swizzled != 0: 128x4 swizzled layout, its padding written as zero; else
+ * [B*H*W, C/32]).
  * With act = FIM_ACT_RELU and swizzled = 1 this replaces ops.depthwise5x5_relu_mxfp8 (flashim/ops/conv.py:30-44;
  * kernel flashim/backends/triton/conv.py:47-130). */
 int fim_dw5x5_mxfp8(const void* value, const void* weight, const float* bias, void* out, void* scales, int swizzled,
