@@ -552,6 +552,13 @@ conv_kernel(const __grid_constant__ CUtensorMap act_map, const __grid_constant__
       tmem_relinquish();
     }
   }
+  if (p.act == kActGelu) {
+    for (int i = threadIdx.x; i < kGeluEntries; i += kBlockThreads) {
+      asm volatile("st.shared.b32 [%0], %1;" ::"r"(smem_gelu + i * 4), "r"(kGeluTable[i]) : "memory");
+    }
+  }
+  grid_release();
+  grid_wait();
   if (warp == 2 && SCALED && !dynamic_a) {
     // static activation scales: one 512-byte tile per 128 input channels, the same 4 bytes in all 128 rows
     const int tiles = (p.cin + 127) / 128;
@@ -572,11 +579,6 @@ conv_kernel(const __grid_constant__ CUtensorMap act_map, const __grid_constant__
     for (int i = threadIdx.x; i < p.tiles_n * BN; i += kBlockThreads) {
       const float value = i < p.cout ? __bfloat162float(p.bias[i]) : 0.0f;
       asm volatile("st.shared.f32 [%0], %1;" ::"r"(smem_bias + i * 4), "f"(value) : "memory");
-    }
-  }
-  if (p.act == kActGelu) {
-    for (int i = threadIdx.x; i < kGeluEntries; i += kBlockThreads) {
-      asm volatile("st.shared.b32 [%0], %1;" ::"r"(smem_gelu + i * 4), "r"(kGeluTable[i]) : "memory");
     }
   }
   tc_fence_before();
@@ -1548,12 +1550,14 @@ mlp_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constant__ CU
     tmem_alloc(&ctl.tmem_base, kTmemColumns);
     tmem_relinquish();
   }
+  for (int i = threadIdx.x; i < kGeluEntries; i += kMlpThreads) {
+    asm volatile("st.shared.b32 [%0], %1;" ::"r"(smem_gelu + i * 4), "r"(kGeluTable[i]) : "memory");
+  }
+  grid_release();
+  grid_wait();
   for (int i = threadIdx.x; i < 3 * C; i += kMlpThreads) {  // both biases widened to fp32 once per CTA
     const float value = __bfloat162float(i < 2 * C ? p.bias1[i] : p.bias2[i - 2 * C]);
     asm volatile("st.shared.f32 [%0], %1;" ::"r"(smem_bias1 + i * 4), "f"(value) : "memory");
-  }
-  for (int i = threadIdx.x; i < kGeluEntries; i += kMlpThreads) {
-    asm volatile("st.shared.b32 [%0], %1;" ::"r"(smem_gelu + i * 4), "r"(kGeluTable[i]) : "memory");
   }
   tc_fence_before();
   __syncthreads();
@@ -2173,21 +2177,8 @@ int launch_conv(const ConvMaps& maps, const ConvParams& p, const Plan& pl, cudaS
     if (e != cudaSuccess) return static_cast<int>(e);
     if (device >= 0 && device < kMaxDevices) configured[device] = true;
   }
-  if (PAIR) {
-    cudaLaunchConfig_t config = {};
-    config.gridDim = dim3(static_cast<unsigned>(pl.ctas), 1, 1);
-    config.blockDim = dim3(kThreads, 1, 1);
-    config.dynamicSmemBytes = pl.smem;
-    config.stream = stream;
-    cudaLaunchAttribute attribute;
-    attribute.id = cudaLaunchAttributeClusterDimension;
-    attribute.val.clusterDim.x = 2, attribute.val.clusterDim.y = 1, attribute.val.clusterDim.z = 1;
-    config.attrs = &attribute;
-    config.numAttrs = 1;
-    return static_cast<int>(cudaLaunchKernelEx(&config, conv_kernel<FMT, BN, BK, PAIR, EPI, CONVERT>, maps.act, maps.weight, maps.out, maps.sfb,
-                                               maps.sfa, maps.out_warp, p));
-  }
-  conv_kernel<FMT, BN, BK, PAIR, EPI, CONVERT><<<pl.ctas, CONVERT ? kConvertThreads : kThreads, pl.smem, stream>>>(maps.act, maps.weight, maps.out, maps.sfb, maps.sfa, maps.out_warp, p);
+  launch_dependent(conv_kernel<FMT, BN, BK, PAIR, EPI, CONVERT>, static_cast<unsigned>(pl.ctas), CONVERT ? kConvertThreads : kThreads, pl.smem, stream,
+                   PAIR ? 2u : 1u, maps.act, maps.weight, maps.out, maps.sfb, maps.sfa, maps.out_warp, p);
   return static_cast<int>(cudaGetLastError());
 }
 
@@ -2502,7 +2493,7 @@ int launch_mlp(const CUtensorMap& x_map, const CUtensorMap& w1_map, const CUtens
     if (e != cudaSuccess) return static_cast<int>(e);
     if (device >= 0 && device < kMaxDevices) configured[device] = true;
   }
-  mlp_kernel<KC><<<ctas, kMlpThreads, smem, stream>>>(x_map, w1_map, w2_map, out_map, res_map, p);
+  launch_dependent(mlp_kernel<KC>, static_cast<unsigned>(ctas), kMlpThreads, smem, stream, 1u, x_map, w1_map, w2_map, out_map, res_map, p);
   return static_cast<int>(cudaGetLastError());
 }
 

@@ -290,6 +290,8 @@ dw5x5_kernel(const __grid_constant__ CUtensorMap in_map, const __grid_constant__
     tma_prefetch_desc(&in_map);
     tma_prefetch_desc(&out_map);
   }
+  grid_release();
+  grid_wait();
   __syncthreads();
 
   const int worker = blockIdx.x * p.cta_quads + quad, group = worker / p.group_quads, member = worker % p.group_quads;
@@ -698,7 +700,7 @@ int launch_kernel(const CUtensorMap& in_map, const CUtensorMap& out_map, const D
     if (e != cudaSuccess) return static_cast<int>(e);
     if (device >= 0 && device < kMaxDevices) configured[act][device] = true;
   }
-  kernel<<<grid, 128 * kQuads, kSmem, s>>>(in_map, out_map, p);
+  launch_dependent(kernel, grid, 128 * kQuads, kSmem, s, 1u, in_map, out_map, p);
   return static_cast<int>(cudaGetLastError());
 }
 

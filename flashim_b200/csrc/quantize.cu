@@ -44,6 +44,9 @@ template <typename T>
 __global__ void __launch_bounds__(kThreads) quantize_mx_static_kernel(const T* __restrict__ in, const int8_t* __restrict__ exps,
                                                                       uint8_t* __restrict__ out, long long rows, int channels,
                                                                       int padded, bool aligned) {
+  grid_release();
+  grid_wait();
+  in = from_here(in), exps = from_here(exps);
   const int chunks = padded / 16;
   const long long total = rows * chunks;
   for (long long i = blockIdx.x * static_cast<long long>(kThreads) + threadIdx.x; i < total;
@@ -70,6 +73,9 @@ template <typename T>
 __global__ void __launch_bounds__(kThreads) quantize_mx_dynamic_kernel(const T* __restrict__ in, uint8_t* __restrict__ out,
                                                                        uint8_t* __restrict__ scales, long long rows, int channels,
                                                                        int swizzled) {
+  grid_release();
+  grid_wait();
+  in = from_here(in);
   const int chunks = channels / 16;
   const int groups = channels / 32;
   const int group_tiles = (groups + 3) / 4;
@@ -112,6 +118,9 @@ __global__ void __launch_bounds__(kThreads) quantize_mx_dynamic_kernel(const T* 
 template <typename T>
 __global__ void __launch_bounds__(kThreads) quantize_int8_kernel(const T* __restrict__ in, const float* __restrict__ scale_ptr,
                                                                  int8_t* __restrict__ out, long long count) {
+  grid_release();
+  grid_wait();
+  in = from_here(in), scale_ptr = from_here(scale_ptr);
   const Int8Quantizer quantizer = make_int8_quantizer(__ldg(scale_ptr));
   const long long chunks = count / 16;
   for (long long i = blockIdx.x * static_cast<long long>(kThreads) + threadIdx.x; i < chunks;
@@ -181,6 +190,9 @@ __global__ void __launch_bounds__(kThreads) quantize_nchw_kernel(const T* __rest
                                                                  int channels, int padded, long long pixels, int pixel_tiles,
                                                                  int channel_tiles) {
   __shared__ __align__(16) uint8_t tile[kTilePixels * kTilePitch];
+  grid_release();
+  grid_wait();
+  in = from_here(in), exps = from_here(exps), scale_ptr = from_here(scale_ptr);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   long long t = blockIdx.x;
   const int ct = static_cast<int>(t % channel_tiles);
@@ -244,6 +256,9 @@ __global__ void __launch_bounds__(kThreads) quantize_nchw_kernel(const T* __rest
 __global__ void __launch_bounds__(kThreads) maxpool2_int8_kernel(const uint4* __restrict__ in, const float* __restrict__ scale_ptr,
                                                                  uint2* __restrict__ out, int batch, int height, int width,
                                                                  int channels) {
+  grid_release();
+  grid_wait();
+  in = from_here(in), scale_ptr = from_here(scale_ptr);
   const Int8Quantizer quantizer = make_int8_quantizer(__ldg(scale_ptr));
   const int ho = height / 2, wo = width / 2, groups = channels / 8;
   const long long total = static_cast<long long>(batch) * ho * wo * groups;
@@ -281,7 +296,7 @@ int launch_nchw(const void* value, int dtype, const int8_t* exponent, const floa
   auto launch = [&](auto zero, auto vec) {
     using T = decltype(zero);
     // one aligned load per four pixels needs every channel row to start on such a boundary
-    quantize_nchw_kernel<T, INT8, decltype(vec)::value><<<grid, kThreads, 0, s>>>(
+    launch_dependent(quantize_nchw_kernel<T, INT8, decltype(vec)::value>, static_cast<unsigned>(grid), kThreads, 0, s, 1u, 
         static_cast<const T*>(value), exponent, scale, static_cast<uint8_t*>(out), channels, padded, pixels,
         static_cast<int>(pixel_tiles), channel_tiles);
   };
@@ -305,6 +320,9 @@ int launch_nchw(const void* value, int dtype, const int8_t* exponent, const floa
 __global__ void __launch_bounds__(kThreads) gelu_quantize_mx_kernel(const __nv_bfloat16* __restrict__ in, const float* __restrict__ bias,
                                                                     const int8_t* __restrict__ exps, uint8_t* __restrict__ out,
                                                                     long long rows, int channels) {
+  grid_release();
+  grid_wait();
+  in = from_here(in), bias = from_here(bias), exps = from_here(exps);
   const int chunks = channels / 16;
   const long long total = rows * chunks;
   for (long long i = blockIdx.x * static_cast<long long>(kThreads) + threadIdx.x; i < total;
@@ -343,10 +361,10 @@ extern "C" int fim_quantize_mxfp8_static(const void* value, int dtype, const int
   const int grid = grid_for(rows * (padded / 16), 16);
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   if (dtype == FIM_DTYPE_BF16) {
-    quantize_mx_static_kernel<__nv_bfloat16><<<grid, kThreads, 0, s>>>(static_cast<const __nv_bfloat16*>(value), exponent,
+    launch_dependent(quantize_mx_static_kernel<__nv_bfloat16>, static_cast<unsigned>(grid), kThreads, 0, s, 1u, static_cast<const __nv_bfloat16*>(value), exponent,
                                                                       static_cast<uint8_t*>(out), rows, channels, padded, vec);
   } else if (dtype == FIM_DTYPE_F32) {
-    quantize_mx_static_kernel<float><<<grid, kThreads, 0, s>>>(static_cast<const float*>(value), exponent,
+    launch_dependent(quantize_mx_static_kernel<float>, static_cast<unsigned>(grid), kThreads, 0, s, 1u, static_cast<const float*>(value), exponent,
                                                               static_cast<uint8_t*>(out), rows, channels, padded, vec);
   } else {
     return kBadArgument;
@@ -363,11 +381,11 @@ extern "C" int fim_quantize_mxfp8_dynamic(const void* value, int dtype, void* ou
   const int grid = grid_for(rows * (channels / 16), 16);
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   if (dtype == FIM_DTYPE_BF16) {
-    quantize_mx_dynamic_kernel<__nv_bfloat16><<<grid, kThreads, 0, s>>>(static_cast<const __nv_bfloat16*>(value),
+    launch_dependent(quantize_mx_dynamic_kernel<__nv_bfloat16>, static_cast<unsigned>(grid), kThreads, 0, s, 1u, static_cast<const __nv_bfloat16*>(value),
                                                                        static_cast<uint8_t*>(out), static_cast<uint8_t*>(scales),
                                                                        rows, channels, swizzled);
   } else if (dtype == FIM_DTYPE_F32) {
-    quantize_mx_dynamic_kernel<float><<<grid, kThreads, 0, s>>>(static_cast<const float*>(value), static_cast<uint8_t*>(out),
+    launch_dependent(quantize_mx_dynamic_kernel<float>, static_cast<unsigned>(grid), kThreads, 0, s, 1u, static_cast<const float*>(value), static_cast<uint8_t*>(out),
                                                                static_cast<uint8_t*>(scales), rows, channels, swizzled);
   } else {
     return kBadArgument;
@@ -383,10 +401,10 @@ extern "C" int fim_quantize_int8_static(const void* value, int dtype, const floa
   const int grid = grid_for(count / 16 + 1, 16);
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   if (dtype == FIM_DTYPE_BF16) {
-    quantize_int8_kernel<__nv_bfloat16><<<grid, kThreads, 0, s>>>(static_cast<const __nv_bfloat16*>(value), scale,
+    launch_dependent(quantize_int8_kernel<__nv_bfloat16>, static_cast<unsigned>(grid), kThreads, 0, s, 1u, static_cast<const __nv_bfloat16*>(value), scale,
                                                                  static_cast<int8_t*>(out), count);
   } else if (dtype == FIM_DTYPE_F32) {
-    quantize_int8_kernel<float><<<grid, kThreads, 0, s>>>(static_cast<const float*>(value), scale, static_cast<int8_t*>(out),
+    launch_dependent(quantize_int8_kernel<float>, static_cast<unsigned>(grid), kThreads, 0, s, 1u, static_cast<const float*>(value), scale, static_cast<int8_t*>(out),
                                                          count);
   } else {
     return kBadArgument;
@@ -413,7 +431,7 @@ extern "C" int fim_maxpool2_quantize_int8(const void* value, const float* scale,
   if (value == nullptr || scale == nullptr || out == nullptr) return kBadArgument;
   if (!aligned16(value) || (reinterpret_cast<uintptr_t>(out) & 7u)) return kBadLayout;
   const long long work = static_cast<long long>(batch) * (height / 2) * (width / 2) * (channels / 8);
-  maxpool2_int8_kernel<<<grid_for(work, 16), kThreads, 0, static_cast<cudaStream_t>(stream)>>>(
+  launch_dependent(maxpool2_int8_kernel, static_cast<unsigned>(grid_for(work, 16)), kThreads, 0, static_cast<cudaStream_t>(stream), 1u, 
       static_cast<const uint4*>(value), scale, static_cast<uint2*>(out), batch, height, width, channels);
   return static_cast<int>(cudaGetLastError());
 }
@@ -424,7 +442,7 @@ extern "C" int fim_gelu_quantize_mxfp8(const void* value, const float* input_bia
   if (value == nullptr || exponent == nullptr || out == nullptr || rows < 0 || channels <= 0) return kBadArgument;
   if (channels % 32) return kBadLayout;
   if (!aligned16(value) || !aligned16(out)) return kBadLayout;
-  gelu_quantize_mx_kernel<<<grid_for(rows * (channels / 16), 16), kThreads, 0, static_cast<cudaStream_t>(stream)>>>(
+  launch_dependent(gelu_quantize_mx_kernel, static_cast<unsigned>(grid_for(rows * (channels / 16), 16)), kThreads, 0, static_cast<cudaStream_t>(stream), 1u, 
       static_cast<const __nv_bfloat16*>(value), input_bias, exponent, static_cast<uint8_t*>(out), rows, channels);
   return static_cast<int>(cudaGetLastError());
 }

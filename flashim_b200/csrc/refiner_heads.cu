@@ -27,6 +27,9 @@ __global__ void __launch_bounds__(kHeadThreads) refiner_heads_kernel(const uint4
                                                                      float* __restrict__ warp_out, float* __restrict__ conf_out,
                                                                      long long rows, int channels, float inv_norm_x, float inv_norm_y) {
   __shared__ __align__(16) float w[kHeadOutputs * kHeadMaxChannels];
+  grid_release();
+  grid_wait();
+  weight = from_here(weight);
   for (int i = threadIdx.x; i < kHeadOutputs * channels; i += kHeadThreads) w[i] = __ldg(weight + i);
   __syncthreads();
   const int part = threadIdx.x & 7;
@@ -129,7 +132,7 @@ extern "C" int fim_romav2_refiner_heads(const void* z, const float* weight, cons
   const long long per_block = (kHeadThreads / 8) * kHeadPixels;
   const long long blocks = (rows + per_block - 1) / per_block;
   const unsigned grid = static_cast<unsigned>(blocks < 148LL * 8 ? blocks : 148LL * 8);
-  refiner_heads_kernel<<<grid, kHeadThreads, 0, static_cast<cudaStream_t>(stream)>>>(
+  launch_dependent(refiner_heads_kernel, grid, kHeadThreads, 0, static_cast<cudaStream_t>(stream), 1u,
       static_cast<const uint4*>(z), weight, bias, prev_warp, prev_confidence, prev_channels, warp, confidence, rows, channels,
       inv_norm_x, inv_norm_y);
   return static_cast<int>(cudaGetLastError());

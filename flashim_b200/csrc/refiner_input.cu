@@ -33,6 +33,8 @@ struct InputParams {
 __device__ __forceinline__ void store_bf16(__nv_bfloat16* at, float v) { *at = __float2bfloat16_rn(v); }
 
 __global__ void __launch_bounds__(32 * kInputWarps) refiner_input_kernel(const InputParams p) {
+  grid_release();
+  grid_wait();
   __shared__ __align__(16) float scaled_a[kInputWarps][kInputMaxFeatures];
   __shared__ float dots[kInputWarps][kInputMaxPatch];
   const int warp_id = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -142,6 +144,8 @@ __global__ void __launch_bounds__(32 * kInputWarps) refiner_input_kernel(const I
 // Refiner input + heads of both directions of a pair, 96x72x64, radius 3: 45 -> 23 us; 200x200x128, radius 2: 225 -> 164.
 template <int NF, int R>
 __global__ void __launch_bounds__(32 * kInputWarps, 3) refiner_input_wide_kernel(const InputParams p) {
+  grid_release();
+  grid_wait();
   constexpr int P = 32 * NF, kAhead = NF >= 4 ? 2 : 8 / NF;  // patch pixels in flight per group of eight lanes
   extern __shared__ __align__(16) __nv_bfloat16 tile[];      // kInputWarps output rows
   __shared__ float dots[kInputWarps][kInputMaxPatch];
@@ -264,6 +268,8 @@ __global__ void __launch_bounds__(32 * kInputWarps, 3) refiner_input_wide_kernel
 // Without a correlation window (radius < 0, RoMaV2's full-resolution refiner with 12 features) a pixel is little work:
 // eight lanes share one, so a warp handles four pixels at a time.
 __global__ void __launch_bounds__(256) refiner_input_plain_kernel(const InputParams p) {
+  grid_release();
+  grid_wait();
   const int P = p.features, E = p.embedding, C = 2 * P + E;
   const unsigned pixels = static_cast<unsigned>(p.batch) * p.height * p.width;
   const int sub = threadIdx.x & 7;
@@ -335,8 +341,8 @@ extern "C" int fim_romav2_refiner_input(const float* f_a, const float* f_b, cons
   if (pixels >= 0x7fffffffLL) return kUnsupported;
   if (radius < 0) {
     const long long plain_blocks = (pixels + 31) / 32;
-    refiner_input_plain_kernel<<<static_cast<unsigned>(plain_blocks < 148LL * 32 ? plain_blocks : 148LL * 32), 256, 0,
-                                 static_cast<cudaStream_t>(stream)>>>(p);
+    launch_dependent(refiner_input_plain_kernel, static_cast<unsigned>(plain_blocks < 148LL * 32 ? plain_blocks : 148LL * 32), 256, 0,
+                     static_cast<cudaStream_t>(stream), 1u, p);
     return static_cast<int>(cudaGetLastError());
   }
   const long long blocks = (pixels + kInputWarps - 1) / kInputWarps;
@@ -349,10 +355,10 @@ extern "C" int fim_romav2_refiner_input(const float* f_a, const float* f_b, cons
         {refiner_input_wide_kernel<4, 0>, refiner_input_wide_kernel<4, 1>, refiner_input_wide_kernel<4, 2>, refiner_input_wide_kernel<4, 3>}};
     const Kernel kernel = kKernels[features == 32 ? 0 : features == 64 ? 1 : 2][radius];
     const unsigned grid = static_cast<unsigned>(blocks < 148LL * 32 ? blocks : 148LL * 32);
-    kernel<<<grid, 32 * kInputWarps, kInputWarps * row_bytes, static_cast<cudaStream_t>(stream)>>>(p);
+    launch_dependent(kernel, grid, 32 * kInputWarps, kInputWarps * row_bytes, static_cast<cudaStream_t>(stream), 1u, p);
     return static_cast<int>(cudaGetLastError());
   }
   const unsigned grid = static_cast<unsigned>(blocks < 148LL * 16 ? blocks : 148LL * 16);
-  refiner_input_kernel<<<grid, 32 * kInputWarps, 0, static_cast<cudaStream_t>(stream)>>>(p);
+  launch_dependent(refiner_input_kernel, grid, 32 * kInputWarps, 0, static_cast<cudaStream_t>(stream), 1u, p);
   return static_cast<int>(cudaGetLastError());
 }
