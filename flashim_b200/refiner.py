@@ -41,11 +41,18 @@ class PointwiseMX(nn.Module):
         self.register_buffer("weight_exponent", packed.scale_exponent)
         self.register_buffer("weight_scales", swizzle_scales(packed.scale_exponent))
         self.register_buffer("bias", (torch.randn(padded_channels(cout), generator=generator) * 0.02).to(torch.bfloat16))
+        self._operands: tuple = (None,)
+
+    def operands(self) -> tuple[Tensor, Tensor, Tensor]:
+        """``(E4M3 weight, swizzled scales, bias)``. The views and look-ups are kept for as long as the weight buffer is the
+        same tensor: made anew for every call they cost more host time than the launch."""
+        weight = self._buffers["weight"]
+        if self._operands[0] is not weight:
+            self._operands = (weight, (weight.view(torch.float8_e4m3fn), self.weight_scales, self.bias))
+        return self._operands[1]
 
     def forward(self, q: Tensor, scales: Tensor, **epilogue):
-        return ops.mxfp8_conv2d_fused(q, scales, self.weight.view(torch.float8_e4m3fn), self.weight_scales, self.bias,
-                                      1, 1, 1, 1, 0, 0, 1, 1, **epilogue)
-
+        return ops.mxfp8_conv2d_fused(q, scales, *self.operands(), 1, 1, 1, 1, 0, 0, 1, 1, **epilogue)
 
     def forward_bf16(self, x: Tensor, **epilogue):
         """The same layer on bf16 activations: quantised per pixel and 32 channels inside the conv kernel where it takes
@@ -53,7 +60,7 @@ class PointwiseMX(nn.Module):
         # (a layer wider than one 256-column tile would quantise every activation tile once per column tile: measured
         # slower than the standalone quantiser at 512 -> 512)
         if self.cin % 128 == 0 and self.cout <= 256:
-            return ops.mxfp8_conv2d_bf16(x, None, self.weight.view(torch.float8_e4m3fn), self.weight_scales, self.bias, **epilogue)
+            return ops.mxfp8_conv2d_bf16(x, None, *self.operands(), **epilogue)
         q, s = ops.quantize_mxfp8_dynamic(x)
         return self.forward(q, s, **epilogue)
 
@@ -74,9 +81,7 @@ class RefinerBlock(nn.Module):
         if c in (128, 256) and x.is_contiguous():
             # up conv, GELU, requantisation, down conv and residual add in one launch: the hidden tensor stays on chip
             # (the same bits as the two launches below)
-            return ops.mxfp8_gelu_mlp_residual(
-                q.view(b, h, w, c), s, self.up.weight.view(torch.float8_e4m3fn), self.up.weight_scales, self.up.bias,
-                self.down.weight.view(torch.float8_e4m3fn), self.down.weight_scales, self.down.bias, x)
+            return ops.mxfp8_gelu_mlp_residual(q.view(b, h, w, c), s, *self.up.operands(), *self.down.operands(), x)
         hq, hs = self.up(q.view(b, h, w, c), s, act="gelu", dynamic_out=True)
         return self.down(hq, hs, residual=x)
 
@@ -94,7 +99,7 @@ class RefinerLevel(nn.Module):
         """bf16 ``[B, H, W, C]`` -> bf16 ``[B, H, W, 32]`` (channels 0-1 warp, 2-3 confidence, the rest padding)."""
         y = self.proj.forward_bf16(x)
         for block in self.blocks:
-            y = block(y)
+            y = block.forward(y)
         return self.head.forward_bf16(y)
 
 
@@ -129,12 +134,14 @@ class RefinerStack(nn.Module):
         for level, x in zip(self.levels, pyramid):
             parts = []
             for i in range(0, x.shape[0], self.chunk):
-                if lanes > 1:
-                    with torch.cuda.stream(streams[turn % lanes]):
-                        parts.append(level(x[i: i + self.chunk]))
-                    turn += 1
+                part = x if x.shape[0] <= self.chunk else x[i: i + self.chunk]
+                lane = streams[turn % lanes] if lanes > 1 else None
+                turn += 1
+                if lane is None or lane is main:
+                    parts.append(level(part))
                 else:
-                    parts.append(level(x[i: i + self.chunk]))
+                    with torch.cuda.stream(lane):
+                        parts.append(level(part))
             outputs.append(parts)
         if lanes > 1:
             for stream in streams[1:]:
