@@ -19,9 +19,9 @@
 //     or 16 bytes per pixel from registers instead costs a shared-memory wavefront per lane.
 //
 // Measured against the fp32-pipe kernel before it (B200, inputs in L2 where they fit):
-//   4x200x200x256: GELU -> bf16 68 -> 52 us, ReLU -> bf16 54 -> 41, GELU -> MXFP8 88 -> 69, ReLU -> INT8 87 -> 51
-//   8x400x400x128: GELU -> bf16 232 -> 163, ReLU -> bf16 183 -> 125 (80 % of the HBM copy rate), GELU -> MXFP8 303 -> 220,
-//   ReLU -> MXFP8 252 -> 174, ReLU -> INT8 299 -> 165
+//   4x200x200x256: GELU -> bf16 68 -> 52 us, ReLU -> bf16 54 -> 41, GELU -> MXFP8 88 -> 66, ReLU -> INT8 87 -> 51
+//   8x400x400x128: GELU -> bf16 232 -> 163, ReLU -> bf16 183 -> 125 (80 % of the HBM copy rate), GELU -> MXFP8 303 -> 213,
+//   ReLU -> MXFP8 252 -> 177, ReLU -> INT8 299 -> 165
 // What bounds the GELU and quantising forms now is the arithmetic of their epilogues on twelve warps per SM (issue slots about
 // half busy); the care for equal results (below) is a quarter of the MXFP8 form's time.
 //
@@ -68,8 +68,9 @@ enum { kOutBf16 = 0, kOutMx = 1, kOutInt8 = 2 };
 // the shared memory leaves hardly any L1 for, they cost a third of the kernel's time.)
 __host__ __device__ constexpr uint32_t panel_bytes(int mode) { return mode == kOutBf16 ? 8192u : 4096u; }
 __host__ __device__ constexpr uint32_t exchange_bytes(int mode) { return mode == kOutMx ? 4096u : 0u; }
-__host__ __device__ constexpr int stages(int mode) { return mode == kOutMx ? 4 : kMaxStages; }
-__host__ __device__ constexpr uint32_t fragment_bytes(int mode) { return mode == kOutMx ? 4u * 12u * 512u : 0u; }
+__host__ __device__ constexpr bool shared_fragments(int mode) { return mode == kOutMx; }
+__host__ __device__ constexpr int stages(int mode) { return shared_fragments(mode) ? 4 : kMaxStages; }
+__host__ __device__ constexpr uint32_t fragment_bytes(int mode) { return shared_fragments(mode) ? 4u * 12u * 512u : 0u; }
 __host__ __device__ constexpr uint32_t quad_bytes(int mode) {
   return (stages(mode) * kChunkBytes + fragment_bytes(mode) + 2 * panel_bytes(mode) + exchange_bytes(mode) + kListBytes + kWeightBytes + kBiasBytes + 1023u) / 1024u * 1024u;
 }
@@ -396,7 +397,7 @@ dw5x5_kernel(const __grid_constant__ CUtensorMap in_map, const __grid_constant__
             bfrag[st][2 * j + 1][h] = __byte_perm(lo[j], hi[j], 0x7632);
           }
         }
-        if (MODE == kOutMx) {
+        if (shared_fragments(MODE)) {
 #pragma unroll
           for (int j = 0; j < 4; ++j) {
             asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(fragments + (st * 4 + j) * 512), "r"(bfrag[st][2 * j][0]),
@@ -429,7 +430,7 @@ dw5x5_kernel(const __grid_constant__ CUtensorMap in_map, const __grid_constant__
         {
           RowPair r2;
           const auto multiply = [&](auto first, const RowPair& upper, const RowPair& lower, int st) {
-            if constexpr (MODE == kOutMx) {
+            if constexpr (shared_fragments(MODE)) {
               multiply_step_shared<decltype(first)::value>(upper, lower, fragments + st * (4 * 512), acc);
             } else {
               multiply_step<decltype(first)::value>(upper, lower, bfrag[st], acc);
@@ -489,6 +490,23 @@ dw5x5_kernel(const __grid_constant__ CUtensorMap in_map, const __grid_constant__
         float inv[4];
         uint32_t unsure = 0;  // MX: bit i for a pixel whose block is to be summed again
         if (MODE == kOutMx) {
+          // A value whose low 20 mantissa bits are within 8 of one half lies within 2**-20 of a boundary between two E4M3 codes,
+          // whatever power of two it is scaled by (codes below 2**-6 of the scale have coarser steps and are not looked at:
+          // the largest of them is 1/28672 of the block's maximum).
+          constexpr uint32_t kToZero = static_cast<uint32_t>(-(0x80000 - 8)) << 12, kWindow = 16u << 12;
+          uint32_t nearest[4] = {~0u, ~0u, ~0u, ~0u};
+#pragma unroll
+          for (int c = 0; c < 8; ++c) {
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+              float lo, hi;
+              unpack2(v[c][h], lo, hi);
+              nearest[2 * h] = min(nearest[2 * h], (__float_as_uint(lo) << 12) + kToZero);
+              nearest[2 * h + 1] = min(nearest[2 * h + 1], (__float_as_uint(hi) << 12) + kToZero);
+            }
+          }
+#pragma unroll
+          for (int i = 0; i < 4; ++i) unsure |= nearest[i] < kWindow ? 1u << i : 0u;
           float amax[4] = {0.0f, 0.0f, 0.0f, 0.0f};
 #pragma unroll
           for (int c = 0; c < 8; c += 2) {
@@ -519,7 +537,7 @@ dw5x5_kernel(const __grid_constant__ CUtensorMap in_map, const __grid_constant__
 #pragma unroll
           for (int i = 0; i < 4; ++i) amax[i] = fmaxf(max_abs(amax[i], theirs[0][i], theirs[1][i]), theirs[2][i]);
           uint32_t bytes[4];
-          unsure = block_scales(amax, bytes, inv);
+          unsure |= block_scales(amax, bytes, inv);
           if (alive && x < p.width && y + piece < p.height) {  // each warp stores the scales of one row
             const uint32_t byte = piece == 0 ? bytes[0] : piece == 1 ? bytes[1] : piece == 2 ? bytes[2] : bytes[3];
             const uint32_t row = scale_row + y * p.width, groups = p.channels >> 5;
@@ -543,41 +561,18 @@ dw5x5_kernel(const __grid_constant__ CUtensorMap in_map, const __grid_constant__
           }
         };
         if (MODE == kOutMx) {
-          // Codes of the values pushed up and down by 2**-20: where they agree, they are the code, and no other order of
-          // summation gives another one.
-          constexpr float kUp = 1.0f + 0x1p-20f, kDown = 1.0f - 0x1p-20f;
-          const uint64_t up[2] = {pack2(inv[0] * kUp, inv[1] * kUp), pack2(inv[2] * kUp, inv[3] * kUp)};
-          const uint64_t down[2] = {pack2(inv[0] * kDown, inv[1] * kDown), pack2(inv[2] * kDown, inv[3] * kDown)};
-          uint32_t differ[4] = {0, 0, 0, 0};
 #pragma unroll
           for (int c = 0; c < 8; c += 4) {
-            float f[4][4], g[4][4];
+            float f[4][4];
 #pragma unroll
             for (int d = 0; d < 4; ++d) {
-#pragma unroll
-              for (int h = 0; h < 2; ++h) {
-                unpack2(mul2(v[c + d][h], up[h]), f[d][2 * h], f[d][2 * h + 1]);
-                unpack2(mul2(v[c + d][h], down[h]), g[d][2 * h], g[d][2 * h + 1]);
-              }
+              unpack2(mul2(v[c + d][0], pack2(inv[0], inv[1])), f[d][0], f[d][1]);
+              unpack2(mul2(v[c + d][1], pack2(inv[2], inv[3])), f[d][2], f[d][3]);
             }
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-              words[i][c / 4] = e4m3x4(f[0][i], f[1][i], f[2][i], f[3][i]);
-              differ[i] |= words[i][c / 4] ^ e4m3x4(g[0][i], g[1][i], g[2][i], g[3][i]);
-            }
+            for (int i = 0; i < 4; ++i) words[i][c / 4] = e4m3x4(f[0][i], f[1][i], f[2][i], f[3][i]);
           }
-          if (((differ[0] | differ[1]) | (differ[2] | differ[3])) != 0 || unsure != 0) {
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-              if (differ[i] != 0) {
-                float f[4], g[4];
-                values_of(0, i, f);
-                values_of(4, i, g);
-                words[i][0] = e4m3x4(f[0] * inv[i], f[1] * inv[i], f[2] * inv[i], f[3] * inv[i]);
-                words[i][1] = e4m3x4(g[0] * inv[i], g[1] * inv[i], g[2] * inv[i], g[3] * inv[i]);
-                unsure |= 1u << i;
-              }
-            }
+          if (unsure != 0) {
 #pragma unroll 1
             for (; unsure != 0; unsure &= unsure - 1) {
               const int row = y + __ffs(unsure) - 1;
