@@ -19,9 +19,9 @@
 //     or 16 bytes per pixel from registers instead costs a shared-memory wavefront per lane.
 //
 // Measured against the fp32-pipe kernel before it (B200, inputs in L2 where they fit):
-//   4x200x200x256: GELU -> bf16 68 -> 52 us, ReLU -> bf16 54 -> 41, GELU -> MXFP8 88 -> 66, ReLU -> INT8 87 -> 51
-//   8x400x400x128: GELU -> bf16 232 -> 163, ReLU -> bf16 183 -> 125 (80 % of the HBM copy rate), GELU -> MXFP8 303 -> 213,
-//   ReLU -> MXFP8 252 -> 177, ReLU -> INT8 299 -> 165
+//   4x200x200x256: GELU -> bf16 68 -> 52 us, ReLU -> bf16 54 -> 41, GELU -> MXFP8 88 -> 70, ReLU -> INT8 87 -> 49
+//   8x400x400x128: GELU -> bf16 232 -> 165, ReLU -> bf16 183 -> 125 (80 % of the HBM copy rate), GELU -> MXFP8 303 -> 225,
+//   ReLU -> MXFP8 252 -> 178, ReLU -> INT8 299 -> 159
 // What bounds the GELU and quantising forms now is the arithmetic of their epilogues on twelve warps per SM (issue slots about
 // half busy); the care for equal results (below) is a quarter of the MXFP8 form's time.
 //
@@ -29,11 +29,11 @@
 // another order; the two differ by about one fp32 ulp of the largest partial sum. Outputs on which that could show are
 // noted in a list of the quad and summed again at its end in the reference's order (ky-major FMA chain, bias last): bf16
 // outputs below 2**-14 of the sums in their column, where bias and products cancel, and MXFP8 blocks with a value within
-// 2**-20 of a rounding boundary of E4M3 or a maximum within a few ulp of one of the exponent rule (with normal data one
-// output in 30000 and one block in 1000). INT8 codes have an absolute resolution far above the difference.
+// 2**-19 of a rounding boundary of E4M3 or a maximum within a few ulp of one of the exponent rule (with normal data one
+// output in 30000 and one block in 700). INT8 codes have an absolute resolution far above the difference.
 //
-// Not-a-number and infinite inputs: a patch value outside an output's 5x5 window is multiplied by a zero of B, so they
-// spoil the outputs of their 6 x 8 patches instead of those of their 5x5 windows.
+// A patch value outside an output's 5x5 window is multiplied by a zero of B, which an infinity or a not-a-number survives. A
+// quad that meets a sum which is not finite therefore does its whole range again in the reference's order at the end.
 //
 // Work: a strip is one (image, 32-column tile) over all rows, cut into steps of four output rows; a span is the part of a
 // range of steps inside one strip. The quads of all CTAs (three per CTA, one CTA per SM) form groups of one quad per
@@ -57,7 +57,7 @@ constexpr int kHaloX = kTileX + 4;
 constexpr uint32_t kPixelBytes = kTileC * 2, kRowBytes = kHaloX * kPixelBytes, kChunkBytes = kStepRows * kRowBytes;
 constexpr int kTaps = 25, kMaxStages = 6;
 constexpr float kCancelled = 16384.0f;  // an output below 1 / kCancelled of the sums it comes from is summed again (bf16)
-constexpr uint32_t kListEntries = 126, kListBytes = 1024;  // {count, -}, then {image row, column * 32 + channel} per entry
+constexpr uint32_t kListEntries = 126, kListBytes = 1024;  // {count, not finite}, then {image row, column * 32 + channel} per entry
 constexpr uint32_t kWeightBytes = kTaps * kTileC * 2, kBiasBytes = kTileC * 8;
 
 enum { kOutBf16 = 0, kOutMx = 1, kOutInt8 = 2 };
@@ -215,6 +215,12 @@ __device__ __forceinline__ void note(uint32_t list, uint32_t row, uint32_t x, ui
   if (at < kListEntries) asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(list + 8 + at * 8), "r"(row), "r"(x * 32 + channel) : "memory");
 }
 
+// max(|a|, |b|, |c|), not a number if one of them is
+__device__ __forceinline__ float max_abs_nan(float a, float b, float c) {
+  float r;
+  asm("max.NaN.abs.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+}
 // min(|a|, |b|, |c|)
 __device__ __forceinline__ float min_abs(float a, float b, float c) {
   float r;
@@ -372,7 +378,7 @@ dw5x5_kernel(const __grid_constant__ CUtensorMap in_map, const __grid_constant__
         asm volatile("st.shared.b32 [%0], %1;" ::"r"(weights_at + i * 4), "r"(word) : "memory");
       }
       if (piece == 0) {
-        if (lane == 0) asm volatile("st.shared.b32 [%0], 0;" ::"r"(list) : "memory");
+        if (lane == 0) asm volatile("st.shared.v2.b32 [%0], {%1, %1};" ::"r"(list), "r"(0u) : "memory");
         const float bias = __ldg(p.bias + c0 + lane);
         asm volatile("st.shared.v2.f32 [%0], {%1, %1};" ::"r"(bias_at + lane * 8), "f"(bias) : "memory");
       }
@@ -445,7 +451,7 @@ dw5x5_kernel(const __grid_constant__ CUtensorMap in_map, const __grid_constant__
         }
         // bias and activation: v[channel][0 / 1] = rows (0, 1) / (2, 3) of the lane's column
         uint64_t v[8][2];
-        float margin = 0.0f;
+        float margin = 0.0f, largest = 0.0f;
 #pragma unroll
         for (int c = 0; c < 8; c += 2) {
           uint64_t bias[2];
@@ -461,12 +467,22 @@ dw5x5_kernel(const __grid_constant__ CUtensorMap in_map, const __grid_constant__
               unpack2(bias[d], b, unused);
               unpack2(v[c + d][0], f[0], f[1]);
               unpack2(v[c + d][1], f[2], f[3]);
-              const float size = max_abs(max_abs(a[0], a[1], a[2]), a[3], b);
+              const float size = max_abs_nan(max_abs_nan(a[0], a[1], a[2]), a[3], b);
+              largest = max_abs_nan(largest, size, size);
               slack[d] = fmaf(min_abs(min_abs(f[0], f[1], f[2]), f[3], f[3]), kCancelled, -size);
             }
           }
-          if (MODE == kOutBf16) margin = fminf(fminf(margin, slack[0]), slack[1]);
+          if (MODE == kOutBf16) {
+            margin = fminf(fminf(margin, slack[0]), slack[1]);
+          } else {
+#pragma unroll
+            for (int d = 0; d < 2; ++d) {
+              largest = max_abs_nan(largest, acc[c + d][0], acc[c + d][1]);
+              largest = max_abs_nan(largest, acc[c + d][2], acc[c + d][3]);
+            }
+          }
         }
+        if (!(largest < __int_as_float(0x7F800000))) asm volatile("st.shared.b32 [%0], %1;" ::"r"(list + 4), "r"(1u) : "memory");
         if (MODE == kOutBf16 && margin < 0.0f) {
           uint32_t cancelled = 0;  // bit 4 c + i
 #pragma unroll
@@ -490,10 +506,10 @@ dw5x5_kernel(const __grid_constant__ CUtensorMap in_map, const __grid_constant__
         float inv[4];
         uint32_t unsure = 0;  // MX: bit i for a pixel whose block is to be summed again
         if (MODE == kOutMx) {
-          // A value whose low 20 mantissa bits are within 8 of one half lies within 2**-20 of a boundary between two E4M3 codes,
+          // A value whose low 20 mantissa bits are within 16 of one half lies within 2**-19 of a boundary between two E4M3 codes,
           // whatever power of two it is scaled by (codes below 2**-6 of the scale have coarser steps and are not looked at:
           // the largest of them is 1/28672 of the block's maximum).
-          constexpr uint32_t kToZero = static_cast<uint32_t>(-(0x80000 - 8)) << 12, kWindow = 16u << 12;
+          constexpr uint32_t kToZero = static_cast<uint32_t>(-(0x80000 - 16)) << 12, kWindow = 32u << 12;
           uint32_t nearest[4] = {~0u, ~0u, ~0u, ~0u};
 #pragma unroll
           for (int c = 0; c < 8; ++c) {
@@ -638,22 +654,20 @@ dw5x5_kernel(const __grid_constant__ CUtensorMap in_map, const __grid_constant__
       if (piece == 0 && stored_b >= 0 && alive) store_panel(panels + (flip ^ 1u) * panel_bytes(MODE), stored_c, stored_x, stored_y, stored_b);
       stored_b = -1;
     }
-    if (MODE != kOutInt8) {
+    {
       // the outputs in the list once more, after the stores of their panels have completed
       named_barrier(quad_barrier, 128);
-      uint32_t count;
-      asm volatile("ld.shared.b32 %0, [%1];" : "=r"(count) : "r"(list));
+      uint32_t count, not_finite;
+      asm volatile("ld.shared.v2.b32 {%0, %1}, [%2];" : "=r"(count), "=r"(not_finite) : "r"(list));
       count = min(count, kListEntries);
-      if (count != 0) {
+      if ((count | not_finite) != 0) {
         if (piece == 0 && elect_one()) bulk_wait_all();
         named_barrier(quad_barrier, 128);
       }
-      if (!alive) count = 0;
-#pragma unroll 1
-      for (uint32_t i = MODE == kOutMx ? piece : threadIdx.x & 127; i < count; i += MODE == kOutMx ? 4 : 128) {
-        uint32_t row, place;
-        asm volatile("ld.shared.v2.b32 {%0, %1}, [%2];" : "=r"(row), "=r"(place) : "r"(list + 8 + i * 8));
-        const int c = MODE == kOutMx ? lane : place & 31, px = place >> 5, b = row / p.height, y = row - b * p.height;
+      if (!alive) count = not_finite = 0;
+      // one output (MXFP8: a warp per block, lane = channel) of image row `row` (of all images one below the other)
+      const auto again = [&](uint32_t row, int px, int c) {
+        const int b = row / p.height, y = row - b * p.height;
         float bias;
         asm volatile("ld.shared.f32 %0, [%1];" : "=f"(bias) : "r"(bias_at + c * 8));
         const float sum = chain_sum(p.value + static_cast<size_t>(b) * p.height * p.width * p.channels + c0 + c, p.height, p.width, p.channels,
@@ -663,11 +677,31 @@ dw5x5_kernel(const __grid_constant__ CUtensorMap in_map, const __grid_constant__
         const size_t pixel = static_cast<size_t>(row) * p.width + px, to = pixel * p.channels + c0 + c;
         if (MODE == kOutBf16) {
           reinterpret_cast<uint16_t*>(p.out)[to] = static_cast<uint16_t>(pack_bf16(out, 0.0f));
-        } else {  // a warp per block
-          const int e = e8m0_exponent(__uint_as_float(redux_max(__float_as_uint(fabsf(out)), 0xffffffffu)));
+        } else if (MODE == kOutInt8) {
+          p.out[to] = static_cast<uint8_t>(int8_pack2(int8, bf16_lo(pack_bf16(out, 0.0f)), 0.0f));
+        } else {
+          // (fmaxf drops a not-a-number, as the block maximum above does)
+          const int e = e8m0_exponent(__uint_as_float(redux_max(__float_as_uint(fmaxf(fabsf(out), 0.0f)), 0xffffffffu)));
           p.out[to] = static_cast<uint8_t>(e4m3x2(out * exp2_int(-e), 0.0f));
           const int groups = p.channels >> 5;
           if (lane == 0) p.scales[p.swizzled ? swizzled_scale_offset(pixel, ct, (groups + 3) >> 2) : pixel * groups + ct] = static_cast<uint8_t>(e + 127);
+        }
+      };
+      if (not_finite != 0) {
+        for (int s = s_begin; s < s_end;) {
+          const Position at = position_of(p, s);
+          const int len = min(p.strip_steps - at.k0, s_end - s), y0 = at.k0 * kStepRows, x0 = at.tx * kTileX;
+          s += len;
+          const int rows = min(len * kStepRows, p.height - y0), columns = min(kTileX, p.width - x0);
+#pragma unroll 1
+          for (int i = piece; i < rows * columns; i += 4) again(at.b * p.height + y0 + i / columns, x0 + i % columns, lane);
+        }
+      } else if (MODE != kOutInt8) {
+#pragma unroll 1
+        for (uint32_t i = MODE == kOutMx ? piece : threadIdx.x & 127; i < count; i += MODE == kOutMx ? 4 : 128) {
+          uint32_t row, place;
+          asm volatile("ld.shared.v2.b32 {%0, %1}, [%2];" : "=r"(row), "=r"(place) : "r"(list + 8 + i * 8));
+          again(row, place >> 5, MODE == kOutMx ? lane : place & 31);
         }
       }
     }

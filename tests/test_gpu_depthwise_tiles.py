@@ -77,3 +77,24 @@ def test_outputs_off_the_tma_alignment(offset):
         assert int(space[3 * n + 32 + at]) == 7 and int(space[2 * n + at]) == 7  # nothing behind the outputs
         outs.append((dense.clone(), codes.clone(), scales))
     assert all(same_bytes(p, q) for p, q in zip(*outs))
+
+
+def test_infinite_and_nan_inputs_stay_in_their_windows(ops):
+    """The kernel multiplies a 6 x 8 patch per eight pixels; what is not finite may only show in the 5x5 windows that hold it."""
+    g = torch.Generator().manual_seed(3)
+    x = torch.randn(2, 64, 21, 70, generator=g).to(BF16).contiguous(memory_format=torch.channels_last)
+    w, b = (torch.randn(25, 64, generator=g) * 0.2).to(BF16), torch.randn(64, generator=g)
+    spoiled = x.clone(memory_format=torch.preserve_format)
+    hit = torch.zeros(2, 21, 70, dtype=torch.bool)
+    for image, c, y, px, v in ((0, 3, 0, 0, float("inf")), (0, 40, 10, 33, float("nan")), (1, 63, 20, 69, float("-inf")), (1, 0, 7, 31, float("nan"))):
+        spoiled[image, c, y, px] = v
+        hit[image, max(0, y - 2): y + 3, max(0, px - 2): px + 3] = True
+    xd, sd, wd, bd = to_dev(x, spoiled, w, b)
+    got, want = ops.depthwise5x5_act(sd, wd, bd, "none").cpu(), oracle.depthwise5x5_act_ext(spoiled, w, b, "none")
+    finite = torch.isfinite(want)
+    assert torch.equal(torch.isnan(got), torch.isnan(want)) and torch.equal(got[~finite & ~torch.isnan(want)], want[~finite & ~torch.isnan(want)])
+    assert int(bf16_ulp_distance(got[finite], want[finite]).max()) <= 1
+    scale = torch.tensor(0.03, device=DEV)
+    for op, extra in ((ops.depthwise5x5_relu_int8, (scale,)), (lambda *a: ops.depthwise5x5_relu_mxfp8(*a)[0], ())):
+        bad, clean = (op(t, wd, bd, *extra).cpu().view(torch.uint8).view(2, 21, 70, 64) for t in (sd, xd))
+        assert float((bad[~hit] != clean[~hit]).float().mean()) < 1e-3
