@@ -2003,7 +2003,6 @@ int make_plan(const FimConvGeometry& g, int fmt, bool per_pixel, bool allow_flat
   if (g_forced_block_n == 64) bn = 64;
   if (fmt == kFmtBf16 && bn == 256) bn = 128;  // BF16 layers on this path are narrow pointwise products
   if (bn == 64 && g.cout > 64 && scaled) bn = 128;  // a 64-wide tile may only start at column 0 of its scale tile
-  pl.block_n = bn;
   pl.flat = pointwise && allow_flat;
   pl.convert = convert;
   if (convert && !(fmt == kFmtMx && pl.flat && pl.block_k == 128)) return kUnsupported;
@@ -2029,8 +2028,20 @@ int make_plan(const FimConvGeometry& g, int fmt, bool per_pixel, bool allow_flat
     }
     pl.tiles_x = ceil_div(out_w, pl.tile_w), pl.tiles_y = ceil_div(out_h, pl.tile_h);
   }
-  pl.tiles_n = ceil_div(g.cout, bn);
   const long long row_tiles = static_cast<long long>(pl.tiles_x) * pl.tiles_y * (pl.flat ? 1 : g.batch);
+  // A problem whose tiles leave half of the SMs without one takes narrower tiles for as long as all of them still run at
+  // once: a layer of one round lasts as long as one tile's main loop and epilogue, both of which shrink with the width. us at
+  // 1x50x50x256 -> 256, 3x3: MXFP8 11.3 -> 9.8 (64 columns are not open to it), INT8 12.4 -> 7.6; INT8 linear 300x3072 -> 768
+  // 14.2 -> 7.7; one tile more than the SMs hold and the narrower form loses (2x50x50x512: 18.4 against 23.4). Not for
+  // converting layers, which would quantise a tile once per column tile, nor where it would cost the layer its patches.
+  {
+    const int device_sms = sm_count(), sms = g_max_ctas > 0 && g_max_ctas < device_sms ? g_max_ctas : device_sms;
+    const bool patch_layer = g.kh * g.kw > 1 && g.stride_h == 1 && g.stride_w == 1 && g.cout <= 128;
+    const int narrowest = scaled || patch_layer ? 128 : 64;
+    while (g_forced_block_n == 0 && !convert && bn > narrowest && row_tiles * ceil_div(g.cout, bn / 2) <= sms) bn /= 2;
+  }
+  pl.block_n = bn;
+  pl.tiles_n = ceil_div(g.cout, bn);
   // CTA pairs for the wide, compute-bound INT8 tiles: a pair owns two consecutive row tiles (the last one may not exist:
   // its loads are zero-filled and its stores clipped). The block-scaled form is correct too but measured slower than
   // single CTAs (its scale copies serialise the pair's tensor pipes): it only runs when asked for (tuning flag 128).
