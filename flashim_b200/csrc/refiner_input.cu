@@ -141,12 +141,14 @@ __global__ void __launch_bounds__(32 * kInputWarps) refiner_input_kernel(const I
 // eight steps are added by one transposing butterfly (7 shuffles instead of 24, each sum over the same pairs of lanes as
 // above; the division by sqrt(P) comes last, once per value), the radius is a constant of the code, and the eight rows of a block, which are contiguous in the output, go through shared memory and
 // leave as 16-byte words instead of single bf16 values. The kernel above waits for one pair of loads per four patch pixels.
-// Refiner input + heads of both directions of a pair, 96x72x64, radius 3: 45 -> 23 us; 200x200x128, radius 2: 225 -> 164.
+// Refiner input + heads of both directions of a pair, 96x72x64, radius 3: 45 -> 23 us; 200x200x128, radius 2: 225 -> 147.
+// (Four CTAs with half as many loads in flight against three with twice as many: 119 against 129 us for the latter's input
+// rows; five or more CTAs spill.)
 template <int NF, int R>
-__global__ void __launch_bounds__(32 * kInputWarps, 3) refiner_input_wide_kernel(const InputParams p) {
+__global__ void __launch_bounds__(32 * kInputWarps, 4) refiner_input_wide_kernel(const InputParams p) {
   grid_release();
   grid_wait();
-  constexpr int P = 32 * NF, kAhead = NF >= 4 ? 2 : 8 / NF;  // patch pixels in flight per group of eight lanes
+  constexpr int P = 32 * NF, kAhead = NF >= 4 ? 2 : 4 / NF;  // patch pixels in flight per group of eight lanes
   extern __shared__ __align__(16) __nv_bfloat16 tile[];      // kInputWarps output rows
   __shared__ float dots[kInputWarps][kInputMaxPatch];
   const int warp_id = threadIdx.x >> 5, lane = threadIdx.x & 31, group = lane >> 3, sub = lane & 7;
