@@ -96,6 +96,7 @@ struct ConvParams {
   int warp_panels;           // flat 1x1 convs: every epilogue warp stages and stores its own 32 rows (no barrier between warps)
   int8_t* pooled;            // kPatch: where that output goes
   int pool;                  // INT8, bf16 output: the 2x2 max pool of the output also leaves the epilogue, as INT8 codes (out_scale)
+  int gelu_copies;  // kPatch: copies of the GELU table (1, 2, 4 or 8)
   uint32_t patch_bytes, patch_pitch, patch_rows;  // kPatch: one channel chunk's patch (rounded up to 1 KB), one patch row, its rows
   int debug;  // probe builds only (FIM_PROBE_BUILD): 1 = no activation loads, 2 = no weight loads, 4 = no output stores, 8 = no scale copies
 };
@@ -139,7 +140,9 @@ __device__ __forceinline__ uint32_t idesc_i8(int block_n, int block_m = kTileM) 
 }
 
 #include "gelu_table.inc"
-constexpr uint32_t kGeluSmemBytes = (kGeluEntries * 4u + 1023u) / 1024u * 1024u;  // keeps the tiles behind it 1024-byte aligned
+// shared memory of the table, or of several interleaved copies of it (a size that keeps the tiles behind it 1024-byte aligned)
+__host__ __device__ constexpr uint32_t gelu_smem_bytes(int copies) { return (kGeluEntries * 4u * copies + 1023u) / 1024u * 1024u; }
+constexpr uint32_t kGeluSmemBytes = gelu_smem_bytes(1);
 
 // GELU of two bf16 values in one word, as bf16: the erf form torch evaluates (x * 0.5 * (1 + erf(x / sqrt 2)) in fp32,
 // rounded to bf16), looked up instead of computed. `table` locates the shared-memory copy of kGeluTable: per magnitude a
@@ -150,11 +153,17 @@ constexpr uint32_t kGeluSmemBytes = (kGeluEntries * 4u + 1023u) / 1024u * 1024u;
 struct GeluTable {
   uint32_t low2;    // the low 16 bits of the table's shared-memory address, in both halves of the word
   uint32_t window;  // its upper 16 bits: zero for a single CTA; in a cluster the CTA's rank sits up there
+  uint32_t stride;  // bytes from one entry to the next
 };
-__device__ __forceinline__ GeluTable gelu_table_at(uint32_t smem_address) {
+// `copies` > 1 (a power of two): entry e of copy c is word e * copies + c, and a lane reads copy lane % copies. Lanes of
+// different copies never share a bank, so the 32 scattered reads of a look-up take about 2.2 passes with eight copies
+// where one copy takes 3.5: what bounds the layers with the shortest main loops (3x3 64 -> 64 at 800x800: shared-memory
+// wavefronts 78 % busy, 176 -> 154 us).
+__device__ __forceinline__ GeluTable gelu_table_at(uint32_t smem_address, uint32_t copies = 1, uint32_t lane = 0) {
   GeluTable t;
-  t.low2 = (smem_address & 0xFFFFu) * 0x00010001u;
+  t.low2 = ((smem_address & 0xFFFFu) + 4u * (lane & (copies - 1u))) * 0x00010001u;
   t.window = smem_address & 0xFFFF0000u;
+  t.stride = 4u * copies;
   return t;
 }
 __device__ __forceinline__ uint32_t gelu_bf16x2(uint32_t r, const GeluTable& table) {
@@ -165,7 +174,7 @@ __device__ __forceinline__ uint32_t gelu_bf16x2(uint32_t r, const GeluTable& tab
   // both entry addresses with one multiply-add: the table sits in the first 64 KB of the CTA's shared window, so the low
   // 16 bits of an address fit a half and neither half carries into the other; a byte permute then puts each half under
   // the window's upper bits
-  const uint32_t at = t * 4u + table.low2;
+  const uint32_t at = t * table.stride + table.low2;
   uint32_t w0, w1, negative;
   asm("ld.shared.b32 %0, [%1];" : "=r"(w0) : "r"(__byte_perm(at, table.window, 0x7610)));
   asm("ld.shared.b32 %0, [%1];" : "=r"(w1) : "r"(__byte_perm(at, table.window, 0x7632)));
@@ -199,8 +208,8 @@ constexpr int kEpiGelu = 1, kEpiDynamic = 2, kEpiResidual = 4, kEpiLean = 8, kEp
 // groups are one patch row apart (the descriptor's stride). The swizzle is a function of the shared-memory address, so a
 // shifted start needs no other layout. Per tile that is one copy and one barrier round instead of one per tap and channel
 // chunk, 1.4 activation bytes per input byte instead of 9 (3x3), and no scale copies: all weight scales stay in tensor memory.
-//   MXFP8 3x3 + bias + GELU + static requantisation, N = 4: 800x800x64 363 -> 176 us, 400x400x128 117 -> 96 (with a plain
-//   bf16 output 107 -> 77); INT8 3x3 + bias: 4x201x199x128 31 -> 22, 4x400x400x64 84 -> 54.
+//   MXFP8 3x3 + bias + GELU + static requantisation, N = 4: 800x800x64 363 -> 154 us, 400x400x128 117 -> 92 (with a plain
+//   bf16 output 107 -> 70); INT8 3x3 + bias: 4x201x199x128 31 -> 20, 4x400x400x64 84 -> 32.
 constexpr int kPatch = 128;
 constexpr int kPatchTileW = 8, kPatchTileH = 16;
 
@@ -494,7 +503,8 @@ conv_kernel(const __grid_constant__ CUtensorMap act_map, const __grid_constant__
   const uint32_t base = (smem_u32(smem_dyn) + 1023u) & ~1023u;
   const uint32_t panel_bytes = 4096u * p.out_elem;
   const uint32_t smem_gelu = base;  // kGeluTable first, when the epilogue applies GELU: within 64 KB of the window's start
-  const uint32_t smem_a = base + (p.act == kActGelu ? kGeluSmemBytes : 0u);
+  const int gelu_copies = PATCH ? p.gelu_copies : 1;
+  const uint32_t smem_a = base + (p.act == kActGelu ? gelu_smem_bytes(gelu_copies) : 0u);
   const uint32_t a_stage = PATCH ? p.patch_bytes * static_cast<uint32_t>(p.k_chunks) : kABytes;
   const uint32_t smem_b = smem_a + p.stages * a_stage;
   const uint32_t smem_out = smem_b + static_cast<uint32_t>(p.b_slots) * kBBytes;
@@ -555,7 +565,10 @@ conv_kernel(const __grid_constant__ CUtensorMap act_map, const __grid_constant__
   }
   if (p.act == kActGelu) {
     for (int i = threadIdx.x; i < kGeluEntries; i += kBlockThreads) {
-      asm volatile("st.shared.b32 [%0], %1;" ::"r"(smem_gelu + i * 4), "r"(kGeluTable[i]) : "memory");
+      const uint32_t entry = kGeluTable[i];
+      for (int c = 0; c < gelu_copies; ++c) {
+        asm volatile("st.shared.b32 [%0], %1;" ::"r"(smem_gelu + (i * gelu_copies + c) * 4), "r"(entry) : "memory");
+      }
     }
   }
   grid_release();
@@ -1265,6 +1278,7 @@ conv_kernel(const __grid_constant__ CUtensorMap act_map, const __grid_constant__
       }
       pool_to = static_cast<uint32_t>(pp) * 32u + static_cast<uint32_t>(slot) * 8u;
     }
+    const GeluTable gelu_table = gelu_table_at(smem_gelu, static_cast<uint32_t>(gelu_copies), static_cast<uint32_t>(lane));
     uint32_t tile_it = 0, chunk_it = 0;
     for (int tile = worker; tile < p.total_tiles; tile += workers, ++tile_it) {
       if (kTileSets == 2 && (tile_it & 1u) != tile_set) continue;  // the other set's tile
@@ -1440,7 +1454,7 @@ conv_kernel(const __grid_constant__ CUtensorMap act_map, const __grid_constant__
           const int n = n0 + cgroup * kGroupColumns + g * 32;
           if (n >= n_end) continue;  // uniform over the four warps of this group
           uint32_t w[16];
-          finish_chunk<INT8>(p, sw, q[g], n, pixel, b, y, x, valid, gelu_table_at(smem_gelu), w);
+          finish_chunk<INT8>(p, sw, q[g], n, pixel, b, y, x, valid, gelu_table, w);
           const uint32_t parity = chunk_it & 1u;
           if constexpr (pool && PATCH) {
             store_pooled(n, pool_in_warp(w));
@@ -1957,7 +1971,7 @@ struct Plan {
   bool pair;  // clusters of two CTAs driving one cta_group::2 instruction stream
   bool convert = false;    // bf16 activations, quantised on chip
   bool patch = false;      // one halo patch of activations per tile (kPatch)
-  int patch_w = 0, patch_h = 0, patch_bytes = 0;
+  int patch_w = 0, patch_h = 0, patch_bytes = 0, gelu_copies = 1;
   bool resident_b = false; // the whole weight matrix stays in shared memory (one output-channel tile, small K)
   int fixed_epilogue = 0;  // kEpiLean | switches when one of the compile-time epilogues serves this call, else 0
   int out_h, out_w;
@@ -2104,14 +2118,22 @@ int make_plan(const FimConvGeometry& g, int fmt, bool per_pixel, bool allow_flat
       const int fit = room / (chunks * chunk);
       if (fit < 2 || pw > 256 || ph > 256 || tiles > 0x3fffffffLL || scale_tiles * 512 > epilogue_groups * panels * 4096 * out_elem) continue;
       if (acc_stages(bn) * bn + 4 * 6 + 4 * ((g.cin + 127) / 128) + 4 * scale_tiles > 512) continue;  // tensor memory
+      // more copies of the GELU table where shared memory has room for them and a CTA has tiles enough to repay filling them
+      // (up to eight: the table's addresses fit 16 bits)
+      int left = fit, copies = 1;
+      while (gelu && copies < 8 && tiles >= 8LL * (g_max_ctas > 0 ? g_max_ctas : sm_count())) {
+        const int next = (room - static_cast<int>(gelu_smem_bytes(2 * copies) - kGeluSmemBytes)) / (chunks * chunk);
+        if (next < (fit < 4 ? fit : 4)) break;
+        copies *= 2, left = next;
+      }
       pl.patch = true, pl.pair = false, pl.resident_b = true;
-      pl.panels_per_half = panels;
-      pl.stages = fit < 6 ? fit : 6;
+      pl.panels_per_half = panels, pl.gelu_copies = copies;
+      pl.stages = left < 6 ? left : 6;
       pl.tile_w = kPatchTileW, pl.tile_h = kPatchTileH;
       pl.patch_w = pw, pl.patch_h = ph, pl.patch_bytes = chunk;
       pl.tiles_x = static_cast<int>(tx), pl.tiles_y = static_cast<int>(ty);
       pl.total_tiles = static_cast<int>(tiles);
-      pl.smem = static_cast<size_t>(kSmemLimit - room) + static_cast<size_t>(pl.stages) * chunks * chunk;
+      pl.smem = static_cast<size_t>(kSmemLimit - room) + gelu_smem_bytes(copies) - kGeluSmemBytes + static_cast<size_t>(pl.stages) * chunks * chunk;
     }
   }
   const int device_sms = sm_count();
@@ -2399,6 +2421,7 @@ int run_conv(int fmt, const void* x, const int8_t* act_exponent, const void* act
   p.out_scale = ep->out_scale;
   p.pool = pool && !pl.patch ? 1 : 0;  // (pooled panels in shared memory)
   p.pooled = static_cast<int8_t*>(pooled);
+  p.gelu_copies = pl.gelu_copies;
   p.patch_bytes = static_cast<uint32_t>(pl.patch_bytes), p.patch_pitch = static_cast<uint32_t>(pl.patch_w * pl.block_k);
   p.patch_rows = static_cast<uint32_t>(pl.patch_h);
   p.status = status;

@@ -720,7 +720,10 @@ template <int MODE>
 int launch_kernel(const CUtensorMap& in_map, const CUtensorMap& out_map, const DwParams& p, int act, unsigned grid, cudaStream_t s) {
   constexpr size_t kSmem = 1024 + kQuads * quad_bytes(MODE);
   static_assert(kSmem <= 227 * 1024, "shared memory of one CTA");
-  auto kernel = act == kActGelu ? dw5x5_kernel<MODE, kActGelu> : act == kActRelu ? dw5x5_kernel<MODE, kActRelu> : dw5x5_kernel<MODE, kActNone>;
+  auto kernel = dw5x5_kernel<MODE, kActRelu>;
+  if constexpr (MODE != kOutInt8) {  // (the INT8 form always ends in a ReLU)
+    if (act != kActRelu) kernel = act == kActGelu ? dw5x5_kernel<MODE, kActGelu> : dw5x5_kernel<MODE, kActNone>;
+  }
   // every instantiation gets the opt-in limit once per device
   static bool configured[3][kMaxDevices] = {};
   const int device = current_device();

@@ -23,6 +23,7 @@ CASES = [  # batch, height, width, cin, cout, kh, kw, ph, pw, dh, dw, most CTAs
     (1, 16, 8, 64, 64, 3, 3, 1, 1, 1, 1, 0), (3, 17, 9, 64, 64, 3, 3, 1, 1, 1, 1, 2), (2, 33, 41, 128, 128, 3, 3, 1, 1, 1, 1, 5),
     (2, 31, 23, 32, 32, 5, 5, 2, 2, 1, 1, 3), (1, 20, 20, 96, 96, 3, 3, 2, 2, 2, 2, 1), (1, 1, 50, 64, 128, 1, 3, 0, 1, 1, 1, 2),
     (2, 12, 7, 128, 64, 3, 1, 0, 0, 3, 1, 0), (1, 6, 6, 64, 64, 3, 3, 0, 0, 1, 1, 0), (1, 40, 30, 192, 64, 3, 3, 1, 1, 1, 1, 4),
+    (4, 40, 40, 64, 64, 3, 3, 1, 1, 1, 1, 1),  # tiles enough for several copies of the GELU table
 ]
 
 
