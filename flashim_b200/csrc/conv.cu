@@ -1505,13 +1505,15 @@ conv_kernel(const __grid_constant__ CUtensorMap act_map, const __grid_constant__
 // tensor memory (they take alternate 32-channel chunks), add bias and residual to the finished second accumulator and
 // store bf16 rows; the residual reaches them by TMA, in panels of the output panels' shape, two chunks ahead. The same
 // MMAs in the same order as the two separate launches, the same epilogue arithmetic: the same bits. KC = C / 128 (1 or
-// 2). 26 warps: TMA producer, MMA issuer, 16 hidden-block warps, 8 output warps. (Four interleaved copies of the GELU
-// table, so that lanes of different copies never share a bank, measured no faster: 267 against 263 us.)
+// 2). 26 warps: TMA producer, MMA issuer, 16 hidden-block warps, 8 output warps.
 constexpr uint32_t kMlpTile = 128u * 128u;  // bytes of one operand tile: 128 rows x 128 bytes of K
 constexpr int kMlpOutWarps = 8;  // output warps: two per lane quarter of tensor memory, which take alternate 32-channel chunks
 constexpr int kMlpThreads = kThreads + 32 * kMlpOutWarps;
 constexpr uint32_t kMlpPanels = 2, kMlpPanelBytes = 32u * 64u;  // output panels per output warp: 32 rows x 32 bf16 channels
 constexpr uint32_t kMlpResidualSlots = 2;  // residual panels (same shape) each output warp keeps in flight
+// Copies of the GELU table: the ring gives up a weight unit or two for them, which nothing waits for (8x400x400x128 260 -> 256
+// us, 8x200x200x256 168 -> 163; two copies give half of that).
+constexpr int kMlpGeluCopies = 4;
 struct MlpParams {
   int rows, row_tiles, stages;
   const uint8_t* x_scales;   // per-pixel scales of x: swizzled tiles, KC per row tile
@@ -1550,7 +1552,7 @@ mlp_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constant__ CU
 
   const uint32_t base = (smem_u32(smem_dyn) + 1023u) & ~1023u;
   const uint32_t smem_gelu = base;
-  const uint32_t smem_x = base + kGeluSmemBytes;
+  const uint32_t smem_x = base + gelu_smem_bytes(kMlpGeluCopies);
   const uint32_t smem_w = smem_x + kUnitBytes;
   const uint32_t smem_h = smem_w + static_cast<uint32_t>(p.stages) * kUnitBytes;
   const uint32_t smem_out = smem_h + 2u * kMlpTile;
@@ -1595,7 +1597,11 @@ mlp_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constant__ CU
     tmem_relinquish();
   }
   for (int i = threadIdx.x; i < kGeluEntries; i += kMlpThreads) {
-    asm volatile("st.shared.b32 [%0], %1;" ::"r"(smem_gelu + i * 4), "r"(kGeluTable[i]) : "memory");
+    const uint32_t entry = kGeluTable[i];
+#pragma unroll
+    for (int c = 0; c < kMlpGeluCopies; ++c) {
+      asm volatile("st.shared.b32 [%0], %1;" ::"r"(smem_gelu + (i * kMlpGeluCopies + c) * 4), "r"(entry) : "memory");
+    }
   }
   grid_release();
   grid_wait();
@@ -1755,7 +1761,7 @@ mlp_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constant__ CU
     // ===== hidden-block warps: lanes 32 * (w % 4) ... of tensor memory, 32 hidden channels (w - 2) / 4 of every block =====
     const int quarter = warp & 3, group = (warp - 2) >> 2;
     const int row = quarter * 32 + lane;
-    const GeluTable gelu2 = gelu_table_at(smem_gelu);
+    const GeluTable gelu2 = gelu_table_at(smem_gelu, kMlpGeluCopies, static_cast<uint32_t>(lane));
     const uint32_t lane_tmem = tmem + (static_cast<uint32_t>(quarter * 32) << 16) + kAcc1 + group * 32;
     // where this lane's 32 hidden bytes go in a K-major 128-byte-swizzled tile, and its scale byte in the scale tile
     const uint32_t h_row = static_cast<uint32_t>(row) * 128u;
@@ -2577,7 +2583,7 @@ int run_mlp(const void* x, const void* x_scales, const void* w1, const void* w1_
   }
   const int kc = channels / 128, c = channels;
   const uint32_t unit = static_cast<uint32_t>(kc) * (kMlpTile + 512u);
-  const uint32_t fixed = 1024u + kGeluSmemBytes + unit + 2u * (kMlpTile + 512u) + kMlpOutWarps * (kMlpPanels + kMlpResidualSlots) * kMlpPanelBytes + 3u * c * 4u;
+  const uint32_t fixed = 1024u + gelu_smem_bytes(kMlpGeluCopies) + unit + 2u * (kMlpTile + 512u) + kMlpOutWarps * (kMlpPanels + kMlpResidualSlots) * kMlpPanelBytes + 3u * c * 4u;
   int stages = static_cast<int>((kSmemLimit - fixed) / unit);
   if (stages > kMaxStages) stages = kMaxStages;
   if (stages < 2) return kUnsupported;
