@@ -27,8 +27,8 @@
 //
 // Precision: the tensor cores add the exact products into fp32 accumulators, as the fp32 chain of the reference does, but in
 // another order; the two differ by about one fp32 ulp of the largest partial sum. Outputs on which that could show are
-// noted in a list of the quad and summed again at its end in the reference's order (ky-major FMA chain, bias last): bf16
-// outputs below 2**-14 of the sums in their column, where bias and products cancel, and MXFP8 blocks with a value within
+// noted in a list of the quad and summed again in the reference's order (ky-major FMA chain, bias last), at the end of its range or
+// when the list fills up; a step whose entries the list cannot take is summed again as a whole. Noted are bf16 outputs below 2**-14 of the sums in their column, where bias and products cancel, and MXFP8 blocks with a value within
 // 2**-19 of a rounding boundary of E4M3 or a maximum within a few ulp of one of the exponent rule (with normal data one
 // output in 30000 and one block in 700). INT8 codes have an absolute resolution far above the difference.
 //
@@ -57,7 +57,11 @@ constexpr int kHaloX = kTileX + 4;
 constexpr uint32_t kPixelBytes = kTileC * 2, kRowBytes = kHaloX * kPixelBytes, kChunkBytes = kStepRows * kRowBytes;
 constexpr int kTaps = 25, kMaxStages = 6;
 constexpr float kCancelled = 16384.0f;  // an output below 1 / kCancelled of the sums it comes from is summed again (bf16)
-constexpr uint32_t kListEntries = 126, kListBytes = 1024;  // {count, not finite}, then {image row, column * 32 + channel} per entry
+// The list of a quad: a header (count; not finite; flush and redo tags by step parity), then one word per entry: whole block |
+// step of the range (19 bits) | row (2) | column (5) | channel (5).
+constexpr uint32_t kListBytes = 1024, kListHeader = 64, kListEntries = (kListBytes - kListHeader) / 4, kFlushAt = 200;
+constexpr uint32_t kListTags = 16, kWholeBlock = 1u << 31;
+constexpr long long kMaxRange = 1 << 19;  // steps of a range that an entry can name
 constexpr uint32_t kWeightBytes = kTaps * kTileC * 2, kBiasBytes = kTileC * 8;
 
 enum { kOutBf16 = 0, kOutMx = 1, kOutInt8 = 2 };
@@ -183,7 +187,7 @@ __device__ __forceinline__ void multiply_step(const RowPair& upper, const RowPai
 // The pre-activation value of one output as the reference sums it: an fp32 FMA chain over the taps, ky-major, bias last.
 // `image`: the channel's first pixel, `weights`: the shared-memory address of its first tap. Five loads are in flight at a
 // time; unrolling all 25 is slower, since the code runs once and is fetched as it runs.
-__device__ __noinline__ float chain_sum(const uint16_t* image, int height, int width, int channels, uint32_t weights, float bias, int y, int x) {
+__device__ __forceinline__ float chain_sum(const uint16_t* image, int height, int width, int channels, uint32_t weights, float bias, int y, int x) {
   float sum = 0.0f;
 #pragma unroll 1
   for (int ky = 0; ky < 5; ++ky) {
@@ -208,11 +212,52 @@ __device__ __noinline__ float chain_sum(const uint16_t* image, int height, int w
   return sum + bias;
 }
 
-// Notes an output (or the block it lies in) in the quad's list. A full list drops it: the output keeps its tensor-core sum.
-__device__ __forceinline__ void note(uint32_t list, uint32_t row, uint32_t x, uint32_t channel) {
+// The same for four neighbouring columns x .. x + 3 (those outside the image are of no use), eight loads in flight.
+__device__ __forceinline__ float4 chain_sum4(const uint16_t* image, int height, int width, int channels, uint32_t weights, float bias, int y, int x) {
+  float sum[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll 1
+  for (int ky = 0; ky < 5; ++ky) {
+    const int iy = y + ky - 2;
+    const bool row_in = static_cast<unsigned>(iy) < static_cast<unsigned>(height);
+    const uint16_t* row = image + static_cast<ptrdiff_t>(row_in ? iy : y) * width * channels;
+    uint16_t v[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const int ix = x + j - 2;
+      const bool in = row_in && static_cast<unsigned>(ix) < static_cast<unsigned>(width);
+      v[j] = __ldg(row + static_cast<ptrdiff_t>(in ? ix : x) * channels);
+      v[j] = in ? v[j] : static_cast<uint16_t>(0);
+    }
+#pragma unroll
+    for (int kx = 0; kx < 5; ++kx) {
+      uint16_t w;
+      asm volatile("ld.shared.u16 %0, [%1];" : "=h"(w) : "r"(weights + (ky * 5 + kx) * (kTileC * 2)));
+#pragma unroll
+      for (int j = 0; j < 4; ++j) sum[j] = fmaf(bf16_lo(v[j + kx]), bf16_lo(w), sum[j]);
+    }
+  }
+  return make_float4(sum[0] + bias, sum[1] + bias, sum[2] + bias, sum[3] + bias);
+}
+
+// Marks of a step in its tags (one pair for even and one for odd steps): flush - the quad empties the list one step later, redo - it
+// does the whole step again then. `at`: the step's pair; `mark`: not 0, the value the readers look for.
+__device__ __forceinline__ void tag_flush(uint32_t at, uint32_t mark) {
+  asm volatile("st.shared.b32 [%0], %1;" ::"r"(at), "r"(mark) : "memory");
+}
+__device__ __forceinline__ void tag_redo(uint32_t at, uint32_t mark) {
+  asm volatile("st.shared.v2.b32 [%0], {%1, %1};" ::"r"(at), "r"(mark) : "memory");
+}
+
+// Notes an output (or the block it lies in) in the quad's list. A step whose entries do not fit is done again as a whole.
+__device__ __forceinline__ void note(uint32_t list, uint32_t tags, uint32_t mark, uint32_t entry) {
   uint32_t at;
   asm volatile("atom.shared.add.u32 %0, [%1], 1;" : "=r"(at) : "r"(list) : "memory");
-  if (at < kListEntries) asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(list + 8 + at * 8), "r"(row), "r"(x * 32 + channel) : "memory");
+  if (at < kListEntries) {
+    asm volatile("st.shared.b32 [%0], %1;" ::"r"(list + kListHeader + at * 4), "r"(entry) : "memory");
+    if (at >= kFlushAt) tag_flush(tags, mark);
+  } else {
+    tag_redo(tags, mark);
+  }
 }
 
 // max(|a|, |b|, |c|), not a number if one of them is
@@ -359,6 +404,7 @@ dw5x5_kernel(const __grid_constant__ CUtensorMap in_map, const __grid_constant__
     if (++slot == kStages) slot = 0, parity ^= 1u;
     return at;
   };
+  uint32_t number = 0;  // MX: steps begun so far
   // MX panels are filled behind the step's barrier and stored behind the next one
   int stored_x = 0, stored_y = 0, stored_c = 0, stored_b = -1;
   auto store_panel = [&](uint32_t panel, int c, int x, int y, int b) {
@@ -378,7 +424,10 @@ dw5x5_kernel(const __grid_constant__ CUtensorMap in_map, const __grid_constant__
         asm volatile("st.shared.b32 [%0], %1;" ::"r"(weights_at + i * 4), "r"(word) : "memory");
       }
       if (piece == 0) {
-        if (lane == 0) asm volatile("st.shared.v2.b32 [%0], {%1, %1};" ::"r"(list), "r"(0u) : "memory");
+        if (lane == 0) {
+          asm volatile("st.shared.v4.b32 [%0], {%1, %1, %1, %1};" ::"r"(list), "r"(0u) : "memory");
+          asm volatile("st.shared.v4.b32 [%0], {%1, %1, %1, %1};" ::"r"(list + kListTags), "r"(0u) : "memory");
+        }
         const float bias = __ldg(p.bias + c0 + lane);
         asm volatile("st.shared.v2.f32 [%0], {%1, %1};" ::"r"(bias_at + lane * 8), "f"(bias) : "memory");
       }
@@ -414,6 +463,82 @@ dw5x5_kernel(const __grid_constant__ CUtensorMap in_map, const __grid_constant__
       }
     }
 
+    // ---- the outputs in the list once more, and steps that are tagged as a whole, after the stores of their panels ----
+    const auto sum_of = [&](int b, int y, int x, int c) {
+      float bias;
+      asm volatile("ld.shared.f32 %0, [%1];" : "=f"(bias) : "r"(bias_at + c * 8));
+      return chain_sum(p.value + static_cast<size_t>(b) * p.height * p.width * p.channels + c0 + c, p.height, p.width, p.channels,
+                       weights_at + c * 2, bias, y, x);
+    };
+    // one output per lane: channel c of image row `row` (of all images one below the other); MXFP8: a warp per block, c = lane
+    const auto put = [&](uint32_t row, int px, int c, float sum) {
+      float out, unused;
+      unpack2(activate2<ACT>(pack2(sum, sum)), out, unused);
+      const size_t pixel = static_cast<size_t>(row) * p.width + px, to = pixel * p.channels + c0 + c;
+      if (MODE == kOutBf16) {
+        reinterpret_cast<uint16_t*>(p.out)[to] = static_cast<uint16_t>(pack_bf16(out, 0.0f));
+      } else if (MODE == kOutInt8) {
+        p.out[to] = static_cast<uint8_t>(int8_exact(int8.scale, bf16_lo(pack_bf16(out, 0.0f))));
+      } else {
+        // (fmaxf drops a not-a-number, as the block maximum of a step does)
+        const int e = e8m0_exponent(__uint_as_float(redux_max(__float_as_uint(fmaxf(fabsf(out), 0.0f)), 0xffffffffu)));
+        p.out[to] = static_cast<uint8_t>(e4m3x2(out * exp2_int(-e), 0.0f));
+        const int groups = p.channels >> 5;
+        if (lane == 0) p.scales[p.swizzled ? swizzled_scale_offset(pixel, ct, (groups + 3) >> 2) : pixel * groups + ct] = static_cast<uint8_t>(e + 127);
+      }
+    };
+    const auto redo_step = [&](const Position& at) {  // a row per warp, a channel per lane, four columns at a time
+      const int row = at.k0 * kStepRows + piece, x0 = at.tx * kTileX, b = at.b;
+      if (row >= p.height) return;
+      float bias;
+      asm volatile("ld.shared.f32 %0, [%1];" : "=f"(bias) : "r"(bias_at + lane * 8));
+      const uint16_t* image = p.value + static_cast<size_t>(b) * p.height * p.width * p.channels + c0 + lane;
+#pragma unroll 1
+      for (int px = x0; px < min(x0 + kTileX, p.width); px += 4) {
+        const float4 sums = chain_sum4(image, p.height, p.width, p.channels, weights_at + lane * 2, bias, row, px);
+#pragma unroll 1
+        for (int j = 0; j < min(4, p.width - px); ++j) {
+          put(b * p.height + row, px + j, lane, j == 0 ? sums.x : j == 1 ? sums.y : j == 2 ? sums.z : sums.w);
+        }
+      }
+    };
+    const auto flush = [&](int step) {  // at the end of a step (flip is already the next one's)
+      named_barrier(quad_barrier, 128);
+      if (MODE == kOutMx) {
+        if (piece == 0 && stored_b >= 0 && alive) store_panel(panels + (flip ^ 1u) * panel_bytes(MODE), stored_c, stored_x, stored_y, stored_b);
+        stored_b = -1;
+      }
+      uint32_t count, not_finite, redo, redo_before;
+      asm volatile("ld.shared.v2.b32 {%0, %1}, [%2];" : "=r"(count), "=r"(not_finite) : "r"(list) : "memory");
+      asm volatile("ld.shared.b32 %0, [%1];" : "=r"(redo) : "r"(list + kListTags + (flip ^ 1u) * 8 + 4) : "memory");
+      asm volatile("ld.shared.b32 %0, [%1];" : "=r"(redo_before) : "r"(list + kListTags + flip * 8 + 4) : "memory");
+      const bool again = redo != 0 && (MODE != kOutMx || redo == number);
+      const bool again_before = redo_before != 0 && (MODE != kOutMx || redo_before == number - 1u);
+      if ((count | not_finite) == 0 && !again && !again_before) return;
+      if (piece == 0 && elect_one()) bulk_wait_all();
+      named_barrier(quad_barrier, 128);  // (all of the quad have read the header)
+      if ((threadIdx.x & 127) == 0) {
+        asm volatile("st.shared.b32 [%0], %1;" ::"r"(list), "r"(0u) : "memory");
+        asm volatile("st.shared.v4.b32 [%0], {%1, %1, %1, %1};" ::"r"(list + kListTags), "r"(0u) : "memory");
+      }
+      if (alive) {
+        count = MODE == kOutInt8 ? 0 : min(count, kListEntries);
+#pragma unroll 1
+        for (uint32_t i = MODE == kOutMx ? piece : threadIdx.x & 127; i < count; i += MODE == kOutMx ? 4 : 128) {
+          uint32_t entry;
+          asm volatile("ld.shared.b32 %0, [%1];" : "=r"(entry) : "r"(list + kListHeader + i * 4) : "memory");
+          const Position at = position_of(p, s_begin + static_cast<int>((entry >> 12) & (kMaxRange - 1)));
+          const int row = at.k0 * kStepRows + static_cast<int>((entry >> 10) & 3u), px = at.tx * kTileX + static_cast<int>((entry >> 5) & 31u);
+          const int c = MODE == kOutMx ? lane : static_cast<int>(entry & 31u);
+          put(at.b * p.height + row, px, c, sum_of(at.b, row, px, c));
+        }
+        const bool all = not_finite != 0 && step + 1 == s_end;
+#pragma unroll 1
+        for (int s = all ? s_begin : again_before ? step - 1 : step; s <= (all || again ? step : step - 1); ++s) redo_step(position_of(p, s));
+      }
+      named_barrier(quad_barrier, 128);  // the entries have been read before new ones are noted
+    };
+
     for (int s = s_begin; s < s_end;) {
       const Position at = position_of(p, s);
       const int len = min(p.strip_steps - at.k0, s_end - s);
@@ -430,6 +555,17 @@ dw5x5_kernel(const __grid_constant__ CUtensorMap in_map, const __grid_constant__
       }
       for (int k = 0; k < len; ++k) {
         const int y = (at.k0 + k) * kStepRows;
+        const int step = s - len + k;
+        const uint32_t entry = static_cast<uint32_t>(step - s_begin) << 12 | static_cast<uint32_t>(lane) << 5;  // + row * 1024 + channel
+        // The flush tag of the step before, in which all warps have to see the same. Dense and INT8 steps are noted ahead of their
+        // barrier: the tag is read ahead of the next one, and the step after this one, which uses its place again, begins behind
+        // that. MXFP8 steps are noted behind their barrier as well: the tag is read behind the next one, and a warp that is ahead may
+        // have left the mark of the step after this one, which differs. (It then found no mark, and nor does this warp.)
+        if (MODE == kOutMx) ++number;
+        const uint32_t mark = MODE == kOutMx ? number : 1u, tags = list + kListTags + flip * 8, tags_before = list + kListTags + (flip ^ 1u) * 8;
+        uint32_t tag = 0;
+        const auto read_tag = [&]() { asm volatile("ld.shared.b32 %0, [%1];" : "=r"(tag) : "r"(tags_before) : "memory"); };
+        if (MODE != kOutMx) read_tag();
         const uint32_t from = take_chunk();
         const uint32_t panel = panels + flip * panel_bytes(MODE);
         float acc[8][4];
@@ -498,7 +634,7 @@ dw5x5_kernel(const __grid_constant__ CUtensorMap in_map, const __grid_constant__
 #pragma unroll 1
           for (; cancelled != 0; cancelled &= cancelled - 1) {
             const int bit = __ffs(cancelled) - 1, row = y + (bit & 3);
-            if (x < p.width && row < p.height) note(list, at.b * p.height + row, x, piece * 8 + (bit >> 2));
+            if (x < p.width && row < p.height) note(list, tags, mark, entry + (bit & 3) * 1024 + piece * 8 + (bit >> 2));
           }
         }
 #pragma unroll
@@ -544,6 +680,7 @@ dw5x5_kernel(const __grid_constant__ CUtensorMap in_map, const __grid_constant__
             if (alive) issue_until(taken + kStages);
           }
           stored_c = c0, stored_x = x0, stored_y = y, stored_b = p.tma_out ? at.b : -1;
+          read_tag();
           float theirs[3][4];
 #pragma unroll
           for (int other = 1; other < 4; ++other) {
@@ -591,8 +728,8 @@ dw5x5_kernel(const __grid_constant__ CUtensorMap in_map, const __grid_constant__
           if (unsure != 0) {
 #pragma unroll 1
             for (; unsure != 0; unsure &= unsure - 1) {
-              const int row = y + __ffs(unsure) - 1;
-              if (x < p.width && row < p.height) note(list, at.b * p.height + row, x, 0);
+              const int i = __ffs(unsure) - 1;
+              if (x < p.width && y + i < p.height) note(list, tags, mark, kWholeBlock | (entry + i * 1024));
             }
           }
         } else {
@@ -647,62 +784,7 @@ dw5x5_kernel(const __grid_constant__ CUtensorMap in_map, const __grid_constant__
           }
         }
         flip ^= 1u;
-      }
-    }
-    if (MODE == kOutMx) {  // the last panel
-      named_barrier(quad_barrier, 128);
-      if (piece == 0 && stored_b >= 0 && alive) store_panel(panels + (flip ^ 1u) * panel_bytes(MODE), stored_c, stored_x, stored_y, stored_b);
-      stored_b = -1;
-    }
-    {
-      // the outputs in the list once more, after the stores of their panels have completed
-      named_barrier(quad_barrier, 128);
-      uint32_t count, not_finite;
-      asm volatile("ld.shared.v2.b32 {%0, %1}, [%2];" : "=r"(count), "=r"(not_finite) : "r"(list));
-      count = min(count, kListEntries);
-      if ((count | not_finite) != 0) {
-        if (piece == 0 && elect_one()) bulk_wait_all();
-        named_barrier(quad_barrier, 128);
-      }
-      if (!alive) count = not_finite = 0;
-      // one output (MXFP8: a warp per block, lane = channel) of image row `row` (of all images one below the other)
-      const auto again = [&](uint32_t row, int px, int c) {
-        const int b = row / p.height, y = row - b * p.height;
-        float bias;
-        asm volatile("ld.shared.f32 %0, [%1];" : "=f"(bias) : "r"(bias_at + c * 8));
-        const float sum = chain_sum(p.value + static_cast<size_t>(b) * p.height * p.width * p.channels + c0 + c, p.height, p.width, p.channels,
-                                    weights_at + c * 2, bias, y, px);
-        float out, unused;
-        unpack2(activate2<ACT>(pack2(sum, sum)), out, unused);
-        const size_t pixel = static_cast<size_t>(row) * p.width + px, to = pixel * p.channels + c0 + c;
-        if (MODE == kOutBf16) {
-          reinterpret_cast<uint16_t*>(p.out)[to] = static_cast<uint16_t>(pack_bf16(out, 0.0f));
-        } else if (MODE == kOutInt8) {
-          p.out[to] = static_cast<uint8_t>(int8_pack2(int8, bf16_lo(pack_bf16(out, 0.0f)), 0.0f));
-        } else {
-          // (fmaxf drops a not-a-number, as the block maximum above does)
-          const int e = e8m0_exponent(__uint_as_float(redux_max(__float_as_uint(fmaxf(fabsf(out), 0.0f)), 0xffffffffu)));
-          p.out[to] = static_cast<uint8_t>(e4m3x2(out * exp2_int(-e), 0.0f));
-          const int groups = p.channels >> 5;
-          if (lane == 0) p.scales[p.swizzled ? swizzled_scale_offset(pixel, ct, (groups + 3) >> 2) : pixel * groups + ct] = static_cast<uint8_t>(e + 127);
-        }
-      };
-      if (not_finite != 0) {
-        for (int s = s_begin; s < s_end;) {
-          const Position at = position_of(p, s);
-          const int len = min(p.strip_steps - at.k0, s_end - s), y0 = at.k0 * kStepRows, x0 = at.tx * kTileX;
-          s += len;
-          const int rows = min(len * kStepRows, p.height - y0), columns = min(kTileX, p.width - x0);
-#pragma unroll 1
-          for (int i = piece; i < rows * columns; i += 4) again(at.b * p.height + y0 + i / columns, x0 + i % columns, lane);
-        }
-      } else if (MODE != kOutInt8) {
-#pragma unroll 1
-        for (uint32_t i = MODE == kOutMx ? piece : threadIdx.x & 127; i < count; i += MODE == kOutMx ? 4 : 128) {
-          uint32_t row, place;
-          asm volatile("ld.shared.v2.b32 {%0, %1}, [%2];" : "=r"(row), "=r"(place) : "r"(list + 8 + i * 8));
-          again(row, place >> 5, MODE == kOutMx ? lane : place & 31);
-        }
+        if ((tag != 0 && (MODE != kOutMx || tag == number - 1u)) || step + 1 == s_end) flush(step);
       }
     }
   }
@@ -792,6 +874,7 @@ int launch(const void* value, const void* weight, const float* bias, void* out, 
   const long long most_groups = sms * kQuads / p.group_quads;
   p.groups = static_cast<int>(steps < most_groups ? steps : most_groups);
   const int quads = p.groups * p.group_quads;
+  if (steps / p.groups >= kMaxRange) return kUnsupported;  // (on a whole GPU a tensor of more than its memory)
   p.cta_quads = ceil_div(quads, sms);
   const unsigned grid = static_cast<unsigned>(ceil_div(quads, p.cta_quads));
   return launch_kernel<MODE>(in_map, out_map, p, act, grid, static_cast<cudaStream_t>(stream));
