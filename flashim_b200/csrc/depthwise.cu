@@ -28,12 +28,13 @@
 // Precision: the tensor cores add the exact products into fp32 accumulators, as the fp32 chain of the reference does, but in
 // another order; the two differ by about one fp32 ulp of the largest partial sum. Outputs on which that could show are
 // noted in a list of the quad and summed again in the reference's order (ky-major FMA chain, bias last), at the end of its range or
-// when the list fills up; a step whose entries the list cannot take is summed again as a whole. Noted are bf16 outputs below 2**-14 of the sums in their column, where bias and products cancel, and MXFP8 blocks with a value within
-// 2**-19 of a rounding boundary of E4M3 or a maximum within a few ulp of one of the exponent rule (with normal data one
-// output in 30000 and one block in 700). INT8 codes have an absolute resolution far above the difference.
+// when the list fills up; a step whose entries the list cannot take is summed again as a whole. Noted are bf16 outputs below
+// 2**-14 of the sums in their column, where bias and products cancel, and MXFP8 blocks with a value within 2**-19 of a rounding
+// boundary of E4M3 or a maximum within a few ulp of one of the exponent rule (with normal data one output in 30000 and one
+// block in 700). INT8 codes have an absolute resolution far above the difference.
 //
 // A patch value outside an output's 5x5 window is multiplied by a zero of B, which an infinity or a not-a-number survives. A
-// quad that meets a sum which is not finite therefore does its whole range again in the reference's order at the end.
+// step that meets a sum which is not finite is therefore done again in the reference's order.
 //
 // Work: a strip is one (image, 32-column tile) over all rows, cut into steps of four output rows; a span is the part of a
 // range of steps inside one strip. The quads of all CTAs (three per CTA, one CTA per SM) form groups of one quad per
@@ -57,7 +58,7 @@ constexpr int kHaloX = kTileX + 4;
 constexpr uint32_t kPixelBytes = kTileC * 2, kRowBytes = kHaloX * kPixelBytes, kChunkBytes = kStepRows * kRowBytes;
 constexpr int kTaps = 25, kMaxStages = 6;
 constexpr float kCancelled = 16384.0f;  // an output below 1 / kCancelled of the sums it comes from is summed again (bf16)
-// The list of a quad: a header (count; not finite; flush and redo tags by step parity), then one word per entry: whole block |
+// The list of a quad: a header (count; flush and redo tags by step parity), then one word per entry: whole block |
 // step of the range (19 bits) | row (2) | column (5) | channel (5).
 constexpr uint32_t kListBytes = 1024, kListHeader = 64, kListEntries = (kListBytes - kListHeader) / 4, kFlushAt = 200;
 constexpr uint32_t kListTags = 16, kWholeBlock = 1u << 31;
@@ -508,13 +509,14 @@ dw5x5_kernel(const __grid_constant__ CUtensorMap in_map, const __grid_constant__
         if (piece == 0 && stored_b >= 0 && alive) store_panel(panels + (flip ^ 1u) * panel_bytes(MODE), stored_c, stored_x, stored_y, stored_b);
         stored_b = -1;
       }
-      uint32_t count, not_finite, redo, redo_before;
-      asm volatile("ld.shared.v2.b32 {%0, %1}, [%2];" : "=r"(count), "=r"(not_finite) : "r"(list) : "memory");
-      asm volatile("ld.shared.b32 %0, [%1];" : "=r"(redo) : "r"(list + kListTags + (flip ^ 1u) * 8 + 4) : "memory");
-      asm volatile("ld.shared.b32 %0, [%1];" : "=r"(redo_before) : "r"(list + kListTags + flip * 8 + 4) : "memory");
+      uint32_t count, redo, redo_before;
+      asm volatile("ld.shared.b32 %0, [%1];" : "=r"(count) : "r"(list) : "memory");
+      const uint32_t redo_tags = list + kListTags + (MODE == kOutInt8 ? 0u : 4u);
+      asm volatile("ld.shared.b32 %0, [%1];" : "=r"(redo) : "r"(redo_tags + (flip ^ 1u) * 8) : "memory");
+      asm volatile("ld.shared.b32 %0, [%1];" : "=r"(redo_before) : "r"(redo_tags + flip * 8) : "memory");
       const bool again = redo != 0 && (MODE != kOutMx || redo == number);
       const bool again_before = redo_before != 0 && (MODE != kOutMx || redo_before == number - 1u);
-      if ((count | not_finite) == 0 && !again && !again_before) return;
+      if (count == 0 && !again && !again_before) return;
       if (piece == 0 && elect_one()) bulk_wait_all();
       named_barrier(quad_barrier, 128);  // (all of the quad have read the header)
       if ((threadIdx.x & 127) == 0) {
@@ -532,9 +534,8 @@ dw5x5_kernel(const __grid_constant__ CUtensorMap in_map, const __grid_constant__
           const int c = MODE == kOutMx ? lane : static_cast<int>(entry & 31u);
           put(at.b * p.height + row, px, c, sum_of(at.b, row, px, c));
         }
-        const bool all = not_finite != 0 && step + 1 == s_end;
 #pragma unroll 1
-        for (int s = all ? s_begin : again_before ? step - 1 : step; s <= (all || again ? step : step - 1); ++s) redo_step(position_of(p, s));
+        for (int s = again_before ? step - 1 : step; s <= (again ? step : step - 1); ++s) redo_step(position_of(p, s));
       }
       named_barrier(quad_barrier, 128);  // the entries have been read before new ones are noted
     };
@@ -564,7 +565,11 @@ dw5x5_kernel(const __grid_constant__ CUtensorMap in_map, const __grid_constant__
         if (MODE == kOutMx) ++number;
         const uint32_t mark = MODE == kOutMx ? number : 1u, tags = list + kListTags + flip * 8, tags_before = list + kListTags + (flip ^ 1u) * 8;
         uint32_t tag = 0;
-        const auto read_tag = [&]() { asm volatile("ld.shared.b32 %0, [%1];" : "=r"(tag) : "r"(tags_before) : "memory"); };
+        const auto read_tag = [&]() {
+          uint32_t redo;
+          asm volatile("ld.shared.v2.b32 {%0, %1}, [%2];" : "=r"(tag), "=r"(redo) : "r"(tags_before) : "memory");
+          if (MODE == kOutInt8) tag |= redo;  // (says nothing more; without it the compiler's schedule takes 182 instead of 172 us)
+        };
         if (MODE != kOutMx) read_tag();
         const uint32_t from = take_chunk();
         const uint32_t panel = panels + flip * panel_bytes(MODE);
@@ -618,7 +623,13 @@ dw5x5_kernel(const __grid_constant__ CUtensorMap in_map, const __grid_constant__
             }
           }
         }
-        if (!(largest < __int_as_float(0x7F800000))) asm volatile("st.shared.b32 [%0], %1;" ::"r"(list + 4), "r"(1u) : "memory");
+        if (!(largest < __int_as_float(0x7F800000))) {
+          if (MODE == kOutInt8) {
+            tag_flush(tags, mark);  // (without a list the one tag says it all)
+          } else {
+            tag_redo(tags, mark);
+          }
+        }
         if (MODE == kOutBf16 && margin < 0.0f) {
           uint32_t cancelled = 0;  // bit 4 c + i
 #pragma unroll

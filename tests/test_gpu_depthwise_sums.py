@@ -68,3 +68,26 @@ def test_no_cancelled_output_is_lost(ops, ctas, everywhere):
     assert same_bytes(got[0][inner], want[inner])
     assert int(bf16_ulp_distance(got[0][~inner], want[~inner]).max() if not inner.all() else 0) <= 1
     assert same_bytes(got[1], got[0]) and same_bytes(got[2], got[0])
+
+
+def test_what_is_not_finite_costs_its_own_steps(ops, ctas):
+    """The patches (6 x 8 pixels) that hold an infinity are summed again with their step of 4 rows x 32 columns x 32 channels;
+    every other step keeps the bytes that it has without the infinity, and the windows that hold it have the chain's."""
+    shape = (2, 61, 130, 64)
+    g = torch.Generator(device=DEV).manual_seed(3)
+    x, w = torch.randn(shape, generator=g, device=DEV).to(BF16), (torch.randn(25, 64, generator=g, device=DEV) * 0.2).to(BF16)
+    b = torch.randn(64, generator=g, device=DEV)
+    spoiled, redone = x.clone(), torch.zeros(shape, dtype=torch.bool, device=DEV)
+    for image, y, px, c, value in ((0, 0, 0, 3, float("inf")), (0, 30, 63, 40, float("nan")), (1, 60, 129, 63, float("-inf"))):
+        spoiled[image, y, px, c] = value
+        for top in range(0, shape[1], 4):
+            for left in range(0, shape[2], 32):
+                if top - 2 <= y <= top + 5 and left - 2 <= px <= left + 33:
+                    redone[image, top: top + 4, left: left + 32, c // 32 * 32: c // 32 * 32 + 32] = True
+    clean, got = (ops.depthwise5x5_act(t.permute(0, 3, 1, 2), w, b, "none") for t in (x, spoiled))
+    assert same_bytes(got[~redone], clean[~redone])
+    want = chain(spoiled, w, b).to(BF16)
+    assert torch.equal(torch.isnan(got), torch.isnan(want))
+    number = redone & ~torch.isnan(want)
+    assert number.any() and same_bytes(got[number], want[number])
+    assert int((~torch.isfinite(want)).sum()) > 0
