@@ -19,19 +19,25 @@
 //     or 16 bytes per pixel from registers instead costs a shared-memory wavefront per lane.
 //
 // Measured against the fp32-pipe kernel before it (B200, inputs in L2 where they fit):
-//   4x200x200x256: GELU -> bf16 68 -> 52 us, ReLU -> bf16 54 -> 41, GELU -> MXFP8 88 -> 70, ReLU -> INT8 87 -> 49
-//   8x400x400x128: GELU -> bf16 232 -> 165, ReLU -> bf16 183 -> 125 (80 % of the HBM copy rate), GELU -> MXFP8 303 -> 225,
-//   ReLU -> MXFP8 252 -> 178, ReLU -> INT8 299 -> 159
+//   4x200x200x256: GELU -> bf16 68 -> 52 us, ReLU -> bf16 54 -> 41, GELU -> MXFP8 88 -> 82, ReLU -> INT8 87 -> 50
+//   8x400x400x128: GELU -> bf16 232 -> 162, ReLU -> bf16 183 -> 124 (80 % of the HBM copy rate), GELU -> MXFP8 303 -> 274,
+//   ReLU -> MXFP8 252 -> 191, ReLU -> INT8 299 -> 165
 // What bounds the GELU and quantising forms now is the arithmetic of their epilogues on twelve warps per SM (issue slots about
-// half busy); the care for equal results (below) is a quarter of the MXFP8 form's time.
+// half busy). The same bytes as the chain (below) cost the MXFP8 form up to a quarter of its time: 225 and 178 us with a test that
+// missed half of the codes that differ. Arguments of the GELU that reach its left tail take 350 us.
 //
-// Precision: the tensor cores add the exact products into fp32 accumulators, as the fp32 chain of the reference does, but in
-// another order; the two differ by about one fp32 ulp of the largest partial sum. Outputs on which that could show are
-// noted in a list of the quad and summed again in the reference's order (ky-major FMA chain, bias last), at the end of its range or
-// when the list fills up; a step whose entries the list cannot take is summed again as a whole. Noted are bf16 outputs below
-// 2**-14 of the sums in their column, where bias and products cancel, and MXFP8 blocks with a value within 2**-19 of a rounding
-// boundary of E4M3 or a maximum within a few ulp of one of the exponent rule (with normal data one output in 30000 and one
-// block in 700). INT8 codes have an absolute resolution far above the difference.
+// Precision: the tensor cores add the exact products into fp32 accumulators, as the fp32 chain of the reference does (ky-major FMA
+// chain, bias last), but in another order; the two differ by up to about two fp32 ulp of the largest partial sum.
+//   MXFP8: the bytes of the chain. Every value has two bounds, itself less and plus the largest difference (error_of); where their
+//     codes differ (with normal data one in 2000) the output is summed again in the chain's order, at once and from shared memory.
+//     Where the exponents of the two bounds of a block's maximum differ, the block is noted in a list of the quad. No code or scale
+//     differed in 2.5 G of normal, wide and sparse data.
+//   bf16: outputs below 2**-14 of the sums in their column, where bias and products cancel, are noted (one in 30000). Others may
+//     lie one ulp of bf16 from the chain's where its sum lies next to a rounding boundary: one in 200000.
+//   INT8: likewise a code may lie one from the chain's: one in 4000000.
+// The outputs and blocks of a list are summed again in the chain's order at the end of the quad's range or when the list fills up; a
+// step with more of them than the list takes, or with more open codes than is worth correcting one by one, is summed again as a
+// whole.
 //
 // A patch value outside an output's 5x5 window is multiplied by a zero of B, which an infinity or a not-a-number survives. A
 // step that meets a sum which is not finite is therefore done again in the reference's order.
@@ -58,11 +64,21 @@ constexpr int kHaloX = kTileX + 4;
 constexpr uint32_t kPixelBytes = kTileC * 2, kRowBytes = kHaloX * kPixelBytes, kChunkBytes = kStepRows * kRowBytes;
 constexpr int kTaps = 25, kMaxStages = 6;
 constexpr float kCancelled = 16384.0f;  // an output below 1 / kCancelled of the sums it comes from is summed again (bf16)
-// The list of a quad: a header (count; flush and redo tags by step parity), then one word per entry: whole block |
-// step of the range (19 bits) | row (2) | column (5) | channel (5).
-constexpr uint32_t kListBytes = 1024, kListHeader = 64, kListEntries = (kListBytes - kListHeader) / 4, kFlushAt = 200;
-constexpr uint32_t kListTags = 16, kWholeBlock = 1u << 31;
-constexpr long long kMaxRange = 1 << 19;  // steps of a range that an entry can name
+// MXFP8: how far a tensor-core sum may lie from the fp32 chain, as a share of the size that error_of forms: 2**-20.75. The largest
+// difference in 46 M outputs of each of 14 kinds of data (normal, ReLU'd, positive, log-normal, smooth and flat images; random,
+// positive, zero-sum, Laplacian and Sobel taps) was 2**-21.35 of it; at most one output in 100000 passed 2**-22.
+constexpr float kSumError = 5.67e-7f;
+// The GELU passes on less than kGeluSlope of an argument's error (|GELU'| <= 1.129), and less than kGeluBase + kGeluGrowth * GELU
+// (|GELU'| <= 0.5 + 1.6 GELU for every argument); both with a tenth for the rounding of the polynomial.
+constexpr float kGeluSlope = 1.25f, kGeluBase = 0.55f, kGeluGrowth = 1.76f;
+// open codes that a warp corrects one by one (about 450 cycles each); with more of them the quad does the step again (20000)
+constexpr int kMostOpen = 32;
+// The list of a quad: a header (count; flush and redo tags by step parity; MXFP8: error bounds of the four warps by step parity,
+// their largest taps and biases), then one word per entry: step of the range (20 bits) | row (2) | column (5) | channel (5; MXFP8:
+// 0, for a block).
+constexpr uint32_t kListBytes = 1024, kListHeader = 96, kListEntries = (kListBytes - kListHeader) / 4, kFlushAt = 200;
+constexpr uint32_t kListTags = 16, kListErrors = 32, kListSizes = 64;
+constexpr long long kMaxRange = 1 << 20;  // steps of a range that an entry can name
 constexpr uint32_t kWeightBytes = kTaps * kTileC * 2, kBiasBytes = kTileC * 8;
 
 enum { kOutBf16 = 0, kOutMx = 1, kOutInt8 = 2 };
@@ -74,6 +90,8 @@ enum { kOutBf16 = 0, kOutMx = 1, kOutInt8 = 2 };
 __host__ __device__ constexpr uint32_t panel_bytes(int mode) { return mode == kOutBf16 ? 8192u : 4096u; }
 __host__ __device__ constexpr uint32_t exchange_bytes(int mode) { return mode == kOutMx ? 4096u : 0u; }
 __host__ __device__ constexpr bool shared_fragments(int mode) { return mode == kOutMx; }
+// chunks of the ring that are kept after their products: MXFP8 corrects codes from the two of the step (it has two on the way then)
+__host__ __device__ constexpr uint32_t kept_chunks(int mode) { return mode == kOutMx ? 2u : 0u; }
 __host__ __device__ constexpr int stages(int mode) { return shared_fragments(mode) ? 4 : kMaxStages; }
 __host__ __device__ constexpr uint32_t fragment_bytes(int mode) { return shared_fragments(mode) ? 4u * 12u * 512u : 0u; }
 __host__ __device__ constexpr uint32_t quad_bytes(int mode) {
@@ -146,6 +164,13 @@ __device__ __forceinline__ void mma_16x8x16(float (&d)[4], uint32_t a0, uint32_t
   }
 }
 
+// max(|m|, |a|, |b|)
+__device__ __forceinline__ float max_abs(float m, float a, float b) {
+  float r;
+  asm("max.abs.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(m), "f"(a), "f"(b));
+  return r;
+}
+
 // Two image rows of the patch for 8 channels, as A operands: [channel][row], patch columns q and q + 4 in one register.
 // `at`: the lane's pixel in the upper row, its 16-byte piece chosen by the swizzle; in the odd row and four columns on, the
 // swizzle phase differs in one bit.
@@ -165,6 +190,18 @@ __device__ __forceinline__ void load_pair(uint32_t at, RowPair& p) {
     p.a[2 * j][1] = __byte_perm(v[2][j], v[3][j], 0x5410);
     p.a[2 * j + 1][1] = __byte_perm(v[2][j], v[3][j], 0x7632);
   }
+}
+
+// The largest magnitude of columns q + 4 in two row pairs, or `big`. As fp32 numbers the words are the values of their upper halves (and
+// up to 2**-7 of them more), three to an instruction; packed bf16 maxima take five times as long.
+__device__ __forceinline__ float size_of(const RowPair& p, const RowPair& q, float big) {
+  float other = 0.0f;
+#pragma unroll
+  for (int c = 0; c < 8; ++c) {
+    asm volatile("max.abs.f32 %0, %0, %1, %2;" : "+f"(big) : "f"(__uint_as_float(p.a[c][0])), "f"(__uint_as_float(p.a[c][1])));
+    asm volatile("max.abs.f32 %0, %0, %1, %2;" : "+f"(other) : "f"(__uint_as_float(q.a[c][0])), "f"(__uint_as_float(q.a[c][1])));
+  }
+  return fmaxf(big, other);
 }
 
 // One K step for the 8 channels: the upper blocks (M rows 0-7) see row pair `upper` of the patch, the blocks below them the
@@ -273,31 +310,53 @@ __device__ __forceinline__ float min_abs(float a, float b, float c) {
   asm("min.abs.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
   return r;
 }
-// max(|m|, |a|, |b|)
-__device__ __forceinline__ float max_abs(float m, float a, float b) {
+__device__ __forceinline__ float max3(float m, float a, float b) {
   float r;
-  asm("max.abs.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(m), "f"(a), "f"(b));
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(m), "f"(a), "f"(b));
   return r;
 }
+// the largest of numbers that are not negative (or a not-a-number), over the warp
+__device__ __forceinline__ float warp_max(float v) { return __uint_as_float(redux_max(__float_as_uint(v), 0xffffffffu)); }
 
-// E8M0 bytes and the factors 2**-e of four block maxima: e = E - 8 + (mantissa > 1.75), one carry away from the exponent field,
-// unless one of them lies in the window where the reference's rule departs from that or is not finite. Returns a bit per
-// maximum that lies in that window or within 8 ulp of it (one block in 150000).
-__device__ __forceinline__ uint32_t block_scales(const float (&amax)[4], uint32_t (&bytes)[4], float (&inv)[4]) {
+// four E4M3 codes, of max(value, 0) for a ReLU
+template <int ACT>
+__device__ __forceinline__ uint32_t codes_of(float a, float b, float c, float d) {
+  if (ACT != kActRelu) return e4m3x4(a, b, c, d);
+  uint16_t lo, hi;
+  asm("cvt.rn.satfinite.relu.e4m3x2.f32 %0, %1, %2;" : "=h"(lo) : "f"(b), "f"(a));
+  asm("cvt.rn.satfinite.relu.e4m3x2.f32 %0, %1, %2;" : "=h"(hi) : "f"(d), "f"(c));
+  return static_cast<uint32_t>(lo) | (static_cast<uint32_t>(hi) << 16);
+}
+
+// Bound on the difference between a sum of the tensor cores plus bias and the same of the fp32 chain. Both err by ulps of
+// their partial sums. `size` is the largest |sum| of the warp or twice the largest product that its patches can hold, whichever is
+// larger: where all sums cancel (flat areas under taps that sum to zero) only the second bounds the partial sums. The bias adds a
+// rounding to an ulp of the result. Sums of zeros are equal. Near the subnormals ulps no longer shrink with the sums: nothing is
+// assumed there.
+__device__ __forceinline__ float error_of(float size, float bias) {
+  const float total = fmaxf(size, bias);
+  return size == 0.0f ? 0.0f : total < 1e-30f ? total : total * kSumError;
+}
+
+// E8M0 bytes and the factors 2**-e of four block maxima that are known to within `error`: e = E - 8 + (mantissa > 1.75), one
+// carry away from the exponent field, unless one of them lies in the window above 1.75 where the reference's rule departs from
+// that, is not finite, or the exponents of its two bounds differ. Returns a bit per maximum whose exponent is open.
+__device__ __forceinline__ uint32_t block_scales(const float (&amax)[4], float error, uint32_t (&bytes)[4], float (&inv)[4]) {
   uint32_t unsure = 0;
   bool rare = false;
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
-    const uint32_t bits = __float_as_uint(amax[i]);
-    bytes[i] = static_cast<uint32_t>(max(static_cast<int>((bits + 0x1FFFFFu) >> 23) - 8, 0));
+    const uint32_t low = __float_as_uint(fmaxf(amax[i] - error, 0.0f)), high = __float_as_uint(fmaxf(amax[i] + error, 0.0f));
+    const uint32_t byte = (high + 0x1FFFFFu) >> 23;
+    bytes[i] = static_cast<uint32_t>(max(static_cast<int>(byte) - 8, 0));
     inv[i] = __uint_as_float((254u - bytes[i]) << 23);
-    rare |= ((bits & 0x7FFFFFu) - 0x5FFFF8u) < 57u || bits >= 0x7F800000u;
+    rare |= ((low + 0x1FFFFFu) >> 23) != byte || ((low & 0x7FFFFFu) - 0x600001u) < 41u || high >= 0x7F800000u;
   }
   if (rare) {
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-      if (((__float_as_uint(amax[i]) & 0x7FFFFFu) - 0x5FFFF8u) < 57u) unsure |= 1u << i;
-      const int e = e8m0_exponent(amax[i]);
+      const int e = e8m0_exponent(fmaxf(amax[i] + error, 0.0f));
+      if (e8m0_exponent(fmaxf(amax[i] - error, 0.0f)) != e) unsure |= 1u << i;
       bytes[i] = static_cast<uint32_t>(e + 127);
       inv[i] = exp2_int(-e);
     }
@@ -395,6 +454,9 @@ dw5x5_kernel(const __grid_constant__ CUtensorMap in_map, const __grid_constant__
   constexpr int kOutBytes = MODE == kOutBf16 ? 2 : 1;
   const uint32_t turn = static_cast<uint32_t>(piece ^ ((lane >> 1) & 3)) << 4;  // the 16-byte piece under the swizzle
   const uint32_t lane_at = ring + lane * kPixelBytes + turn;
+  // from there to the lane's share of columns 0 - 3 of a chunk: row lane / 8, column lane / 2 % 4, four channels
+  const uint32_t first_pixel = (lane >> 3) * kHaloX + ((lane >> 1) & 3);
+  const uint32_t first_at = first_pixel * kPixelBytes + (((piece ^ (first_pixel >> 1)) & 3u) << 4) + (lane & 1) * 8 - (lane * kPixelBytes + turn);
 
   uint32_t taken = 0, slot = 0, parity = 0, flip = 0;  // chunks taken so far, the next one's ring position; panel in use
   bool alive = true;
@@ -433,6 +495,17 @@ dw5x5_kernel(const __grid_constant__ CUtensorMap in_map, const __grid_constant__
         asm volatile("st.shared.v2.f32 [%0], {%1, %1};" ::"r"(bias_at + lane * 8), "f"(bias) : "memory");
       }
       named_barrier(quad_barrier, 128);
+      if (MODE == kOutMx) {  // the largest |tap| and |bias| of the warp's channels
+        uint32_t tap[4] = {};
+        if (lane < kTaps) lds128(weights_at + lane * (kTileC * 2) + piece * 16, tap);
+        float bias, size = 0.0f;
+        asm volatile("ld.shared.f32 %0, [%1];" : "=f"(bias) : "r"(bias_at + (piece * 8 + (lane & 7)) * 8));
+#pragma unroll
+        for (int j = 0; j < 4; ++j) size = max_abs(size, bf16_lo(tap[j]), bf16_hi(tap[j]));
+        const float largest_tap = warp_max(size), largest_bias = warp_max(fabsf(bias));
+        if (lane == 0) asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(list + kListSizes + piece * 8), "f"(largest_tap), "f"(largest_bias) : "memory");
+        __syncwarp();
+      }
       // B[k][n] = w[row - dy][column - dx] for patch position k = (row, column) and output pixel n = (dx, dy), else 0; this
       // lane holds columns q and q + 4 of pixel n
       const int q = lane & 3, dx = lane >> 3, dy = (lane >> 2) & 1;
@@ -529,7 +602,7 @@ dw5x5_kernel(const __grid_constant__ CUtensorMap in_map, const __grid_constant__
         for (uint32_t i = MODE == kOutMx ? piece : threadIdx.x & 127; i < count; i += MODE == kOutMx ? 4 : 128) {
           uint32_t entry;
           asm volatile("ld.shared.b32 %0, [%1];" : "=r"(entry) : "r"(list + kListHeader + i * 4) : "memory");
-          const Position at = position_of(p, s_begin + static_cast<int>((entry >> 12) & (kMaxRange - 1)));
+          const Position at = position_of(p, s_begin + static_cast<int>(entry >> 12));
           const int row = at.k0 * kStepRows + static_cast<int>((entry >> 10) & 3u), px = at.tx * kTileX + static_cast<int>((entry >> 5) & 31u);
           const int c = MODE == kOutMx ? lane : static_cast<int>(entry & 31u);
           put(at.b * p.height + row, px, c, sum_of(at.b, row, px, c));
@@ -548,11 +621,19 @@ dw5x5_kernel(const __grid_constant__ CUtensorMap in_map, const __grid_constant__
       // (rows of the scale matrix fit 32 bits: one more would be 256 GB of input)
       const uint32_t scale_row = (static_cast<uint32_t>(at.b) * p.height + piece) * p.width + x;
       const uint32_t scale_tile_bytes = ((p.channels >> 5) + 3) / 4 * 512, scale_at = (ct >> 2) * 512 + (ct & 3);
+      // MX: the largest |value| of four channels of a pixel in the first four columns of a chunk, which size_of leaves out
+      const auto first_columns = [&](uint32_t from) {
+        uint32_t v[2];
+        asm volatile("ld.shared.v2.b32 {%0, %1}, [%2];" : "=r"(v[0]), "=r"(v[1]) : "r"(from + first_at));
+        return max_abs(max_abs(0.0f, bf16_lo(v[0]), __uint_as_float(v[0])), bf16_lo(v[1]), __uint_as_float(v[1]));
+      };
       RowPair r0, r1;  // the two row pairs above the ones a step brings
+      float size_above = 0.0f;  // MX: the largest |value| that the lane has seen of their chunk
       {
         const uint32_t from = take_chunk();
         load_pair(from, r0);
         load_pair(from + 2 * kRowBytes, r1);
+        if (MODE == kOutMx) size_above = size_of(r0, r1, first_columns(from));
       }
       for (int k = 0; k < len; ++k) {
         const int y = (at.k0 + k) * kStepRows;
@@ -574,7 +655,13 @@ dw5x5_kernel(const __grid_constant__ CUtensorMap in_map, const __grid_constant__
         const uint32_t from = take_chunk();
         const uint32_t panel = panels + flip * panel_bytes(MODE);
         float acc[8][4];
+        float size_product = 0.0f, largest_tap = 0.0f, largest_bias = 0.0f;  // MX: twice the largest product that the lane knows of
         {
+          float first = 0.0f;
+          if (MODE == kOutMx) {
+            first = first_columns(from);
+            asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(largest_tap), "=f"(largest_bias) : "r"(list + kListSizes + piece * 8));
+          }
           RowPair r2;
           const auto multiply = [&](auto first, const RowPair& upper, const RowPair& lower, int st) {
             if constexpr (shared_fragments(MODE)) {
@@ -589,6 +676,12 @@ dw5x5_kernel(const __grid_constant__ CUtensorMap in_map, const __grid_constant__
           r0 = r2;
           load_pair(from + 2 * kRowBytes, r1);
           multiply(std::false_type{}, r0, r1, 2);
+          if (MODE == kOutMx) {
+            const float size = size_of(r0, r1, first), both = fmaxf(size, size_above);
+            size_product = 2.0f * largest_tap * both;
+            if (size_product < 1e-36f && largest_tap > 0.0f && both > 0.0f) size_product = 1e-36f;  // (underflow)
+            size_above = size;
+          }
         }
         // bias and activation: v[channel][0 / 1] = rows (0, 1) / (2, 3) of the lane's column
         uint64_t v[8][2];
@@ -623,7 +716,14 @@ dw5x5_kernel(const __grid_constant__ CUtensorMap in_map, const __grid_constant__
             }
           }
         }
-        if (!(largest < __int_as_float(0x7F800000))) {
+        float error = 0.0f;  // MX: a bound on the error of the warp's arguments
+        float limit = __int_as_float(0x7F800000), reached = largest;
+        if (MODE == kOutMx) {
+          reached = warp_max(max_abs_nan(largest, size_product, size_product));
+          error = error_of(reached, largest_bias);
+          limit = 1e37f;  // (near the end of the range the chain may overflow where these sums do not)
+        }
+        if (!(reached < limit)) {
           if (MODE == kOutInt8) {
             tag_flush(tags, mark);  // (without a list the one tag says it all)
           } else {
@@ -648,29 +748,37 @@ dw5x5_kernel(const __grid_constant__ CUtensorMap in_map, const __grid_constant__
             if (x < p.width && row < p.height) note(list, tags, mark, entry + (bit & 3) * 1024 + piece * 8 + (bit >> 2));
           }
         }
+        // MX: whether the warp may hold many values in the left tail of the GELU. There they err by less than (1 + |x|) times the
+        // argument's error *of themselves* (|GELU'| <= |x| |GELU|), far below the bound for all: the codes of values near zero would
+        // look open everywhere. (Arguments of a standard deviation below 1.5 have fewer such values, at -4 and below, than looking
+        // for them is worth.)
+        constexpr bool kTails = MODE == kOutMx && ACT == kActGelu;
+        uint32_t tails = 0;  // bit c * 4 + i * 4 + d, c = 0, 4: channel c + d of pixel i is below -1, before the activation
+        bool tail_warp = false;
+        if (kTails) {
+          tail_warp = error < 0.01f && __any_sync(0xffffffffu, largest + largest_bias > 5.0f);
+          if (tail_warp) {
 #pragma unroll
-        for (int c = 0; c < 8; ++c) v[c][0] = activate2<ACT>(v[c][0]), v[c][1] = activate2<ACT>(v[c][1]);
-        float inv[4];
-        uint32_t unsure = 0;  // MX: bit i for a pixel whose block is to be summed again
-        if (MODE == kOutMx) {
-          // A value whose low 20 mantissa bits are within 16 of one half lies within 2**-19 of a boundary between two E4M3 codes,
-          // whatever power of two it is scaled by (codes below 2**-6 of the scale have coarser steps and are not looked at:
-          // the largest of them is 1/28672 of the block's maximum).
-          constexpr uint32_t kToZero = static_cast<uint32_t>(-(0x80000 - 16)) << 12, kWindow = 32u << 12;
-          uint32_t nearest[4] = {~0u, ~0u, ~0u, ~0u};
+            for (int n = 7; n >= 0; --n) {
 #pragma unroll
-          for (int c = 0; c < 8; ++c) {
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-              float lo, hi;
-              unpack2(v[c][h], lo, hi);
-              nearest[2 * h] = min(nearest[2 * h], (__float_as_uint(lo) << 12) + kToZero);
-              nearest[2 * h + 1] = min(nearest[2 * h + 1], (__float_as_uint(hi) << 12) + kToZero);
+              for (int d = 3; d >= 0; --d) {
+                float lo, hi;
+                unpack2(add2(v[(n >> 2) * 4 + d][(n & 3) >> 1], pack2(1.0f, 1.0f)), lo, hi);
+                tails = __funnelshift_l(__float_as_uint(n & 1 ? hi : lo), tails, 1);
+              }
             }
           }
+        }
+        // (the quantiser of a ReLU clips: its bounds lie on both sides of zero)
+        if (MODE != kOutMx || ACT != kActRelu) {
 #pragma unroll
-          for (int i = 0; i < 4; ++i) unsure |= nearest[i] < kWindow ? 1u << i : 0u;
-          float amax[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+          for (int c = 0; c < 8; ++c) v[c][0] = activate2<ACT>(v[c][0]), v[c][1] = activate2<ACT>(v[c][1]);
+        }
+        float inv[4];
+        uint32_t unsure = 0;  // MX: bit i for a pixel whose block exponent is open
+        if (MODE == kOutMx) {
+          constexpr float kNone = ACT == kActRelu ? -__builtin_huge_valf() : 0.0f;
+          float amax[4] = {kNone, kNone, kNone, kNone};  // (of a ReLU: the largest value, below zero as it is)
 #pragma unroll
           for (int c = 0; c < 8; c += 2) {
 #pragma unroll
@@ -678,17 +786,20 @@ dw5x5_kernel(const __grid_constant__ CUtensorMap in_map, const __grid_constant__
               float lo0, hi0, lo1, hi1;
               unpack2(v[c][h], lo0, hi0);
               unpack2(v[c + 1][h], lo1, hi1);
-              amax[2 * h] = max_abs(amax[2 * h], lo0, lo1), amax[2 * h + 1] = max_abs(amax[2 * h + 1], hi0, hi1);
+              amax[2 * h] = ACT == kActRelu ? max3(amax[2 * h], lo0, lo1) : max_abs(amax[2 * h], lo0, lo1);
+              amax[2 * h + 1] = ACT == kActRelu ? max3(amax[2 * h + 1], hi0, hi1) : max_abs(amax[2 * h + 1], hi0, hi1);
             }
           }
           const uint32_t mine = exchange + flip * 2048 + lane * 16;
           asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(mine + piece * 512), "f"(amax[0]), "f"(amax[1]), "f"(amax[2]), "f"(amax[3])
                        : "memory");
+          const uint32_t errors = list + kListErrors + flip * 16;
+          if (lane == 0) asm volatile("st.shared.f32 [%0], %1;" ::"r"(errors + piece * 4), "f"(ACT == kActGelu ? error * kGeluSlope : error) : "memory");
           if (piece == 0 && elect_one()) bulk_wait_read<0>();  // the store of the panel before the last
           named_barrier(quad_barrier, 128);
           if (piece == 0) {
             if (stored_b >= 0) store_panel(panels + (flip ^ 1u) * panel_bytes(MODE), stored_c, stored_x, stored_y, stored_b);
-            if (alive) issue_until(taken + kStages);
+            if (alive) issue_until(taken + kStages - kept_chunks(MODE));
           }
           stored_c = c0, stored_x = x0, stored_y = y, stored_b = p.tma_out ? at.b : -1;
           read_tag();
@@ -699,9 +810,13 @@ dw5x5_kernel(const __grid_constant__ CUtensorMap in_map, const __grid_constant__
             asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(t[0]), "=f"(t[1]), "=f"(t[2]), "=f"(t[3]) : "r"(mine + (piece ^ other) * 512));
           }
 #pragma unroll
-          for (int i = 0; i < 4; ++i) amax[i] = fmaxf(max_abs(amax[i], theirs[0][i], theirs[1][i]), theirs[2][i]);
+          for (int i = 0; i < 4; ++i) {
+            amax[i] = fmaxf(ACT == kActRelu ? max3(amax[i], theirs[0][i], theirs[1][i]) : max_abs(amax[i], theirs[0][i], theirs[1][i]), theirs[2][i]);
+          }
           uint32_t bytes[4];
-          unsure |= block_scales(amax, bytes, inv);
+          float e[4];
+          asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(e[0]), "=f"(e[1]), "=f"(e[2]), "=f"(e[3]) : "r"(errors));
+          unsure = block_scales(amax, fmaxf(max3(e[0], e[1], e[2]), e[3]), bytes, inv);
           if (alive && x < p.width && y + piece < p.height) {  // each warp stores the scales of one row
             const uint32_t byte = piece == 0 ? bytes[0] : piece == 1 ? bytes[1] : piece == 2 ? bytes[2] : bytes[3];
             const uint32_t row = scale_row + y * p.width, groups = p.channels >> 5;
@@ -716,31 +831,79 @@ dw5x5_kernel(const __grid_constant__ CUtensorMap in_map, const __grid_constant__
         // the lane's 8 channels of each of its four pixels, as they are stored
         constexpr int kWords = 2 * kOutBytes;
         uint32_t words[4][kWords];
-        const auto values_of = [&](int c, int i, float (&f)[4]) {  // channels c .. c + 3 of pixel i
-#pragma unroll
-          for (int d = 0; d < 4; ++d) {
-            float lo, hi;
-            unpack2(v[c + d][i >> 1], lo, hi);
-            f[d] = i & 1 ? hi : lo;
-          }
-        };
+        uint32_t pending = 0;  // MX: open codes of the lane: channel 4 j + b of pixel i in bit 8 b + 7 - (2 i + j)
         if (MODE == kOutMx) {
+          // the codes of both bounds of every value; where they are the same it is the code of the fp32 chain, too
+          uint32_t open[4][2];  // a byte other than 0 for a code that is open
 #pragma unroll
-          for (int c = 0; c < 8; c += 4) {
-            float f[4][4];
+          for (int h = 0; h < 2; ++h) {
+            float tail_share[2] = {};
+            if (kTails && tail_warp) {
+              // (|GELU(x)| < exp(-x^2 / 2) / sqrt(2 pi) bounds |x| where the value is more than 2**-11 of the scale; below, both bounds
+              // are zeros)
 #pragma unroll
-            for (int d = 0; d < 4; ++d) {
-              unpack2(mul2(v[c + d][0], pack2(inv[0], inv[1])), f[d][0], f[d][1]);
-              unpack2(mul2(v[c + d][1], pack2(inv[2], inv[3])), f[d][2], f[d][3]);
+              for (int i = 0; i < 2; ++i) {
+                const float far = fmaxf(1.3863f * static_cast<float>(static_cast<int>(__float_as_uint(inv[2 * h + i]) >> 23) - 127 + 11) - 1.83f, 0.0f);
+                tail_share[i] = kGeluSlope * error * (2.0f + __fsqrt_rn(far));
+              }
             }
 #pragma unroll
-            for (int i = 0; i < 4; ++i) words[i][c / 4] = e4m3x4(f[0][i], f[1][i], f[2][i], f[3][i]);
+            for (int c = 0; c < 8; c += 4) {
+              uint32_t codes[2][2];
+#pragma unroll
+              for (int side = 0; side < 2; ++side) {
+                const float bound = (side ? error : -error) * (ACT == kActGelu ? kGeluBase : 1.0f);
+                const float grown = ACT == kActGelu ? 1.0f + (side ? error : -error) * kGeluGrowth : 1.0f;
+                const uint64_t bounds = pack2(bound * inv[2 * h], bound * inv[2 * h + 1]), scale = pack2(grown * inv[2 * h], grown * inv[2 * h + 1]);
+                float f[4][2];
+#pragma unroll
+                for (int d = 0; d < 4; ++d) unpack2(fma2(v[c + d][h], scale, bounds), f[d][0], f[d][1]);
+#pragma unroll
+                for (int i = 0; i < 2; ++i) codes[side][i] = codes_of<ACT>(f[0][i], f[1][i], f[2][i], f[3][i]);
+              }
+#pragma unroll
+              for (int i = 0; i < 2; ++i) words[2 * h + i][c / 4] = codes[0][i], open[2 * h + i][c / 4] = codes[0][i] ^ codes[1][i];
+              if (kTails && tail_warp) {
+                // codes of the values themselves, and for those in the tail the bounds that hold there
+#pragma unroll
+                for (int i = 0; i < 2; ++i) {
+                  float f[4], low[4], up[4];
+#pragma unroll
+                  for (int d = 0; d < 4; ++d) {
+                    float first, second;
+                    unpack2(v[c + d][h], first, second);
+                    f[d] = (i ? second : first) * inv[2 * h + i];
+                    low[d] = fmaf(f[d], -tail_share[i], f[d]), up[d] = fmaf(f[d], tail_share[i], f[d]);
+                  }
+                  const uint32_t in_tail = ((tails >> (c * 4 + (2 * h + i) * 4) & 15u) * 0x204081u & 0x01010101u) * 0xFFu;
+                  const uint32_t differ = codes_of<ACT>(low[0], low[1], low[2], low[3]) ^ codes_of<ACT>(up[0], up[1], up[2], up[3]);
+                  open[2 * h + i][c / 4] = (open[2 * h + i][c / 4] & ~in_tail) | (differ & in_tail);
+                  words[2 * h + i][c / 4] = codes_of<ACT>(f[0], f[1], f[2], f[3]);
+                }
+              }
+            }
           }
-          if (unsure != 0) {
+          uint32_t any = 0;
+#pragma unroll
+          for (int i = 0; i < 4; ++i) any |= open[i][0] | open[i][1];
+          if (__any_sync(0xffffffffu, any != 0)) {
+#pragma unroll
+            for (int k = 0; k < 8; ++k) {
+              const uint32_t bytes = open[k >> 1][k & 1];
+              pending |= ((((bytes & 0x7F7F7F7Fu) + 0x7F7F7F7Fu) | bytes) & 0x80808080u) >> k;
+            }
+            const int rows = min(p.height - y, kStepRows);
+            pending = x < p.width ? pending & ((0xFF00u >> (2 * rows) & 0xFFu) * 0x01010101u) : 0;
+            if (__reduce_add_sync(0xffffffffu, __popc(pending)) > kMostOpen) {
+              tag_redo(tags, mark);
+              pending = 0;
+            }
+          }
+          if (piece == 0 && unsure != 0 && x < p.width) {
 #pragma unroll 1
             for (; unsure != 0; unsure &= unsure - 1) {
               const int i = __ffs(unsure) - 1;
-              if (x < p.width && y + i < p.height) note(list, tags, mark, kWholeBlock | (entry + i * 1024));
+              if (y + i < p.height) note(list, tags, mark, entry + i * 1024);
             }
           }
         } else {
@@ -748,8 +911,13 @@ dw5x5_kernel(const __grid_constant__ CUtensorMap in_map, const __grid_constant__
           for (int c = 0; c < 8; c += 4) {
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
-              float f[4];
-              values_of(c, i, f);
+              float f[4];  // channels c .. c + 3 of pixel i
+#pragma unroll
+              for (int d = 0; d < 4; ++d) {
+                float lo, hi;
+                unpack2(v[c + d][i >> 1], lo, hi);
+                f[d] = i & 1 ? hi : lo;
+              }
               const uint32_t w0 = pack_bf16(f[0], f[1]), w1 = pack_bf16(f[2], f[3]);
               if (MODE == kOutBf16) {
                 words[i][c / 2] = w0;
@@ -774,7 +942,6 @@ dw5x5_kernel(const __grid_constant__ CUtensorMap in_map, const __grid_constant__
                            : "memory");
             }
           }
-          fence_async_proxy();
         } else if (alive) {
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
@@ -786,6 +953,52 @@ dw5x5_kernel(const __grid_constant__ CUtensorMap in_map, const __grid_constant__
             }
           }
         }
+        if (MODE == kOutMx) {
+          // The sum of one output at a time as the chain forms it, from the two chunks of the ring that hold its window: a product per
+          // lane into the scratch, the chain in every lane, the code from the lane it belongs to. (Listed for the end of the range, when
+          // the rows have left the L2, the corrections took three times as long.) Scratch is the warp's part of the exchange of the
+          // step before: nobody else looks at it until the warp writes the next maxima.
+          const uint32_t scratch = exchange + (flip ^ 1u) * 2048 + piece * 512;
+#pragma unroll 1
+          for (uint32_t holders; (holders = __ballot_sync(0xffffffffu, pending != 0)) != 0;) {
+            const uint32_t owner = __ffs(holders) - 1, bit = __ffs(__shfl_sync(0xffffffffu, pending, owner)) - 1, k = 7 - (bit & 7u);
+            if (lane == owner) pending &= pending - 1;
+            const uint32_t c = piece * 8 + (k & 1u) * 4 + (bit >> 3), i = k >> 1;
+            const uint32_t below = slot == 0 ? kStages - 1 : slot - 1, above = below == 0 ? kStages - 1 : below - 1;
+            float bias;
+            asm volatile("ld.shared.f32 %0, [%1];" : "=f"(bias) : "r"(bias_at + c * 8));
+            if (lane < kTaps) {
+              const uint32_t ky = lane / 5, row = i + ky, pixel = (row & 3u) * kHaloX + owner + (lane - ky * 5);
+              uint16_t value, tap;
+              asm volatile("ld.shared.u16 %0, [%1];" : "=h"(value) : "r"(ring + (row < 4 ? above : below) * kChunkBytes + pixel * kPixelBytes +
+                                                                       (((c >> 3) ^ ((pixel >> 1) & 3u)) << 4) + (c & 7u) * 2));
+              asm volatile("ld.shared.u16 %0, [%1];" : "=h"(tap) : "r"(weights_at + lane * (kTileC * 2) + c * 2));
+              asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(scratch + lane * 8), "f"(bf16_lo(value)), "f"(bf16_lo(tap)) : "memory");
+            }
+            __syncwarp();
+            float sum = 0.0f;
+#pragma unroll
+            for (int t = 0; t < kTaps; t += 2) {
+              uint32_t pair[4];
+              lds128(scratch + t * 8, pair);
+              sum = fmaf(__uint_as_float(pair[0]), __uint_as_float(pair[1]), sum);
+              if (t + 1 < kTaps) sum = fmaf(__uint_as_float(pair[2]), __uint_as_float(pair[3]), sum);
+            }
+            __syncwarp();
+            sum += bias;
+            float out, unused;
+            unpack2(activate2<ACT>(pack2(sum, sum)), out, unused);
+            const uint32_t code = e4m3x2(out * (i == 0 ? inv[0] : i == 1 ? inv[1] : i == 2 ? inv[2] : inv[3]), 0.0f);
+            if (lane == owner) {
+              if (p.tma_out) {
+                asm volatile("st.shared.u8 [%0], %1;" ::"r"(panel + (i * kTileX + lane) * 32 + (((piece >> 1) ^ ((lane >> 2) & 1)) << 4) + (c & 15u)), "r"(code) : "memory");
+              } else if (alive) {
+                p.out[((static_cast<size_t>(at.b) * p.height + y + i) * p.width + x) * p.channels + c0 + c] = static_cast<uint8_t>(code);
+              }
+            }
+          }
+        }
+        if (p.tma_out) fence_async_proxy();
         if (MODE != kOutMx) {
           if (piece == 0 && elect_one()) bulk_wait_read<0>();  // the store of the other panel
           named_barrier(quad_barrier, 128);

@@ -91,3 +91,103 @@ def test_what_is_not_finite_costs_its_own_steps(ops, ctas):
     number = redone & ~torch.isnan(want)
     assert number.any() and same_bytes(got[number], want[number])
     assert int((~torch.isfinite(want)).sum()) > 0
+
+
+# ---- MXFP8: codes and scales of the chain ------------------------------------------------------------------------------
+
+ACTS = {"none": 0, "relu": 1, "gelu": 2}
+
+
+def quantise(values, act):
+    """E4M3 codes ``[rows, C]`` and E8M0 bytes ``[rows, C / 32]`` of fp32 pre-activation values, by the op's own activation and
+    quantiser: its sums over an image of zeros are zero in every order, so the bias of a channel passes through as it is."""
+    from flashim_b200 import _native
+
+    lib, rows, c = _native.library(), values.shape[0], values.shape[1]
+    flat, step = values.reshape(-1).contiguous(), 1 << 20
+    codes, scales = torch.empty(flat.numel(), dtype=torch.uint8, device=DEV), torch.empty(flat.numel() // 32, dtype=torch.uint8, device=DEV)
+    x, w = torch.zeros(step, dtype=BF16, device=DEV), torch.zeros(25 * step, dtype=BF16, device=DEV)
+    for at in range(0, flat.numel(), step):
+        n = min(step, flat.numel() - at)
+        part_codes, part_scales = torch.empty(n, dtype=torch.uint8, device=DEV), torch.empty(n // 32, dtype=torch.uint8, device=DEV)
+        bias = flat[at: at + n].clone()
+        assert lib.fim_dw5x5_mxfp8(x.data_ptr(), w.data_ptr(), bias.data_ptr(), part_codes.data_ptr(), part_scales.data_ptr(), 0, 1, 1, 1, n,
+                                   ACTS[act], None, torch.cuda.current_stream().cuda_stream) == 0
+        codes[at: at + n], scales[at // 32: (at + n) // 32] = part_codes, part_scales
+    return codes.view(rows, c), scales.view(rows, c // 32)
+
+
+def dw_mxfp8(x, w, b, act):
+    from flashim_b200 import _native
+
+    batch, height, width, c = x.shape
+    rows = batch * height * width
+    codes, scales = torch.empty(rows, c, dtype=torch.uint8, device=DEV), torch.empty(rows, c // 32, dtype=torch.uint8, device=DEV)
+    assert _native.library().fim_dw5x5_mxfp8(x.data_ptr(), w.data_ptr(), b.data_ptr(), codes.data_ptr(), scales.data_ptr(), 0, batch, height, width, c,
+                                             ACTS[act], None, torch.cuda.current_stream().cuda_stream) == 0
+    return codes, scales
+
+
+def data(kind, shape, seed):
+    g = torch.Generator(device=DEV).manual_seed(seed)
+    batch, height, width, c = shape
+    rand = lambda *s: torch.randn(s, generator=g, device=DEV)  # noqa: E731
+    x, w, b = rand(*shape), rand(25, c) * 0.05, rand(c) * 0.02
+    zero_sum = rand(25, c) * 0.05
+    zero_sum = (zero_sum - zero_sum.mean(0)).to(BF16).float()
+    zero_sum[24] -= zero_sum.sum(0)  # (up to the rounding of one tap)
+    if kind == "wide":  # arguments of the GELU of +-20: half of them in its tail
+        w = w * 20
+    elif kind == "smooth":
+        x, w, b = F.interpolate(rand(batch, c, height // 8, width // 8), size=(height, width), mode="bicubic").permute(0, 2, 3, 1) + 10, zero_sum, b * 0
+    elif kind == "flat":  # the sum of every window inside is what the roundings leave of zero
+        x, w, b = rand(batch, 1, 1, c).expand(shape), zero_sum, b * 0
+    elif kind == "heavy":
+        x, w = (2 * x).exp() * rand(*shape).sign(), (2 * rand(25, c)).exp() * rand(25, c).sign()
+    elif kind == "sparse":
+        x = torch.where(F.avg_pool2d(rand(batch, 1, height, width), 9, 1, 4).permute(0, 2, 3, 1) > 0, x.relu(), 0.0)
+    elif kind == "tiny":
+        # (products of 2**-112 and down to 2**-133, below which 16 bits no longer fit and the product of the chain here would round)
+        x, w, b = x * 1e-18, w * 1e-16, b * 0
+    return x.to(BF16).contiguous(), w.to(BF16), b
+
+
+@pytest.mark.parametrize("act", ["gelu", "relu", "none"])
+@pytest.mark.parametrize("kind", ["normal", "wide", "smooth", "flat", "heavy", "sparse", "tiny"])
+def test_mxfp8_is_that_of_the_chain(ctas, kind, act):
+    """Every code and scale, on data whose sums keep their size and on data whose sums cancel (in a flat image every output is
+    open), by the whole grid and by one CTA."""
+    shape = (1, 67, 133, 96) if ctas == 1 else (2, 200, 201, 128)
+    for seed in range(1 if ctas == 1 else 4):
+        x, w, b = data(kind, shape, 10 + seed)
+        want = quantise(chain(x, w, b).view(-1, shape[3]), act)
+        got, again = dw_mxfp8(x, w, b, act), dw_mxfp8(x, w, b, act)
+        codes, scales = int((got[0] != want[0]).sum()), int((got[1] != want[1]).sum())
+        assert codes == 0 and scales == 0, f"{codes} of {want[0].numel()} codes, {scales} of {want[1].numel()} scales differ"
+        assert torch.equal(again[0], got[0]) and torch.equal(again[1], got[1])
+
+
+def test_stack_on_chain_sums(ops, monkeypatch):
+    """The refiner stack on four image pairs: the same bytes as with every depthwise layer summed by the chain."""
+    import flashim_b200
+    from flashim_b200 import refiner
+    from flashim_b200.quant import swizzle_scales
+
+    levels = ((50, 512), (100, 256), (200, 128))
+    model = flashim_b200.load("refiner-stack", "fp8", device=DEV, engine="eager", overrides={"arch.levels": [list(v) for v in levels]})
+    g = torch.Generator(device=DEV).manual_seed(9)
+    pyramid = [torch.randn(8, size, size, c, generator=g, device=DEV).to(BF16) for size, c in levels]
+    got = model(pyramid)
+
+    class ChainSummed:
+        def __getattr__(self, name):
+            return getattr(ops, name)
+
+        def depthwise5x5_act_mxfp8(self, value, weight, bias, act):
+            pixels = value.permute(0, 2, 3, 1).contiguous()
+            codes, scales = quantise(chain(pixels, weight, bias).view(-1, pixels.shape[3]), act)
+            return codes.view(torch.float8_e4m3fn), swizzle_scales((scales.int() - 127).to(torch.int8))
+
+    monkeypatch.setattr(refiner, "ops", ChainSummed())
+    for mine, want in zip(got, model(pyramid)):
+        assert same_bytes(mine, want)
