@@ -277,6 +277,7 @@ PyObject* shape_tuple(const Tensor& t) {
 // one shape and version of it. At most 512 entries, the least recently used one goes first. Guarded by the interpreter lock.
 
 struct Swizzled {
+  const void* key;
   Tensor source, packed;
   uint32_t version;
 };
@@ -284,32 +285,40 @@ std::list<Swizzled> swizzled;
 std::unordered_map<const void*, std::list<Swizzled>::iterator> swizzled_at;
 constexpr size_t kSwizzledEntries = 512;
 
-// nullptr: not for the cache (inference tensors have no version)
-const Tensor* swizzled_scales(const Tensor& exponent) {
-  if (exponent.is_inference()) return nullptr;
+void drop_swizzled(std::unordered_map<const void*, std::list<Swizzled>::iterator>::iterator at) {
+  std::list<Swizzled> gone;  // (destroyed last: the tables are whole again by then)
+  gone.splice(gone.begin(), swizzled, at->second);
+  swizzled_at.erase(at);
+}
+
+// The packed scales, held by the caller: another thread may take the entry out while this one runs without the interpreter
+// lock. Undefined: not for the cache (inference tensors have no version).
+Tensor swizzled_scales(const Tensor& exponent) {
+  if (exponent.is_inference()) return {};
   const void* key = exponent.data_ptr();
   auto hit = swizzled_at.find(key);
   if (hit != swizzled_at.end()) {
     const Swizzled& e = *hit->second;
     if (e.version == exponent._version() && e.source.sizes() == exponent.sizes() && e.source.strides() == exponent.strides()) {
       swizzled.splice(swizzled.begin(), swizzled, hit->second);
-      return &e.packed;
+      return e.packed;
     }
-    swizzled.erase(hit->second);
-    swizzled_at.erase(hit);
+    drop_swizzled(hit);
   }
+  const auto version = static_cast<uint32_t>(exponent._version());
   PyObject* source = wrap(exponent);
-  PyObject* packed = PyObject_CallFunctionObjArgs(py_swizzle, source, nullptr);
+  PyObject* made = PyObject_CallFunctionObjArgs(py_swizzle, source, nullptr);
   Py_DECREF(source);
-  if (packed == nullptr) failed();
-  swizzled.push_front({exponent, THPVariable_Unpack(packed), static_cast<uint32_t>(exponent._version())});
-  Py_DECREF(packed);
+  if (made == nullptr) failed();
+  const Tensor packed = THPVariable_Unpack(made);
+  Py_DECREF(made);
+  // (the call may have let another thread in, which may have made the same entry: one per key)
+  hit = swizzled_at.find(key);
+  if (hit != swizzled_at.end()) drop_swizzled(hit);
+  swizzled.push_front({key, exponent, packed, version});
   swizzled_at[key] = swizzled.begin();
-  if (swizzled.size() > kSwizzledEntries) {
-    swizzled_at.erase(swizzled.back().source.data_ptr());
-    swizzled.pop_back();
-  }
-  return &swizzled.front().packed;
+  if (swizzled.size() > kSwizzledEntries) drop_swizzled(swizzled_at.find(swizzled.back().key));
+  return packed;
 }
 
 // ---- convs: geometry and epilogue ------------------------------------------------------------------------------------
@@ -500,9 +509,9 @@ PyObject* mxfp8_conv2d(Args a) {
   }
   Call call;
   if (!call.begin(*x) || !call.here(e, w, we, bias, res, oe)) return nullptr;
-  const Tensor* packed = swizzled_scales(*we);
-  if (packed == nullptr) return nullptr;
-  return mx_conv(*x, e, nullptr, *w, *packed, bias, g, res, flag(a[13]) ? FIM_ACT_RELU : FIM_ACT_NONE,
+  const Tensor packed = swizzled_scales(*we);
+  if (!packed.defined()) return nullptr;
+  return mx_conv(*x, e, nullptr, *w, packed, bias, g, res, flag(a[13]) ? FIM_ACT_RELU : FIM_ACT_NONE,
                  oe == nullptr ? FIM_OUT_BF16 : FIM_OUT_E4M3_STATIC, oe, call);
 }
 
@@ -685,9 +694,9 @@ PyObject* mxfp8_linear(Args a) {  // activation, bias, weight
   if (!linear_operands(v, e, w, we) || !optional_tensor(a[1], &bias) || !bias_ok(bias, w->size(0))) return nullptr;
   Call call;
   if (!call.begin(*v) || !call.here(e, w, we, bias)) return nullptr;
-  const Tensor* packed = swizzled_scales(*we);
-  if (packed == nullptr) return nullptr;
-  return wrap(mx_gemm(*v, v->numel() / w->size(1), e, nullptr, *w, *packed, bias, call, "mxfp8_linear"));
+  const Tensor packed = swizzled_scales(*we);
+  if (!packed.defined()) return nullptr;
+  return wrap(mx_gemm(*v, v->numel() / w->size(1), e, nullptr, *w, packed, bias, call, "mxfp8_linear"));
 }
 
 PyObject* mxfp8_gelu_mlp(Args a) {  // x, w1, b1, hidden_exponent, w2
@@ -703,11 +712,8 @@ PyObject* mxfp8_gelu_mlp(Args a) {  // x, w1, b1, hidden_exponent, w2
   }
   Call call;
   if (!call.begin(*v) || !call.here(e, w1, e1, b1, he, w2, e2)) return nullptr;
-  const Tensor* found1 = swizzled_scales(*e1);
-  if (found1 == nullptr) return nullptr;
-  const Tensor packed1 = *found1;  // (the second look-up may move the first entry out)
-  const Tensor* packed2 = swizzled_scales(*e2);
-  if (packed2 == nullptr) return nullptr;
+  const Tensor packed1 = swizzled_scales(*e1), packed2 = swizzled_scales(*e2);
+  if (!packed1.defined() || !packed2.defined()) return nullptr;
   // the reference's rounding points: the first product rounds to bf16 before b1 is added, GELU runs in fp32 on that sum,
   // and the second product has no bias
   const Tensor bias = b1->scalar_type() == kF32 && b1->is_contiguous() ? *b1 : b1->to(kF32).contiguous();
@@ -717,7 +723,7 @@ PyObject* mxfp8_gelu_mlp(Args a) {  // x, w1, b1, hidden_exponent, w2
     return abi.fim_gelu_quantize_mxfp8(h.data_ptr(), static_cast<const float*>(bias.data_ptr()), static_cast<const int8_t*>(he->data_ptr()),
                                        q.data_ptr(), rows, hidden, call.stream);
   });
-  return wrap(mx_gemm(q, rows, he, nullptr, *w2, *packed2, nullptr, call, "mxfp8_gelu_mlp"));
+  return wrap(mx_gemm(q, rows, he, nullptr, *w2, packed2, nullptr, call, "mxfp8_gelu_mlp"));
 }
 
 PyObject* mxfp8_scaled_mm(Args a) {  // a, b_t, a_scale, b_scale, bias
@@ -1050,8 +1056,8 @@ PyObject* bind(PyObject*, PyObject* args) {
 PyObject* cached_swizzle(PyObject*, PyObject* o) {
   if (!THPVariable_Check(o)) Py_RETURN_NONE;
   try {
-    const Tensor* t = swizzled_scales(THPVariable_Unpack(o));
-    if (t != nullptr) return wrap(*t);
+    Tensor t = swizzled_scales(THPVariable_Unpack(o));
+    if (t.defined()) return wrap(std::move(t));
   } catch (const Failed&) {
     return nullptr;
   } catch (const std::exception& e) {
