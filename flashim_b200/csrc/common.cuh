@@ -55,9 +55,11 @@ __device__ __forceinline__ bool elect_one() {
 }
 
 // ---- launches that overlap their prologue with the kernel before them (launch_dependent below) ----------------------------
-// Every kernel launched that way calls grid_release first and grid_wait once, before its first access to global memory: the
+// Every kernel launched that way calls grid_release early and grid_wait once, before its first access to global memory: the
 // kernel before it has completed then, and its writes are visible. What comes ahead of grid_wait (barriers, tensor
-// memory, constant tables) runs while that kernel drains.
+// memory, constant tables) runs while that kernel drains. The next kernel may start once a thread of every CTA has called
+// grid_release, and a CTA of it that finds room beside one of this kernel may allocate tensor memory at once and then waits for
+// this kernel: in a kernel that allocates tensor memory only the warp that does so calls grid_release, and behind the allocation.
 __device__ __forceinline__ void grid_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 // A pointer the compiler cannot use before this point (a read-only load could otherwise move ahead of grid_wait).

@@ -562,6 +562,7 @@ conv_kernel(const __grid_constant__ CUtensorMap act_map, const __grid_constant__
       tmem_alloc(&ctl.tmem_base, kTmemColumns);
       tmem_relinquish();
     }
+    grid_release();
   }
   if (p.act == kActGelu) {
     for (int i = threadIdx.x; i < kGeluEntries; i += kBlockThreads) {
@@ -571,7 +572,6 @@ conv_kernel(const __grid_constant__ CUtensorMap act_map, const __grid_constant__
       }
     }
   }
-  grid_release();
   grid_wait();
   if (warp == 2 && SCALED && !dynamic_a) {
     // static activation scales: one 512-byte tile per 128 input channels, the same 4 bytes in all 128 rows
@@ -1595,6 +1595,7 @@ mlp_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constant__ CU
   if (warp == 1) {
     tmem_alloc(&ctl.tmem_base, kTmemColumns);
     tmem_relinquish();
+    grid_release();
   }
   for (int i = threadIdx.x; i < kGeluEntries; i += kMlpThreads) {
     const uint32_t entry = kGeluTable[i];
@@ -1603,7 +1604,6 @@ mlp_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constant__ CU
       asm volatile("st.shared.b32 [%0], %1;" ::"r"(smem_gelu + (i * kMlpGeluCopies + c) * 4), "r"(entry) : "memory");
     }
   }
-  grid_release();
   grid_wait();
   for (int i = threadIdx.x; i < 3 * C; i += kMlpThreads) {  // both biases widened to fp32 once per CTA
     const float value = __bfloat162float(i < 2 * C ? p.bias1[i] : p.bias2[i - 2 * C]);
