@@ -36,8 +36,8 @@
 //     lie one ulp of bf16 from the chain's where its sum lies next to a rounding boundary: one in 200000.
 //   INT8: likewise a code may lie one from the chain's: one in 4000000.
 // The outputs and blocks of a list are summed again in the chain's order at the end of the quad's range or when the list fills up; a
-// step with more of them than the list takes, or with more open codes than is worth correcting one by one, is summed again as a
-// whole.
+// step with more of them, or with more open codes, than is worth doing one by one is summed again as a whole. The bits of all
+// outputs thus depend on their own step alone, not on how the work is cut.
 //
 // A patch value outside an output's 5x5 window is multiplied by a zero of B, which an infinity or a not-a-number survives. A
 // step that meets a sum which is not finite is therefore done again in the reference's order.
@@ -76,7 +76,11 @@ constexpr int kMostOpen = 32;
 // The list of a quad: a header (count; flush and redo tags by step parity; MXFP8: error bounds of the four warps by step parity,
 // their largest taps and biases), then one word per entry: step of the range (20 bits) | row (2) | column (5) | channel (5; MXFP8:
 // 0, for a block).
-constexpr uint32_t kListBytes = 1024, kListHeader = 96, kListEntries = (kListBytes - kListHeader) / 4, kFlushAt = 200;
+constexpr uint32_t kListBytes = 1024, kListHeader = 96, kListEntries = (kListBytes - kListHeader) / 4, kFlushAt = 32;
+// bf16: outputs that a warp notes in a step; with more of them the quad does the step again. A list below kFlushAt takes those of two
+// steps, so which steps are done again is a matter of their own data alone, and so are the bits of the other outputs in them.
+constexpr int kMostNoted = 24;
+static_assert(kFlushAt + 2 * 4 * kMostNoted <= kListEntries, "the notes of the step that fills the list, and of the next");
 constexpr uint32_t kListTags = 16, kListErrors = 32, kListSizes = 64;
 constexpr long long kMaxRange = 1 << 20;  // steps of a range that an entry can name
 constexpr uint32_t kWeightBytes = kTaps * kTileC * 2, kBiasBytes = kTileC * 8;
@@ -286,7 +290,7 @@ __device__ __forceinline__ void tag_redo(uint32_t at, uint32_t mark) {
   asm volatile("st.shared.v2.b32 [%0], {%1, %1};" ::"r"(at), "r"(mark) : "memory");
 }
 
-// Notes an output (or the block it lies in) in the quad's list. A step whose entries do not fit is done again as a whole.
+// Notes an output (or the block it lies in) in the quad's list. A step whose entries do not fit is done again as a whole (MXFP8).
 __device__ __forceinline__ void note(uint32_t list, uint32_t tags, uint32_t mark, uint32_t entry) {
   uint32_t at;
   asm volatile("atom.shared.add.u32 %0, [%1], 1;" : "=r"(at) : "r"(list) : "memory");
@@ -730,7 +734,7 @@ dw5x5_kernel(const __grid_constant__ CUtensorMap in_map, const __grid_constant__
             tag_redo(tags, mark);
           }
         }
-        if (MODE == kOutBf16 && margin < 0.0f) {
+        if (MODE == kOutBf16 && __any_sync(0xffffffffu, margin < 0.0f)) {
           uint32_t cancelled = 0;  // bit 4 c + i
 #pragma unroll
           for (int c = 0; c < 8; ++c) {
@@ -742,10 +746,15 @@ dw5x5_kernel(const __grid_constant__ CUtensorMap in_map, const __grid_constant__
 #pragma unroll
             for (int i = 0; i < 4; ++i) cancelled |= fabsf(f[i]) <= size ? 1u << (4 * c + i) : 0u;
           }
+          if (!(margin < 0.0f)) cancelled = 0;
+          if (__reduce_add_sync(0xffffffffu, __popc(cancelled)) > kMostNoted) {
+            tag_redo(tags, mark);
+            cancelled = 0;
+          }
 #pragma unroll 1
           for (; cancelled != 0; cancelled &= cancelled - 1) {
-            const int bit = __ffs(cancelled) - 1, row = y + (bit & 3);
-            if (x < p.width && row < p.height) note(list, tags, mark, entry + (bit & 3) * 1024 + piece * 8 + (bit >> 2));
+            const int bit = __ffs(cancelled) - 1;
+            if (x < p.width && y + (bit & 3) < p.height) note(list, tags, mark, entry + (bit & 3) * 1024 + piece * 8 + (bit >> 2));
           }
         }
         // MX: whether the warp may hold many values in the left tail of the GELU. There they err by less than (1 + |x|) times the

@@ -191,3 +191,24 @@ def test_stack_on_chain_sums(ops, monkeypatch):
     monkeypatch.setattr(refiner, "ops", ChainSummed())
     for mine, want in zip(got, model(pyramid)):
         assert same_bytes(mine, want)
+
+
+def test_bits_do_not_depend_on_how_the_work_is_cut(ops):
+    """Which steps are summed again as a whole is a matter of their own data, not of what a list holds already: areas that cancel
+    in a few, in some and in most pixels of a step, on grids that cut the steps into different ranges and one image at a time."""
+    from flashim_b200 import _native
+
+    lib, shape = _native.library(), (4, 200, 201, 96)
+    g = torch.Generator(device=DEV).manual_seed(6)
+    density = torch.rand(shape[0], 1, 1, generator=g, device=DEV) * 0.002
+    x, w, b = cancelling(shape, 7, torch.rand(shape[:3], generator=g, device=DEV) < density)
+    image = x.permute(0, 3, 1, 2)
+    want = ops.depthwise5x5_act(image, w, b, "none")
+    try:
+        for ctas in (1, 5, 40):
+            lib.fim_dw_tune(ctas, 0)
+            assert same_bytes(ops.depthwise5x5_act(image, w, b, "none"), want)
+    finally:
+        lib.fim_dw_tune(0, 0)
+    for i in range(shape[0]):
+        assert same_bytes(ops.depthwise5x5_act(x[i: i + 1].permute(0, 3, 1, 2), w, b, "none"), want[i: i + 1])
