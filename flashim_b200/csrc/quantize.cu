@@ -142,7 +142,7 @@ __global__ void __launch_bounds__(kThreads) quantize_int8_kernel(const T* __rest
 
 int grid_for(long long work_items, int multiple) {
   const long long blocks = (work_items + kThreads - 1) / kThreads;
-  const long long cap = 148LL * multiple;
+  const long long cap = static_cast<long long>(sm_count()) * multiple;
   return static_cast<int>(blocks < 1 ? 1 : (blocks < cap ? blocks : cap));
 }
 
@@ -295,7 +295,7 @@ int launch_nchw(const void* value, int dtype, const int8_t* exponent, const floa
   auto launch = [&](auto zero, auto vec) {
     using T = decltype(zero);
     // one aligned load per four pixels needs every channel row to start on such a boundary
-    launch_dependent(quantize_nchw_kernel<T, INT8, decltype(vec)::value>, static_cast<unsigned>(grid), kThreads, 0, s, 1u, 
+    launch_dependent(quantize_nchw_kernel<T, INT8, decltype(vec)::value>, static_cast<unsigned>(grid), kThreads, 0, s, 1u,
         static_cast<const T*>(value), exponent, scale, static_cast<uint8_t*>(out), channels, padded, pixels,
         static_cast<int>(pixel_tiles), channel_tiles);
   };
@@ -442,7 +442,7 @@ extern "C" int fim_maxpool2_quantize_int8(const void* value, const float* scale,
   if (value == nullptr || scale == nullptr || out == nullptr) return kBadArgument;
   if (!aligned16(value) || (reinterpret_cast<uintptr_t>(out) & 7u)) return kBadLayout;
   const long long work = static_cast<long long>(batch) * (height / 2) * (width / 2) * (channels / 8);
-  launch_dependent(maxpool2_int8_kernel, static_cast<unsigned>(grid_for(work, 16)), kThreads, 0, static_cast<cudaStream_t>(stream), 1u, 
+  launch_dependent(maxpool2_int8_kernel, static_cast<unsigned>(grid_for(work, 16)), kThreads, 0, static_cast<cudaStream_t>(stream), 1u,
       static_cast<const uint4*>(value), scale, static_cast<uint2*>(out), batch, height, width, channels);
   return static_cast<int>(cudaGetLastError());
 }
@@ -458,7 +458,7 @@ extern "C" int fim_gelu_quantize_mxfp8(const void* value, const float* input_bia
     launch_dependent(kernel, static_cast<unsigned>(grid_for(values / per_thread, 16)), kThreads, 0, static_cast<cudaStream_t>(stream), 1u,
                      static_cast<const __nv_bfloat16*>(value), input_bias, exponent, static_cast<uint8_t*>(out), rows, channels);
   };
-  if (values / 16 < 148LL * 8 * kThreads) {
+  if (values / 16 < static_cast<long long>(sm_count()) * 8 * kThreads) {
     go(gelu_quantize_mx_kernel<4>, 4);
   } else {
     go(gelu_quantize_mx_kernel<16>, 16);

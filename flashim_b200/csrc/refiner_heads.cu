@@ -131,7 +131,7 @@ extern "C" int fim_romav2_refiner_heads(const void* z, const float* weight, cons
   }
   const long long per_block = (kHeadThreads / 8) * kHeadPixels;
   const long long blocks = (rows + per_block - 1) / per_block;
-  const unsigned grid = static_cast<unsigned>(blocks < 148LL * 8 ? blocks : 148LL * 8);
+  const unsigned grid = static_cast<unsigned>(blocks < sm_count() * 8LL ? blocks : sm_count() * 8LL);
   launch_dependent(refiner_heads_kernel, grid, kHeadThreads, 0, static_cast<cudaStream_t>(stream), 1u,
       static_cast<const uint4*>(z), weight, bias, prev_warp, prev_confidence, prev_channels, warp, confidence, rows, channels,
       inv_norm_x, inv_norm_y);

@@ -343,7 +343,7 @@ extern "C" int fim_romav2_refiner_input(const float* f_a, const float* f_b, cons
   if (pixels >= 0x7fffffffLL) return kUnsupported;
   if (radius < 0) {
     const long long plain_blocks = (pixels + 31) / 32;
-    launch_dependent(refiner_input_plain_kernel, static_cast<unsigned>(plain_blocks < 148LL * 32 ? plain_blocks : 148LL * 32), 256, 0,
+    launch_dependent(refiner_input_plain_kernel, static_cast<unsigned>(plain_blocks < sm_count() * 32LL ? plain_blocks : sm_count() * 32LL), 256, 0,
                      static_cast<cudaStream_t>(stream), 1u, p);
     return static_cast<int>(cudaGetLastError());
   }
@@ -356,11 +356,11 @@ extern "C" int fim_romav2_refiner_input(const float* f_a, const float* f_b, cons
         {refiner_input_wide_kernel<2, 0>, refiner_input_wide_kernel<2, 1>, refiner_input_wide_kernel<2, 2>, refiner_input_wide_kernel<2, 3>},
         {refiner_input_wide_kernel<4, 0>, refiner_input_wide_kernel<4, 1>, refiner_input_wide_kernel<4, 2>, refiner_input_wide_kernel<4, 3>}};
     const Kernel kernel = kKernels[features == 32 ? 0 : features == 64 ? 1 : 2][radius];
-    const unsigned grid = static_cast<unsigned>(blocks < 148LL * 32 ? blocks : 148LL * 32);
+    const unsigned grid = static_cast<unsigned>(blocks < sm_count() * 32LL ? blocks : sm_count() * 32LL);
     launch_dependent(kernel, grid, 32 * kInputWarps, kInputWarps * row_bytes, static_cast<cudaStream_t>(stream), 1u, p);
     return static_cast<int>(cudaGetLastError());
   }
-  const unsigned grid = static_cast<unsigned>(blocks < 148LL * 16 ? blocks : 148LL * 16);
+  const unsigned grid = static_cast<unsigned>(blocks < sm_count() * 16LL ? blocks : sm_count() * 16LL);
   launch_dependent(refiner_input_kernel, grid, 32 * kInputWarps, 0, static_cast<cudaStream_t>(stream), 1u, p);
   return static_cast<int>(cudaGetLastError());
 }
