@@ -1135,9 +1135,6 @@ extern "C" int fim_dw5x5_relu_int8(const void* value, const void* weight, const 
   return launch<kOutInt8>(value, weight, bias, out, nullptr, scale, 0, batch, height, width, channels, kActRelu, status, stream);
 }
 
-extern "C" void fim_dw_tune(int variant, int probe_flags) {
-  g_dw_max_ctas = variant;
-  (void)probe_flags;
-}
+extern "C" void fim_dw_tune(int max_ctas, int /* reserved */) { g_dw_max_ctas = max_ctas; }
 
 extern "C" int fim_abi_version(void) { return FIM_ABI_VERSION; }

@@ -33,9 +33,9 @@ extern "C" {
  * (two of its hidden-block warps print their cycle counts per block). */
 void fim_conv_tune(int block_n, int max_ctas, int flags);
 
-/* Depthwise launches: `variant` caps the grid at that many CTAs (0 = automatic), so that a small problem makes every quad
- * of warps walk several spans and channel tiles; the results are the same bits. `probe_flags` is not used. */
-void fim_dw_tune(int variant, int probe_flags);
+/* Depthwise launches: `max_ctas` caps the grid at that many CTAs (0 = automatic), so that a small problem makes every quad
+ * of warps walk several spans and channel tiles; the results are the same bits. `reserved` is ignored: pass 0. */
+void fim_dw_tune(int max_ctas, int reserved);
 
 #ifdef __cplusplus
 }
