@@ -76,16 +76,18 @@ constexpr int kMostOpen = 32;
 // The list of a quad: a header (count; flush and redo tags by step parity; MXFP8: error bounds of the four warps by step parity,
 // their largest taps and biases), then one word per entry: step of the range (20 bits) | row (2) | column (5) | channel (5; MXFP8:
 // 0, for a block).
-constexpr uint32_t kListBytes = 1024, kListHeader = 96, kListEntries = (kListBytes - kListHeader) / 4, kFlushAt = 32;
-// bf16: outputs that a warp notes in a step; with more of them the quad does the step again. A list below kFlushAt takes those of two
+constexpr uint32_t kListHeader = 96, kListTags = 16, kListErrors = 32, kListSizes = 64, kFlushAt = 32;
+// bf16: outputs that a lane notes in a step; with more of them the quad does the step again. A list below kFlushAt takes those of two
 // steps, so which steps are done again is a matter of their own data alone, and so are the bits of the other outputs in them.
-constexpr int kMostNoted = 24;
-static_assert(kFlushAt + 2 * 4 * kMostNoted <= kListEntries, "the notes of the step that fills the list, and of the next");
-constexpr uint32_t kListTags = 16, kListErrors = 32, kListSizes = 64;
+constexpr int kMostNoted = 2;
 constexpr long long kMaxRange = 1 << 20;  // steps of a range that an entry can name
 constexpr uint32_t kWeightBytes = kTaps * kTileC * 2, kBiasBytes = kTileC * 8;
 
 enum { kOutBf16 = 0, kOutMx = 1, kOutInt8 = 2 };
+
+__host__ __device__ constexpr uint32_t list_bytes(int mode) { return mode == kOutBf16 ? 3072u : 1024u; }
+__host__ __device__ constexpr uint32_t list_entries(int mode) { return (list_bytes(mode) - kListHeader) / 4; }
+static_assert(kFlushAt + 2 * 128 * kMostNoted <= list_entries(kOutBf16), "the notes of the step that fills the list, and of the next");
 
 // shared memory of one quad: ring, two output panels (128 pixels x 32 channels), block maxima of two steps, list, B fragments,
 // weights, bias. The MXFP8 form holds its values across a barrier and has no registers left for the B fragments (48): it reads
@@ -99,7 +101,7 @@ __host__ __device__ constexpr uint32_t kept_chunks(int mode) { return mode == kO
 __host__ __device__ constexpr int stages(int mode) { return shared_fragments(mode) ? 4 : kMaxStages; }
 __host__ __device__ constexpr uint32_t fragment_bytes(int mode) { return shared_fragments(mode) ? 4u * 12u * 512u : 0u; }
 __host__ __device__ constexpr uint32_t quad_bytes(int mode) {
-  return (stages(mode) * kChunkBytes + fragment_bytes(mode) + 2 * panel_bytes(mode) + exchange_bytes(mode) + kListBytes + kWeightBytes + kBiasBytes + 1023u) / 1024u * 1024u;
+  return (stages(mode) * kChunkBytes + fragment_bytes(mode) + 2 * panel_bytes(mode) + exchange_bytes(mode) + list_bytes(mode) + kWeightBytes + kBiasBytes + 1023u) / 1024u * 1024u;
 }
 
 struct DwParams {
@@ -291,10 +293,11 @@ __device__ __forceinline__ void tag_redo(uint32_t at, uint32_t mark) {
 }
 
 // Notes an output (or the block it lies in) in the quad's list. A step whose entries do not fit is done again as a whole (MXFP8).
+template <int MODE>
 __device__ __forceinline__ void note(uint32_t list, uint32_t tags, uint32_t mark, uint32_t entry) {
   uint32_t at;
   asm volatile("atom.shared.add.u32 %0, [%1], 1;" : "=r"(at) : "r"(list) : "memory");
-  if (at < kListEntries) {
+  if (at < list_entries(MODE)) {
     asm volatile("st.shared.b32 [%0], %1;" ::"r"(list + kListHeader + at * 4), "r"(entry) : "memory");
     if (at >= kFlushAt) tag_flush(tags, mark);
   } else {
@@ -394,8 +397,8 @@ dw5x5_kernel(const __grid_constant__ CUtensorMap in_map, const __grid_constant__
   const int quad = warp >> 2, piece = warp & 3;  // piece: which 8 of the 32 channels
   const uint32_t ring = ((smem_u32(smem_raw) + 1023u) & ~1023u) + quad * quad_bytes(MODE);
   const uint32_t panels = ring + kStages * kChunkBytes, exchange = panels + 2 * panel_bytes(MODE);
-  const uint32_t list = exchange + exchange_bytes(MODE), fragments = list + kListBytes + piece * (12 * 512) + lane * 16;
-  const uint32_t weights_at = list + kListBytes + fragment_bytes(MODE), bias_at = weights_at + kWeightBytes;
+  const uint32_t list = exchange + exchange_bytes(MODE), fragments = list + list_bytes(MODE) + piece * (12 * 512) + lane * 16;
+  const uint32_t weights_at = list + list_bytes(MODE) + fragment_bytes(MODE), bias_at = weights_at + kWeightBytes;
   const uint32_t full0 = smem_u32(&full_bar[quad * kStages]);
 
   if (threadIdx.x == 0) {
@@ -601,7 +604,7 @@ dw5x5_kernel(const __grid_constant__ CUtensorMap in_map, const __grid_constant__
         asm volatile("st.shared.v4.b32 [%0], {%1, %1, %1, %1};" ::"r"(list + kListTags), "r"(0u) : "memory");
       }
       if (alive) {
-        count = MODE == kOutInt8 ? 0 : min(count, kListEntries);
+        count = MODE == kOutInt8 ? 0 : min(count, list_entries(MODE));
 #pragma unroll 1
         for (uint32_t i = MODE == kOutMx ? piece : threadIdx.x & 127; i < count; i += MODE == kOutMx ? 4 : 128) {
           uint32_t entry;
@@ -734,7 +737,7 @@ dw5x5_kernel(const __grid_constant__ CUtensorMap in_map, const __grid_constant__
             tag_redo(tags, mark);
           }
         }
-        if (MODE == kOutBf16 && __any_sync(0xffffffffu, margin < 0.0f)) {
+        if (MODE == kOutBf16 && margin < 0.0f) {
           uint32_t cancelled = 0;  // bit 4 c + i
 #pragma unroll
           for (int c = 0; c < 8; ++c) {
@@ -746,15 +749,14 @@ dw5x5_kernel(const __grid_constant__ CUtensorMap in_map, const __grid_constant__
 #pragma unroll
             for (int i = 0; i < 4; ++i) cancelled |= fabsf(f[i]) <= size ? 1u << (4 * c + i) : 0u;
           }
-          if (!(margin < 0.0f)) cancelled = 0;
-          if (__reduce_add_sync(0xffffffffu, __popc(cancelled)) > kMostNoted) {
+          if (__popc(cancelled) > kMostNoted) {
             tag_redo(tags, mark);
             cancelled = 0;
           }
 #pragma unroll 1
           for (; cancelled != 0; cancelled &= cancelled - 1) {
             const int bit = __ffs(cancelled) - 1;
-            if (x < p.width && y + (bit & 3) < p.height) note(list, tags, mark, entry + (bit & 3) * 1024 + piece * 8 + (bit >> 2));
+            if (x < p.width && y + (bit & 3) < p.height) note<MODE>(list, tags, mark, entry + (bit & 3) * 1024 + piece * 8 + (bit >> 2));
           }
         }
         // MX: whether the warp may hold many values in the left tail of the GELU. There they err by less than (1 + |x|) times the
@@ -912,7 +914,7 @@ dw5x5_kernel(const __grid_constant__ CUtensorMap in_map, const __grid_constant__
 #pragma unroll 1
             for (; unsure != 0; unsure &= unsure - 1) {
               const int i = __ffs(unsure) - 1;
-              if (y + i < p.height) note(list, tags, mark, entry + i * 1024);
+              if (y + i < p.height) note<MODE>(list, tags, mark, entry + i * 1024);
             }
           }
         } else {
