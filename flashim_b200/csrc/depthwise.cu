@@ -19,9 +19,9 @@
 //     or 16 bytes per pixel from registers instead costs a shared-memory wavefront per lane.
 //
 // Measured against the fp32-pipe kernel before it (B200, inputs in L2 where they fit):
-//   4x200x200x256: GELU -> bf16 68 -> 52 us, ReLU -> bf16 54 -> 41, GELU -> MXFP8 88 -> 82, ReLU -> INT8 87 -> 50
-//   8x400x400x128: GELU -> bf16 232 -> 162, ReLU -> bf16 183 -> 124 (80 % of the HBM copy rate), GELU -> MXFP8 303 -> 274,
-//   ReLU -> MXFP8 252 -> 191, ReLU -> INT8 299 -> 165
+//   4x200x200x256: GELU -> bf16 68 -> 52 us, ReLU -> bf16 54 -> 42, GELU -> MXFP8 88 -> 83, ReLU -> INT8 87 -> 51
+//   8x400x400x128: GELU -> bf16 232 -> 160, ReLU -> bf16 183 -> 127 (80 % of the HBM copy rate), GELU -> MXFP8 303 -> 275,
+//   ReLU -> MXFP8 252 -> 189, ReLU -> INT8 299 -> 165
 // What bounds the GELU and quantising forms now is the arithmetic of their epilogues on twelve warps per SM (issue slots about
 // half busy). The same bytes as the chain (below) cost the MXFP8 form up to a quarter of its time: 225 and 178 us with a test that
 // missed half of the codes that differ. Arguments of the GELU that reach its left tail take 350 us.
