@@ -29,7 +29,7 @@
 // Precision: the tensor cores add the exact products into fp32 accumulators, as the fp32 chain of the reference does (ky-major FMA
 // chain, bias last), but in another order; the two differ by up to about two fp32 ulp of the largest partial sum.
 //   MXFP8: the bytes of the chain. Every value has two bounds, itself less and plus the largest difference (error_of); where their
-//     codes differ (with normal data one in 2000) the output is summed again in the chain's order, at once and from shared memory.
+//     codes differ (with normal data one in 1300) the output is summed again in the chain's order, at once and from shared memory.
 //     Where the exponents of the two bounds of a block's maximum differ, the block is noted in a list of the quad. No code or scale
 //     differed in 2.5 G of normal, wide and sparse data.
 //   bf16: outputs below 2**-14 of the sums in their column, where bias and products cancel, are noted (one in 30000). Others may
@@ -64,17 +64,18 @@ constexpr int kHaloX = kTileX + 4;
 constexpr uint32_t kPixelBytes = kTileC * 2, kRowBytes = kHaloX * kPixelBytes, kChunkBytes = kStepRows * kRowBytes;
 constexpr int kTaps = 25, kMaxStages = 6;
 constexpr float kCancelled = 16384.0f;  // an output below 1 / kCancelled of the sums it comes from is summed again (bf16)
-// MXFP8: how far a tensor-core sum may lie from the fp32 chain, as a share of the size that error_of forms: 2**-20.75. The largest
-// difference in 46 M outputs of each of 14 kinds of data (normal, ReLU'd, positive, log-normal, smooth and flat images; random,
-// positive, zero-sum, Laplacian and Sobel taps) was 2**-21.35 of it; at most one output in 100000 passed 2**-22.
-constexpr float kSumError = 5.67e-7f;
+// MXFP8: how far a tensor-core sum may lie from the fp32 chain, as a share of the size that error_of forms: 2**-20.1. The largest
+// difference in three times 46 M outputs of each of 88 kinds of data (normal, ReLU'd, positive, uniform, log-normal, smooth and flat
+// images under random, positive, zero-sum, edge, Gaussian and log-normal taps) was 2**-20.6 of it, for edge filters on a smooth
+// image; it is 2**-21.2 of the largest partial sum at most, and where sums cancel that is at most twice the size.
+constexpr float kSumError = 8.9e-7f;
 // The GELU passes on less than kGeluSlope of an argument's error (|GELU'| <= 1.129), and less than kGeluBase + kGeluGrowth * GELU
 // (|GELU'| <= 0.5 + 1.6 GELU for every argument); both with a tenth for the rounding of the polynomial.
 constexpr float kGeluSlope = 1.25f, kGeluBase = 0.55f, kGeluGrowth = 1.76f;
-// open codes that a warp corrects one by one (about 450 cycles each); with more of them the quad does the step again (20000)
+// open codes that a warp corrects two by two (about 500 cycles); with more of them the quad does the step again (20000)
 constexpr int kMostOpen = 32;
 // The list of a quad: a header (count; flush and redo tags by step parity; MXFP8: error bounds of the four warps by step parity,
-// their largest taps and biases), then one word per entry: step of the range (20 bits) | row (2) | column (5) | channel (5; MXFP8:
+// the sizes of their taps and biases), then one word per entry: step of the range (20 bits) | row (2) | column (5) | channel (5; MXFP8:
 // 0, for a block).
 constexpr uint32_t kListHeader = 96, kListTags = 16, kListErrors = 32, kListSizes = 64, kFlushAt = 32;
 // bf16: outputs that a lane notes in a step; with more of them the quad does the step again. A list below kFlushAt takes those of two
@@ -336,9 +337,9 @@ __device__ __forceinline__ uint32_t codes_of(float a, float b, float c, float d)
 }
 
 // Bound on the difference between a sum of the tensor cores plus bias and the same of the fp32 chain. Both err by ulps of
-// their partial sums. `size` is the largest |sum| of the warp or twice the largest product that its patches can hold, whichever is
-// larger: where all sums cancel (flat areas under taps that sum to zero) only the second bounds the partial sums. The bias adds a
-// rounding to an ulp of the result. Sums of zeros are equal. Near the subnormals ulps no longer shrink with the sums: nothing is
+// their partial sums. `size` is the largest |sum| of the warp or, if that is larger, its largest |value| times twice the largest |tap| or
+// a quarter of the sum of a channel's |taps|: where all sums cancel (flat areas under taps that sum to zero) only the second bounds the
+// partial sums. The bias adds a rounding to an ulp of the result. Sums of zeros are equal. Near the subnormals ulps no longer shrink with the sums: nothing is
 // assumed there.
 __device__ __forceinline__ float error_of(float size, float bias) {
   const float total = fmaxf(size, bias);
@@ -502,15 +503,21 @@ dw5x5_kernel(const __grid_constant__ CUtensorMap in_map, const __grid_constant__
         asm volatile("st.shared.v2.f32 [%0], {%1, %1};" ::"r"(bias_at + lane * 8), "f"(bias) : "memory");
       }
       named_barrier(quad_barrier, 128);
-      if (MODE == kOutMx) {  // the largest |tap| and |bias| of the warp's channels
-        uint32_t tap[4] = {};
-        if (lane < kTaps) lds128(weights_at + lane * (kTileC * 2) + piece * 16, tap);
-        float bias, size = 0.0f;
-        asm volatile("ld.shared.f32 %0, [%1];" : "=f"(bias) : "r"(bias_at + (piece * 8 + (lane & 7)) * 8));
+      if (MODE == kOutMx) {  // the size of the taps (see error_of) and the largest |bias| of the warp's channels; four lanes per channel
+        const uint32_t c = piece * 8 + (lane & 7);
+        float bias, sum = 0.0f, most = 0.0f;
+        asm volatile("ld.shared.f32 %0, [%1];" : "=f"(bias) : "r"(bias_at + c * 8));
 #pragma unroll
-        for (int j = 0; j < 4; ++j) size = max_abs(size, bf16_lo(tap[j]), bf16_hi(tap[j]));
-        const float largest_tap = warp_max(size), largest_bias = warp_max(fabsf(bias));
-        if (lane == 0) asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(list + kListSizes + piece * 8), "f"(largest_tap), "f"(largest_bias) : "memory");
+        for (int i = 0; i < 7; ++i) {
+          const int t = i * 4 + (lane >> 3);
+          uint16_t tap = 0;
+          if (t < kTaps) asm volatile("ld.shared.u16 %0, [%1];" : "=h"(tap) : "r"(weights_at + t * (kTileC * 2) + c * 2));
+          sum += fabsf(bf16_lo(tap)), most = fmaxf(most, fabsf(bf16_lo(tap)));
+        }
+        sum += __shfl_xor_sync(0xffffffffu, sum, 8);
+        sum += __shfl_xor_sync(0xffffffffu, sum, 16);
+        const float tap_size = warp_max(fmaxf(2.0f * most, 0.25f * sum)), largest_bias = warp_max(fabsf(bias));
+        if (lane == 0) asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(list + kListSizes + piece * 8), "f"(tap_size), "f"(largest_bias) : "memory");
         __syncwarp();
       }
       // B[k][n] = w[row - dy][column - dx] for patch position k = (row, column) and output pixel n = (dx, dy), else 0; this
@@ -662,12 +669,12 @@ dw5x5_kernel(const __grid_constant__ CUtensorMap in_map, const __grid_constant__
         const uint32_t from = take_chunk();
         const uint32_t panel = panels + flip * panel_bytes(MODE);
         float acc[8][4];
-        float size_product = 0.0f, largest_tap = 0.0f, largest_bias = 0.0f;  // MX: twice the largest product that the lane knows of
+        float size_product = 0.0f, tap_size = 0.0f, largest_bias = 0.0f;  // MX: largest |value| that the lane knows of times the size of the taps
         {
           float first = 0.0f;
           if (MODE == kOutMx) {
             first = first_columns(from);
-            asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(largest_tap), "=f"(largest_bias) : "r"(list + kListSizes + piece * 8));
+            asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(tap_size), "=f"(largest_bias) : "r"(list + kListSizes + piece * 8));
           }
           RowPair r2;
           const auto multiply = [&](auto first, const RowPair& upper, const RowPair& lower, int st) {
@@ -685,8 +692,8 @@ dw5x5_kernel(const __grid_constant__ CUtensorMap in_map, const __grid_constant__
           multiply(std::false_type{}, r0, r1, 2);
           if (MODE == kOutMx) {
             const float size = size_of(r0, r1, first), both = fmaxf(size, size_above);
-            size_product = 2.0f * largest_tap * both;
-            if (size_product < 1e-36f && largest_tap > 0.0f && both > 0.0f) size_product = 1e-36f;  // (underflow)
+            size_product = tap_size * both;
+            if (size_product < 1e-36f && tap_size > 0.0f && both > 0.0f) size_product = 1e-36f;  // (underflow)
             size_above = size;
           }
         }
@@ -965,33 +972,43 @@ dw5x5_kernel(const __grid_constant__ CUtensorMap in_map, const __grid_constant__
           }
         }
         if (MODE == kOutMx) {
-          // The sum of one output at a time as the chain forms it, from the two chunks of the ring that hold its window: a product per
-          // lane into the scratch, the chain in every lane, the code from the lane it belongs to. (Listed for the end of the range, when
+          // The sums of two outputs at a time as the chain forms them, from the two chunks of the ring that hold their windows: a product
+          // per lane into the scratch, a chain in every lane, the codes from the lanes they belong to. One at a time takes 292 us for
+          // GELU at 8x400x400x128 instead of 280, an output per lane without scratch 303. (Listed for the end of the range, when
           // the rows have left the L2, the corrections took three times as long.) Scratch is the warp's part of the exchange of the
           // step before: nobody else looks at it until the warp writes the next maxima.
           const uint32_t scratch = exchange + (flip ^ 1u) * 2048 + piece * 512;
+          const uint32_t below = slot == 0 ? kStages - 1 : slot - 1, above = below == 0 ? kStages - 1 : below - 1;
 #pragma unroll 1
           for (uint32_t holders; (holders = __ballot_sync(0xffffffffu, pending != 0)) != 0;) {
-            const uint32_t owner = __ffs(holders) - 1, bit = __ffs(__shfl_sync(0xffffffffu, pending, owner)) - 1, k = 7 - (bit & 7u);
-            if (lane == owner) pending &= pending - 1;
-            const uint32_t c = piece * 8 + (k & 1u) * 4 + (bit >> 3), i = k >> 1;
-            const uint32_t below = slot == 0 ? kStages - 1 : slot - 1, above = below == 0 ? kStages - 1 : below - 1;
+            // the first open codes of two lanes
+            const uint32_t first = __ffs(holders) - 1, others = holders & (holders - 1), second = others != 0 ? __ffs(others) - 1 : first;
+            const uint32_t mine = __ffs(pending) - 1;
+            pending = lane == first || lane == second ? pending & (pending - 1) : pending;
+            const auto channel = [&](uint32_t bit) { return piece * 8 + (~bit & 1u) * 4 + (bit >> 3); };
+            const auto row_of = [&](uint32_t bit) { return (7 - (bit & 7u)) >> 1; };
+            const auto products = [&](uint32_t owner, uint32_t to) {
+              const uint32_t bit = __shfl_sync(0xffffffffu, mine, owner), c = channel(bit);
+              if (lane < kTaps) {
+                const uint32_t ky = lane / 5, row = row_of(bit) + ky, pixel = (row & 3u) * kHaloX + owner + (lane - ky * 5);
+                uint16_t value, tap;
+                asm volatile("ld.shared.u16 %0, [%1];" : "=h"(value) : "r"(ring + (row < 4 ? above : below) * kChunkBytes + pixel * kPixelBytes +
+                                                                         (((c >> 3) ^ ((pixel >> 1) & 3u)) << 4) + (c & 7u) * 2));
+                asm volatile("ld.shared.u16 %0, [%1];" : "=h"(tap) : "r"(weights_at + lane * (kTileC * 2) + c * 2));
+                asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(to + lane * 8), "f"(bf16_lo(value)), "f"(bf16_lo(tap)) : "memory");
+              }
+            };
+            products(first, scratch);
+            if (others != 0) products(second, scratch + 208);
+            const uint32_t from = lane == second && others != 0 ? scratch + 208 : scratch, c = channel(mine & 31u), i = row_of(mine & 31u);
             float bias;
             asm volatile("ld.shared.f32 %0, [%1];" : "=f"(bias) : "r"(bias_at + c * 8));
-            if (lane < kTaps) {
-              const uint32_t ky = lane / 5, row = i + ky, pixel = (row & 3u) * kHaloX + owner + (lane - ky * 5);
-              uint16_t value, tap;
-              asm volatile("ld.shared.u16 %0, [%1];" : "=h"(value) : "r"(ring + (row < 4 ? above : below) * kChunkBytes + pixel * kPixelBytes +
-                                                                       (((c >> 3) ^ ((pixel >> 1) & 3u)) << 4) + (c & 7u) * 2));
-              asm volatile("ld.shared.u16 %0, [%1];" : "=h"(tap) : "r"(weights_at + lane * (kTileC * 2) + c * 2));
-              asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(scratch + lane * 8), "f"(bf16_lo(value)), "f"(bf16_lo(tap)) : "memory");
-            }
             __syncwarp();
             float sum = 0.0f;
 #pragma unroll
             for (int t = 0; t < kTaps; t += 2) {
               uint32_t pair[4];
-              lds128(scratch + t * 8, pair);
+              lds128(from + t * 8, pair);
               sum = fmaf(__uint_as_float(pair[0]), __uint_as_float(pair[1]), sum);
               if (t + 1 < kTaps) sum = fmaf(__uint_as_float(pair[2]), __uint_as_float(pair[3]), sum);
             }
@@ -1000,7 +1017,7 @@ dw5x5_kernel(const __grid_constant__ CUtensorMap in_map, const __grid_constant__
             float out, unused;
             unpack2(activate2<ACT>(pack2(sum, sum)), out, unused);
             const uint32_t code = e4m3x2(out * (i == 0 ? inv[0] : i == 1 ? inv[1] : i == 2 ? inv[2] : inv[3]), 0.0f);
-            if (lane == owner) {
+            if (lane == first || lane == second) {
               if (p.tma_out) {
                 asm volatile("st.shared.u8 [%0], %1;" ::"r"(panel + (i * kTileX + lane) * 32 + (((piece >> 1) ^ ((lane >> 2) & 1)) << 4) + (c & 15u)), "r"(code) : "memory");
               } else if (alive) {
