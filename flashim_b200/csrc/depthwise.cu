@@ -72,6 +72,7 @@ constexpr float kSumError = 8.9e-7f;
 // The GELU passes on less than kGeluSlope of an argument's error (|GELU'| <= 1.129), and less than kGeluBase + kGeluGrowth * GELU
 // (|GELU'| <= 0.5 + 1.6 GELU for every argument); both with a tenth for the rounding of the polynomial.
 constexpr float kGeluSlope = 1.25f, kGeluBase = 0.55f, kGeluGrowth = 1.76f;
+constexpr float kGeluUnderflow = 12.743085f;  // minus the argument at which 2**q of gelu_phi2 falls below 2**-126
 // open codes that a warp corrects two by two (about 500 cycles); with more of them the quad does the step again (20000)
 constexpr int kMostOpen = 32;
 // The list of a quad: a header (count; flush and redo tags by step parity; MXFP8: error bounds of the four warps by step parity,
@@ -772,6 +773,7 @@ dw5x5_kernel(const __grid_constant__ CUtensorMap in_map, const __grid_constant__
         // for them is worth.)
         constexpr bool kTails = MODE == kOutMx && ACT == kActGelu;
         uint32_t tails = 0;  // bit c * 4 + i * 4 + d, c = 0, 4: channel c + d of pixel i is below -1, before the activation
+        uint32_t edge = 0;  // (as `pending` below) an argument at the underflow of Phi
         bool tail_warp = false;
         if (kTails) {
           tail_warp = error < 0.01f && __any_sync(0xffffffffu, largest + largest_bias > 5.0f);
@@ -783,6 +785,29 @@ dw5x5_kernel(const __grid_constant__ CUtensorMap in_map, const __grid_constant__
                 float lo, hi;
                 unpack2(add2(v[(n >> 2) * 4 + d][(n & 3) >> 1], pack2(1.0f, 1.0f)), lo, hi);
                 tails = __funnelshift_l(__float_as_uint(n & 1 ? hi : lo), tails, 1);
+              }
+            }
+            if (__any_sync(0xffffffffu, largest + largest_bias > 12.0f)) {
+              // where Phi underflows the value goes from below zero to +0, and its code from 0x80 to 0x00
+              float nearest = 1.0f;
+#pragma unroll
+              for (int c = 0; c < 8; ++c) {
+                float f[4];
+                unpack2(add2(v[c][0], pack2(kGeluUnderflow, kGeluUnderflow)), f[0], f[1]);
+                unpack2(add2(v[c][1], pack2(kGeluUnderflow, kGeluUnderflow)), f[2], f[3]);
+                nearest = min_abs(min_abs(nearest, f[0], f[1]), f[2], f[3]);
+              }
+              if (nearest < 2.0f * error + 1e-5f) {
+#pragma unroll
+                for (int c = 0; c < 8; ++c) {
+                  float f[4];
+                  unpack2(v[c][0], f[0], f[1]);
+                  unpack2(v[c][1], f[2], f[3]);
+#pragma unroll
+                  for (int i = 0; i < 4; ++i) {
+                    edge |= fabsf(f[i] + kGeluUnderflow) < 2.0f * error + 1e-5f ? 1u << (8 * (c & 3) + 7 - (2 * i + (c >> 2))) : 0u;
+                  }
+                }
               }
             }
           }
@@ -901,7 +926,7 @@ dw5x5_kernel(const __grid_constant__ CUtensorMap in_map, const __grid_constant__
               }
             }
           }
-          uint32_t any = 0;
+          uint32_t any = edge;
 #pragma unroll
           for (int i = 0; i < 4; ++i) any |= open[i][0] | open[i][1];
           if (__any_sync(0xffffffffu, any != 0)) {
@@ -910,6 +935,7 @@ dw5x5_kernel(const __grid_constant__ CUtensorMap in_map, const __grid_constant__
               const uint32_t bytes = open[k >> 1][k & 1];
               pending |= ((((bytes & 0x7F7F7F7Fu) + 0x7F7F7F7Fu) | bytes) & 0x80808080u) >> k;
             }
+            pending |= edge;
             const int rows = min(p.height - y, kStepRows);
             pending = x < p.width ? pending & ((0xFF00u >> (2 * rows) & 0xFFu) * 0x01010101u) : 0;
             if (__reduce_add_sync(0xffffffffu, __popc(pending)) > kMostOpen) {

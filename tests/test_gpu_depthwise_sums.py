@@ -144,6 +144,10 @@ def data(kind, shape, seed):
         x = F.interpolate(rand(batch, c, height // 8, width // 8), size=(height, width), mode="bicubic").permute(0, 2, 3, 1) + 3
         amplitude = torch.rand(5, 1, c, generator=g, device=DEV) * torch.tensor([1.0, 1.0, 0.0, -1.0, -1.0], device=DEV)[:, None, None]
         w, b = (amplitude.expand(5, 5, c) + 0.02 * rand(5, 5, c)).reshape(25, c), b * 0
+    elif kind == "underflow":  # flat, with arguments at -12.743085, where the GELU goes from below zero to +0
+        x, w, channel = rand(1, 1, 1, c).expand(shape).to(BF16), (rand(25, c) * 8).to(BF16), torch.arange(c, device=DEV)
+        at = torch.where(channel % 32 == 5, 3.0, -12.743084 + (channel % 9 - 4) * 1e-6)
+        b = (at - (x[0, 0, 0].double() * w.double()).sum(0)).float()
     elif kind == "flat":  # the sum of every window inside is what the roundings leave of zero
         x, w, b = rand(batch, 1, 1, c).expand(shape), zero_sum, b * 0
     elif kind == "heavy":
@@ -157,7 +161,7 @@ def data(kind, shape, seed):
 
 
 @pytest.mark.parametrize("act", ["gelu", "relu", "none"])
-@pytest.mark.parametrize("kind", ["normal", "wide", "smooth", "edges", "flat", "heavy", "sparse", "tiny"])
+@pytest.mark.parametrize("kind", ["normal", "wide", "smooth", "edges", "underflow", "flat", "heavy", "sparse", "tiny"])
 def test_mxfp8_is_that_of_the_chain(ctas, kind, act):
     """Every code and scale, on data whose sums keep their size and on data whose sums cancel (in a flat image every output is
     open), by the whole grid and by one CTA."""
