@@ -19,22 +19,24 @@
 //     or 16 bytes per pixel from registers instead costs a shared-memory wavefront per lane.
 //
 // Measured against the fp32-pipe kernel before it (B200, inputs in L2 where they fit):
-//   4x200x200x256: GELU -> bf16 68 -> 52 us, ReLU -> bf16 54 -> 42, GELU -> MXFP8 88 -> 83, ReLU -> INT8 87 -> 51
-//   8x400x400x128: GELU -> bf16 232 -> 160, ReLU -> bf16 183 -> 127 (80 % of the HBM copy rate), GELU -> MXFP8 303 -> 275,
-//   ReLU -> MXFP8 252 -> 189, ReLU -> INT8 299 -> 165
+//   4x200x200x256: GELU -> bf16 68 -> 52 us, ReLU -> bf16 54 -> 42, GELU -> MXFP8 88 -> 85, ReLU -> INT8 87 -> 51
+//   8x400x400x128: GELU -> bf16 232 -> 160, ReLU -> bf16 183 -> 127 (80 % of the HBM copy rate), GELU -> MXFP8 303 -> 282,
+//   ReLU -> MXFP8 252 -> 198, ReLU -> INT8 299 -> 165
 // What bounds the GELU and quantising forms now is the arithmetic of their epilogues on twelve warps per SM (issue slots about
 // half busy). The same bytes as the chain (below) cost the MXFP8 form up to a quarter of its time: 225 and 178 us with a test that
-// missed half of the codes that differ. Arguments of the GELU that reach its left tail take 350 us.
+// missed half of the codes that differ. Where the arguments of the GELU reach far into its left tail (a standard deviation of 1.5 and
+// up) it takes 360 us, more than the fp32-pipe kernel.
 //
 // Precision: the tensor cores add the exact products into fp32 accumulators, as the fp32 chain of the reference does (ky-major FMA
 // chain, bias last), but in another order; the two differ by up to about two fp32 ulp of the largest partial sum.
 //   MXFP8: the bytes of the chain. Every value has two bounds, itself less and plus the largest difference (error_of); where their
 //     codes differ (with normal data one in 1300) the output is summed again in the chain's order, at once and from shared memory.
 //     Where the exponents of the two bounds of a block's maximum differ, the block is noted in a list of the quad. No code or scale
-//     differed in 2.5 G of normal, wide and sparse data.
+//     differed in 4 G of normal, wide, sparse, smooth, edge-filtered and heavy-tailed data.
 //   bf16: outputs below 2**-14 of the sums in their column, where bias and products cancel, are noted (one in 30000). Others may
-//     lie one ulp of bf16 from the chain's where its sum lies next to a rounding boundary: one in 200000.
-//   INT8: likewise a code may lie one from the chain's: one in 4000000.
+//     lie one ulp of bf16 from the chain's where its sum lies next to a rounding boundary: one in 200000 of normal data, up to one in
+//     25000 where sums cancel.
+//   INT8: likewise a code may lie one from the chain's: one in 4000000, up to one in 400000.
 // The outputs and blocks of a list are summed again in the chain's order at the end of the quad's range or when the list fills up; a
 // step with more of them, or with more open codes, than is worth doing one by one is summed again as a whole. The bits of all
 // outputs thus depend on their own step alone, not on how the work is cut.
