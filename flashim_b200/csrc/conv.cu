@@ -34,6 +34,7 @@ constexpr int kConverterWarps = 8, kConvertThreads = kThreads + 32 * kConverterW
 constexpr int kRawStages = 2;                       // landing ring of bf16 tiles
 constexpr uint32_t kRawBytes = 128u * 128u * 2u;    // 128 pixels x 128 channels of bf16
 constexpr int kTileM = 128;
+constexpr uint32_t kSetupBarrier = 8;  // named barrier of all warps but the producer (1 to 4: the groups of the epilogue)
 constexpr uint32_t kTmemColumns = 512;
 constexpr int kMaxStages = 12;  // a short K loop is bound by the latency of a stage's round trip: more stages in flight
 constexpr int kSmemLimit = 226 * 1024;
@@ -564,8 +565,18 @@ conv_kernel(const __grid_constant__ CUtensorMap act_map, const __grid_constant__
     }
     grid_release();
   }
-  if (p.act == kActGelu) {
-    for (int i = threadIdx.x; i < kGeluEntries; i += kBlockThreads) {
+  tc_fence_before();
+  __syncthreads();  // barriers and tensor memory
+  if (PAIR) cluster_sync();  // the other CTA's barriers exist before anything refers to them
+  tc_fence_after();
+  const uint32_t tmem = ctl.tmem_base;
+  // The producer warp goes straight to its copies; what the others need from memory (the GELU table, the static activation scales,
+  // the bias) arrives beside them and is joined by a barrier of those warps alone. A pair's scales are read by its leader's copies to
+  // tensor memory in both CTAs: there both meet once more, producers included.
+  constexpr bool kEarlyCopies = !(PAIR && SCALED);
+  constexpr int kSetupThreads = kBlockThreads - 32;
+  if (warp != 0 && p.act == kActGelu) {
+    for (int i = threadIdx.x - 32; i < kGeluEntries; i += kSetupThreads) {
       const uint32_t entry = kGeluTable[i];
       for (int c = 0; c < gelu_copies; ++c) {
         asm volatile("st.shared.b32 [%0], %1;" ::"r"(smem_gelu + (i * gelu_copies + c) * 4), "r"(entry) : "memory");
@@ -588,18 +599,19 @@ conv_kernel(const __grid_constant__ CUtensorMap act_map, const __grid_constant__
     }
     fence_async_proxy();
   }
-  if (p.bias != nullptr) {
+  if (warp != 0 && p.bias != nullptr) {
     // the bias widened to fp32 once per CTA (zero for the columns a ragged last tile pads)
-    for (int i = threadIdx.x; i < p.tiles_n * BN; i += kBlockThreads) {
+    for (int i = threadIdx.x - 32; i < p.tiles_n * BN; i += kSetupThreads) {
       const float value = i < p.cout ? __bfloat162float(p.bias[i]) : 0.0f;
       asm volatile("st.shared.f32 [%0], %1;" ::"r"(smem_bias + i * 4), "f"(value) : "memory");
     }
   }
-  tc_fence_before();
-  __syncthreads();
-  if (PAIR) cluster_sync();  // the other CTA's barriers and static scale tiles exist before anything refers to them
-  tc_fence_after();
-  const uint32_t tmem = ctl.tmem_base;
+  if (!kEarlyCopies) {
+    __syncthreads();
+    cluster_sync();
+  } else if (warp != 0) {
+    named_barrier(kSetupBarrier, kSetupThreads);
+  }
   const uint32_t full0 = smem_u32(&ctl.full[0]), empty0 = smem_u32(&ctl.empty[0]);
   const uint32_t tfull0 = smem_u32(&ctl.tmem_full[0]), tempty0 = smem_u32(&ctl.tmem_empty[0]);
   const uint32_t raw_full0 = smem_u32(&ctl.raw_full[0]), raw_empty0 = smem_u32(&ctl.raw_empty[0]);
@@ -1597,22 +1609,29 @@ mlp_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constant__ CU
     tmem_relinquish();
     grid_release();
   }
-  for (int i = threadIdx.x; i < kGeluEntries; i += kMlpThreads) {
-    const uint32_t entry = kGeluTable[i];
+  tc_fence_before();
+  __syncthreads();  // barriers and tensor memory
+  tc_fence_after();
+  const uint32_t tmem = ctl.tmem_base;
+  // (as in conv_kernel: the producer warp goes straight to its copies)
+  constexpr int kSetupThreads = kMlpThreads - 32;
+  if (warp != 0) {
+    for (int i = threadIdx.x - 32; i < kGeluEntries; i += kSetupThreads) {
+      const uint32_t entry = kGeluTable[i];
 #pragma unroll
-    for (int c = 0; c < kMlpGeluCopies; ++c) {
-      asm volatile("st.shared.b32 [%0], %1;" ::"r"(smem_gelu + (i * kMlpGeluCopies + c) * 4), "r"(entry) : "memory");
+      for (int c = 0; c < kMlpGeluCopies; ++c) {
+        asm volatile("st.shared.b32 [%0], %1;" ::"r"(smem_gelu + (i * kMlpGeluCopies + c) * 4), "r"(entry) : "memory");
+      }
     }
   }
   grid_wait();
-  for (int i = threadIdx.x; i < 3 * C; i += kMlpThreads) {  // both biases widened to fp32 once per CTA
-    const float value = __bfloat162float(i < 2 * C ? p.bias1[i] : p.bias2[i - 2 * C]);
-    asm volatile("st.shared.f32 [%0], %1;" ::"r"(smem_bias1 + i * 4), "f"(value) : "memory");
+  if (warp != 0) {
+    for (int i = threadIdx.x - 32; i < 3 * C; i += kSetupThreads) {  // both biases widened to fp32 once per CTA
+      const float value = __bfloat162float(i < 2 * C ? p.bias1[i] : p.bias2[i - 2 * C]);
+      asm volatile("st.shared.f32 [%0], %1;" ::"r"(smem_bias1 + i * 4), "f"(value) : "memory");
+    }
+    named_barrier(kSetupBarrier, kSetupThreads);
   }
-  tc_fence_before();
-  __syncthreads();
-  tc_fence_after();
-  const uint32_t tmem = ctl.tmem_base;
   volatile int* abort_flag = &ctl.abort_flag;
   const uint32_t w_full0 = smem_u32(&ctl.w_full[0]), w_empty0 = smem_u32(&ctl.w_empty[0]);
   const uint32_t x_full = smem_u32(&ctl.x_full), x_empty = smem_u32(&ctl.x_empty);
