@@ -607,7 +607,7 @@ __device__ __forceinline__ float gelu_fast(float x) {
   return lo;
 }
 
-constexpr int kActNone = 0, kActRelu = 1, kActGelu = 2, kActReluEarly = 3;
+constexpr int kActNone = 0, kActRelu = 1, kActGelu = 2, kActReluEarly = 3, kActGeluSum = 4;
 __device__ __forceinline__ float activate(float x, int act) {
   if (act == kActRelu) return fmaxf(x, 0.0f);
   if (act == kActGelu) return gelu_erf(x);

@@ -201,6 +201,11 @@ __device__ __forceinline__ uint32_t idesc_bf16(int block_n, int block_m = kTileM
 // bf16 output that also writes the 2x2 max pool of its tiles as INT8 codes.
 constexpr uint32_t kPoolPanelBytes = 1024;  // 32 pooled pixels x 32 INT8 channels
 constexpr int kEpiGelu = 1, kEpiDynamic = 2, kEpiResidual = 4, kEpiLean = 8, kEpiFixed = 16, kEpiStatic = 32, kEpiPool = 64;
+// kEpiGeluSum (with kEpiFixed | kEpiStatic): the first product of a GELU MLP, whose bias is added behind the bf16 rounding and whose
+// GELU takes the fp32 sum, so that no table serves it: bf16(erf GELU(bf16(acc) + bias)) -> E4M3, the steps of
+// gelu_quantize_mx_kernel on the same values. A lane evaluates 32 error functions per chunk, which the main loop of a short K does not
+// hide; still the hidden tensor crosses memory once and as bytes, and a launch goes (MLP of 1000 x 256 x 1024: 18.0 -> 14.2 us, 20000 x 384 x 1536: 119 -> 69).
+constexpr int kEpiGeluSum = 256;
 
 // kPatch (with any of the epilogues above): a spatial conv whose whole weight matrix stays in shared memory and whose
 // activations arrive as one halo patch per tile instead of one shifted tile per tap. A tile is 8 columns x 16 rows of output
@@ -217,22 +222,23 @@ constexpr int kPatchTileW = 8, kPatchTileH = 16;
 struct EpilogueSwitches {
   int act, out_mode;
   uint32_t out_elem, panels;  // bytes per output element; output panels per group
-  bool has_bias, has_residual;
+  bool has_bias, has_residual, gelu_sum;  // gelu_sum: kEpiGeluSum, in the fixed epilogues alone
 };
 template <int EPI>
 __device__ __forceinline__ EpilogueSwitches epilogue_switches(const ConvParams& p) {
   EpilogueSwitches sw;
   if constexpr ((EPI & kEpiFixed) != 0) {
     sw.act = (EPI & kEpiGelu) ? kActGelu : kActNone;
+    sw.gelu_sum = (EPI & kEpiGeluSum) != 0;
     sw.out_mode = (EPI & kEpiStatic) ? FIM_OUT_E4M3_STATIC : ((EPI & kEpiDynamic) ? FIM_OUT_E4M3_DYNAMIC : FIM_OUT_BF16);
     sw.out_elem = sw.out_mode == FIM_OUT_BF16 ? 2u : 1u;
     sw.panels = (EPI & kPatch) != 0 ? static_cast<uint32_t>(p.panels_per_half) : 2u;
-    sw.has_bias = true;
+    sw.has_bias = !sw.gelu_sum;  // ahead of the bf16 rounding
     sw.has_residual = (EPI & kEpiResidual) != 0;
   } else {
     sw.act = p.act, sw.out_mode = p.out_mode;
     sw.out_elem = static_cast<uint32_t>(p.out_elem), sw.panels = static_cast<uint32_t>(p.panels_per_half);
-    sw.has_bias = p.bias != nullptr, sw.has_residual = p.residual != nullptr;
+    sw.has_bias = p.bias != nullptr, sw.has_residual = p.residual != nullptr, sw.gelu_sum = false;
   }
   return sw;
 }
@@ -336,9 +342,21 @@ __device__ __forceinline__ void round_chunk(const ConvParams& p, const EpilogueS
 // output format.
 template <bool INT8>
 __device__ __forceinline__ void finish_chunk(const ConvParams& p, const EpilogueSwitches& sw, uint32_t (&r)[16], int n, size_t pixel,
-                                             int b, int y, int x, bool valid, const GeluTable& gelu_table, uint32_t (&w)[16]) {
+                                             int b, int y, int x, bool valid, const GeluTable& gelu_table, uint32_t bias_at, uint32_t (&w)[16]) {
   const bool has_res = sw.has_residual;
-  if (sw.act == kActGelu) {
+  if (sw.gelu_sum) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      uint64_t b0, b1;
+      load_bias_pairs(bias_at, i, b0, b1);
+      float b[4];
+      unpack2(b0, b[0], b[1]);
+      unpack2(b1, b[2], b[3]);
+      const uint32_t v0 = r[2 * i], v1 = r[2 * i + 1];
+      r[2 * i] = pack_bf16(gelu_erf(bf16_lo(v0) + b[0]), gelu_erf(bf16_hi(v0) + b[1]));
+      r[2 * i + 1] = pack_bf16(gelu_erf(bf16_lo(v1) + b[2]), gelu_erf(bf16_hi(v1) + b[3]));
+    }
+  } else if (sw.act == kActGelu) {
 #pragma unroll
     for (int i = 0; i < 16; ++i) r[i] = gelu_bf16x2(r[i], gelu_table);
   } else if (sw.act == kActReluEarly || (sw.act == kActRelu && !has_res)) {
@@ -1466,7 +1484,7 @@ conv_kernel(const __grid_constant__ CUtensorMap act_map, const __grid_constant__
           const int n = n0 + cgroup * kGroupColumns + g * 32;
           if (n >= n_end) continue;  // uniform over the four warps of this group
           uint32_t w[16];
-          finish_chunk<INT8>(p, sw, q[g], n, pixel, b, y, x, valid, gelu_table, w);
+          finish_chunk<INT8>(p, sw, q[g], n, pixel, b, y, x, valid, gelu_table, smem_bias + static_cast<uint32_t>(n) * 4u, w);
           const uint32_t parity = chunk_it & 1u;
           if constexpr (pool && PATCH) {
             store_pooled(n, pool_in_warp(w));
@@ -2309,6 +2327,10 @@ int launch_conv_k(const ConvMaps& maps, const ConvParams& p, const Plan& pl, cud
         if (pl.block_k == 128) return launch_conv<FMT, BN, 128, false, kGeluStatic>(maps, p, pl, stream);
       }
     }
+    if (pl.fixed_epilogue == (kEpiFixed | kEpiStatic | kEpiGeluSum)) {
+      if constexpr (BN >= 128) return launch_conv<FMT, BN, 128, false, kEpiFixed | kEpiStatic | kEpiGeluSum>(maps, p, pl, stream);
+      return kUnsupported;
+    }
   }
   if constexpr (FMT == kFmtI8) {
     if (pl.fixed_epilogue == kEpiPool) {  // the general epilogue + the pooled second output
@@ -2366,7 +2388,7 @@ int run_conv(int fmt, const void* x, const int8_t* act_exponent, const void* act
   if (geometry == nullptr || ep == nullptr) return kBadArgument;
   if (geometry->batch == 0 || geometry->height == 0 || geometry->width == 0) return kOk;
   if (x == nullptr || weight == nullptr || out == nullptr) return kBadArgument;
-  if (ep->act < 0 || ep->act > 3 || ep->out_mode < 0 || ep->out_mode > 5) return kBadArgument;
+  if (ep->act < 0 || ep->act > 4 || ep->out_mode < 0 || ep->out_mode > 5) return kBadArgument;
   // the kernel counts K in bytes: a BF16 layer is a layer of 2 * Cin one-byte channels
   FimConvGeometry bytes = *geometry;
   if (fmt == kFmtBf16) {
@@ -2402,7 +2424,8 @@ int run_conv(int fmt, const void* x, const int8_t* act_exponent, const void* act
   bool allow_flat = !pool;  // pooling windows need the tile to be a patch of the image
   Plan pl;
   Schedule sc;
-  const bool gelu = ep->act == FIM_ACT_GELU;
+  const bool gelu = ep->act == FIM_ACT_GELU, gelu_sum = ep->act == FIM_ACT_GELU_SUM;
+  if (gelu_sum && (fmt != kFmtMx || convert || ep->out_mode != FIM_OUT_E4M3_STATIC || ep->bias == nullptr || ep->residual != nullptr)) return kUnsupported;
   int rc = plan_for(*g, fmt, per_pixel, allow_flat, out_elem, gelu, convert, pool, &pl, &sc);
   if (rc == kOk && allow_flat && pl.flat && ep->residual != nullptr) {
     const long long c = ep->res_stride[3], xs = ep->res_stride[2], ys = ep->res_stride[1], bs = ep->res_stride[0];
@@ -2410,6 +2433,7 @@ int run_conv(int fmt, const void* x, const int8_t* act_exponent, const void* act
     if (!dense) rc = plan_for(*g, fmt, per_pixel, false, out_elem, gelu, convert, pool, &pl, &sc);
   }
   if (rc != kOk) return rc;
+  if (gelu_sum && (!pl.flat || pl.pair || pl.block_n < 128 || pl.block_k != 128 || pl.panels_per_half != 2)) return kUnsupported;
   if (pool && (pl.out_h < 2 || pl.out_w < 2 || (pl.panels_per_half != 2 && !pl.patch))) return kUnsupported;  // no whole window: nothing to pool
 
   ConvParams p;
@@ -2539,6 +2563,7 @@ int run_conv(int fmt, const void* x, const int8_t* act_exponent, const void* act
   }
 
   if (pool) pl.fixed_epilogue = kEpiPool;
+  if (p.act == kActGeluSum) pl.fixed_epilogue = kEpiFixed | kEpiStatic | kEpiGeluSum;
 
   // scale tiles as tensors of 128 four-byte words per 512-byte tile: the loads of a CTA pair go through these
   maps.sfb = act_map, maps.sfa = act_map;

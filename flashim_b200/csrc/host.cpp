@@ -716,13 +716,27 @@ PyObject* mxfp8_gelu_mlp(Args a) {  // x, w1, b1, hidden_exponent, w2
   if (!packed1.defined() || !packed2.defined()) return nullptr;
   // the reference's rounding points: the first product rounds to bf16 before b1 is added, GELU runs in fp32 on that sum,
   // and the second product has no bias
-  const Tensor bias = b1->scalar_type() == kF32 && b1->is_contiguous() ? *b1 : b1->to(kF32).contiguous();
-  Tensor h = mx_gemm(*v, rows, e, nullptr, *w1, packed1, nullptr, call, "mxfp8_gelu_mlp");
   Tensor q = call.empty({rows, hidden}, kE4M3);
-  call.launch("mxfp8_gelu_mlp", [&] {
-    return abi.fim_gelu_quantize_mxfp8(h.data_ptr(), static_cast<const float*>(bias.data_ptr()), static_cast<const int8_t*>(he->data_ptr()),
-                                       q.data_ptr(), rows, hidden, call.stream);
-  });
+  int code = FIM_ERR_UNSUPPORTED;
+  if (b1->scalar_type() == kBF16 && b1->is_contiguous() && at16(*b1)) {  // all of it in the epilogue of the first product
+    const FimConvGeometry g = pointwise(rows, w1->size(1), hidden);
+    FimConvEpilogue ep = {};
+    ep.bias = b1->data_ptr(), ep.act = FIM_ACT_GELU_SUM, ep.out_mode = FIM_OUT_E4M3_STATIC;
+    ep.out_exponent = static_cast<const int8_t*>(he->data_ptr());
+    call.launch("mxfp8_gelu_mlp", [&] {
+      code = abi.fim_mxfp8_conv2d(v->data_ptr(), static_cast<const int8_t*>(e->data_ptr()), nullptr, w1->data_ptr(), packed1.data_ptr(), &g, &ep,
+                                  q.data_ptr(), call.status, call.stream);
+      return code == FIM_ERR_UNSUPPORTED ? 0 : code;
+    });
+  }
+  if (code == FIM_ERR_UNSUPPORTED) {  // a bias of another type, input channels that are no multiple of 128
+    const Tensor bias = b1->scalar_type() == kF32 && b1->is_contiguous() ? *b1 : b1->to(kF32).contiguous();
+    Tensor h = mx_gemm(*v, rows, e, nullptr, *w1, packed1, nullptr, call, "mxfp8_gelu_mlp");
+    call.launch("mxfp8_gelu_mlp", [&] {
+      return abi.fim_gelu_quantize_mxfp8(h.data_ptr(), static_cast<const float*>(bias.data_ptr()), static_cast<const int8_t*>(he->data_ptr()),
+                                         q.data_ptr(), rows, hidden, call.stream);
+    });
+  }
   return wrap(mx_gemm(q, rows, he, nullptr, *w2, packed2, nullptr, call, "mxfp8_gelu_mlp"));
 }
 

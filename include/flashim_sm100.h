@@ -37,6 +37,8 @@ extern "C" {
 #define FIM_ACT_RELU 1
 #define FIM_ACT_GELU 2
 #define FIM_ACT_RELU_EARLY 3 /* conv epilogues: ReLU before the residual add (the order of flashim/ops/gemm.py:87-98) */
+#define FIM_ACT_GELU_SUM 4   /* block-scaled 1x1 convs with a bias and FIM_OUT_E4M3_STATIC (cin % 128 == 0, else FIM_ERR_UNSUPPORTED): erf
+                              * GELU of bf16(product) + bias, the sum in fp32 (the order of flashim/ops/gemm.py:146-157) */
 
 /* What the conv epilogue writes. */
 #define FIM_OUT_BF16 0         /* bf16 [B,Ho,Wo,Cout] */

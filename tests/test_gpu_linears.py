@@ -152,3 +152,22 @@ def test_strided_golden_cases(ops, golden):
         want8 = g(f"i8{i}_out") if requant else g(f"i8{i}_out", BF16)
         assert same_bytes(got8.cpu(), want8), f"int8 golden case {i}"
     assert seen >= 1
+
+
+@pytest.mark.parametrize("rows,cin,hidden,bias", [
+    (1, 128, 32, BF16), (127, 128, 96, BF16), (129, 384, 512, BF16), (300, 256, 1056, BF16), (3000, 128, 288, BF16),
+    (40, 96, 128, BF16), (40, 128, 128, torch.float32),  # a separate GELU launch: channels, type of the bias
+])
+def test_gelu_mlp_in_the_epilogue_agrees_with_its_steps(ops, rows, cin, hidden, bias):
+    """GELU of the bf16 product plus bias and the quantiser behind it, in the epilogue of the first product: the bytes of the product,
+    gelu_quantize and the second product called one after another."""
+    from flashim_b200.quant import QuantizedWeight, calibrate_block32_exponent
+
+    g = torch.Generator(device=DEV).manual_seed(rows + cin)
+    rand = lambda *shape: torch.randn(shape, generator=g, device=DEV)  # noqa: E731
+    value = (rand(rows, cin) * 4).to(BF16)  # arguments of the GELU out to both of its ends
+    x = ops.quantize_mxfp8(value, calibrate_block32_exponent(value))
+    w1, w2 = QuantizedWeight.from_float(rand(hidden, cin) * cin ** -0.5), QuantizedWeight.from_float(rand(64, hidden) * hidden ** -0.5)
+    b1, exponent = rand(hidden).to(bias), torch.full((hidden // 32,), -6, dtype=torch.int8, device=DEV)
+    codes = ops.gelu_quantize(ops.mxfp8_linear(x, None, w1), exponent, input_bias=b1)
+    assert same_bytes(ops.mxfp8_gelu_mlp(x, w1, b1, exponent, w2), ops.mxfp8_linear(codes, None, w2))
