@@ -27,7 +27,27 @@ constexpr int kStatusWaitRows = 0x105;       // depthwise row ring barrier never
 
 __host__ __device__ constexpr int ceil_div(int a, int b) { return (a + b - 1) / b; }
 
+// Division of an index (of a tile, a pixel) by a run-time constant without the integer-division sequence (some forty instructions,
+// which a warp that owns 32 columns of a tile would pay several times per tile): q = floor(x * floor(2**32 / d) / 2**32) is the
+// quotient or one below it for every x < 2**32, so one compare-and-step finishes it. `magic` = floor(2**32 / d), or
+// 2**32 - 1 for d = 1 (which the same two steps turn into x).
+struct FastDiv {
+  uint32_t divisor, magic;
+};
+inline FastDiv make_fastdiv(int divisor) {
+  FastDiv f;
+  f.divisor = static_cast<uint32_t>(divisor < 1 ? 1 : divisor);
+  f.magic = f.divisor == 1 ? 0xFFFFFFFFu : static_cast<uint32_t>((1ull << 32) / f.divisor);
+  return f;
+}
 #if defined(__CUDACC__)
+
+__device__ __forceinline__ void divmod(int x, const FastDiv& f, int& quotient, int& remainder) {
+  uint32_t q = __umulhi(static_cast<uint32_t>(x), f.magic);
+  uint32_t r = static_cast<uint32_t>(x) - q * f.divisor;
+  if (r >= f.divisor) ++q, r -= f.divisor;
+  quotient = static_cast<int>(q), remainder = static_cast<int>(r);
+}
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return static_cast<uint32_t>(__cvta_generic_to_shared(p)); }
 

@@ -40,26 +40,6 @@ constexpr int kMaxStages = 12;  // a short K loop is bound by the latency of a s
 constexpr int kSmemLimit = 226 * 1024;
 constexpr int kMaxWeightSteps = 32;  // patch kernels: K steps (tap, channel chunk) whose weights have a barrier of their own
 
-// Division of a tile index by a run-time constant without the integer-division sequence (some forty instructions, which a
-// warp that owns 32 columns of a tile would pay several times per tile): q = floor(x * floor(2**32 / d) / 2**32) is the
-// quotient or one below it for every x < 2**32, so one compare-and-step finishes it. `magic` = floor(2**32 / d), or
-// 2**32 - 1 for d = 1 (which the same two steps turn into x).
-struct FastDiv {
-  uint32_t divisor, magic;
-};
-__host__ inline FastDiv make_fastdiv(int divisor) {
-  FastDiv f;
-  f.divisor = static_cast<uint32_t>(divisor < 1 ? 1 : divisor);
-  f.magic = f.divisor == 1 ? 0xFFFFFFFFu : static_cast<uint32_t>((1ull << 32) / f.divisor);
-  return f;
-}
-__device__ __forceinline__ void divmod(int x, const FastDiv& f, int& quotient, int& remainder) {
-  uint32_t q = __umulhi(static_cast<uint32_t>(x), f.magic);
-  uint32_t r = static_cast<uint32_t>(x) - q * f.divisor;
-  if (r >= f.divisor) ++q, r -= f.divisor;
-  quotient = static_cast<int>(q), remainder = static_cast<int>(r);
-}
-
 struct ConvParams {
   int cin, cout, out_h, out_w;
   int kh, kw, pad_h, pad_w, dil_h, dil_w, stride_h, stride_w;

@@ -8,6 +8,8 @@
 // dot products of f_a / sqrt(P) with each pixel of the patch (eight lanes per patch pixel, f_a from shared memory),
 // then every correlation value is the bilinear blend of four neighbouring dot products: (2r+2)^2 reads of P channels
 // instead of 4 (2r+1)^2. The four centre pixels of the patch are also the corners of the f_b sample.
+#include <type_traits>
+
 #include "common.cuh"
 #include "flashim_sm100.h"
 
@@ -28,6 +30,8 @@ struct InputParams {
   __nv_bfloat16* out;       // [B, h, w, 2P + E + K]
   int batch, height, width, features, embedding, radius, pair;
   float scale_x, scale_y, root_features;
+  FastDiv div_width, div_height;  // and the reciprocals of both
+  float inv_width, inv_height;
 };
 
 __device__ __forceinline__ void store_bf16(__nv_bfloat16* at, float v) { *at = __float2bfloat16_rn(v); }
@@ -136,14 +140,42 @@ __global__ void __launch_bounds__(32 * kInputWarps) refiner_input_kernel(const I
   }
 }
 
-// The same rows for P = 32 NF features (the widths RoMaV2 uses), arranged for latency and for whole sectors: f_a stays in
+// N consecutive floats, loaded as one word
+template <int N>
+struct Floats {
+  float v[N];
+};
+template <int N>
+__device__ __forceinline__ Floats<N> load_floats(const float* at) {
+  Floats<N> r;
+  if constexpr (N == 1) {
+    r.v[0] = __ldg(at);
+  } else if constexpr (N == 2) {
+    const float2 q = __ldg(reinterpret_cast<const float2*>(at));
+    r.v[0] = q.x, r.v[1] = q.y;
+  } else {
+    const float4 q = __ldg(reinterpret_cast<const float4*>(at));
+    r.v[0] = q.x, r.v[1] = q.y, r.v[2] = q.z, r.v[3] = q.w;
+  }
+  return r;
+}
+
+// n / d from inv = RN(1 / d): the quotient, corrected once by its exact residual
+__device__ __forceinline__ float divided(float n, float d, float inv) {
+  const float q = n * inv;
+  return fmaf(fmaf(-q, d, n), inv, q);
+}
+
+// The same rows for P = 32 NF features (the widths RoMaV2 uses), arranged for instructions, latency and whole sectors: f_a stays in
 // registers, the patch pixels of several steps are in flight together, the eight partial sums a group of lanes gathers in
 // eight steps are added by one transposing butterfly (7 shuffles instead of 24, each sum over the same pairs of lanes as
 // above; the division by sqrt(P) comes last, once per value), the radius is a constant of the code, and the eight rows of a block, which are contiguous in the output, go through shared memory and
 // leave as 16-byte words instead of single bf16 values. The kernel above waits for one pair of loads per four patch pixels.
-// Refiner input + heads of both directions of a pair, 96x72x64, radius 3: 45 -> 23 us; 200x200x128, radius 2: 225 -> 147.
-// (Four CTAs with half as many loads in flight against three with twice as many: 119 against 129 us for the latter's input
-// rows; five or more CTAs spill.)
+// What bounds it is the issue of instructions (62 % of the slots while an SM had work, 960 per pixel of 96x72x64 with radius 3, of which
+// 128 are the products). A patch that lies inside the image (nearly all do) therefore takes code without a bounds test,
+// a select or an address per load. Input rows, before -> after (us): 2x96x72x64, radius 3 18.4 -> 17.1; 2x100x140x64, radius 2 29.2 -> 23.9;
+// 4x300x300x64, radius 3 453 -> 394; 2x200x200x128, radius 2 120 -> 109; 2x100x100x32, radius 3 19.5 -> 16.3. (Three CTAs, or twice the
+// loads in flight, are slower at most sizes.)
 template <int NF, int R>
 __global__ void __launch_bounds__(32 * kInputWarps, 4) refiner_input_wide_kernel(const InputParams p) {
   grid_release();
@@ -160,10 +192,10 @@ __global__ void __launch_bounds__(32 * kInputWarps, 4) refiner_input_wide_kernel
   for (unsigned first = blockIdx.x * kInputWarps; first < pixels; first += gridDim.x * kInputWarps) {
     const unsigned flat = first + warp_id;
     if (flat < pixels) {
-      const int x = static_cast<int>(flat % static_cast<unsigned>(p.width));
-      const int y = static_cast<int>((flat / static_cast<unsigned>(p.width)) % static_cast<unsigned>(p.height));
-      const int b = static_cast<int>(flat / (static_cast<unsigned>(p.width) * static_cast<unsigned>(p.height)));
-      const int b_other = p.pair > 0 ? (b + p.batch - p.pair) % p.batch : b;
+      int x, y, b;
+      divmod(static_cast<int>(flat), p.div_width, y, x);
+      divmod(y, p.div_height, b, y);
+      const int b_other = p.pair > 0 ? (b >= p.pair ? b - p.pair : b + p.batch - p.pair) : b;
       const float* other = p.f_b + static_cast<long long>(b_other) * p.height * p.width * P;
       const float2 at = __ldg(reinterpret_cast<const float2*>(p.warp) + flat);
       float4 a[NF];  // channels 4 sub + 32 i, in every group
@@ -176,78 +208,102 @@ __global__ void __launch_bounds__(32 * kInputWarps, 4) refiner_input_wide_kernel
       const int x0 = static_cast<int>(fminf(fmaxf(fx0, -16.0f), static_cast<float>(p.width) + 16.0f));
       const int y0 = static_cast<int>(fminf(fmaxf(fy0, -16.0f), static_cast<float>(p.height) + 16.0f));
       const bool finite = fabsf(ix) < 1e9f && fabsf(iy) < 1e9f;
-      const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
-      // f_b at the warp: a lane per four channels; the corners are patch pixels too
-      if (lane < P / 4) {
+      const long long line = static_cast<long long>(p.width) * P;  // floats of an image row
+      // (uniform over the warp)
+      const bool inside = finite && x0 >= R && y0 >= R && x0 + R + 1 < p.width && y0 + R + 1 < p.height;
+      // f_b at the warp, NF channels per lane; the corners are patch pixels too
+      {
         const bool north = finite && y0 >= 0 && y0 < p.height, south = finite && y0 + 1 >= 0 && y0 + 1 < p.height;
         const bool west = x0 >= 0 && x0 < p.width, east = x0 + 1 >= 0 && x0 + 1 < p.width;
-        const float* base = other + (static_cast<long long>(y0) * p.width + x0) * P + 4 * lane;
-        const long long down = static_cast<long long>(p.width) * P;
-        const float4 nw = north && west ? __ldg(reinterpret_cast<const float4*>(base)) : zero;
-        const float4 ne = north && east ? __ldg(reinterpret_cast<const float4*>(base + P)) : zero;
-        const float4 sw = south && west ? __ldg(reinterpret_cast<const float4*>(base + down)) : zero;
-        const float4 se = south && east ? __ldg(reinterpret_cast<const float4*>(base + down + P)) : zero;
-        __nv_bfloat16* to = row + P + 4 * lane;
-        store_bf16(to, nw.x * w_nw + ne.x * w_ne + sw.x * w_sw + se.x * w_se);
-        store_bf16(to + 1, nw.y * w_nw + ne.y * w_ne + sw.y * w_sw + se.y * w_se);
-        store_bf16(to + 2, nw.z * w_nw + ne.z * w_ne + sw.z * w_sw + se.z * w_se);
-        store_bf16(to + 3, nw.w * w_nw + ne.w * w_ne + sw.w * w_sw + se.w * w_se);
-      }
-      if (group == 0) {
-#pragma unroll
-        for (int i = 0; i < NF; ++i) {
-          __nv_bfloat16* to = row + 32 * i + 4 * sub;
-          store_bf16(to, a[i].x), store_bf16(to + 1, a[i].y), store_bf16(to + 2, a[i].z), store_bf16(to + 3, a[i].w);
+        const float* base = other + y0 * line + static_cast<long long>(x0) * P + NF * lane;
+        Floats<NF> nw = {}, ne = {}, sw = {}, se = {};
+        if (inside) {
+          nw = load_floats<NF>(base), ne = load_floats<NF>(base + P), sw = load_floats<NF>(base + line), se = load_floats<NF>(base + line + P);
+        } else {
+          if (north && west) nw = load_floats<NF>(base);
+          if (north && east) ne = load_floats<NF>(base + P);
+          if (south && west) sw = load_floats<NF>(base + line);
+          if (south && east) se = load_floats<NF>(base + line + P);
         }
+#pragma unroll
+        for (int i = 0; i < NF; ++i) store_bf16(row + P + NF * lane + i, nw.v[i] * w_nw + ne.v[i] * w_ne + sw.v[i] * w_sw + se.v[i] * w_se);
+      }
+      // f_a itself: every lane one of the four channels that its group and the three others hold
+#pragma unroll
+      for (int i = 0; i < NF; ++i) {
+        const float lower = group & 1 ? a[i].y : a[i].x, upper = group & 1 ? a[i].w : a[i].z;
+        store_bf16(row + 32 * i + 4 * sub + group, group & 2 ? upper : lower);
       }
       // dot products with the patch pixels, a group of eight lanes per pixel, eight pixels of a group per butterfly
+      const auto form_dots = [&](auto unchecked) {
+        constexpr bool kInside = decltype(unchecked)::value;
+        const float* corner = other + (y0 - R) * line + static_cast<long long>(x0 - R) * P + 4 * sub;
+        if (kInside && side % 4 == 0) corner += group * P;
 #pragma unroll
-      for (int base = 0; base < side * side; base += 32) {
-        float sum[8];
+        for (int base = 0; base < side * side; base += 32) {
+          float sum[8];
 #pragma unroll
-        for (int ahead = 0; ahead < 8; ahead += kAhead) {
-          float4 v[kAhead][NF];
+          for (int ahead = 0; ahead < 8; ahead += kAhead) {
+            float4 v[kAhead][NF];
 #pragma unroll
-          for (int q = 0; q < kAhead; ++q) {
-            const int pos = base + 4 * (ahead + q) + group;
-            const int yy = y0 - R + pos / side, xx = x0 - R + pos % side;
-            const bool in = base + 4 * (ahead + q) < side * side && finite && pos < side * side &&
-                            static_cast<unsigned>(yy) < static_cast<unsigned>(p.height) && static_cast<unsigned>(xx) < static_cast<unsigned>(p.width);
-            const float* src = other + static_cast<long long>(yy * p.width + xx) * P;  // (below 2**31 pixels)
+            for (int q = 0; q < kAhead; ++q) {
+              const int step = base + 4 * (ahead + q), pos = step + group;  // `step`: a constant of the unrolled code
+              if (kInside && step < side * side) {
+                const float* src;
+                if (side % 4 == 0) {  // the four groups' pixels are neighbours
+                  src = corner + step / side * line + step % side * P;
+                } else {  // (36 pixels, or 4)
+                  src = corner + pos / side * line + pos % side * P;
+                }
 #pragma unroll
-            for (int i = 0; i < NF; ++i) v[q][i] = in ? __ldg(reinterpret_cast<const float4*>(src + 32 * i) + sub) : zero;
-          }
+                for (int i = 0; i < NF; ++i) v[q][i] = __ldg(reinterpret_cast<const float4*>(src + 32 * i));
+              } else {
+                const int yy = y0 - R + pos / side, xx = x0 - R + pos % side;
+                const bool in = step < side * side && finite && static_cast<unsigned>(yy) < static_cast<unsigned>(p.height) &&
+                                static_cast<unsigned>(xx) < static_cast<unsigned>(p.width);
+                const float* src = corner + pos / side * line + pos % side * P;
 #pragma unroll
-          for (int q = 0; q < kAhead; ++q) {
-            float t = 0.0f;
-#pragma unroll
-            for (int i = 0; i < NF; ++i) {
-              t = fmaf(a[i].x, v[q][i].x, t), t = fmaf(a[i].y, v[q][i].y, t), t = fmaf(a[i].z, v[q][i].z, t), t = fmaf(a[i].w, v[q][i].w, t);
+                for (int i = 0; i < NF; ++i) v[q][i] = in ? __ldg(reinterpret_cast<const float4*>(src + 32 * i)) : make_float4(0.f, 0.f, 0.f, 0.f);
+              }
             }
-            sum[ahead + q] = t;
+#pragma unroll
+            for (int q = 0; q < kAhead; ++q) {
+              float t = 0.0f;
+#pragma unroll
+              for (int i = 0; i < NF; ++i) {
+                t = fmaf(a[i].x, v[q][i].x, t), t = fmaf(a[i].y, v[q][i].y, t), t = fmaf(a[i].z, v[q][i].z, t), t = fmaf(a[i].w, v[q][i].w, t);
+              }
+              sum[ahead + q] = t;
+            }
           }
-        }
-        float half[4], quarter[2];
-        const bool odd = sub & 1, second = sub & 2, fourth = sub & 4;
+          float half[4], quarter[2];
+          const bool odd = sub & 1, second = sub & 2, fourth = sub & 4;
 #pragma unroll
-        for (int i = 0; i < 4; ++i) half[i] = (odd ? sum[2 * i + 1] : sum[2 * i]) + __shfl_xor_sync(0xffffffffu, odd ? sum[2 * i] : sum[2 * i + 1], 1);
+          for (int i = 0; i < 4; ++i) half[i] = (odd ? sum[2 * i + 1] : sum[2 * i]) + __shfl_xor_sync(0xffffffffu, odd ? sum[2 * i] : sum[2 * i + 1], 1);
 #pragma unroll
-        for (int i = 0; i < 2; ++i) {
-          quarter[i] = (second ? half[2 * i + 1] : half[2 * i]) + __shfl_xor_sync(0xffffffffu, second ? half[2 * i] : half[2 * i + 1], 2);
+          for (int i = 0; i < 2; ++i) {
+            quarter[i] = (second ? half[2 * i + 1] : half[2 * i]) + __shfl_xor_sync(0xffffffffu, second ? half[2 * i] : half[2 * i + 1], 2);
+          }
+          const float total = (fourth ? quarter[1] : quarter[0]) + __shfl_xor_sync(0xffffffffu, fourth ? quarter[0] : quarter[1], 4);
+          const int pos = base + 4 * sub + group;  // the lane's own step
+          if (pos < side * side) dot[pos] = NF == 2 ? total * 0.125f : total / p.root_features;  // (64 features: exact either way)
         }
-        const float total = (fourth ? quarter[1] : quarter[0]) + __shfl_xor_sync(0xffffffffu, fourth ? quarter[0] : quarter[1], 4);
-        const int pos = base + 4 * sub + group;  // the lane's own step
-        if (pos < side * side) dot[pos] = total / p.root_features;
+      };
+      if (inside) {
+        form_dots(std::true_type{});
+      } else {
+        form_dots(std::false_type{});
       }
       {
-        const float dx = p.scale_x * (at.x - (-1.0f + (2.0f * x + 1.0f) / p.width));
-        const float dy = p.scale_y * (at.y - (-1.0f + (2.0f * y + 1.0f) / p.height));
+        const float dx = p.scale_x * (at.x - (-1.0f + divided(2.0f * x + 1.0f, p.width, p.inv_width)));
+        const float dy = p.scale_y * (at.y - (-1.0f + divided(2.0f * y + 1.0f, p.height, p.inv_height)));
         for (int e = lane; e < E; e += 32) {
           const float2 weight = __ldg(reinterpret_cast<const float2*>(p.emb_weight) + e);
           store_bf16(row + 2 * P + e, fmaf(weight.y, dy, weight.x * dx) + __ldg(p.emb_bias + e));
         }
       }
       __syncwarp();
+#pragma unroll
       for (int k = lane; k < K; k += 32) {
         const int at_patch = (k / window) * side + k % window;
         const float v = dot[at_patch] * w_nw + dot[at_patch + 1] * w_ne + dot[at_patch + side] * w_sw + dot[at_patch + side + 1] * w_se;
@@ -339,6 +395,8 @@ extern "C" int fim_romav2_refiner_input(const float* f_a, const float* f_b, cons
   p.batch = batch, p.height = height, p.width = width, p.features = features, p.embedding = embedding, p.radius = radius, p.pair = pair;
   p.scale_x = scale_x, p.scale_y = scale_y;
   p.root_features = static_cast<float>(sqrt(static_cast<double>(features)));
+  p.div_width = make_fastdiv(width), p.div_height = make_fastdiv(height);
+  p.inv_width = 1.0f / static_cast<float>(width), p.inv_height = 1.0f / static_cast<float>(height);
   const long long pixels = static_cast<long long>(batch) * height * width;
   if (pixels >= 0x7fffffffLL) return kUnsupported;
   if (radius < 0) {

@@ -85,3 +85,23 @@ def test_refiner_input_golden(ops, golden):
             *to_dev(g(f"rin{i}_fa"), g(f"rin{i}_fb"), g(f"rin{i}_warp"), g(f"rin{i}_ew"), g(f"rin{i}_eb"), torch.tensor([3.0, 2.0])),
             radius, pair)
         _close(got.permute(0, 2, 3, 1), g(f"rin{i}_out", BF16), f"golden case {i}")
+
+
+@pytest.mark.parametrize("case", [(2, 41, 36, 64, 32, 3, 1), (1, 33, 47, 32, 8, 2, 0), (2, 30, 31, 128, 16, 3, 1), (1, 40, 9, 64, 1, 1, 0), (1, 7, 50, 32, 3, 0, 0)])
+def test_refiner_input_patches_inside_and_across_the_edges(ops, case):
+    """A patch inside the image is read without bounds tests: images of which most pixels, and only some, have one, with positions
+    that end exactly at the edges."""
+    test_refiner_input(ops, case)
+    b, h, w, p, e, radius, pair = case
+    g = torch.Generator().manual_seed(9)
+    f = torch.randn(b, h, w, p, generator=g)
+    gy, gx = torch.meshgrid((torch.arange(h) * 2 + 1) / h - 1, (torch.arange(w) * 2 + 1) / w - 1, indexing="ij")
+    # whole and half pixels beside the pixel's own place
+    warp = torch.stack((gx, gy), -1) + torch.randint(-3, 4, (b, h, w, 2), generator=g) * torch.tensor([1.0 / w, 1.0 / h])
+    rest = torch.randn(e, 2, 1, 1, generator=g), torch.randn(e, generator=g), torch.tensor([3.0, 2.0])
+    want = oracle.romav2_refiner_input(f, f, warp, *rest, radius, pair)
+    got = ops.romav2_refiner_input(*to_dev(f, f, warp, *rest), radius, pair).cpu()
+    # Positions that fall on a pixel may round to either side of it: four roundings of up to 48 pixels (2e-6 each) move a sample, or
+    # a correlation, by at most 8e-6 times the difference of two neighbours, below 10 for these values.
+    bad = (bf16_ulp_distance(got, want) > 1) & ((got.float() - want.float()).abs() > 1e-4)
+    assert not bad.any()
