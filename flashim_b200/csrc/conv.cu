@@ -1259,8 +1259,13 @@ conv_kernel(const __grid_constant__ CUtensorMap act_map, const __grid_constant__
     const float a_scale = INT8 && p.a_scale != nullptr ? __ldg(p.a_scale) : 1.0f;
     const uint32_t panels = smem_out + group * sw.panels * panel_bytes_;
     // A flat 1x1 conv (a tile = 128 consecutive rows of the pixel matrix) lets every warp stage and store its own 32 rows:
-    // the four warps of a group then never wait for each other. The panels take the same shared memory either way.
-    const bool own = p.warp_panels != 0;
+    // the four warps of a group then never wait for each other. The panels take the same shared memory either way. So does a patch
+    // tile, of which a warp has four image rows of eight pixels: three barriers per chunk less. Only a 64-wide tile whose epilogue is
+    // little more than its store (the host's choice) keeps the shared panels, since four times as many stores cost it more. us at
+    // 4x800x800x64, GELU + requantisation 153 -> 135, plain 114 with shared panels, 117 with own ones; INT8 4x201x199x128 21.4 -> 19.4,
+    // with the pooled output 25.4 -> 21.8, 4x400x400x64 39.5 -> 33.8.
+    constexpr bool kAlwaysOwn = PATCH && (BN == 128 || (EPI & (kEpiFixed | kEpiPool)) != 0);
+    const bool own = kAlwaysOwn || p.warp_panels != 0;
     const uint32_t own_bytes = 1024u * sw.out_elem;
     const uint32_t own_panels = smem_out + static_cast<uint32_t>(warp - 2) * sw.panels * own_bytes;
     const bool store = !(probe_flags(p) & 4);
@@ -1361,7 +1366,7 @@ conv_kernel(const __grid_constant__ CUtensorMap act_map, const __grid_constant__
         if (own) {
           __syncwarp();
           if (store && elect_one()) {
-            tma_store_4d(&out_warp_map, panel, n * static_cast<int>(sw.out_elem), x0 + quarter * 32, y0, b);
+            tma_store_4d(&out_warp_map, panel, n * static_cast<int>(sw.out_elem), PATCH ? x0 : x0 + quarter * 32, PATCH ? y0 + quarter * 4 : y0, b);
             bulk_commit();
           }
           return;
@@ -2517,7 +2522,12 @@ int run_conv(int fmt, const void* x, const int8_t* act_exponent, const void* act
       if (rcw != kOk) return rcw;
       p.warp_panels = 1;
     }
-    if (pool) {  // the pooled output [B, Ho / 2, Wo / 2, Cout] INT8, stored in boxes of a quarter tile x 32 channels
+    if (pl.patch) {  // (a patch kernel's warps store four image rows of a tile each)
+      const uint32_t warp_box[4] = {static_cast<uint32_t>(32 * out_elem), kPatchTileW, kPatchTileH / 4, 1};
+      const int rcw = make_tensor_map(&maps.out_warp, CU_TENSOR_MAP_DATA_TYPE_UINT8, 4, out, dims, strides, warp_box, swizzle_for_bytes(32 * out_elem));
+      if (rcw != kOk) return rcw;
+      p.warp_panels = pl.block_n == 128 || out_elem == 1 || p.act == kActGelu || p.residual != nullptr ? 1 : 0;
+    } else if (pool) {  // the pooled output [B, Ho / 2, Wo / 2, Cout] INT8, stored in boxes of a quarter tile x 32 channels
       const uint64_t prow = static_cast<uint64_t>(g->cout), ph = static_cast<uint64_t>(pl.out_h / 2), pw = static_cast<uint64_t>(pl.out_w / 2);
       const uint64_t pdims[4] = {prow, pw, ph, static_cast<uint64_t>(o_b)};
       const uint64_t pstrides[3] = {prow, pw * prow, ph * pw * prow};

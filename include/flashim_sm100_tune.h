@@ -20,7 +20,7 @@ extern "C" {
  *   128  enables pairs for block-scaled 256-wide tiles too;
  *   256  reloads the weight scales for every tile instead of keeping the first K iterations resident in tensor memory;
  *   512  makes the four warps of an epilogue group of a 1x1 conv share one output panel and one store (as the spatial
- *        convs do) instead of one per warp;
+ *        convs without halo patches do) instead of one per warp;
  *  1024  sends every call through the general epilogue instead of the ones whose switches are fixed at compile time;
  *  2048  streams the weights of a layer (and the activations tap by tap, instead of one halo patch per tile) through the
  *        stage ring even where they are kept in shared memory by default;
