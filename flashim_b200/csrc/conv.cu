@@ -50,6 +50,7 @@ struct ConvParams {
   int batch;       // images (rows of a flattened 1x1 conv count as one)
   int full_tiles;  // tiles [0, full_tiles) are BN wide; the rest are the halves (BN / 2 columns) of the last few tiles
   int k_chunks, stages;
+  int last_steps;  // 32-channel MMAs of a tap's last channel chunk: all of them, or fewer with ragged K steps (kKSteps = 4 only)
   int resident_k;  // weight-scale tiles of the first resident_k K iterations stay in tensor memory from tile to tile
   int panels_per_half;  // output panels each column group of the epilogue rotates through (1 or 2)
   // scales (MXFP8)
@@ -197,6 +198,13 @@ constexpr int kEpiGeluSum = 256;
 //   MXFP8 3x3 + bias + GELU + static requantisation, N = 4: 800x800x64 363 -> 154 us, 400x400x128 117 -> 92 (with a plain
 //   bf16 output 107 -> 70); INT8 3x3 + bias: 4x201x199x128 31 -> 20, 4x400x400x64 84 -> 32.
 constexpr int kPatch = 128;
+// Ragged K steps: input channels that 128 does not divide (96, 160, 192, ...) go in 128-byte steps all the same. The last step of a tap
+// has only as many MMAs as it has 32-channel blocks; what its boxes bring beyond them (zeros of the activations, the next tap's weights)
+// is not multiplied. A step's weight scales may then lie in two scale tiles, so all of them stay in tensor memory: a step brings the
+// one that begins in it when the tile's output channels are new. Steps of 64 or 32 bytes, the widest that divide such channel counts,
+// took two or three barrier rounds and copies (of a strided conv: element by element) for the same MMAs. us: MXFP8 3x3 3x75x101x96 ->
+// 160, stride 2 14.4 -> 11.4; 2x200x190x192 68.5 -> 60.5; 3x100x120x96 15.4 -> 13.9; 1x1 4x200x200x192 + residual 50.2 -> 46.2;
+// INT8 3x175x101x96 -> 160, stride 2 14.0 -> 10.3; 1x1 4x100x90x160 10.7 -> 9.2.
 constexpr int kPatchTileW = 8, kPatchTileH = 16;
 
 struct EpilogueSwitches {
@@ -641,6 +649,9 @@ conv_kernel(const __grid_constant__ CUtensorMap act_map, const __grid_constant__
       bool alive = true;
       int last_n0 = -1;
       const bool resident_b = in_register(static_cast<uint32_t>(p.weights_resident)) != 0;
+      // bytes of a tap's last channel chunk along the weight's K axis
+      const int last_bytes = static_cast<int>(in_register(static_cast<uint32_t>(BK == 128 ? p.last_steps * 32 : BK)));
+      const bool ragged = BK == 128 && last_bytes != BK;
       if constexpr (PATCH) {
         // one patch per tile; behind the first one the weights, K step by K step, which the first tile's MMAs wait for singly
         const int k_total = kh * kw * k_chunks;
@@ -661,11 +672,14 @@ conv_kernel(const __grid_constant__ CUtensorMap act_map, const __grid_constant__
           if (first) {
             first = false;
             const uint32_t step0 = smem_u32(&ctl.weights_step[0]);
-            const int scale_tiles = SCALED ? (k_total * kKSteps + 3) / 4 : 0;
-            for (int ki = 0; ki < k_total; ++ki) {
+            const int scale_tiles = SCALED ? p.weight_scale_tiles : 0;
+            for (int ki = 0, j = 0, k0 = 0; ki < k_total; ++ki) {
               mbar_expect_tx_addr(step0 + 8 * ki, kBBytes + (ki == 0 ? scale_tiles * 512u : 0u));
               if (ki == 0 && SCALED) bulk_load_addr(smem_sfb, p.weight_scales, scale_tiles * 512u, step0);
-              tma_load_2d_addr(smem_b + ki * kBBytes, &weight_map, step0 + 8 * ki, ki * BK, 0);
+              tma_load_2d_addr(smem_b + ki * kBBytes, &weight_map, step0 + 8 * ki, k0, 0);
+              const bool last = ++j == k_chunks;
+              k0 += last ? last_bytes : BK;
+              if (last) j = 0;
             }
           }
         }
@@ -675,12 +689,14 @@ conv_kernel(const __grid_constant__ CUtensorMap act_map, const __grid_constant__
         // and scale tiles are copied once and stay; the loop below then moves activations only.
         const int k_total = kh * kw * k_chunks;
         mbar_expect_tx_addr(smem_u32(&ctl.weights_ready), static_cast<uint32_t>(k_total) * (kBBytes + (SCALED ? kScaleTilesB * 512u : 0u)));
-        for (int ki = 0; ki < k_total; ++ki) {
+        for (int ki = 0, j = 0, k0 = 0; ki < k_total; ++ki) {
 #pragma unroll
           for (int part = 0; part < BN / kWeightBoxRows; ++part) {
-            tma_load_2d_addr(smem_b + ki * kBBytes + part * kWeightBoxRows * BK, &weight_map, smem_u32(&ctl.weights_ready), ki * BK,
-                             part * kWeightBoxRows);
+            tma_load_2d_addr(smem_b + ki * kBBytes + part * kWeightBoxRows * BK, &weight_map, smem_u32(&ctl.weights_ready), k0, part * kWeightBoxRows);
           }
+          const bool last = ++j == k_chunks;
+          k0 += last ? last_bytes : BK;
+          if (last) j = 0;
           if (SCALED) {
 #pragma unroll
             for (int i = 0; i < kScaleTilesB; ++i) {
@@ -726,7 +742,11 @@ conv_kernel(const __grid_constant__ CUtensorMap act_map, const __grid_constant__
         for (int ky = 0; ky < kh && alive; ++ky) {
           for (int kx = 0; kx < kw && alive; ++kx) {
             const int cx = x0 + kx * dil_w, cy = y0 + ky * dil_h;
-            for (int j = 0; j < k_chunks; ++j, k0 += BK) {
+            for (int j = 0; j < k_chunks; ++j) {
+              const int step_bytes = BK == 128 && j + 1 == k_chunks ? last_bytes : BK;
+              // ragged: the scale tile that begins in this step, if any
+              const int new_tile = (k0 + step_bytes - 32) >> 7;
+              const bool begins = new_tile != (k0 - 32) >> 7;
               if (CONVERT) {
                 // the bf16 tile of this K step into the landing ring: 128 rows of the pixel matrix x 128 channels
                 if (!loop_wait(raw_empty0 + 8 * raw_s, raw_phase ^ 1, kStatusWaitEmpty)) {
@@ -744,7 +764,7 @@ conv_kernel(const __grid_constant__ CUtensorMap act_map, const __grid_constant__
                 break;
               }
               const uint32_t bar = PAIR ? ((full0 + 8 * s) & ~kPeerBit) : full0 + 8 * s;
-              const bool load_sfb = SCALED && !resident_b && (fresh || k0 >= resident_bytes);
+              const bool load_sfb = SCALED && !resident_b && (ragged ? fresh && begins : fresh || k0 >= resident_bytes);
               const uint32_t tx_bytes = (PAIR ? 2u : 1u) * (operand_bytes + (load_sfb ? sfb_bytes : 0u));
               const bool issuer = kLaneLoop || elect_one();
               if (issuer && (!PAIR || rank == 0)) {
@@ -775,6 +795,7 @@ conv_kernel(const __grid_constant__ CUtensorMap act_map, const __grid_constant__
                 }
                 }
                 if (++s == stages) s = 0, phase ^= 1;
+                k0 += step_bytes;
                 continue;
               }
               if (issuer) {
@@ -788,7 +809,7 @@ conv_kernel(const __grid_constant__ CUtensorMap act_map, const __grid_constant__
                 }
               }
               if (SCALED) {
-                const int w_tile = k0 >> 7;
+                const int w_tile = ragged ? new_tile : k0 >> 7;
 #pragma unroll
                 for (int i = 0; i < kScaleTilesB; ++i) {
                   if (i < scale_tiles && load_sfb) {
@@ -799,6 +820,7 @@ conv_kernel(const __grid_constant__ CUtensorMap act_map, const __grid_constant__
               }
               }
               if (++s == stages) s = 0, phase ^= 1;
+              k0 += step_bytes;
             }
           }
         }
@@ -820,6 +842,8 @@ conv_kernel(const __grid_constant__ CUtensorMap act_map, const __grid_constant__
       const uint32_t sfa_base = in_register(tmem + sfa_column), sfb_stage_base = in_register(tmem + kSfbColumn);
       const uint32_t sfb_resident_base = in_register(tmem + resident_column);
       const bool per_stage_a = in_register(dynamic_a ? 1u : 0u) != 0;
+      const int last_steps = static_cast<int>(in_register(static_cast<uint32_t>(BK == 128 ? p.last_steps : kKSteps)));
+      const bool ragged = BK == 128 && last_steps != kKSteps;
       if (SCALED && !dynamic_a && (kLaneLoop || elect_one())) {
         // static activation scales never change: all tiles go to tensor memory once, ahead of the first MMA
         const int tiles = (p.cin + 127) / 128;
@@ -846,6 +870,21 @@ conv_kernel(const __grid_constant__ CUtensorMap act_map, const __grid_constant__
         const uint32_t b_low0 = in_register(static_cast<uint32_t>(b_desc0)), b_high = in_register(static_cast<uint32_t>(b_desc0 >> 32));
         const auto desc = [](uint32_t low, uint32_t high) { return static_cast<uint64_t>(high) << 32 | low; };
         const uint32_t idesc = in_register(INT8 ? idesc_i8(BN) : idesc_mxf8(BN));
+        // the same for a ragged K step of `steps` MMAs, whose blocks may lie in two scale tiles
+        const auto multiply_ragged = [&](uint32_t d_tmem, uint32_t a_low, uint32_t b_low, uint32_t kb, uint32_t kb_a, uint32_t accumulate, int steps) {
+#pragma unroll
+          for (int k = 0; k < kKSteps; ++k) {
+            if (k < steps) {
+              const uint64_t a = desc(a_low + 2 * k, a_high), b = desc(b_low + 2 * k, b_high);
+              if (INT8) {
+                tc_mma_i8(d_tmem, a, b, idesc, k > 0 ? 1u : accumulate);
+              } else {
+                tc_mma_mxf8(d_tmem, a, b, idesc + ((static_cast<uint32_t>(k) << 29) | (((kb + k) & 3u) << 4)), sfa_base + 4 * (kb_a >> 2),
+                            sfb_resident_base + kSfbColumns * ((kb + k) >> 2), k > 0 ? 1u : accumulate);
+              }
+            }
+          }
+        };
         // the MMAs of one K step (a tap's channel chunk): A from the patch at `a_low`, block `kb` along the weight's K axis
         const auto multiply = [&](uint32_t d_tmem, uint32_t a_low, uint32_t b_low, uint32_t kb, uint32_t kb_a, uint32_t accumulate) {
           const uint32_t scaled0 = idesc + (((kb_a & 3u) << 29) | ((kb & 3u) << 4));
@@ -885,14 +924,19 @@ conv_kernel(const __grid_constant__ CUtensorMap act_map, const __grid_constant__
               if (!loop_wait(step0 + 8 * ki, 0, kStatusWaitFull)) return false;
               tc_fence_after();
               if (ki == 0 && copy_scales) {
-                for (int t = 0; t < (k_iters * kKSteps + 3) / 4; ++t) {
+                for (int t = 0; t < p.weight_scale_tiles; ++t) {
                   tc_copy_scales(sfb_resident_base + kSfbColumns * t, sfb_desc0 + static_cast<uint64_t>((t * 512) >> 4));
                 }
               }
             }
-            multiply(tmem + acc * BN, tap_low + (chunk >> 4), b_low, kb, static_cast<uint32_t>(j) * kKSteps, ki > 0 ? 1u : 0u);
+            const int steps = BK == 128 && j + 1 == k_chunks ? last_steps : kKSteps;
+            if (ragged) {
+              multiply_ragged(tmem + acc * BN, tap_low + (chunk >> 4), b_low, kb, static_cast<uint32_t>(j) * kKSteps, ki > 0 ? 1u : 0u, steps);
+            } else {
+              multiply(tmem + acc * BN, tap_low + (chunk >> 4), b_low, kb, static_cast<uint32_t>(j) * kKSteps, ki > 0 ? 1u : 0u);
+            }
             b_low += kBBytes >> 4;
-            kb += kKSteps;
+            kb += steps;
             chunk += chunk_at;
             if (++j == k_chunks) {
               j = 0, chunk = 0;
@@ -910,7 +954,7 @@ conv_kernel(const __grid_constant__ CUtensorMap act_map, const __grid_constant__
         int tile = worker;
         if (tile < p.total_tiles && general_tile(true)) {
           tile += workers;
-          if (taps == 9 && taps_w == 3 && k_chunks == 1) {
+          if (taps == 9 && taps_w == 3 && k_chunks == 1 && !ragged) {
             // 3x3 with one channel chunk, unrolled: every offset along K is an immediate, so the issuing lane spends its time
             // on the MMAs (the general loop takes about 150 cycles for each)
             for (; tile < p.total_tiles; tile += workers) {
@@ -955,6 +999,7 @@ conv_kernel(const __grid_constant__ CUtensorMap act_map, const __grid_constant__
         last_n0 = n0;
         int j = 0;            // channel chunk within the tap
         uint32_t b_id = 0;    // (32-channel block index along the weight's K) mod 4 at the start of the stage
+        uint32_t kb = 0;      // ragged: that index itself
 #if FIM_PROBE_BUILD
         c_tile += clock64() - c_t0;
 #endif
@@ -992,7 +1037,42 @@ conv_kernel(const __grid_constant__ CUtensorMap act_map, const __grid_constant__
           const bool copy_b = copy_scales && (fresh || !resident), copy_a = copy_scales && per_stage_a;
           const uint32_t scaled0 = idesc | (a_id << 29) | (b_id << 4);  // the scale ids advance by one per K step
           const uint32_t first = ki > 0 ? 1u : 0u;
-          if (kLaneLoop || elect_one()) {
+          if (BK == 128 && ragged) {
+            const int steps = j + 1 == k_chunks ? last_steps : kKSteps;
+            const uint32_t new_tile = (kb + steps - 1) >> 2;
+            const bool begins = kb == 0 || new_tile != (kb - 1) >> 2;
+            if (kLaneLoop || elect_one()) {
+              if constexpr (SCALED && !PAIR) {
+#pragma unroll
+                for (int i = 0; i < kScaleTilesB; ++i) {
+                  if (i < scale_tiles && copy_scales && fresh && begins) tc_copy_scales(sfb_resident_base + kSfbColumns * new_tile + 4 * i, sfb_from + 32 * i);
+                }
+              }
+#pragma unroll
+              for (int k = 0; k < kKSteps; ++k) {
+                if (k < steps) {
+                  const uint32_t accumulate = k > 0 ? 1u : first;
+                  if (INT8) {
+                    if (PAIR) {
+                      tc_mma_i8_pair(d_tmem, a_desc + 2 * k, b_desc + 2 * k, idesc, accumulate);
+                    } else {
+                      tc_mma_i8(d_tmem, a_desc + 2 * k, b_desc + 2 * k, idesc, accumulate);
+                    }
+                  } else if constexpr (SCALED && !PAIR) {
+                    tc_mma_mxf8(d_tmem, a_desc + 2 * k, b_desc + 2 * k, idesc | (static_cast<uint32_t>(k) << 29) | (((kb + k) & 3u) << 4), sfa_tmem,
+                                sfb_resident_base + kSfbColumns * ((kb + k) >> 2), accumulate);
+                  }
+                }
+              }
+              if (PAIR) {
+                tc_commit_pair(empty0 + 8 * s);
+                tc_commit_pair((empty0 + 8 * s) | kPeerBit);
+              } else {
+                tc_commit(&ctl.empty[s]);
+              }
+            }
+            kb += static_cast<uint32_t>(steps);
+          } else if (kLaneLoop || elect_one()) {
 #pragma unroll
             for (int i = 0; i < kScaleTilesB; ++i) {
               if (i < scale_tiles && copy_b) {
@@ -1144,6 +1224,7 @@ conv_kernel(const __grid_constant__ CUtensorMap act_map, const __grid_constant__
       for (int tile = worker; tile < p.total_tiles; tile += workers, ++tile_it) {
         int m, n0, width;
         decode_tile<BN>(p, tile, m, n0, width);
+        width = min(width, p.cout - n0);  // (columns behind the last output channel have nothing to write)
         const int pixel = m * kTileM + row;  // the host keeps rows below 2**31
         const bool valid = pixel < p.out_w;
         const uint32_t acc = kAccStages == 2 ? (tile_it & 1u) : 0u;
@@ -1169,7 +1250,7 @@ conv_kernel(const __grid_constant__ CUtensorMap act_map, const __grid_constant__
             __syncwarp();
             if (lane == 0) mbar_arrive_addr(tempty0 + 8 * acc);
           }
-          if (column0 + g * 32 >= width) continue;  // a half-width tile of a split last round: nothing behind this chunk
+          if (column0 + g * 32 >= width) continue;  // a half-width tile of a split last round, a partial last tile
           const uint32_t bias_chunk = bias_at + static_cast<uint32_t>(n0 + g * 32) * 4u;
 #pragma unroll
           for (int i = 0; i < 8; ++i) {
@@ -2000,6 +2081,8 @@ struct Plan {
   bool convert = false;    // bf16 activations, quantised on chip
   bool patch = false;      // one halo patch of activations per tile (kPatch)
   int patch_w = 0, patch_h = 0, patch_bytes = 0, gelu_copies = 1;
+  int k_chunks = 0;        // K steps per tap
+  bool ragged = false;     // 128-byte K steps that do not divide the input channels
   bool resident_b = false; // the whole weight matrix stays in shared memory (one output-channel tile, small K)
   int fixed_epilogue = 0;  // kEpiLean | switches when one of the compile-time epilogues serves this call, else 0
   int out_h, out_w;
@@ -2015,8 +2098,8 @@ int out_elem_bytes(int out_mode) {
   }
 }
 
-int make_plan(const FimConvGeometry& g, int fmt, bool per_pixel, bool allow_flat, int out_elem, bool gelu, Plan* plan,
-              bool convert = false, bool pool = false) {
+int plan_with(const FimConvGeometry& g, int fmt, bool per_pixel, bool allow_flat, int out_elem, bool gelu, bool convert, bool pool, bool ragged,
+              Plan* plan) {
   // `g.cin` counts bytes of K per tap here (a BF16 layer arrives with its channel count doubled)
   const bool int8 = fmt == kFmtI8, scaled = fmt == kFmtMx;
   if (g.batch <= 0 || g.height <= 0 || g.width <= 0 || g.cin <= 0 || g.cout <= 0) return kBadArgument;
@@ -2032,7 +2115,10 @@ int make_plan(const FimConvGeometry& g, int fmt, bool per_pixel, bool allow_flat
   if (scaled && !per_pixel && (g.cin + 127) / 128 > kMaxStaticScaleTiles) return kUnsupported;
   Plan pl;
   pl.out_h = out_h, pl.out_w = out_w;
-  pl.block_k = g.cin % 128 == 0 ? 128 : (g.cin % 64 == 0 ? 64 : 32);
+  pl.ragged = ragged;
+  pl.block_k = g.cin % 128 == 0 || ragged ? 128 : (g.cin % 64 == 0 ? 64 : 32);
+  pl.k_chunks = ceil_div(g.cin, pl.block_k);
+  const int all_scale_tiles = ceil_div(g.kh * g.kw * g.cin, 128);
   // Output-channel tile: 256 halves the activation re-reads of a wide layer; narrower layers keep two accumulators in
   // tensor memory so the epilogue overlaps the next tile.
   // A block-scaled 1x1 layer that writes at least as much as it reads is bound by its epilogue: the wide tile halves the
@@ -2087,13 +2173,13 @@ int make_plan(const FimConvGeometry& g, int fmt, bool per_pixel, bool allow_flat
   // CTA pairs for the wide, compute-bound INT8 tiles: a pair owns two consecutive row tiles (the last one may not exist:
   // its loads are zero-filled and its stores clipped). The block-scaled form is correct too but measured slower than
   // single CTAs (its scale copies serialise the pair's tensor pipes): it only runs when asked for (tuning flag 128).
-  pl.pair = bn == 256 && row_tiles >= 2 && !(g_debug_flags & 64) && (int8 || (g_debug_flags & 128)) && !convert;
+  pl.pair = bn == 256 && row_tiles >= 2 && !(g_debug_flags & 64) && (int8 || ((g_debug_flags & 128) && !ragged)) && !convert;
   // A 128-wide block-scaled tile moves as many operand bytes through shared memory per MMA as the tensor pipe takes
   // twice as fast; a pair halves the weight bytes per CTA (64 rows each). Worth it for a spatial conv with many tiles
   // (3x3 128 -> 128 at 400 x 400: 118 -> 107 us), not for a small one, not for a flat 1x1 layer, whose short epilogue
   // serves single CTAs only, and not with a GELU epilogue (117 -> 123 us: the two epilogues of a pair release one shared
   // accumulator barrier, and the heavier they are the longer the MMAs wait for the slower one); flag 16384 forces it.
-  if (bn == 128 && scaled && pl.block_k == 128 && row_tiles >= 2 && !convert && !(g_debug_flags & 64) &&
+  if (bn == 128 && scaled && pl.block_k == 128 && !ragged && row_tiles >= 2 && !convert && !(g_debug_flags & 64) &&
       ((g_debug_flags & 16384) || (!pl.flat && !gelu && row_tiles >= 8LL * sm_count()))) {
     pl.pair = true;
   }
@@ -2102,7 +2188,7 @@ int make_plan(const FimConvGeometry& g, int fmt, bool per_pixel, bool allow_flat
   pl.total_tiles = static_cast<int>(total);
   // shared memory: alignment slack + output panels + static activation-scale tiles + the stage ring. A layer with few
   // K iterations per tile is bound by its stores: it gets more panels in flight; a long main loop gets the stages.
-  const int k_iters = g.kh * g.kw * (g.cin / pl.block_k);
+  const int k_iters = g.kh * g.kw * pl.k_chunks;
   pl.panels_per_half = out_elem == 4 || convert ? 1 : 2;  // 16 KB panels of a 4-byte output: one per column group
   (void)k_iters;
   const int stage_bytes = kTileM * pl.block_k + (pl.pair ? bn / 2 : bn) * pl.block_k + scale_tiles_b(bn) * 512 + 512;
@@ -2122,7 +2208,7 @@ int make_plan(const FimConvGeometry& g, int fmt, bool per_pixel, bool allow_flat
   // scale tiles) are copied once per CTA instead of once per tile and K step, which leaves the producer one copy per K
   // step. Used for 64-wide tiles, where the producer's copies are what a K step waits for (3x3 64 -> 64: 377 -> 345 us);
   // measured without gain at 128 and slower at 256 columns (1x1 128 -> 256: 163 -> 175 us), flag 4096 asks for it there.
-  if (pl.tiles_n == 1 && !pl.pair && !convert && g.cout <= bn && !(g_debug_flags & 2048) && (bn == 64 || (g_debug_flags & 4096))) {
+  if (pl.tiles_n == 1 && !pl.pair && !convert && !(scaled && ragged) && g.cout <= bn && !(g_debug_flags & 2048) && (bn == 64 || (g_debug_flags & 4096))) {
     const int all_b = k_iters * (bn * pl.block_k + scale_tiles_b(bn) * 512);
     const int a_stage = kTileM * pl.block_k + 512;
     if (fixed + all_b + 3 * a_stage <= kSmemLimit) {
@@ -2138,8 +2224,8 @@ int make_plan(const FimConvGeometry& g, int fmt, bool per_pixel, bool allow_flat
   if (g.kh * g.kw > 1 && g.stride_h == 1 && g.stride_w == 1 && fmt != kFmtBf16 && !per_pixel && !convert && bn <= 128 && pl.tiles_n == 1 &&
       !(g_debug_flags & (2048 | 16384)) && k_iters <= kMaxWeightSteps) {
     const int pw = kPatchTileW + g.dil_w * (g.kw - 1), ph = kPatchTileH + g.dil_h * (g.kh - 1);
-    const int chunk = (pw * ph * pl.block_k + 1023) / 1024 * 1024, chunks = g.cin / pl.block_k;
-    const int scale_tiles = scaled ? (k_iters * (pl.block_k / 32) + 3) / 4 : 0;
+    const int chunk = (pw * ph * pl.block_k + 1023) / 1024 * 1024, chunks = pl.k_chunks;
+    const int scale_tiles = scaled ? all_scale_tiles : 0;
     const long long tx = ceil_div(out_w, kPatchTileW), ty = ceil_div(out_h, kPatchTileH), tiles = tx * ty * g.batch;
     for (int panels = pl.panels_per_half; panels >= 1 && !pl.patch; --panels) {
       const int room = kSmemLimit - (1024 + epilogue_groups * panels * 4096 * out_elem + ((g.cin + 127) / 128) * 512 + bias_bytes + gelu_bytes) - k_iters * bn * pl.block_k;
@@ -2164,12 +2250,35 @@ int make_plan(const FimConvGeometry& g, int fmt, bool per_pixel, bool allow_flat
       pl.smem = static_cast<size_t>(kSmemLimit - room) + gelu_smem_bytes(copies) - kGeluSmemBytes + static_cast<size_t>(pl.stages) * chunks * chunk;
     }
   }
+  // (ragged, tiles through the stage ring: tensor memory has to hold every weight scale)
+  if (ragged && scaled && !pl.patch &&
+      acc_stages(bn) * bn + (pl.stages + all_scale_tiles) * (bn < 128 ? 4 : bn / 32) + 4 * ceil_div(g.cin, 128) > 512) {
+    return kUnsupported;
+  }
   const int device_sms = sm_count();
   const int sms = g_max_ctas > 0 && g_max_ctas < device_sms ? g_max_ctas : device_sms;
   pl.ctas = pl.total_tiles < sms ? pl.total_tiles : sms;
   if (pl.pair) pl.ctas = 2 * (pl.total_tiles < sms / 2 ? pl.total_tiles : sms / 2);
   *plan = pl;
   return kOk;
+}
+
+// Ragged K steps for the channel counts that only 32- or 64-byte steps divide, where tensor and shared memory have room for them. Not
+// for INT8 layers that 64-byte steps divide, which are bound by shared-memory bandwidth (2x200x190x192: 50 against 53 us; MXFP8 68
+// against 60), and not where the divided steps give a layer its halo patches and the ragged ones do not, or it has many tiles to walk:
+// then the larger patches and fewer stages cost more than the rounds (MXFP8 3x100x120x96 15.4 -> 13.3 us, 4x400x400x96 39.8 -> 41.2).
+int make_plan(const FimConvGeometry& g, int fmt, bool per_pixel, bool allow_flat, int out_elem, bool gelu, Plan* plan, bool convert = false,
+              bool pool = false) {
+  if (g.cin > 64 && g.cin % 128 != 0 && g.cin % 32 == 0 && (fmt == kFmtMx || (fmt == kFmtI8 && g.cin % 64 != 0)) && !per_pixel && !convert &&
+      !(g_debug_flags & 32768)) {
+    Plan divided;
+    const int rc = plan_with(g, fmt, per_pixel, allow_flat, out_elem, gelu, convert, pool, true, plan);
+    if (rc == kOk && (plan->patch ? plan->total_tiles <= 6 * plan->ctas :
+                      plan_with(g, fmt, per_pixel, allow_flat, out_elem, gelu, convert, pool, false, &divided) != kOk || !divided.patch)) {
+      return kOk;
+    }
+  }
+  return plan_with(g, fmt, per_pixel, allow_flat, out_elem, gelu, convert, pool, false, plan);
 }
 
 // What the persistent CTAs walk: the tile list (with the last partial round cut into half-width tiles when that halves
@@ -2191,7 +2300,10 @@ Schedule make_schedule(const FimConvGeometry& g, const Plan& pl, bool int8, bool
       sc.total_tiles = sc.full_tiles + 2 * rest;
     }
   }
-  if (!int8 && pl.block_k == 128 && !(g_debug_flags & 256)) {
+  if (pl.ragged) {
+    // every scale tile stays where it pays (resident_k has no part in it); a short K is bound by its stores, which go out row by row
+    sc.n_major = !int8 && g.kh * g.kw * pl.k_chunks >= 8 ? 1 : 0;
+  } else if (!int8 && pl.block_k == 128 && !(g_debug_flags & 256)) {
     // Tensor-memory columns left after the accumulators, the per-stage scale sets and the activation scales hold the
     // weight scales of the first K iterations for as long as consecutive tiles of a CTA share their output channels.
     // That needs the row tiles of one channel tile to follow each other, which re-reads the activations once per channel
@@ -2199,7 +2311,7 @@ Schedule make_schedule(const FimConvGeometry& g, const Plan& pl, bool int8, bool
     const int sfb_columns = pl.block_n < 128 ? 4 : pl.block_n / 32;
     const int sfa_columns = 4 * (per_pixel ? pl.stages : (g.cin + 127) / 128);
     const int room = 512 - acc_stages(pl.block_n) * pl.block_n - pl.stages * sfb_columns - sfa_columns;
-    const int k_iters = g.kh * g.kw * (g.cin / pl.block_k);
+    const int k_iters = g.kh * g.kw * pl.k_chunks;
     const long long activation_bytes = static_cast<long long>(g.batch) * g.height * g.width * g.cin;
     const bool cheap_reread = pl.tiles_n == 1 || k_iters >= 8 || activation_bytes <= (48LL << 20);
     if (room >= sfb_columns && cheap_reread) {
@@ -2430,7 +2542,8 @@ int run_conv(int fmt, const void* x, const int8_t* act_exponent, const void* act
   p.total_tiles = sc.total_tiles;
   p.full_tiles = sc.full_tiles;
   p.batch = pl.flat ? 1 : g->batch;
-  p.k_chunks = g->cin / pl.block_k, p.stages = pl.stages, p.panels_per_half = pl.panels_per_half;
+  p.k_chunks = pl.k_chunks, p.last_steps = (g->cin - (pl.k_chunks - 1) * pl.block_k) / 32;
+  p.stages = pl.stages, p.panels_per_half = pl.panels_per_half;
   p.row_tiles = pl.total_tiles / pl.tiles_n;
   p.div_row_tiles = make_fastdiv(p.row_tiles), p.div_tiles_n = make_fastdiv(pl.tiles_n);
   p.div_tiles_x = make_fastdiv(pl.tiles_x), p.div_tiles_y = make_fastdiv(pl.tiles_y);
@@ -2438,7 +2551,7 @@ int run_conv(int fmt, const void* x, const int8_t* act_exponent, const void* act
   p.act_exponent = act_exponent;
   p.convert_static = convert && act_exponent != nullptr ? 1 : 0;
   p.weights_resident = pl.resident_b ? 1 : 0;
-  p.b_slots = pl.resident_b ? g->kh * g->kw * (g->cin / pl.block_k) : pl.stages;
+  p.b_slots = pl.resident_b ? g->kh * g->kw * pl.k_chunks : pl.stages;
   p.act_scales = static_cast<const uint8_t*>(act_scales);
   p.act_scale_tiles = (g->cin / 32 + 3) / 4;
   p.weight_scales = static_cast<const uint8_t*>(weight_scales);

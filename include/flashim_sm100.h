@@ -37,7 +37,7 @@ extern "C" {
 #define FIM_ACT_RELU 1
 #define FIM_ACT_GELU 2
 #define FIM_ACT_RELU_EARLY 3 /* conv epilogues: ReLU before the residual add (the order of flashim/ops/gemm.py:87-98) */
-#define FIM_ACT_GELU_SUM 4   /* block-scaled 1x1 convs with a bias and FIM_OUT_E4M3_STATIC (cin % 128 == 0, else FIM_ERR_UNSUPPORTED): erf
+#define FIM_ACT_GELU_SUM 4   /* block-scaled 1x1 convs with a bias and FIM_OUT_E4M3_STATIC (cin and cout above 64, else FIM_ERR_UNSUPPORTED): erf
                               * GELU of bf16(product) + bias, the sum in fp32 (the order of flashim/ops/gemm.py:146-157) */
 
 /* What the conv epilogue writes. */

@@ -25,6 +25,7 @@ extern "C" {
  *  2048  streams the weights of a layer (and the activations tap by tap, instead of one halo patch per tile) through the
  *        stage ring even where they are kept in shared memory by default;
  *  4096  keeps them resident for every tile width where they fit (by default only 64-wide tiles do);
+ * 32768  divides K into steps that divide the input channels (32, 64 or 128 bytes), also where 128-byte steps with a short last one serve;
  * 16384  runs 128-wide block-scaled tiles as CTA pairs whatever the size of the layer.
  * A library built with -DFIM_PROBE_BUILD=1 (never shipped) also honours bits 1, 2, 4, 8 (skip activation loads / weight
  * loads / stores / scale copies), which make results invalid, and 8192 (the MMA warp of CTA 0 prints its cycle counts).
