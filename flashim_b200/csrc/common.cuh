@@ -475,7 +475,11 @@ __device__ __forceinline__ uint16_t e4m3x2(float lo, float hi) {
   return r;
 }
 __device__ __forceinline__ uint32_t e4m3x4(float a, float b, float c, float d) {
-  return static_cast<uint32_t>(e4m3x2(a, b)) | (static_cast<uint32_t>(e4m3x2(c, d)) << 16);
+  uint32_t r;  // (one assembly block: the second conversion then writes the upper half beside the first, without a merge behind both)
+  asm("{\n\t.reg .b16 lo, hi;\n\tcvt.rn.satfinite.e4m3x2.f32 lo, %2, %1;\n\tcvt.rn.satfinite.e4m3x2.f32 hi, %4, %3;\n\tmov.b32 %0, {lo, hi};\n\t}"
+      : "=r"(r)
+      : "f"(a), "f"(b), "f"(c), "f"(d));
+  return r;
 }
 
 // round_half_even(value / scale) saturated to [-127, 127]: a true IEEE division, as the reference's quantiser.
