@@ -485,6 +485,7 @@ conv_kernel(const __grid_constant__ CUtensorMap act_map, const __grid_constant__
   constexpr int kAccStages = acc_stages(BN);
   constexpr int kScaleTilesB = scale_tiles_b(BN);
   constexpr int kKSteps = BK / 32;
+  constexpr bool kMayBeRagged = BK == 128 && BN <= 128;  // (256-wide tiles lose 1 % to the tests: 4x100x100x512 78 -> 79 us)
   constexpr uint32_t kABytes = kTileM * BK, kBBytes = (PAIR ? BN / 2 : BN) * BK;  // per CTA
   constexpr int kWeightBoxRows = BN < 128 ? BN : 128;  // rows of one weight TMA box
   constexpr uint32_t kSfbColumns = BN < 128 ? 4 : BN / 32;
@@ -650,8 +651,8 @@ conv_kernel(const __grid_constant__ CUtensorMap act_map, const __grid_constant__
       int last_n0 = -1;
       const bool resident_b = in_register(static_cast<uint32_t>(p.weights_resident)) != 0;
       // bytes of a tap's last channel chunk along the weight's K axis
-      const int last_bytes = static_cast<int>(in_register(static_cast<uint32_t>(BK == 128 ? p.last_steps * 32 : BK)));
-      const bool ragged = BK == 128 && last_bytes != BK;
+      const int last_bytes = static_cast<int>(in_register(static_cast<uint32_t>(kMayBeRagged ? p.last_steps * 32 : BK)));
+      const bool ragged = kMayBeRagged && last_bytes != BK;
       if constexpr (PATCH) {
         // one patch per tile; behind the first one the weights, K step by K step, which the first tile's MMAs wait for singly
         const int k_total = kh * kw * k_chunks;
@@ -743,7 +744,7 @@ conv_kernel(const __grid_constant__ CUtensorMap act_map, const __grid_constant__
           for (int kx = 0; kx < kw && alive; ++kx) {
             const int cx = x0 + kx * dil_w, cy = y0 + ky * dil_h;
             for (int j = 0; j < k_chunks; ++j) {
-              const int step_bytes = BK == 128 && j + 1 == k_chunks ? last_bytes : BK;
+              const int step_bytes = kMayBeRagged && j + 1 == k_chunks ? last_bytes : BK;
               // ragged: the scale tile that begins in this step, if any
               const int new_tile = (k0 + step_bytes - 32) >> 7;
               const bool begins = new_tile != (k0 - 32) >> 7;
@@ -842,8 +843,8 @@ conv_kernel(const __grid_constant__ CUtensorMap act_map, const __grid_constant__
       const uint32_t sfa_base = in_register(tmem + sfa_column), sfb_stage_base = in_register(tmem + kSfbColumn);
       const uint32_t sfb_resident_base = in_register(tmem + resident_column);
       const bool per_stage_a = in_register(dynamic_a ? 1u : 0u) != 0;
-      const int last_steps = static_cast<int>(in_register(static_cast<uint32_t>(BK == 128 ? p.last_steps : kKSteps)));
-      const bool ragged = BK == 128 && last_steps != kKSteps;
+      const int last_steps = static_cast<int>(in_register(static_cast<uint32_t>(kMayBeRagged ? p.last_steps : kKSteps)));
+      const bool ragged = kMayBeRagged && last_steps != kKSteps;
       if (SCALED && !dynamic_a && (kLaneLoop || elect_one())) {
         // static activation scales never change: all tiles go to tensor memory once, ahead of the first MMA
         const int tiles = (p.cin + 127) / 128;
@@ -929,7 +930,7 @@ conv_kernel(const __grid_constant__ CUtensorMap act_map, const __grid_constant__
                 }
               }
             }
-            const int steps = BK == 128 && j + 1 == k_chunks ? last_steps : kKSteps;
+            const int steps = kMayBeRagged && j + 1 == k_chunks ? last_steps : kKSteps;
             if (ragged) {
               multiply_ragged(tmem + acc * BN, tap_low + (chunk >> 4), b_low, kb, static_cast<uint32_t>(j) * kKSteps, ki > 0 ? 1u : 0u, steps);
             } else {
@@ -1037,7 +1038,7 @@ conv_kernel(const __grid_constant__ CUtensorMap act_map, const __grid_constant__
           const bool copy_b = copy_scales && (fresh || !resident), copy_a = copy_scales && per_stage_a;
           const uint32_t scaled0 = idesc | (a_id << 29) | (b_id << 4);  // the scale ids advance by one per K step
           const uint32_t first = ki > 0 ? 1u : 0u;
-          if (BK == 128 && ragged) {
+          if (kMayBeRagged && ragged) {
             const int steps = j + 1 == k_chunks ? last_steps : kKSteps;
             const uint32_t new_tile = (kb + steps - 1) >> 2;
             const bool begins = kb == 0 || new_tile != (kb - 1) >> 2;
@@ -2131,6 +2132,7 @@ int plan_with(const FimConvGeometry& g, int fmt, bool per_pixel, bool allow_flat
   if (g_forced_block_n == 64) bn = 64;
   if (fmt == kFmtBf16 && bn == 256) bn = 128;  // BF16 layers on this path are narrow pointwise products
   if (bn == 64 && g.cout > 64 && scaled) bn = 128;  // a 64-wide tile may only start at column 0 of its scale tile
+  if (bn == 256 && ragged) return kUnsupported;
   pl.flat = pointwise && allow_flat;
   pl.convert = convert;
   if (convert && !(fmt == kFmtMx && pl.flat && pl.block_k == 128)) return kUnsupported;

@@ -13,7 +13,7 @@ E4M3, BF16 = torch.float8_e4m3fn, torch.bfloat16
 CASES = [  # batch, height, width, cin, cout, kernel, stride, padding, dilation, most CTAs, forced tile width
     (3, 38, 51, 96, 160, 3, 2, 1, 1, 0, 0), (1, 17, 9, 160, 128, 3, 1, 1, 1, 2, 0), (2, 20, 23, 192, 192, 3, 1, 1, 1, 3, 0),
     (1, 19, 21, 96, 96, 3, 1, 1, 1, 2, 0), (1, 19, 21, 96, 64, 3, 1, 2, 2, 1, 0), (1, 30, 20, 224, 64, 1, 1, 0, 1, 2, 0),
-    (2, 13, 13, 480, 256, 3, 1, 1, 1, 2, 256), (1, 40, 45, 288, 512, 1, 1, 0, 1, 5, 256), (1, 15, 14, 96, 32, 5, 3, 2, 1, 0, 0),
+    (2, 13, 13, 480, 256, 3, 1, 1, 1, 2, 128), (1, 40, 45, 288, 512, 1, 1, 0, 1, 5, 128), (1, 15, 14, 96, 32, 5, 3, 2, 1, 0, 0),
     (1, 16, 16, 672, 128, 3, 1, 1, 1, 0, 0), (1, 129, 1, 96, 288, 1, 1, 0, 1, 1, 0), (1, 5, 5, 1120, 64, 3, 1, 1, 1, 0, 0),
 ]
 
@@ -53,12 +53,12 @@ def test_ragged_steps_equal_divided_steps(case):
 
 
 def test_plans_take_ragged_steps_where_they_serve():
-    """Widths of the K steps: 128 bytes for channels that 64 does not divide, or 64 does (MXFP8 alone); not for two blocks or fewer."""
+    """Widths of the K steps: 128 bytes for channels that 64 does not divide, or 64 does (MXFP8 alone); not for two blocks or fewer, nor 256-wide tiles."""
     from flashim_b200 import _native
 
     lib = _native.library()
 
-    def step(cin, int8, k=3, cout=256):
+    def step(cin, int8, k=3, cout=160):
         geometry = _native.ConvGeometry(1, 40, 40, cin, cout, k, k, 1, 1, k // 2, k // 2, 1, 1)
         plan = (ctypes.c_int * 6)()
         assert lib.fim_conv_plan(ctypes.byref(geometry), int8, 0, ctypes.byref(plan)) == 0
@@ -68,3 +68,4 @@ def test_plans_take_ragged_steps_where_they_serve():
     assert [step(c, 1) for c in (32, 64, 96, 128, 160, 192)] == [32, 64, 128, 128, 128, 64]
     assert step(992, 0) == 32 and step(992, 0, k=1) == 128  # weight scales of nine taps: more than tensor memory holds
     assert step(192, 0, cout=64) == 64  # keeps its halo patches
+    assert step(192, 0, cout=256) == 64
