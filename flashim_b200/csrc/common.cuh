@@ -590,6 +590,17 @@ __device__ __forceinline__ uint32_t bf16x2_absmax(uint32_t a, uint32_t b) {
   asm("max.xorsign.abs.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
   return d;
 }
+// the same, a not-a-number if one of them is, and the minimum likewise
+__device__ __forceinline__ uint32_t bf16x2_absmax_nan(uint32_t a, uint32_t b) {
+  uint32_t d;
+  asm("max.NaN.xorsign.abs.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
+  return d;
+}
+__device__ __forceinline__ uint32_t bf16x2_min_nan(uint32_t a, uint32_t b) {
+  uint32_t d;
+  asm("min.NaN.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
+  return d;
+}
 
 // GELU through the complementary error function in the rational-exponential form of Abramowitz & Stegun 7.1.26
 // (|error of erf| <= 1.5e-7): gelu(x) = x/2 * (2 - c) for x >= 0 and x/2 * c for x < 0 with c = erfc(|x|/sqrt 2).

@@ -167,6 +167,125 @@ __device__ __forceinline__ uint32_t gelu_bf16x2(uint32_t r, const GeluTable& tab
   return __viaddmax_s16x2(a, delta, 0u) | (r & 0x80008000u);
 }
 
+// The same GELU by arithmetic, for the epilogues that go on to E4M3: max(x, 0) - |x| 2**q(-|x|) in fp32, rounded to bf16, with q of degree
+// five. Its coefficients solve the linear inequalities that make the rounded result torch's for EVERY bf16 value from -3.515625 up
+// (make_gelu_table.py checks them, with a margin for the roundings of the evaluation); a minimax polynomial of that degree misses
+// some. Below, torch's own result is the rounding noise of 1 + erf, which no polynomial follows, but the E4M3 codes of both are the
+// same under every exponent from -9 up, except those of one value under -6 and of one under -2. What is left, with infinities and
+// not-a-numbers, takes the table. As many issue slots as the look-up, and none of the shared-memory wavefronts that bounded these
+// epilogues (32 scattered reads take 3.3 passes, 2.9 with eight copies of the table): us, table -> arithmetic:
+// 3x3 4x800x800x64 135 -> 122, 4x400x400x128 89 -> 74; 1x1 8x100x100x512 -> 1024 65 -> 59; residual MLP 8x400x400x128 255 -> 229 (arguments of
+// a standard deviation of 1.4, many of them in the tail: 243), 8x200x200x256 164 -> 140.
+__device__ __forceinline__ uint32_t gelu_arithmetic_bf16x2(uint32_t r) {
+  float x0, x1;  // the halves in fp32
+  asm("{\n\t.reg .b16 a, b, one, z;\n\tmov.b32 {a, b}, %2;\n\tmov.b32 {one, z}, %3;\n\t"
+      "fma.rn.f32.bf16 %0, a, one, 0f80000000;\n\tfma.rn.f32.bf16 %1, b, one, 0f80000000;\n\t}"
+      : "=f"(x0), "=f"(x1)
+      : "r"(r), "r"(0x3F803F80u));
+  const uint64_t u = pack2(fminf(x0, -x0), fminf(x1, -x1));
+  uint64_t q = pack2(4.492032749e-04f, 4.492032749e-04f);
+  q = fma2(q, u, pack2(7.005445193e-03f, 7.005445193e-03f));
+  q = fma2(q, u, pack2(5.192643777e-02f, 5.192643777e-02f));
+  q = fma2(q, u, pack2(-4.595530033e-01f, -4.595530033e-01f));
+  q = fma2(q, u, pack2(1.151077390e+00f, 1.151077390e+00f));
+  q = fma2(q, u, pack2(-9.999969602e-01f, -9.999969602e-01f));
+  float q0, q1;
+  unpack2(q, q0, q1);
+  // (a negative zero keeps the sign of a result that vanishes)
+  const uint64_t g = fma2(u, pack2(ex2_approx(q0), ex2_approx(q1)), pack2(fmaxf(x0, -0.0f), fmaxf(x1, -0.0f)));
+  unpack2(g, q0, q1);
+  return pack_bf16(q0, q1);
+}
+constexpr uint32_t kGeluTail = 0xC061u;  // the last argument for which it is exact, -3.515625; larger ones (unsigned) lie below
+// the one argument whose code differs under an exponent (-4.5, -3.53125; 0: none)
+__device__ __forceinline__ uint32_t gelu_exception(int e) { return e == -6 ? 0xC090u : (e == -2 ? 0xC062u : 0u); }
+__device__ __forceinline__ bool contains(const uint32_t (&r)[16], uint32_t value) {
+  uint32_t hit = 0;
+#pragma unroll
+  for (int i = 0; i < 16; ++i) {
+    const uint32_t t = r[i] ^ (value * 0x00010001u);
+    hit |= (t - 0x00010001u) & ~t;  // the top bit of a half that is zero (or, above one, of a half that may not be)
+  }
+  return (hit & 0x80008000u) != 0;
+}
+
+// the largest positive argument (bits; negative without one)
+__device__ __forceinline__ int gelu_highest(const uint32_t (&r)[16]) {
+  uint32_t high = r[0];
+#pragma unroll
+  for (int i = 1; i < 16; ++i) high = __vmaxs2(high, r[i]);
+  return max(static_cast<int>(high) >> 16, static_cast<int>(static_cast<int16_t>(high & 0xFFFFu)));
+}
+
+// GELU of 32 values, by arithmetic unless one of the warp's lanes asks for the table (its one copy: little reaches it)
+__device__ __forceinline__ void gelu_chunk(uint32_t (&r)[16], bool look_up, const GeluTable& table) {
+  if (__any_sync(0xffffffffu, look_up)) {
+#pragma unroll
+    for (int i = 0; i < 16; ++i) r[i] = gelu_bf16x2(r[i], table);
+  } else {
+#pragma unroll
+    for (int i = 0; i < 16; ++i) r[i] = gelu_arithmetic_bf16x2(r[i]);
+  }
+}
+
+// ... under a static exponent
+__device__ __forceinline__ void gelu_chunk_static(uint32_t (&r)[16], int e, const GeluTable& table) {
+  uint32_t low = r[0], high = r[0];
+#pragma unroll
+  for (int i = 1; i < 16; ++i) low = __vmaxu2(low, r[i]), high = __vmaxs2(high, r[i]);
+  const uint32_t lowest = max(low & 0xFFFFu, low >> 16);  // (as unsigned halves: of two negative values the larger magnitude)
+  const int highest = max(static_cast<int>(high) >> 16, static_cast<int>(static_cast<int16_t>(high & 0xFFFFu)));
+  bool look_up = !(lowest < 0xFF80u && highest < 0x7F80);
+  if ((e < -9 || e == -6 || e == -2) && lowest > kGeluTail) {
+    const bool differ = contains(r, e == -6 ? gelu_exception(-6) : gelu_exception(-2));
+    look_up |= e < -9 || differ;
+  }
+  gelu_chunk(r, look_up, table);
+}
+
+// the largest magnitude of 32 values, bf16 bits (KEEP_NAN: above 0x7F80 if one is not a number, which does not count otherwise)
+template <bool KEEP_NAN = false>
+__device__ __forceinline__ uint32_t largest_magnitude(const uint32_t (&r)[16]) {
+  const auto larger = [](uint32_t a, uint32_t b) { return KEEP_NAN ? bf16x2_absmax_nan(a, b) : bf16x2_absmax(a, b); };
+  uint32_t m[8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) m[i] = larger(r[2 * i], r[2 * i + 1]);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) m[i] = larger(m[2 * i], m[2 * i + 1]);
+  m[0] = larger(larger(m[0], m[1]), larger(m[2], m[3]));
+  return max(m[0] & 0x7FFFu, (m[0] >> 16) & 0x7FFFu);
+}
+
+// ... that form a block with an exponent of its own, which it returns. Where arguments lie in the tail the exponent has to be known ahead:
+// it is that of the largest result, which is the GELU of the largest argument from 0.703 up (results below zero stay above -0.17).
+// One minimum per word tells the tail, negative infinities and not-a-numbers; behind those a result that is not a number comes from
+// a positive infinity.
+__device__ __forceinline__ int gelu_chunk_dynamic(uint32_t (&r)[16], const GeluTable& table) {
+  uint32_t low = r[0];
+#pragma unroll
+  for (int i = 1; i < 16; ++i) low = bf16x2_min_nan(low, r[i]);
+  const uint32_t lowest = max(low & 0xFFFFu, low >> 16);  // (negative halves are the larger ones; a not-a-number is 0x7FFF)
+  bool look_up = false;
+  const bool not_a_number = max(low & 0x7FFFu, (low >> 16) & 0x7FFFu) > 0x7F80u;
+  if (lowest > kGeluTail || not_a_number) {
+    const int highest = gelu_highest(r);
+    look_up = not_a_number || lowest >= 0xFF80u || highest >= 0x7F80 || highest < 0x3F34;                        // the last: may be below -9
+    if (highest >= 0x4060 && highest <= 0x40E0 && lowest >= gelu_exception(-6)) look_up |= contains(r, gelu_exception(-6));  // 3.5 to 7
+    if (highest >= 0x4260 && highest <= 0x42E0) look_up |= contains(r, gelu_exception(-2));                                  // 56 to 112
+  }
+  gelu_chunk(r, look_up, table);
+  uint32_t top = largest_magnitude<true>(r);
+  if (top > 0x7F80u) {
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+      if ((r[i] & 0x7FFFu) > 0x7F80u && !look_up) r[i] = (r[i] & 0xFFFF0000u) | 0x7F80u;
+      if ((r[i] & 0x7FFF0000u) > 0x7F800000u && !look_up) r[i] = (r[i] & 0xFFFFu) | 0x7F800000u;
+    }
+    top = largest_magnitude<false>(r);
+  }
+  return e8m0_exponent_bits(top << 16);
+}
+
 __device__ __forceinline__ uint32_t idesc_bf16(int block_n, int block_m = kTileM) {
   // F32 accumulator (1), BF16 A and B (1), both K-major, M = block_m, N = block_n (kind::f16)
   return (1u << 4) | (1u << 7) | (1u << 10) | (static_cast<uint32_t>(block_n >> 3) << 17) |
@@ -187,6 +306,10 @@ constexpr int kEpiGelu = 1, kEpiDynamic = 2, kEpiResidual = 4, kEpiLean = 8, kEp
 // gelu_quantize_mx_kernel on the same values. A lane evaluates 32 error functions per chunk, which the main loop of a short K does not
 // hide; still the hidden tensor crosses memory once and as bytes, and a launch goes (MLP of 1000 x 256 x 1024: 18.0 -> 14.2 us, 20000 x 384 x 1536: 119 -> 69).
 constexpr int kEpiGeluSum = 256;
+// kEpiArithmetic (with kEpiFixed | kEpiGelu | kEpiStatic): the GELU by arithmetic. For patches and layers with a short K, whose epilogue is
+// what a tile waits for; behind a long main loop, which the power limit governs, the table is the cheaper one (4x100x100x512 3x3,
+// inputs not in L2: 95 us against 99).
+constexpr int kEpiArithmetic = 512;
 
 // kPatch (with any of the epilogues above): a spatial conv whose whole weight matrix stays in shared memory and whose
 // activations arrive as one halo patch per tile instead of one shifted tile per tap. A tile is 8 columns x 16 rows of output
@@ -210,14 +333,14 @@ constexpr int kPatchTileW = 8, kPatchTileH = 16;
 struct EpilogueSwitches {
   int act, out_mode;
   uint32_t out_elem, panels;  // bytes per output element; output panels per group
-  bool has_bias, has_residual, gelu_sum;  // gelu_sum: kEpiGeluSum, in the fixed epilogues alone
+  bool has_bias, has_residual, gelu_sum, gelu_static;  // the last two: kEpiGeluSum, kEpiArithmetic, in the fixed epilogues alone
 };
 template <int EPI>
 __device__ __forceinline__ EpilogueSwitches epilogue_switches(const ConvParams& p) {
   EpilogueSwitches sw;
   if constexpr ((EPI & kEpiFixed) != 0) {
     sw.act = (EPI & kEpiGelu) ? kActGelu : kActNone;
-    sw.gelu_sum = (EPI & kEpiGeluSum) != 0;
+    sw.gelu_sum = (EPI & kEpiGeluSum) != 0, sw.gelu_static = (EPI & kEpiArithmetic) != 0;
     sw.out_mode = (EPI & kEpiStatic) ? FIM_OUT_E4M3_STATIC : ((EPI & kEpiDynamic) ? FIM_OUT_E4M3_DYNAMIC : FIM_OUT_BF16);
     sw.out_elem = sw.out_mode == FIM_OUT_BF16 ? 2u : 1u;
     sw.panels = (EPI & kPatch) != 0 ? static_cast<uint32_t>(p.panels_per_half) : 2u;
@@ -226,7 +349,7 @@ __device__ __forceinline__ EpilogueSwitches epilogue_switches(const ConvParams& 
   } else {
     sw.act = p.act, sw.out_mode = p.out_mode;
     sw.out_elem = static_cast<uint32_t>(p.out_elem), sw.panels = static_cast<uint32_t>(p.panels_per_half);
-    sw.has_bias = p.bias != nullptr, sw.has_residual = p.residual != nullptr, sw.gelu_sum = false;
+    sw.has_bias = p.bias != nullptr, sw.has_residual = p.residual != nullptr, sw.gelu_sum = sw.gelu_static = false;
   }
   return sw;
 }
@@ -344,6 +467,8 @@ __device__ __forceinline__ void finish_chunk(const ConvParams& p, const Epilogue
       r[2 * i] = pack_bf16(gelu_erf(bf16_lo(v0) + b[0]), gelu_erf(bf16_hi(v0) + b[1]));
       r[2 * i + 1] = pack_bf16(gelu_erf(bf16_lo(v1) + b[2]), gelu_erf(bf16_hi(v1) + b[3]));
     }
+  } else if (sw.gelu_static) {
+    gelu_chunk_static(r, static_cast<int>(__ldg(p.out_exponent + (n >> 5))), gelu_table);
   } else if (sw.act == kActGelu) {
 #pragma unroll
     for (int i = 0; i < 16; ++i) r[i] = gelu_bf16x2(r[i], gelu_table);
@@ -399,13 +524,7 @@ __device__ __forceinline__ void finish_chunk(const ConvParams& p, const Epilogue
   } else {
     // block maximum of |value| on bf16x2 words: max.xorsign.abs keeps the larger magnitude in both halves (signs are
     // masked off at the end); a bf16 magnitude shifted left by 16 is the same number in fp32
-    uint32_t m[8];
-#pragma unroll
-    for (int i = 0; i < 8; ++i) m[i] = bf16x2_absmax(r[2 * i], r[2 * i + 1]);
-#pragma unroll
-    for (int i = 0; i < 4; ++i) m[i] = bf16x2_absmax(m[2 * i], m[2 * i + 1]);
-    m[0] = bf16x2_absmax(bf16x2_absmax(m[0], m[1]), bf16x2_absmax(m[2], m[3]));
-    const uint32_t top = max(m[0] & 0x7FFFu, (m[0] >> 16) & 0x7FFFu);
+    const uint32_t top = largest_magnitude(r);
     e = e8m0_exponent_bits(top << 16);
     if (valid) {
       const int groups = p.cout >> 5;
@@ -1268,10 +1387,9 @@ conv_kernel(const __grid_constant__ CUtensorMap act_map, const __grid_constant__
         for (int g = 0; g < kChunksPerWarp; ++g) {
           if (column0 + g * 32 >= width) continue;
           uint32_t(&r)[16] = q[g];
-          if (kGelu) {
-#pragma unroll
-            for (int i = 0; i < 16; ++i) r[i] = gelu_bf16x2(r[i], gelu2);
-          }
+          static_assert(!kGelu || (kDynamic && !kResidual), "the GELU of a flat layer is followed by its block's exponent");
+          int e = 0;
+          if (kGelu) e = gelu_chunk_dynamic(r, gelu2);
           if (kResidual) {
             if (valid) {
               const uint4* r4 = reinterpret_cast<const uint4*>(res_row + g * 32);
@@ -1289,14 +1407,7 @@ conv_kernel(const __grid_constant__ CUtensorMap act_map, const __grid_constant__
           ++chunk_it;
           const uint32_t at = panel + row_at;
           if (kDynamic) {
-            uint32_t mx[8];
-#pragma unroll
-            for (int i = 0; i < 8; ++i) mx[i] = bf16x2_absmax(r[2 * i], r[2 * i + 1]);
-#pragma unroll
-            for (int i = 0; i < 4; ++i) mx[i] = bf16x2_absmax(mx[2 * i], mx[2 * i + 1]);
-            mx[0] = bf16x2_absmax(bf16x2_absmax(mx[0], mx[1]), bf16x2_absmax(mx[2], mx[3]));
-            const uint32_t top = max(mx[0] & 0x7FFFu, (mx[0] >> 16) & 0x7FFFu);
-            const int e = e8m0_exponent_bits(top << 16);
+            if (!kGelu) e = e8m0_exponent_bits(largest_magnitude(r) << 16);
             if (valid) {
               const int kg = (n0 + column0 + g * 32) >> 5;
               p.out_scales[(static_cast<size_t>(m) * scale_tiles + (kg >> 2)) * 512 + scale_at + (kg & 3)] = static_cast<uint8_t>(e + 127);
@@ -1608,9 +1719,6 @@ constexpr int kMlpOutWarps = 8;  // output warps: two per lane quarter of tensor
 constexpr int kMlpThreads = kThreads + 32 * kMlpOutWarps;
 constexpr uint32_t kMlpPanels = 2, kMlpPanelBytes = 32u * 64u;  // output panels per output warp: 32 rows x 32 bf16 channels
 constexpr uint32_t kMlpResidualSlots = 2;  // residual panels (same shape) each output warp keeps in flight
-// Copies of the GELU table: the ring gives up a weight unit or two for them, which nothing waits for (8x400x400x128 260 -> 256
-// us, 8x200x200x256 168 -> 163; two copies give half of that).
-constexpr int kMlpGeluCopies = 4;
 struct MlpParams {
   int rows, row_tiles, stages;
   const uint8_t* x_scales;   // per-pixel scales of x: swizzled tiles, KC per row tile
@@ -1649,7 +1757,7 @@ mlp_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constant__ CU
 
   const uint32_t base = (smem_u32(smem_dyn) + 1023u) & ~1023u;
   const uint32_t smem_gelu = base;
-  const uint32_t smem_x = base + gelu_smem_bytes(kMlpGeluCopies);
+  const uint32_t smem_x = base + kGeluSmemBytes;
   const uint32_t smem_w = smem_x + kUnitBytes;
   const uint32_t smem_h = smem_w + static_cast<uint32_t>(p.stages) * kUnitBytes;
   const uint32_t smem_out = smem_h + 2u * kMlpTile;
@@ -1702,11 +1810,7 @@ mlp_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constant__ CU
   constexpr int kSetupThreads = kMlpThreads - 32;
   if (warp != 0) {
     for (int i = threadIdx.x - 32; i < kGeluEntries; i += kSetupThreads) {
-      const uint32_t entry = kGeluTable[i];
-#pragma unroll
-      for (int c = 0; c < kMlpGeluCopies; ++c) {
-        asm volatile("st.shared.b32 [%0], %1;" ::"r"(smem_gelu + (i * kMlpGeluCopies + c) * 4), "r"(entry) : "memory");
-      }
+      asm volatile("st.shared.b32 [%0], %1;" ::"r"(smem_gelu + i * 4), "r"(kGeluTable[i]) : "memory");
     }
   }
   grid_wait();
@@ -1865,7 +1969,7 @@ mlp_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constant__ CU
     // ===== hidden-block warps: lanes 32 * (w % 4) ... of tensor memory, 32 hidden channels (w - 2) / 4 of every block =====
     const int quarter = warp & 3, group = (warp - 2) >> 2;
     const int row = quarter * 32 + lane;
-    const GeluTable gelu2 = gelu_table_at(smem_gelu, kMlpGeluCopies, static_cast<uint32_t>(lane));
+    const GeluTable gelu2 = gelu_table_at(smem_gelu);
     const uint32_t lane_tmem = tmem + (static_cast<uint32_t>(quarter * 32) << 16) + kAcc1 + group * 32;
     // where this lane's 32 hidden bytes go in a K-major 128-byte-swizzled tile, and its scale byte in the scale tile
     const uint32_t h_row = static_cast<uint32_t>(row) * 128u;
@@ -1910,16 +2014,7 @@ mlp_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constant__ CU
       int e = 0;
       uint32_t w[8];
       if (!(probe_flags(p) & 4)) {
-#pragma unroll
-      for (int i = 0; i < 16; ++i) r[i] = gelu_bf16x2(r[i], gelu2);
-      uint32_t mx[8];
-#pragma unroll
-      for (int i = 0; i < 8; ++i) mx[i] = bf16x2_absmax(r[2 * i], r[2 * i + 1]);
-#pragma unroll
-      for (int i = 0; i < 4; ++i) mx[i] = bf16x2_absmax(mx[2 * i], mx[2 * i + 1]);
-      mx[0] = bf16x2_absmax(bf16x2_absmax(mx[0], mx[1]), bf16x2_absmax(mx[2], mx[3]));
-      const uint32_t top = max(mx[0] & 0x7FFFu, (mx[0] >> 16) & 0x7FFFu);
-      e = e8m0_exponent_bits(top << 16);
+      e = gelu_chunk_dynamic(r, gelu2);
       scale_to_e4m3(r, e, w);
       } else {
 #pragma unroll
@@ -2070,6 +2165,10 @@ mlp_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constant__ CU
 
 // ---- host ------------------------------------------------------------------------------------------------------------
 
+// how the epilogue of a layer comes by its GELU (none: 0)
+constexpr int kGeluByTable = 1, kGeluByArithmetic = 2;
+constexpr int kArithmeticSteps = 4;  // K steps up to which kEpiArithmetic serves tiles that come through the stage ring
+
 int g_forced_block_n = 0;
 int g_max_ctas = 0;
 int g_debug_flags = 0;
@@ -2099,7 +2198,7 @@ int out_elem_bytes(int out_mode) {
   }
 }
 
-int plan_with(const FimConvGeometry& g, int fmt, bool per_pixel, bool allow_flat, int out_elem, bool gelu, bool convert, bool pool, bool ragged,
+int plan_with(const FimConvGeometry& g, int fmt, bool per_pixel, bool allow_flat, int out_elem, int gelu, bool convert, bool pool, bool ragged,
               Plan* plan) {
   // `g.cin` counts bytes of K per tap here (a BF16 layer arrives with its channel count doubled)
   const bool int8 = fmt == kFmtI8, scaled = fmt == kFmtMx;
@@ -2237,7 +2336,7 @@ int plan_with(const FimConvGeometry& g, int fmt, bool per_pixel, bool allow_flat
       // more copies of the GELU table where shared memory has room for them and a CTA has tiles enough to repay filling them
       // (up to eight: the table's addresses fit 16 bits)
       int left = fit, copies = 1;
-      while (gelu && copies < 8 && tiles >= 8LL * (g_max_ctas > 0 ? g_max_ctas : sm_count())) {
+      while (gelu == kGeluByTable && copies < 8 && tiles >= 8LL * (g_max_ctas > 0 ? g_max_ctas : sm_count())) {
         const int next = (room - static_cast<int>(gelu_smem_bytes(2 * copies) - kGeluSmemBytes)) / (chunks * chunk);
         if (next < (fit < 4 ? fit : 4)) break;
         copies *= 2, left = next;
@@ -2269,7 +2368,7 @@ int plan_with(const FimConvGeometry& g, int fmt, bool per_pixel, bool allow_flat
 // for INT8 layers that 64-byte steps divide, which are bound by shared-memory bandwidth (2x200x190x192: 50 against 53 us; MXFP8 68
 // against 60), and not where the divided steps give a layer its halo patches and the ragged ones do not, or it has many tiles to walk:
 // then the larger patches and fewer stages cost more than the rounds (MXFP8 3x100x120x96 15.4 -> 13.3 us, 4x400x400x96 39.8 -> 41.2).
-int make_plan(const FimConvGeometry& g, int fmt, bool per_pixel, bool allow_flat, int out_elem, bool gelu, Plan* plan, bool convert = false,
+int make_plan(const FimConvGeometry& g, int fmt, bool per_pixel, bool allow_flat, int out_elem, int gelu, Plan* plan, bool convert = false,
               bool pool = false) {
   if (g.cin > 64 && g.cin % 128 != 0 && g.cin % 32 == 0 && (fmt == kFmtMx || (fmt == kFmtI8 && g.cin % 64 != 0)) && !per_pixel && !convert &&
       !(g_debug_flags & 32768)) {
@@ -2338,7 +2437,7 @@ struct PlanEntry {
 };
 constexpr unsigned kPlanEntries = 64;
 
-int plan_for(const FimConvGeometry& g, int fmt, bool per_pixel, bool allow_flat, int out_elem, bool gelu, bool convert, bool pool, Plan* plan,
+int plan_for(const FimConvGeometry& g, int fmt, bool per_pixel, bool allow_flat, int out_elem, int gelu, bool convert, bool pool, Plan* plan,
              Schedule* schedule) {
   static thread_local PlanEntry table[kPlanEntries];
   PlanKey key;
@@ -2400,7 +2499,7 @@ int launch_conv_k(const ConvMaps& maps, const ConvParams& p, const Plan& pl, cud
   if constexpr (FMT != kFmtBf16 && BN <= 128) {
     if (pl.patch) {
       if constexpr (FMT == kFmtMx) {
-        if (pl.fixed_epilogue == (kEpiFixed | kEpiGelu | kEpiStatic)) return launch_patch<FMT, BN, kEpiFixed | kEpiGelu | kEpiStatic>(maps, p, pl, stream);
+        if (pl.fixed_epilogue == (kEpiFixed | kEpiGelu | kEpiStatic)) return launch_patch<FMT, BN, kEpiFixed | kEpiGelu | kEpiStatic | kEpiArithmetic>(maps, p, pl, stream);
       } else {
         if (pl.fixed_epilogue == kEpiPool) return launch_patch<FMT, BN, kEpiPool>(maps, p, pl, stream);
       }
@@ -2421,9 +2520,10 @@ int launch_conv_k(const ConvMaps& maps, const ConvParams& p, const Plan& pl, cud
   if constexpr (FMT == kFmtMx) {
     if (pl.fixed_epilogue == kGeluStatic && !pl.pair) {
       if constexpr (BN == 64) {
-        if (pl.block_k == 64) return launch_conv<FMT, BN, 64, false, kGeluStatic>(maps, p, pl, stream);
-      } else {
-        if (pl.block_k == 128) return launch_conv<FMT, BN, 128, false, kGeluStatic>(maps, p, pl, stream);
+        if (pl.block_k == 64) return launch_conv<FMT, BN, 64, false, kGeluStatic | kEpiArithmetic>(maps, p, pl, stream);
+      } else if (pl.block_k == 128) {
+        return p.kh * p.kw * pl.k_chunks <= kArithmeticSteps ? launch_conv<FMT, BN, 128, false, kGeluStatic | kEpiArithmetic>(maps, p, pl, stream)
+                                                             : launch_conv<FMT, BN, 128, false, kGeluStatic>(maps, p, pl, stream);
       }
     }
     if (pl.fixed_epilogue == (kEpiFixed | kEpiStatic | kEpiGeluSum)) {
@@ -2523,7 +2623,10 @@ int run_conv(int fmt, const void* x, const int8_t* act_exponent, const void* act
   bool allow_flat = !pool;  // pooling windows need the tile to be a patch of the image
   Plan pl;
   Schedule sc;
-  const bool gelu = ep->act == FIM_ACT_GELU, gelu_sum = ep->act == FIM_ACT_GELU_SUM;
+  // (the layers of the fixed epilogue below)
+  const bool by_arithmetic = fmt == kFmtMx && ep->out_mode == FIM_OUT_E4M3_STATIC && ep->bias != nullptr && ep->residual == nullptr && !(g_debug_flags & 1024);
+  const int gelu = ep->act != FIM_ACT_GELU ? 0 : (by_arithmetic ? kGeluByArithmetic : kGeluByTable);
+  const bool gelu_sum = ep->act == FIM_ACT_GELU_SUM;
   if (gelu_sum && (fmt != kFmtMx || convert || ep->out_mode != FIM_OUT_E4M3_STATIC || ep->bias == nullptr || ep->residual != nullptr)) return kUnsupported;
   int rc = plan_for(*g, fmt, per_pixel, allow_flat, out_elem, gelu, convert, pool, &pl, &sc);
   if (rc == kOk && allow_flat && pl.flat && ep->residual != nullptr) {
@@ -2732,7 +2835,7 @@ int run_mlp(const void* x, const void* x_scales, const void* w1, const void* w1_
   }
   const int kc = channels / 128, c = channels;
   const uint32_t unit = static_cast<uint32_t>(kc) * (kMlpTile + 512u);
-  const uint32_t fixed = 1024u + gelu_smem_bytes(kMlpGeluCopies) + unit + 2u * (kMlpTile + 512u) + kMlpOutWarps * (kMlpPanels + kMlpResidualSlots) * kMlpPanelBytes + 3u * c * 4u;
+  const uint32_t fixed = 1024u + kGeluSmemBytes + unit + 2u * (kMlpTile + 512u) + kMlpOutWarps * (kMlpPanels + kMlpResidualSlots) * kMlpPanelBytes + 3u * c * 4u;
   int stages = static_cast<int>((kSmemLimit - fixed) / unit);
   if (stages > kMaxStages) stages = kMaxStages;
   if (stages < 2) return kUnsupported;

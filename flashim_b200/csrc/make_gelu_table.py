@@ -12,6 +12,12 @@ sign bit of the result is the sign bit of the input. ``t = clamp(a - (BASE - 1),
 magnitude below BASE (delta -0x80: the exponent drops by one, magnitudes below the smallest normal number become zero)
 and the last entry every magnitude from TOP on (delta 0 for positive values, -0x8000 for negative ones: zero).
 
+The epilogues that requantise to E4M3 evaluate GELU by arithmetic instead (``gelu_arithmetic_bf16x2`` in conv.cu). ``verify_arithmetic``
+restates it with the coefficients read from that source: for every bf16 value from ``EXACT_FROM`` up the result is torch's, and below
+the E4M3 codes of the two are the same under every exponent from ``CODES_FROM`` up but for the values in ``EXCEPTIONS``, with room
+for the error of the evaluation. The coefficients are a point of the polytope these conditions span (each bounds log2 of Phi(-|x|),
+which is linear in them, from both sides), found by linear programming with the largest distance from all of its sides.
+
 Run ``python flashim_b200/csrc/make_gelu_table.py`` to rewrite the file; ``--check`` only verifies the committed one.
 Deviations from torch that the check allows: subnormal bf16 inputs (flushed to zero), NaN payloads, and the top binade
 (``|x| >= 2**127``), where torch's own expression overflows to infinity.
@@ -19,6 +25,7 @@ Deviations from torch that the check allows: subnormal bf16 inputs (flushed to z
 
 from __future__ import annotations
 
+import re
 import sys
 from pathlib import Path
 
@@ -74,6 +81,38 @@ def verify(base: int, words: list[int]) -> None:
     assert int(got[0x7F80]) == 0x7F80  # +inf
 
 
+EXACT_FROM, CODES_FROM, EXCEPTIONS = -3.515625, -9, {-6: -4.5, -2: -3.53125}
+P_ERROR = 1.5e-6  # relative: the last roundings of q (|q| <= 13, and half an ulp of it in the exponent) and of ex2.approx (2**-22)
+
+
+def verify_arithmetic() -> None:
+    text = (OUT.parent / "conv.cu").read_text()
+    body = text[text.index("gelu_arithmetic_bf16x2(uint32_t r) {"):]
+    numbers = re.findall(r"pack2\((-?\d\.\d+e[-+]\d+)f, \1f\)", body[: body.index("ex2_approx")])
+    coefficients = [torch.tensor(float(n), dtype=torch.float32) for n in numbers]
+    assert len(coefficients) == 6
+    bits, want = torch_gelu_bits()
+    x = bits.to(torch.int16).view(torch.bfloat16).float()
+    u, relu = torch.minimum(x, -x), torch.where(bits >= 0x8000, torch.tensor(-0.0), x)
+    q = coefficients[0].expand(65536)
+    for c in coefficients[1:]:
+        q = (q.double() * u.double() + c.double()).float()  # one rounding, as an fma
+    a = bits & 0x7FFF
+    checked = (a >= 0x100) & (a < 0x7F00)
+    expected = want.to(torch.int16).view(torch.bfloat16)
+    for error in (-P_ERROR, 0.0, P_ERROR):
+        p = torch.where(q < -126, torch.tensor(0.0, dtype=torch.float64), torch.exp2(q.double()) * (1 + error))
+        value = (u.double() * p + relu.double()).float()
+        value = torch.where((p == 0) & (bits >= 0x8000), torch.tensor(-0.0), value)
+        got = value.to(torch.bfloat16)
+        same = (got.view(torch.int16).to(torch.int32) & 0xFFFF) == want
+        assert bool(same[checked & (x >= EXACT_FROM)].all()), "not exact"
+        for e in range(CODES_FROM, 128):
+            codes = [(t.double() * 2.0 ** -e).clamp(-448, 448).float().to(torch.float8_e4m3fn).view(torch.uint8) for t in (got, expected)]
+            differ = checked & (codes[0] != codes[1])
+            assert not bool((differ & (x != EXCEPTIONS.get(e, 1e30))).any()), f"codes differ under the exponent {e}"
+
+
 def render(base: int, top: int, words: list[int]) -> str:
     lines = [
         "// Generated by make_gelu_table.py from torch's erf-form GELU; do not edit.",
@@ -90,6 +129,7 @@ def render(base: int, top: int, words: list[int]) -> str:
 def main() -> None:
     base, top, words = build()
     verify(base, words)
+    verify_arithmetic()
     text = render(base, top, words)
     if "--check" in sys.argv:
         assert OUT.read_text() == text, f"{OUT.name} is stale: run make_gelu_table.py"
