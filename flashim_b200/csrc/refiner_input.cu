@@ -173,9 +173,10 @@ __device__ __forceinline__ float divided(float n, float d, float inv) {
 // leave as 16-byte words instead of single bf16 values. The kernel above waits for one pair of loads per four patch pixels.
 // What bounds it is the issue of instructions (62 % of the slots while an SM had work, 960 per pixel of 96x72x64 with radius 3, of which
 // 128 are the products). A patch that lies inside the image (nearly all do) therefore takes code without a bounds test,
-// a select or an address per load. Input rows, before -> after (us): 2x96x72x64, radius 3 18.4 -> 17.1; 2x100x140x64, radius 2 29.2 -> 23.9;
-// 4x300x300x64, radius 3 453 -> 394; 2x200x200x128, radius 2 120 -> 109; 2x100x100x32, radius 3 19.5 -> 16.3. (Three CTAs, or twice the
-// loads in flight, are slower at most sizes.)
+// a select or an address per load. Input rows, before -> after (us): 2x96x72x64, radius 3 18.4 -> 15.9; 2x100x140x64, radius 2 29.2 -> 23.7;
+// 4x300x300x64, radius 3 453 -> 357; 2x200x200x128, radius 2 120 -> 109; 2x100x100x32, radius 3 19.4 -> 15.7. (Three CTAs, or twice the
+// loads in flight, are slower at most sizes; so are four pixels per warp over the union of their patches, 22.5 at the first size: fewer
+// loads, but too few warps for their latency.)
 template <int NF, int R>
 __global__ void __launch_bounds__(32 * kInputWarps, 4) refiner_input_wide_kernel(const InputParams p) {
   grid_release();
@@ -211,29 +212,34 @@ __global__ void __launch_bounds__(32 * kInputWarps, 4) refiner_input_wide_kernel
       const long long line = static_cast<long long>(p.width) * P;  // floats of an image row
       // (uniform over the warp)
       const bool inside = finite && x0 >= R && y0 >= R && x0 + R + 1 < p.width && y0 + R + 1 < p.height;
-      // f_b at the warp, NF channels per lane; the corners are patch pixels too
-      {
-        const bool north = finite && y0 >= 0 && y0 < p.height, south = finite && y0 + 1 >= 0 && y0 + 1 < p.height;
-        const bool west = x0 >= 0 && x0 < p.width, east = x0 + 1 >= 0 && x0 + 1 < p.width;
-        const float* base = other + y0 * line + static_cast<long long>(x0) * P + NF * lane;
-        Floats<NF> nw = {}, ne = {}, sw = {}, se = {};
-        if (inside) {
-          nw = load_floats<NF>(base), ne = load_floats<NF>(base + P), sw = load_floats<NF>(base + line), se = load_floats<NF>(base + line + P);
-        } else {
-          if (north && west) nw = load_floats<NF>(base);
-          if (north && east) ne = load_floats<NF>(base + P);
-          if (south && west) sw = load_floats<NF>(base + line);
-          if (south && east) se = load_floats<NF>(base + line + P);
+      // f_b at the warp, NF channels per lane, and f_a itself. The corners are patch pixels too: with up to 64 features this comes behind
+      // the dot products, when the L1 holds them (2x96x72x64, radius 3: 17.1 -> 15.9 us); with 128 it costs registers that the products need
+      // (2x200x200x128, radius 2: 109 -> 117).
+      const auto copy_rows = [&]() {
+        {
+          const bool north = finite && y0 >= 0 && y0 < p.height, south = finite && y0 + 1 >= 0 && y0 + 1 < p.height;
+          const bool west = x0 >= 0 && x0 < p.width, east = x0 + 1 >= 0 && x0 + 1 < p.width;
+          const float* base = other + y0 * line + static_cast<long long>(x0) * P + NF * lane;
+          Floats<NF> nw = {}, ne = {}, sw = {}, se = {};
+          if (inside) {
+            nw = load_floats<NF>(base), ne = load_floats<NF>(base + P), sw = load_floats<NF>(base + line), se = load_floats<NF>(base + line + P);
+          } else {
+            if (north && west) nw = load_floats<NF>(base);
+            if (north && east) ne = load_floats<NF>(base + P);
+            if (south && west) sw = load_floats<NF>(base + line);
+            if (south && east) se = load_floats<NF>(base + line + P);
+          }
+#pragma unroll
+          for (int i = 0; i < NF; ++i) store_bf16(row + P + NF * lane + i, fmaf(se.v[i], w_se, fmaf(sw.v[i], w_sw, fmaf(nw.v[i], w_nw, ne.v[i] * w_ne))));
         }
+        // f_a itself: every lane one of the four channels that its group and the three others hold
 #pragma unroll
-        for (int i = 0; i < NF; ++i) store_bf16(row + P + NF * lane + i, nw.v[i] * w_nw + ne.v[i] * w_ne + sw.v[i] * w_sw + se.v[i] * w_se);
-      }
-      // f_a itself: every lane one of the four channels that its group and the three others hold
-#pragma unroll
-      for (int i = 0; i < NF; ++i) {
-        const float lower = group & 1 ? a[i].y : a[i].x, upper = group & 1 ? a[i].w : a[i].z;
-        store_bf16(row + 32 * i + 4 * sub + group, group & 2 ? upper : lower);
-      }
+        for (int i = 0; i < NF; ++i) {
+          const float lower = group & 1 ? a[i].y : a[i].x, upper = group & 1 ? a[i].w : a[i].z;
+          store_bf16(row + 32 * i + 4 * sub + group, group & 2 ? upper : lower);
+        }
+      };
+      if (NF == 4) copy_rows();
       // dot products with the patch pixels, a group of eight lanes per pixel, eight pixels of a group per butterfly
       const auto form_dots = [&](auto unchecked) {
         constexpr bool kInside = decltype(unchecked)::value;
@@ -294,6 +300,7 @@ __global__ void __launch_bounds__(32 * kInputWarps, 4) refiner_input_wide_kernel
       } else {
         form_dots(std::false_type{});
       }
+      if (NF != 4) copy_rows();
       {
         const float dx = p.scale_x * (at.x - (-1.0f + divided(2.0f * x + 1.0f, p.width, p.inv_width)));
         const float dy = p.scale_y * (at.y - (-1.0f + divided(2.0f * y + 1.0f, p.height, p.inv_height)));
