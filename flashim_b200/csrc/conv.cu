@@ -138,9 +138,9 @@ struct GeluTable {
   uint32_t stride;  // bytes from one entry to the next
 };
 // `copies` > 1 (a power of two): entry e of copy c is word e * copies + c, and a lane reads copy lane % copies. Lanes of
-// different copies never share a bank, so the 32 scattered reads of a look-up take about 2.2 passes with eight copies
-// where one copy takes 3.5: what bounds the layers with the shortest main loops (3x3 64 -> 64 at 800x800: shared-memory
-// wavefronts 78 % busy, 176 -> 154 us).
+// different copies never share a bank, so the 32 scattered reads of a look-up take about 2.9 passes with eight copies
+// where one copy takes 3.4: what bounds layers with short main loops whose outputs are bf16 or have exponents per pixel (with static
+// exponents, before the arithmetic below: 3x3 64 -> 64 at 800x800 176 -> 154 us).
 __device__ __forceinline__ GeluTable gelu_table_at(uint32_t smem_address, uint32_t copies = 1, uint32_t lane = 0) {
   GeluTable t;
   t.low2 = ((smem_address & 0xFFFFu) + 4u * (lane & (copies - 1u))) * 0x00010001u;
@@ -318,8 +318,8 @@ constexpr int kEpiArithmetic = 512;
 // groups are one patch row apart (the descriptor's stride). The swizzle is a function of the shared-memory address, so a
 // shifted start needs no other layout. Per tile that is one copy and one barrier round instead of one per tap and channel
 // chunk, 1.4 activation bytes per input byte instead of 9 (3x3), and no scale copies: all weight scales stay in tensor memory.
-//   MXFP8 3x3 + bias + GELU + static requantisation, N = 4: 800x800x64 363 -> 154 us, 400x400x128 117 -> 92 (with a plain
-//   bf16 output 107 -> 70); INT8 3x3 + bias: 4x201x199x128 31 -> 20, 4x400x400x64 84 -> 32.
+//   MXFP8 3x3 + bias + GELU + static requantisation, N = 4: 800x800x64 363 -> 154 us (122 with what came after), 400x400x128 117 -> 92 (73;
+//   with a plain bf16 output 107 -> 70); INT8 3x3 + bias: 4x201x199x128 31 -> 20, 4x400x400x64 84 -> 31.
 constexpr int kPatch = 128;
 // Ragged K steps: input channels that 128 does not divide (96, 160, 192, ...) go in 128-byte steps all the same. The last step of a tap
 // has only as many MMAs as it has 32-channel blocks; what its boxes bring beyond them (zeros of the activations, the next tap's weights)

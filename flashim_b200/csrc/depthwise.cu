@@ -20,10 +20,11 @@
 //
 // Measured against the fp32-pipe kernel before it (B200, inputs in L2 where they fit):
 //   4x200x200x256: GELU -> bf16 68 -> 52 us, ReLU -> bf16 54 -> 42, GELU -> MXFP8 88 -> 85, ReLU -> INT8 87 -> 51
-//   8x400x400x128: GELU -> bf16 232 -> 160, ReLU -> bf16 183 -> 127 (80 % of the HBM copy rate), GELU -> MXFP8 303 -> 282,
+//   8x400x400x128: GELU -> bf16 232 -> 160, ReLU -> bf16 183 -> 127 (80 % of the HBM copy rate), GELU -> MXFP8 303 -> 281,
 //   ReLU -> MXFP8 252 -> 198, ReLU -> INT8 299 -> 165
-// What bounds the GELU and quantising forms now is the arithmetic of their epilogues on twelve warps per SM (issue slots about
-// half busy). The same bytes as the chain (below) cost the MXFP8 form up to a quarter of its time: 225 and 178 us with a test that
+// What bounds the GELU and quantising forms now is what the schedulers can dispatch: packed FMAs, permutes, integer and conversion
+// instructions take two cycles each and the MMAs of twelve warps 11.4, one after the other (MXFP8: about 90 % of the 1900 cycles per warp and
+// step; bf16 GELU: 72 % of 1240). Sixteen warps with one set of B fragments per CTA were slower (bf16 GELU 57 -> 61 us). The same bytes as the chain (below) cost the MXFP8 form up to a quarter of its time: 225 and 178 us with a test that
 // missed half of the codes that differ. Where the arguments of the GELU reach far into its left tail (a standard deviation of 1.5 and
 // up) it takes 360 us, more than the fp32-pipe kernel.
 //
