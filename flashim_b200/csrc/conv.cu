@@ -2728,24 +2728,17 @@ int run_conv(int fmt, const void* x, const int8_t* act_exponent, const void* act
     const uint64_t row = static_cast<uint64_t>(g->cout) * out_elem;
     const uint64_t dims[4] = {row, static_cast<uint64_t>(o_w), static_cast<uint64_t>(o_h), static_cast<uint64_t>(o_b)};
     const uint64_t strides[3] = {row, static_cast<uint64_t>(o_w) * row, static_cast<uint64_t>(o_h) * o_w * row};
-    const uint32_t box[4] = {static_cast<uint32_t>(32 * out_elem), static_cast<uint32_t>(pl.tile_w), static_cast<uint32_t>(pl.tile_h), 1};
+    // one store per group of warps: a tile; or per warp: 32 rows of the pixel matrix, or four image rows of a patch tile
+    const bool own = (pl.flat && !(g_debug_flags & 512)) ||
+                     (pl.patch && (pl.block_n == 128 || out_elem == 1 || p.act == kActGelu || p.residual != nullptr || pool));
+    const uint32_t box_w = static_cast<uint32_t>(!own ? pl.tile_w : pl.flat ? 32 : kPatchTileW);
+    const uint32_t box_h = static_cast<uint32_t>(!own ? pl.tile_h : pl.flat ? 1 : kPatchTileH / 4);
+    const uint32_t box[4] = {static_cast<uint32_t>(32 * out_elem), box_w, box_h, 1};
     const int rcm = make_tensor_map(&out_map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 4, out, dims, strides, box, swizzle_for_bytes(32 * out_elem));
     if (rcm != kOk) return rcm;
     maps.out_warp = out_map;
-    p.warp_panels = 0;
-    if (pl.flat && !(g_debug_flags & 512)) {  // one store per warp: 32 rows of the pixel matrix x 32 channels
-      const uint32_t warp_box[4] = {static_cast<uint32_t>(32 * out_elem), 32, 1, 1};
-      const int rcw = make_tensor_map(&maps.out_warp, CU_TENSOR_MAP_DATA_TYPE_UINT8, 4, out, dims, strides, warp_box,
-                                      swizzle_for_bytes(32 * out_elem));
-      if (rcw != kOk) return rcw;
-      p.warp_panels = 1;
-    }
-    if (pl.patch) {  // (a patch kernel's warps store four image rows of a tile each)
-      const uint32_t warp_box[4] = {static_cast<uint32_t>(32 * out_elem), kPatchTileW, kPatchTileH / 4, 1};
-      const int rcw = make_tensor_map(&maps.out_warp, CU_TENSOR_MAP_DATA_TYPE_UINT8, 4, out, dims, strides, warp_box, swizzle_for_bytes(32 * out_elem));
-      if (rcw != kOk) return rcw;
-      p.warp_panels = pl.block_n == 128 || out_elem == 1 || p.act == kActGelu || p.residual != nullptr ? 1 : 0;
-    } else if (pool) {  // the pooled output [B, Ho / 2, Wo / 2, Cout] INT8, stored in boxes of a quarter tile x 32 channels
+    p.warp_panels = own ? 1 : 0;
+    if (pool && !pl.patch) {  // the pooled output [B, Ho / 2, Wo / 2, Cout] INT8, stored in boxes of a quarter tile x 32 channels
       const uint64_t prow = static_cast<uint64_t>(g->cout), ph = static_cast<uint64_t>(pl.out_h / 2), pw = static_cast<uint64_t>(pl.out_w / 2);
       const uint64_t pdims[4] = {prow, pw, ph, static_cast<uint64_t>(o_b)};
       const uint64_t pstrides[3] = {prow, pw * prow, ph * pw * prow};
