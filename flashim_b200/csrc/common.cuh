@@ -601,6 +601,12 @@ __device__ __forceinline__ uint32_t bf16x2_min_nan(uint32_t a, uint32_t b) {
   asm("min.NaN.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
   return d;
 }
+// ones in the halves whose numbers are equal
+__device__ __forceinline__ uint32_t bf16x2_equal(uint32_t a, uint32_t b) {
+  uint32_t d;
+  asm("set.eq.u32.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
+  return d;
+}
 
 // GELU through the complementary error function in the rational-exponential form of Abramowitz & Stegun 7.1.26
 // (|error of erf| <= 1.5e-7): gelu(x) = x/2 * (2 - c) for x >= 0 and x/2 * c for x < 0 with c = erfc(|x|/sqrt 2).

@@ -171,8 +171,8 @@ __device__ __forceinline__ uint32_t gelu_bf16x2(uint32_t r, const GeluTable& tab
 // five. Its coefficients solve the linear inequalities that make the rounded result torch's for EVERY bf16 value from -3.515625 up
 // (make_gelu_table.py checks them, with a margin for the roundings of the evaluation); a minimax polynomial of that degree misses
 // some. Below, torch's own result is the rounding noise of 1 + erf, which no polynomial follows, but the E4M3 codes of both are the
-// same under every exponent from -9 up, except those of one value under -6 and of one under -2. What is left, with infinities and
-// not-a-numbers, takes the table. As many issue slots as the look-up, and none of the shared-memory wavefronts that bounded these
+// same under every exponent from -9 up, except those of one value under -6 and of one under -2 (gelu_replace). Arguments in that tail under
+// smaller exponents, infinities and not-a-numbers take the table. As many issue slots as the look-up, and none of the shared-memory wavefronts that bounded these
 // epilogues (32 scattered reads take 3.3 passes, 2.9 with eight copies of the table): us, table -> arithmetic:
 // 3x3 4x800x800x64 135 -> 122, 4x400x400x128 89 -> 74; 1x1 8x100x100x512 -> 1024 65 -> 59; residual MLP 8x400x400x128 255 -> 229 (arguments of
 // a standard deviation of 1.4, many of them in the tail: 243), 8x200x200x256 164 -> 140.
@@ -197,16 +197,14 @@ __device__ __forceinline__ uint32_t gelu_arithmetic_bf16x2(uint32_t r) {
   return pack_bf16(q0, q1);
 }
 constexpr uint32_t kGeluTail = 0xC061u;  // the last argument for which it is exact, -3.515625; larger ones (unsigned) lie below
-// the one argument whose code differs under an exponent (-4.5, -3.53125; 0: none)
-__device__ __forceinline__ uint32_t gelu_exception(int e) { return e == -6 ? 0xC090u : (e == -2 ? 0xC062u : 0u); }
-__device__ __forceinline__ bool contains(const uint32_t (&r)[16], uint32_t value) {
-  uint32_t hit = 0;
+// the one argument whose code differs under an exponent (-4.5 under -6, -3.53125 under -2)
+__device__ __forceinline__ uint32_t gelu_exception(int e) { return e == -6 ? 0xC090u : 0xC062u; }
+// The next bf16 value towards zero takes the place of an exception: its code by arithmetic is torch's of the exception under that exponent,
+// under the two below and under all above. Two instructions a word. (While an exception sent its warp to the table, 3x3 4x800x800x64 under
+// -6 took 181 us at arguments of a standard deviation of 3 instead of 136, the residual MLP 8x400x400x128 281 at 2.5 instead of 268.)
+__device__ __forceinline__ void gelu_replace(uint32_t (&r)[16], uint32_t exception) {
 #pragma unroll
-  for (int i = 0; i < 16; ++i) {
-    const uint32_t t = r[i] ^ (value * 0x00010001u);
-    hit |= (t - 0x00010001u) & ~t;  // the top bit of a half that is zero (or, above one, of a half that may not be)
-  }
-  return (hit & 0x80008000u) != 0;
+  for (int i = 0; i < 16; ++i) r[i] = __viaddmax_s16x2(r[i], bf16x2_equal(r[i], exception * 0x00010001u), 0x80008000u);
 }
 
 // the largest positive argument (bits; negative without one)
@@ -217,30 +215,25 @@ __device__ __forceinline__ int gelu_highest(const uint32_t (&r)[16]) {
   return max(static_cast<int>(high) >> 16, static_cast<int>(static_cast<int16_t>(high & 0xFFFFu)));
 }
 
-// GELU of 32 values, by arithmetic unless one of the warp's lanes asks for the table (its one copy: little reaches it)
-__device__ __forceinline__ void gelu_chunk(uint32_t (&r)[16], bool look_up, const GeluTable& table) {
-  if (__any_sync(0xffffffffu, look_up)) {
-#pragma unroll
-    for (int i = 0; i < 16; ++i) r[i] = gelu_bf16x2(r[i], table);
-  } else {
-#pragma unroll
-    for (int i = 0; i < 16; ++i) r[i] = gelu_arithmetic_bf16x2(r[i]);
-  }
-}
-
-// ... under a static exponent
+// GELU of 32 values under a static exponent: by arithmetic, unless one of the warp's lanes asks for the table. One vote decides where most
+// exponents leave it: a warp's time for its chunk is what a tile of a patch layer waits for, and a second vote on that way costs 3 to 5 %.
 __device__ __forceinline__ void gelu_chunk_static(uint32_t (&r)[16], int e, const GeluTable& table) {
   uint32_t low = r[0], high = r[0];
 #pragma unroll
   for (int i = 1; i < 16; ++i) low = __vmaxu2(low, r[i]), high = __vmaxs2(high, r[i]);
   const uint32_t lowest = max(low & 0xFFFFu, low >> 16);  // (as unsigned halves: of two negative values the larger magnitude)
   const int highest = max(static_cast<int>(high) >> 16, static_cast<int>(static_cast<int16_t>(high & 0xFFFFu)));
-  bool look_up = !(lowest < 0xFF80u && highest < 0x7F80);
-  if ((e < -9 || e == -6 || e == -2) && lowest > kGeluTail) {
-    const bool differ = contains(r, e == -6 ? gelu_exception(-6) : gelu_exception(-2));
-    look_up |= e < -9 || differ;
+  const uint32_t from = e < -9 || e == -6 || e == -2 ? kGeluTail : 0xFF7Fu;
+  if (__any_sync(0xffffffffu, lowest > from || highest >= 0x7F80)) {
+    if (__any_sync(0xffffffffu, lowest >= 0xFF80u || highest >= 0x7F80 || e < -9)) {
+#pragma unroll
+      for (int i = 0; i < 16; ++i) r[i] = gelu_bf16x2(r[i], table);
+      return;
+    }
+    gelu_replace(r, e == -6 ? gelu_exception(-6) : gelu_exception(-2));
   }
-  gelu_chunk(r, look_up, table);
+#pragma unroll
+  for (int i = 0; i < 16; ++i) r[i] = gelu_arithmetic_bf16x2(r[i]);
 }
 
 // the largest magnitude of 32 values, bf16 bits (KEEP_NAN: above 0x7F80 if one is not a number, which does not count otherwise)
@@ -256,30 +249,44 @@ __device__ __forceinline__ uint32_t largest_magnitude(const uint32_t (&r)[16]) {
   return max(m[0] & 0x7FFFu, (m[0] >> 16) & 0x7FFFu);
 }
 
-// ... that form a block with an exponent of its own, which it returns. Where arguments lie in the tail the exponent has to be known ahead:
-// it is that of the largest result, which is the GELU of the largest argument from 0.703 up (results below zero stay above -0.17).
+// GELU of 32 values that form a block with an exponent of its own, which it returns. Where arguments lie in the tail the exponent has to be
+// known ahead: it is that of the largest result, which is the GELU of the largest argument from 0.703 up (results below zero stay above -0.17).
 // One minimum per word tells the tail, negative infinities and not-a-numbers; behind those a result that is not a number comes from
-// a positive infinity.
-__device__ __forceinline__ int gelu_chunk_dynamic(uint32_t (&r)[16], const GeluTable& table) {
-  uint32_t low = r[0];
+// a positive infinity. Blocks that need the table come together (channels of mostly negative arguments), so behind two in a row the
+// warp's next seven go there unseen, which is right for any argument; `streak` (zero at first) counts them (residual MLP 8x400x400x128,
+// arguments of mean -2: 285 -> 272 us, what the table alone takes).
+__device__ __forceinline__ int gelu_chunk_dynamic(uint32_t (&r)[16], const GeluTable& table, int& streak) {
+  bool look_up = streak > 1;
+  if (look_up) {
+    --streak;
+  } else {
+    uint32_t low = r[0];
 #pragma unroll
-  for (int i = 1; i < 16; ++i) low = bf16x2_min_nan(low, r[i]);
-  const uint32_t lowest = max(low & 0xFFFFu, low >> 16);  // (negative halves are the larger ones; a not-a-number is 0x7FFF)
-  bool look_up = false;
-  const bool not_a_number = max(low & 0x7FFFu, (low >> 16) & 0x7FFFu) > 0x7F80u;
-  if (lowest > kGeluTail || not_a_number) {
-    const int highest = gelu_highest(r);
-    look_up = not_a_number || lowest >= 0xFF80u || highest >= 0x7F80 || highest < 0x3F34;                        // the last: may be below -9
-    if (highest >= 0x4060 && highest <= 0x40E0 && lowest >= gelu_exception(-6)) look_up |= contains(r, gelu_exception(-6));  // 3.5 to 7
-    if (highest >= 0x4260 && highest <= 0x42E0) look_up |= contains(r, gelu_exception(-2));                                  // 56 to 112
+    for (int i = 1; i < 16; ++i) low = bf16x2_min_nan(low, r[i]);
+    const uint32_t lowest = max(low & 0xFFFFu, low >> 16);  // (negative halves are the larger ones; a not-a-number is 0x7FFF)
+    const bool not_a_number = max(low & 0x7FFFu, (low >> 16) & 0x7FFFu) > 0x7F80u;
+    if (lowest > kGeluTail || not_a_number) {
+      const int highest = gelu_highest(r);
+      look_up = not_a_number || lowest >= 0xFF80u || highest >= 0x7F80 || highest < 0x3F34;                             // the last: may be below -9
+      if (highest >= 0x4060 && highest <= 0x40E0 && lowest >= gelu_exception(-6)) gelu_replace(r, gelu_exception(-6));  // 3.5 to 7
+      if (highest >= 0x4260 && highest <= 0x42E0) gelu_replace(r, gelu_exception(-2));                                  // 56 to 112
+    }
+    look_up = __any_sync(0xffffffffu, look_up);
+    streak = look_up ? (streak == 1 ? 8 : 1) : 0;
   }
-  gelu_chunk(r, look_up, table);
+  if (look_up) {
+#pragma unroll
+    for (int i = 0; i < 16; ++i) r[i] = gelu_bf16x2(r[i], table);
+    return e8m0_exponent_bits(largest_magnitude(r) << 16);
+  }
+#pragma unroll
+  for (int i = 0; i < 16; ++i) r[i] = gelu_arithmetic_bf16x2(r[i]);
   uint32_t top = largest_magnitude<true>(r);
   if (top > 0x7F80u) {
 #pragma unroll
     for (int i = 0; i < 16; ++i) {
-      if ((r[i] & 0x7FFFu) > 0x7F80u && !look_up) r[i] = (r[i] & 0xFFFF0000u) | 0x7F80u;
-      if ((r[i] & 0x7FFF0000u) > 0x7F800000u && !look_up) r[i] = (r[i] & 0xFFFFu) | 0x7F800000u;
+      if ((r[i] & 0x7FFFu) > 0x7F80u) r[i] = (r[i] & 0xFFFF0000u) | 0x7F80u;
+      if ((r[i] & 0x7FFF0000u) > 0x7F800000u) r[i] = (r[i] & 0xFFFFu) | 0x7F800000u;
     }
     top = largest_magnitude<false>(r);
   }
@@ -1336,6 +1343,7 @@ conv_kernel(const __grid_constant__ CUtensorMap act_map, const __grid_constant__
       const uint32_t bias_at = smem_bias + static_cast<uint32_t>(group * kGroupColumns) * 4u;
       const uint32_t lane_tmem = tmem + (static_cast<uint32_t>(quarter * 32) << 16) + group * kGroupColumns;
       const GeluTable gelu2 = gelu_table_at(smem_gelu);
+      int gelu_streak = 0;
       const int row = quarter * 32 + lane;
       const int scale_tiles = ((p.cout >> 5) + 3) >> 2;         // 4-group tiles per row tile of the output scales
       const uint32_t scale_at = static_cast<uint32_t>(lane * 16 + quarter * 4);
@@ -1389,7 +1397,7 @@ conv_kernel(const __grid_constant__ CUtensorMap act_map, const __grid_constant__
           uint32_t(&r)[16] = q[g];
           static_assert(!kGelu || (kDynamic && !kResidual), "the GELU of a flat layer is followed by its block's exponent");
           int e = 0;
-          if (kGelu) e = gelu_chunk_dynamic(r, gelu2);
+          if (kGelu) e = gelu_chunk_dynamic(r, gelu2, gelu_streak);
           if (kResidual) {
             if (valid) {
               const uint4* r4 = reinterpret_cast<const uint4*>(res_row + g * 32);
@@ -1718,6 +1726,8 @@ constexpr uint32_t kMlpTile = 128u * 128u;  // bytes of one operand tile: 128 ro
 constexpr int kMlpOutWarps = 8;  // output warps: two per lane quarter of tensor memory, which take alternate 32-channel chunks
 constexpr int kMlpThreads = kThreads + 32 * kMlpOutWarps;
 constexpr uint32_t kMlpPanels = 2, kMlpPanelBytes = 32u * 64u;  // output panels per output warp: 32 rows x 32 bf16 channels
+// copies of the GELU table (with one, arguments of mean -2, most of whose blocks go there, take 1 % longer at 128 channels and 2 % at 256)
+constexpr int kMlpGeluCopies = 4;
 constexpr uint32_t kMlpResidualSlots = 2;  // residual panels (same shape) each output warp keeps in flight
 struct MlpParams {
   int rows, row_tiles, stages;
@@ -1757,7 +1767,7 @@ mlp_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constant__ CU
 
   const uint32_t base = (smem_u32(smem_dyn) + 1023u) & ~1023u;
   const uint32_t smem_gelu = base;
-  const uint32_t smem_x = base + kGeluSmemBytes;
+  const uint32_t smem_x = base + gelu_smem_bytes(kMlpGeluCopies);
   const uint32_t smem_w = smem_x + kUnitBytes;
   const uint32_t smem_h = smem_w + static_cast<uint32_t>(p.stages) * kUnitBytes;
   const uint32_t smem_out = smem_h + 2u * kMlpTile;
@@ -1810,7 +1820,11 @@ mlp_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constant__ CU
   constexpr int kSetupThreads = kMlpThreads - 32;
   if (warp != 0) {
     for (int i = threadIdx.x - 32; i < kGeluEntries; i += kSetupThreads) {
-      asm volatile("st.shared.b32 [%0], %1;" ::"r"(smem_gelu + i * 4), "r"(kGeluTable[i]) : "memory");
+      const uint32_t entry = kGeluTable[i];
+#pragma unroll
+      for (int c = 0; c < kMlpGeluCopies; ++c) {
+        asm volatile("st.shared.b32 [%0], %1;" ::"r"(smem_gelu + (i * kMlpGeluCopies + c) * 4), "r"(entry) : "memory");
+      }
     }
   }
   grid_wait();
@@ -1969,7 +1983,8 @@ mlp_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constant__ CU
     // ===== hidden-block warps: lanes 32 * (w % 4) ... of tensor memory, 32 hidden channels (w - 2) / 4 of every block =====
     const int quarter = warp & 3, group = (warp - 2) >> 2;
     const int row = quarter * 32 + lane;
-    const GeluTable gelu2 = gelu_table_at(smem_gelu);
+    const GeluTable gelu2 = gelu_table_at(smem_gelu, kMlpGeluCopies, static_cast<uint32_t>(lane));
+    int gelu_streak = 0;
     const uint32_t lane_tmem = tmem + (static_cast<uint32_t>(quarter * 32) << 16) + kAcc1 + group * 32;
     // where this lane's 32 hidden bytes go in a K-major 128-byte-swizzled tile, and its scale byte in the scale tile
     const uint32_t h_row = static_cast<uint32_t>(row) * 128u;
@@ -2014,7 +2029,7 @@ mlp_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constant__ CU
       int e = 0;
       uint32_t w[8];
       if (!(probe_flags(p) & 4)) {
-      e = gelu_chunk_dynamic(r, gelu2);
+      e = gelu_chunk_dynamic(r, gelu2, gelu_streak);
       scale_to_e4m3(r, e, w);
       } else {
 #pragma unroll
@@ -2338,7 +2353,7 @@ int plan_with(const FimConvGeometry& g, int fmt, bool per_pixel, bool allow_flat
       // more copies of the GELU table where shared memory has room for them and a CTA has tiles enough to repay filling them
       // (up to eight: the table's addresses fit 16 bits)
       int left = fit, copies = 1;
-      while (gelu == kGeluByTable && copies < 8 && tiles >= 8LL * (g_max_ctas > 0 ? g_max_ctas : sm_count())) {
+      while (gelu != 0 && copies < 8 && tiles >= 8LL * (g_max_ctas > 0 ? g_max_ctas : sm_count())) {
         const int next = (room - static_cast<int>(gelu_smem_bytes(2 * copies) - kGeluSmemBytes)) / (chunks * chunk);
         if (next < (fit < 4 ? fit : 4)) break;
         copies *= 2, left = next;
@@ -2830,7 +2845,7 @@ int run_mlp(const void* x, const void* x_scales, const void* w1, const void* w1_
   }
   const int kc = channels / 128, c = channels;
   const uint32_t unit = static_cast<uint32_t>(kc) * (kMlpTile + 512u);
-  const uint32_t fixed = 1024u + kGeluSmemBytes + unit + 2u * (kMlpTile + 512u) + kMlpOutWarps * (kMlpPanels + kMlpResidualSlots) * kMlpPanelBytes + 3u * c * 4u;
+  const uint32_t fixed = 1024u + gelu_smem_bytes(kMlpGeluCopies) + unit + 2u * (kMlpTile + 512u) + kMlpOutWarps * (kMlpPanels + kMlpResidualSlots) * kMlpPanelBytes + 3u * c * 4u;
   int stages = static_cast<int>((kSmemLimit - fixed) / unit);
   if (stages > kMaxStages) stages = kMaxStages;
   if (stages < 2) return kUnsupported;

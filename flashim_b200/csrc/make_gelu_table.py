@@ -14,8 +14,9 @@ and the last entry every magnitude from TOP on (delta 0 for positive values, -0x
 
 The epilogues that requantise to E4M3 evaluate GELU by arithmetic instead (``gelu_arithmetic_bf16x2`` in conv.cu). ``verify_arithmetic``
 restates it with the coefficients read from that source: for every bf16 value from ``EXACT_FROM`` up the result is torch's, and below
-the E4M3 codes of the two are the same under every exponent from ``CODES_FROM`` up but for the values in ``EXCEPTIONS``, with room
-for the error of the evaluation. The coefficients are a point of the polytope these conditions span (each bounds log2 of Phi(-|x|),
+the E4M3 codes of the two are the same under every exponent from ``CODES_FROM`` up but for the values in ``EXCEPTIONS``, whose upper
+neighbours have the right codes there and under every exponent not more than ``REPLACED_BELOW`` less, with room for the error of the
+evaluation. The coefficients are a point of the polytope these conditions span (each bounds log2 of Phi(-|x|),
 which is linear in them, from both sides), found by linear programming with the largest distance from all of its sides.
 
 Run ``python flashim_b200/csrc/make_gelu_table.py`` to rewrite the file; ``--check`` only verifies the committed one.
@@ -81,7 +82,7 @@ def verify(base: int, words: list[int]) -> None:
     assert int(got[0x7F80]) == 0x7F80  # +inf
 
 
-EXACT_FROM, CODES_FROM, EXCEPTIONS = -3.515625, -9, {-6: -4.5, -2: -3.53125}
+EXACT_FROM, CODES_FROM, EXCEPTIONS, REPLACED_BELOW = -3.515625, -9, {-6: -4.5, -2: -3.53125}, 2
 P_ERROR = 1.5e-6  # relative: the last roundings of q (|q| <= 13, and half an ulp of it in the exponent) and of ex2.approx (2**-22)
 
 
@@ -91,6 +92,9 @@ def verify_arithmetic() -> None:
     numbers = re.findall(r"pack2\((-?\d\.\d+e[-+]\d+)f, \1f\)", body[: body.index("ex2_approx")])
     coefficients = [torch.tensor(float(n), dtype=torch.float32) for n in numbers]
     assert len(coefficients) == 6
+    exceptions = re.search(r"gelu_exception\(int e\) { return e == (-\d+) \? (0x\w+)u : (0x\w+)u; }", text)
+    as_float = lambda code: float(torch.tensor([int(code, 16) - 0x10000], dtype=torch.int16).view(torch.bfloat16))  # noqa: E731
+    assert {int(exceptions[1]): as_float(exceptions[2]), -2: as_float(exceptions[3])} == EXCEPTIONS
     bits, want = torch_gelu_bits()
     x = bits.to(torch.int16).view(torch.bfloat16).float()
     u, relu = torch.minimum(x, -x), torch.where(bits >= 0x8000, torch.tensor(-0.0), x)
@@ -111,6 +115,9 @@ def verify_arithmetic() -> None:
             codes = [(t.double() * 2.0 ** -e).clamp(-448, 448).float().to(torch.float8_e4m3fn).view(torch.uint8) for t in (got, expected)]
             differ = checked & (codes[0] != codes[1])
             assert not bool((differ & (x != EXCEPTIONS.get(e, 1e30))).any()), f"codes differ under the exponent {e}"
+            for exponent, value in EXCEPTIONS.items():
+                at = int((x == value).nonzero())
+                assert e < exponent - REPLACED_BELOW or codes[0][at - 1] == codes[1][at], f"the neighbour of {value} under the exponent {e}"
 
 
 def render(base: int, top: int, words: list[int]) -> str:
