@@ -21,9 +21,13 @@
 #include <dlfcn.h>
 #include <torch/csrc/autograd/python_variable.h>
 
+#include <atomic>
 #include <cstdint>
 #include <list>
+#include <memory>
+#include <mutex>
 #include <unordered_map>
+#include <vector>
 
 #include "flashim_sm100.h"
 
@@ -275,6 +279,10 @@ PyObject* shape_tuple(const Tensor& t) {
 // ---- swizzled weight scales, once per exponent tensor ----------------------------------------------------------------
 // Keyed on the storage; an entry holds its source, so the address cannot be reused while the entry lives, and is valid for
 // one shape and version of it. At most 512 entries, the least recently used one goes first. Guarded by the interpreter lock.
+//
+// A graph under capture reads at its replays, any number of times and long after the call. Scales that it finds here stay for as long
+// as it (or an executable made from it) does, whatever becomes of their entry; scales that it has to form are formed by
+// every replay, so the call's own result never exists and is not kept here.
 
 struct Swizzled {
   const void* key;
@@ -291,16 +299,61 @@ void drop_swizzled(std::unordered_map<const void*, std::list<Swizzled>::iterator
   swizzled_at.erase(at);
 }
 
+// Tensors whose last graph has gone. A graph lets go of them on a thread and at a time of the driver's choosing, where no call may be
+// made that frees them, so they wait here for the next look-up. (The list is never destroyed: graphs may go while the process ends.)
+std::mutex released_mutex;
+std::vector<Tensor*>& released = *new std::vector<Tensor*>;
+std::atomic<bool> any_released{false};
+
+void release_to_next_call(void* tensor) {
+  const std::lock_guard<std::mutex> lock(released_mutex);
+  released.push_back(static_cast<Tensor*>(tensor));
+  any_released = true;
+}
+
+void free_released() {
+  if (!any_released) return;
+  std::vector<Tensor*> gone;
+  {
+    const std::lock_guard<std::mutex> lock(released_mutex);
+    gone.swap(released);
+    any_released = false;
+  }
+  for (Tensor* t : gone) delete t;
+}
+
+// The graph that the current stream of the tensor's device is captured into; nullptr: none.
+cudaGraph_t graph_under_capture(const Tensor& t) {
+  if (!t.is_cuda()) return nullptr;
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  unsigned long long id = 0;
+  cudaGraph_t graph = nullptr;
+  const cudaError_t rc = cudaStreamGetCaptureInfo_v2(at::cuda::getCurrentCUDAStream(t.get_device()).stream(), &status, &id, &graph);
+  if (rc != cudaSuccess) (void)cudaGetLastError();  // (a legacy stream beside another thread's capture: not captured itself)
+  return rc == cudaSuccess && status == cudaStreamCaptureStatusActive ? graph : nullptr;
+}
+
+void keep_for_graph(cudaGraph_t graph, const Tensor& packed) {
+  auto held = std::make_unique<Tensor>(packed);
+  cudaUserObject_t object;
+  C10_CUDA_CHECK(cudaUserObjectCreate(&object, held.get(), release_to_next_call, 1, cudaUserObjectNoDestructorSync));
+  held.release();
+  C10_CUDA_CHECK(cudaGraphRetainUserObject(graph, object, 1, cudaGraphUserObjectMove));
+}
+
 // The packed scales, held by the caller: another thread may take the entry out while this one runs without the interpreter
 // lock. Undefined: not for the cache (inference tensors have no version).
 Tensor swizzled_scales(const Tensor& exponent) {
   if (exponent.is_inference()) return {};
+  free_released();
+  cudaGraph_t graph = graph_under_capture(exponent);
   const void* key = exponent.data_ptr();
   auto hit = swizzled_at.find(key);
   if (hit != swizzled_at.end()) {
     const Swizzled& e = *hit->second;
     if (e.version == exponent._version() && e.source.sizes() == exponent.sizes() && e.source.strides() == exponent.strides()) {
       swizzled.splice(swizzled.begin(), swizzled, hit->second);
+      if (graph != nullptr) keep_for_graph(graph, e.packed);
       return e.packed;
     }
     drop_swizzled(hit);
@@ -312,6 +365,7 @@ Tensor swizzled_scales(const Tensor& exponent) {
   if (made == nullptr) failed();
   const Tensor packed = THPVariable_Unpack(made);
   Py_DECREF(made);
+  if (graph != nullptr) return packed;
   // (the call may have let another thread in, which may have made the same entry: one per key)
   hit = swizzled_at.find(key);
   if (hit != swizzled_at.end()) drop_swizzled(hit);

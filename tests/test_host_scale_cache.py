@@ -1,6 +1,8 @@
 """The cache of swizzled weight scales in the native host path (csrc/host.cpp), which all threads share."""
 
+import gc
 import threading
+import time
 
 import pytest
 import torch
@@ -101,4 +103,66 @@ def test_two_threads_and_an_exponent_that_changes_in_place():
     for thread in threads:
         thread.join()
     assert not wrong
+    ops.reset_call_counts()
+
+
+def linear(seed, rows=96):
+    from flashim_b200.quant import QuantizedTensor, QuantizedWeight
+
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    weight = QuantizedWeight.from_float(torch.randn(256, 128, generator=g, device="cuda") * 0.1)
+    x = torch.randn(rows, 128, generator=g, device="cuda").to(torch.float8_e4m3fn)
+    return QuantizedTensor(x, torch.zeros(4, dtype=torch.int8, device="cuda"), (rows, 128)), torch.zeros(256, dtype=torch.bfloat16, device="cuda"), weight
+
+
+def expected(x, bias, weight):
+    return (x.dequantize().double() @ weight.dequantize().double().t()).float()
+
+
+def evict():
+    for _ in range(ENTRIES):
+        kernels._host().swizzled_scales(exponents(1))
+
+
+@pytest.mark.gpu
+def test_graph_keeps_the_scales_that_it_reads():
+    """The entry goes while the graph lives: the graph reads the same scales, and their memory comes back once it has gone."""
+    from flashim_b200 import ops
+
+    args = linear(2)
+    want = ops.mxfp8_linear(*args)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        out = ops.mxfp8_linear(*args)
+    evict()
+    others = [torch.full((1024,), 255, dtype=torch.uint8, device="cuda") for _ in range(64)]  # (256 x 128 weights have 1 KB of scales)
+    out.zero_()
+    graph.replay()
+    assert torch.equal(out, want) and len(others) == 64
+    torch.cuda.synchronize()
+    held = torch.cuda.memory_allocated()
+    del graph
+    gc.collect()
+    deadline = time.monotonic() + 10
+    while torch.cuda.memory_allocated() >= held and time.monotonic() < deadline:
+        evict()
+    assert torch.cuda.memory_allocated() < held
+    ops.reset_call_counts()
+
+
+@pytest.mark.gpu
+def test_first_use_inside_a_capture():
+    """Scales that only the graph's replays form are not there for calls outside of it."""
+    from flashim_b200 import ops
+
+    ops.mxfp8_linear(*linear(3))  # (kernels loaded)
+    args = linear(4)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        out = ops.mxfp8_linear(*args)
+    got = ops.mxfp8_linear(*args)
+    assert float((got.float() - expected(*args)).norm() / expected(*args).norm()) < 4e-3  # (one bf16 rounding: 2**-9 at most)
+    graph.replay()
+    assert torch.equal(out, got)
     ops.reset_call_counts()
