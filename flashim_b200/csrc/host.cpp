@@ -17,16 +17,20 @@
 #include <ATen/cuda/EmptyTensor.h>
 #include <c10/core/GradMode.h>
 #include <c10/core/impl/TorchDispatchModeTLS.h>
+#include <c10/cuda/CUDACachingAllocator.h>
+#include <c10/cuda/CUDAGraphsC10Utils.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <dlfcn.h>
 #include <torch/csrc/autograd/python_variable.h>
 
+#include <algorithm>
 #include <atomic>
 #include <cstdint>
 #include <list>
 #include <memory>
 #include <mutex>
 #include <unordered_map>
+#include <utility>
 #include <vector>
 
 #include "flashim_sm100.h"
@@ -284,10 +288,22 @@ PyObject* shape_tuple(const Tensor& t) {
 // as it (or an executable made from it) does, whatever becomes of their entry; scales that it has to form are formed by
 // every replay, so the call's own result never exists and is not kept here.
 
+//
+// Any stream may find an entry. Until its scales are known to be formed (`formed`: an event behind the kernels that form them), each
+// call's stream waits for that; and the allocator learns of each stream that reads them beside the one they were allocated on, so that
+// their memory is not given to another tensor before those reads are done.
+
 struct Swizzled {
   const void* key;
   Tensor source, packed;
   uint32_t version;
+  cudaEvent_t formed = nullptr;
+  std::vector<cudaStream_t> readers;  // the first: where the scales were formed
+  Swizzled(const void* k, Tensor s, Tensor p, uint32_t v) : key(k), source(std::move(s)), packed(std::move(p)), version(v) {}
+  Swizzled(const Swizzled&) = delete;
+  ~Swizzled() {
+    if (formed != nullptr) cudaEventDestroy(formed);
+  }
 };
 std::list<Swizzled> swizzled;
 std::unordered_map<const void*, std::list<Swizzled>::iterator> swizzled_at;
@@ -341,6 +357,40 @@ void keep_for_graph(cudaGraph_t graph, const Tensor& packed) {
   C10_CUDA_CHECK(cudaGraphRetainUserObject(graph, object, 1, cudaGraphUserObjectMove));
 }
 
+// Behind the kernels that formed an entry's scales on the current stream of their device
+void mark_formed(Swizzled& e) {
+  if (!e.packed.is_cuda()) return;
+  const c10::cuda::CUDAGuard guard(e.packed.device());
+  const cudaStream_t stream = at::cuda::getCurrentCUDAStream(e.packed.get_device()).stream();
+  C10_CUDA_CHECK(cudaEventCreateWithFlags(&e.formed, cudaEventDisableTiming));
+  C10_CUDA_CHECK(cudaEventRecord(e.formed, stream));
+  e.readers.push_back(stream);
+}
+
+// Ahead of a call that reads them on that stream; false: under capture, and they may not be formed yet (a graph cannot wait for that)
+bool order_reader(Swizzled& e, bool captured) {
+  if (!e.packed.is_cuda()) return true;
+  const auto stream = at::cuda::getCurrentCUDAStream(e.packed.get_device());
+  if (e.formed != nullptr) {
+    // (relaxed: a query counts as unsafe while any thread captures a graph)
+    c10::cuda::CUDAStreamCaptureModeGuard mode(cudaStreamCaptureModeRelaxed);
+    const cudaError_t rc = cudaEventQuery(e.formed);
+    if (rc == cudaSuccess) {
+      C10_CUDA_CHECK(cudaEventDestroy(std::exchange(e.formed, nullptr)));
+    } else {
+      (void)cudaGetLastError();
+      if (rc != cudaErrorNotReady) C10_CUDA_CHECK(rc);
+      if (captured) return false;
+      C10_CUDA_CHECK(cudaStreamWaitEvent(stream.stream(), e.formed, 0));
+    }
+  }
+  if (!captured && std::find(e.readers.begin(), e.readers.end(), stream.stream()) == e.readers.end()) {
+    c10::cuda::CUDACachingAllocator::recordStream(e.packed.storage().data_ptr(), stream);
+    e.readers.push_back(stream.stream());
+  }
+  return true;
+}
+
 // The packed scales, held by the caller: another thread may take the entry out while this one runs without the interpreter
 // lock. Undefined: not for the cache (inference tensors have no version).
 Tensor swizzled_scales(const Tensor& exponent) {
@@ -350,13 +400,14 @@ Tensor swizzled_scales(const Tensor& exponent) {
   const void* key = exponent.data_ptr();
   auto hit = swizzled_at.find(key);
   if (hit != swizzled_at.end()) {
-    const Swizzled& e = *hit->second;
-    if (e.version == exponent._version() && e.source.sizes() == exponent.sizes() && e.source.strides() == exponent.strides()) {
+    Swizzled& e = *hit->second;
+    const bool valid = e.version == exponent._version() && e.source.sizes() == exponent.sizes() && e.source.strides() == exponent.strides();
+    if (valid && order_reader(e, graph != nullptr)) {
       swizzled.splice(swizzled.begin(), swizzled, hit->second);
       if (graph != nullptr) keep_for_graph(graph, e.packed);
       return e.packed;
     }
-    drop_swizzled(hit);
+    if (!valid) drop_swizzled(hit);
   }
   const auto version = static_cast<uint32_t>(exponent._version());
   PyObject* source = wrap(exponent);
@@ -369,8 +420,9 @@ Tensor swizzled_scales(const Tensor& exponent) {
   // (the call may have let another thread in, which may have made the same entry: one per key)
   hit = swizzled_at.find(key);
   if (hit != swizzled_at.end()) drop_swizzled(hit);
-  swizzled.push_front({key, exponent, packed, version});
+  swizzled.emplace_front(key, exponent, packed, version);
   swizzled_at[key] = swizzled.begin();
+  mark_formed(swizzled.front());
   if (swizzled.size() > kSwizzledEntries) drop_swizzled(swizzled_at.find(swizzled.back().key));
   return packed;
 }

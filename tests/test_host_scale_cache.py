@@ -166,3 +166,63 @@ def test_first_use_inside_a_capture():
     graph.replay()
     assert torch.equal(out, got)
     ops.reset_call_counts()
+
+
+BUSY = 200_000_000  # clock ticks: a tenth of a second and more
+
+
+@pytest.fixture()
+def streams():
+    """Two streams with memory of their own, and calls that do not read the status word (which would wait for them)."""
+    from flashim_b200 import ops
+
+    kernels._host().bind(str(_native.LIBRARY_PATH), lambda index: kernels.status_word(torch.device("cuda", index)), _native.check, None,
+                         swizzle_scales, kernels.QuantizedTensor, kernels.Int8Tensor)
+    pair = torch.cuda.Stream(), torch.cuda.Stream()
+    for stream in pair:
+        with torch.cuda.stream(stream):
+            ops.mxfp8_linear(*linear(6))
+    torch.cuda.synchronize()
+    yield pair
+    torch.cuda.synchronize()
+    kernels._host.cache_clear()
+    kernels._host()
+    ops.reset_call_counts()
+
+
+@pytest.mark.gpu
+def test_a_stream_waits_for_the_scales_of_another(streams):
+    """The kernels that form the scales stand behind a long one on their stream; a call on a second stream finds the entry meanwhile."""
+    from flashim_b200 import ops
+
+    args, (first, second) = linear(5), streams
+    want = expected(*args)
+    torch.cuda.synchronize()
+    with torch.cuda.stream(first):
+        torch.cuda._sleep(BUSY)
+        here = ops.mxfp8_linear(*args)
+    with torch.cuda.stream(second):
+        there = ops.mxfp8_linear(*args)
+    assert not first.query()
+    torch.cuda.synchronize()
+    assert torch.equal(here, there) and float((here.float() - want).norm() / want.norm()) < 4e-3  # (one bf16 rounding)
+
+
+@pytest.mark.gpu
+def test_memory_of_scales_that_another_stream_reads(streams):
+    """The entry goes while a call on a second stream has yet to read its scales: the first stream must not get their memory."""
+    from flashim_b200 import ops
+
+    args, (first, second) = linear(7), streams
+    with torch.cuda.stream(first):
+        want = ops.mxfp8_linear(*args)
+    torch.cuda.synchronize()
+    with torch.cuda.stream(second):
+        torch.cuda._sleep(BUSY)
+        got = ops.mxfp8_linear(*args)
+    evict()
+    with torch.cuda.stream(first):
+        others = [torch.full((1024,), 255, dtype=torch.uint8, device="cuda") for _ in range(64)]
+    assert not second.query() and len(others) == 64
+    torch.cuda.synchronize()
+    assert torch.equal(got, want)
