@@ -2248,7 +2248,6 @@ int plan_with(const FimConvGeometry& g, int fmt, bool per_pixel, bool allow_flat
   if (g_forced_block_n == 64) bn = 64;
   if (fmt == kFmtBf16 && bn == 256) bn = 128;  // BF16 layers on this path are narrow pointwise products
   if (bn == 64 && g.cout > 64 && scaled) bn = 128;  // a 64-wide tile may only start at column 0 of its scale tile
-  if (bn == 256 && ragged) return kUnsupported;
   pl.flat = pointwise && allow_flat;
   pl.convert = convert;
   if (convert && !(fmt == kFmtMx && pl.flat && pl.block_k == 128)) return kUnsupported;
@@ -2286,6 +2285,7 @@ int plan_with(const FimConvGeometry& g, int fmt, bool per_pixel, bool allow_flat
     const int narrowest = scaled || patch_layer ? 128 : 64;
     while (g_forced_block_n == 0 && !convert && bn > narrowest && row_tiles * ceil_div(g.cout, bn / 2) <= sms) bn /= 2;
   }
+  if (bn == 256 && ragged) return kUnsupported;  // (the width that the tiles have in the end; the kernel has no such form)
   pl.block_n = bn;
   pl.tiles_n = ceil_div(g.cout, bn);
   // CTA pairs for the wide, compute-bound INT8 tiles: a pair owns two consecutive row tiles (the last one may not exist:
@@ -2385,6 +2385,8 @@ int plan_with(const FimConvGeometry& g, int fmt, bool per_pixel, bool allow_flat
 // for INT8 layers that 64-byte steps divide, which are bound by shared-memory bandwidth (2x200x190x192: 50 against 53 us; MXFP8 68
 // against 60), and not where the divided steps give a layer its halo patches and the ragged ones do not, or it has many tiles to walk:
 // then the larger patches and fewer stages cost more than the rounds (MXFP8 3x100x120x96 15.4 -> 13.3 us, 4x400x400x96 39.8 -> 41.2).
+// A layer whose 256-wide tiles a small problem makes narrower takes them too (us, divided -> ragged: MXFP8 3x3 1x40x40x192 -> 256 10.4 -> 9.5,
+// 2x40x40x480 -> 512 33.1 -> 16.4; 1x1 1000x160 -> 1024 5.4 -> 4.3; INT8 3x3 1x40x40x96 -> 256 8.1 -> 5.8).
 int make_plan(const FimConvGeometry& g, int fmt, bool per_pixel, bool allow_flat, int out_elem, int gelu, Plan* plan, bool convert = false,
               bool pool = false) {
   if (g.cin > 64 && g.cin % 128 != 0 && g.cin % 32 == 0 && (fmt == kFmtMx || (fmt == kFmtI8 && g.cin % 64 != 0)) && !per_pixel && !convert &&

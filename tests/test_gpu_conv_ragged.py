@@ -15,6 +15,8 @@ CASES = [  # batch, height, width, cin, cout, kernel, stride, padding, dilation,
     (1, 19, 21, 96, 96, 3, 1, 1, 1, 2, 0), (1, 19, 21, 96, 64, 3, 1, 2, 2, 1, 0), (1, 30, 20, 224, 64, 1, 1, 0, 1, 2, 0),
     (2, 13, 13, 480, 256, 3, 1, 1, 1, 2, 128), (1, 40, 45, 288, 512, 1, 1, 0, 1, 5, 128), (1, 15, 14, 96, 32, 5, 3, 2, 1, 0, 0),
     (1, 16, 16, 672, 128, 3, 1, 1, 1, 0, 0), (1, 129, 1, 96, 288, 1, 1, 0, 1, 1, 0), (1, 5, 5, 1120, 64, 3, 1, 1, 1, 0, 0),
+    # tiles of 256 columns, made narrower for few of them
+    (1, 40, 40, 192, 256, 3, 1, 1, 1, 0, 0), (1, 21, 19, 160, 512, 3, 2, 1, 1, 0, 0), (1, 40, 40, 96, 256, 1, 1, 0, 1, 0, 0),
 ]
 
 
@@ -53,19 +55,26 @@ def test_ragged_steps_equal_divided_steps(case):
 
 
 def test_plans_take_ragged_steps_where_they_serve():
-    """Widths of the K steps: 128 bytes for channels that 64 does not divide, or 64 does (MXFP8 alone); not for two blocks or fewer, nor 256-wide tiles."""
+    """Widths of the tiles and of their K steps: 128 bytes for channels that 64 does not divide, or 64 does (MXFP8 alone); not for two blocks or
+    fewer, nor for tiles that are 256 wide in the end."""
     from flashim_b200 import _native
 
     lib = _native.library()
 
-    def step(cin, int8, k=3, cout=160):
-        geometry = _native.ConvGeometry(1, 40, 40, cin, cout, k, k, 1, 1, k // 2, k // 2, 1, 1)
+    def plan(cin, int8, k=3, cout=160, size=40):
+        geometry = _native.ConvGeometry(1, size, size, cin, cout, k, k, 1, 1, k // 2, k // 2, 1, 1)
         plan = (ctypes.c_int * 6)()
         assert lib.fim_conv_plan(ctypes.byref(geometry), int8, 0, ctypes.byref(plan)) == 0
-        return plan[3]
+        return plan[2], plan[3]
+
+    def step(*args, **kw):
+        return plan(*args, **kw)[1]
 
     assert [step(c, 0) for c in (32, 64, 96, 128, 160, 192)] == [32, 64, 128, 128, 128, 128]
     assert [step(c, 1) for c in (32, 64, 96, 128, 160, 192)] == [32, 64, 128, 128, 128, 64]
     assert step(992, 0) == 32 and step(992, 0, k=1) == 128  # weight scales of nine taps: more than tensor memory holds
     assert step(192, 0, cout=64) == 64  # keeps its halo patches
-    assert step(192, 0, cout=256) == 64
+    # a 256-wide tile, and one that few tiles make narrower
+    assert plan(192, 0, cout=256, size=200) == (256, 64) and plan(192, 0, cout=256) == (128, 128) and plan(192, 0, cout=512, size=50) == (128, 128)
+    assert plan(96, 0, k=1, cout=256, size=200) == (256, 32) and plan(96, 0, k=1, cout=256) == (128, 128)
+    assert plan(160, 1, cout=256, size=200) == (256, 32) and plan(160, 1, cout=256, size=20) == (64, 128)
