@@ -835,7 +835,7 @@ PyObject* mxfp8_gelu_mlp(Args a) {  // x, w1, b1, hidden_exponent, w2
       return code == FIM_ERR_UNSUPPORTED ? 0 : code;
     });
   }
-  if (code == FIM_ERR_UNSUPPORTED) {  // a bias of another type, 64 channels or fewer
+  if (code == FIM_ERR_UNSUPPORTED) {  // a bias of another type, a plan without 128-byte K steps or with 64-wide tiles
     const Tensor bias = b1->scalar_type() == kF32 && b1->is_contiguous() ? *b1 : b1->to(kF32).contiguous();
     Tensor h = mx_gemm(*v, rows, e, nullptr, *w1, packed1, nullptr, call, "mxfp8_gelu_mlp");
     call.launch("mxfp8_gelu_mlp", [&] {

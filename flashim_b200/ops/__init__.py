@@ -48,7 +48,7 @@ mxfp8_linear = Op("mxfp8_linear", doc="(activation QuantizedTensor [rows, K], bi
 gelu_quantize = Op("gelu_quantize", doc="(value bf16 [..., C], scale_exponent, approximate='none', *, input_bias=None) -> "
                    "QuantizedTensor: quantize_static(GELU(value [+ input_bias])) (flashim/ops/quantize.py:62-74)")
 mxfp8_gelu_mlp = Op("mxfp8_gelu_mlp", doc="(x QuantizedTensor, w1 QuantizedWeight, b1, hidden_exponent, w2 QuantizedWeight) -> bf16 "
-                    "[rows, N2]: linear, GELU(+ b1), static requantisation, linear (flashim/ops/gemm.py:146-157)")
+                    "[rows, N2]: linear, GELU(+ b1), static requantisation, linear (flashim/ops/gemm.py:146-157); hidden widths up to 2048")
 depthwise5x5_relu_pointwise = Op("depthwise5x5_relu_pointwise", doc="(value [B, C, H, W], dw_weight bf16 [25, C], dw_bias [C], pw_weight "
                                  "bf16 [N, C], pw_bias bf16 [N]) -> bf16 channels-last [B, N, H, W]: the bf16 refiner block "
                                  "(flashim/ops/conv.py:67-87)")

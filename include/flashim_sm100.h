@@ -37,8 +37,11 @@ extern "C" {
 #define FIM_ACT_RELU 1
 #define FIM_ACT_GELU 2
 #define FIM_ACT_RELU_EARLY 3 /* conv epilogues: ReLU before the residual add (the order of flashim/ops/gemm.py:87-98) */
-#define FIM_ACT_GELU_SUM 4   /* block-scaled 1x1 convs with a bias and FIM_OUT_E4M3_STATIC (cin and cout above 64, else FIM_ERR_UNSUPPORTED): erf
-                              * GELU of bf16(product) + bias, the sum in fp32 (the order of flashim/ops/gemm.py:146-157) */
+#define FIM_ACT_GELU_SUM 4   /* block-scaled 1x1 convs (stride 1, unpadded) with a bias, without a residual, and FIM_OUT_E4M3_STATIC: erf GELU of
+                              * bf16(product) + bias, the sum in fp32 (the order of flashim/ops/gemm.py:146-157). Only where the chosen
+                              * plan (fim_conv_plan) has tiles of 128 or 256 channels and K steps of 128 bytes, FIM_ERR_UNSUPPORTED
+                              * elsewhere: cin or cout of at most 64; cin that 128 does not divide under 256-wide tiles (cout a multiple of
+                              * 256, cout >= cin, and more 128-wide tiles than SMs), as 4000 rows of 192 -> 768 */
 
 /* What the conv epilogue writes. */
 #define FIM_OUT_BF16 0         /* bf16 [B,Ho,Wo,Cout] */
@@ -178,7 +181,8 @@ typedef struct FimConvEpilogue {
 
 /* Block-scaled MXFP8 conv: x E4M3 NHWC; activation scales either static (`act_exponent` int8 [cin/32], shared by every
  * pixel and tap) or per pixel (`act_scales_swizzled`: E8M0 bytes in the 128x4 swizzled layout over rows = B*H*W; 1x1
- * stride-1 unpadded convs only). Strides 1 to 4 are supported (a strided conv reads every stride-th pixel through the
+ * stride-1 unpadded convs only). Static exponents serve at most 2048 input channels (FIM_ERR_UNSUPPORTED above), which also limits the hidden
+ * width of the GELU MLP built from two calls. Strides 1 to 4 are supported (a strided conv reads every stride-th pixel through the
  * tensor map's element strides); weight E4M3 [cout, kh*kw*cin]; `weight_scales_swizzled`: E8M0 bytes of the
  * [cout, kh*kw*cin/32] exponents in the 128x4 swizzled layout. fp32 accumulation in tensor memory, epilogue
  * bias -> bf16 rounding -> GELU -> residual add (one more bf16 rounding) -> ReLU -> requantisation, as `epilogue` selects:

@@ -156,7 +156,9 @@ def test_strided_golden_cases(ops, golden):
 
 @pytest.mark.parametrize("rows,cin,hidden,bias", [
     (1, 128, 32, BF16), (127, 128, 96, BF16), (129, 384, 512, BF16), (300, 256, 1056, BF16), (3000, 128, 288, BF16),
-    (40, 64, 128, BF16), (40, 128, 128, torch.float32),  # a separate GELU launch: channels, type of the bias
+    (300, 192, 768, BF16), (300, 160, 1024, BF16),  # ragged K steps, since few tiles are narrowed to 128 columns
+    # a separate GELU launch: channels, 256-wide tiles without ragged K steps, type of the bias
+    (40, 64, 128, BF16), (4000, 192, 768, BF16), (40, 128, 128, torch.float32),
 ])
 def test_gelu_mlp_in_the_epilogue_agrees_with_its_steps(ops, rows, cin, hidden, bias):
     """GELU of the bf16 product plus bias and the quantiser behind it, in the epilogue of the first product: the bytes of the product,
@@ -171,3 +173,26 @@ def test_gelu_mlp_in_the_epilogue_agrees_with_its_steps(ops, rows, cin, hidden, 
     b1, exponent = rand(hidden).to(bias), torch.full((hidden // 32,), -6, dtype=torch.int8, device=DEV)
     codes = ops.gelu_quantize(ops.mxfp8_linear(x, None, w1), exponent, input_bias=b1)
     assert same_bytes(ops.mxfp8_gelu_mlp(x, w1, b1, exponent, w2), ops.mxfp8_linear(codes, None, w2))
+
+
+def test_where_the_gelu_of_a_sum_is_supported(ops):
+    """The plans that the header names for FIM_ACT_GELU_SUM, by what the C call returns."""
+    import ctypes
+
+    from flashim_b200 import _native
+
+    def code(rows, cin, cout):
+        z = lambda *shape: torch.zeros(shape, dtype=torch.uint8, device=DEV)  # noqa: E731
+        x, exponent, weight, scales = z(rows, cin), z(cin // 32), z(cout, cin), z((cout + 127) // 128 * 128 * ((cin // 32 + 3) // 4) * 4)
+        bias, out, hidden, status = z(2 * cout), z(rows, cout), z(cout // 32), torch.zeros(1, dtype=torch.int32, device=DEV)
+        geometry = _native.ConvGeometry(1, 1, rows, cin, cout, 1, 1, 1, 1, 0, 0, 1, 1)
+        epilogue = _native.ConvEpilogue()
+        epilogue.bias, epilogue.act, epilogue.out_mode, epilogue.out_exponent = bias.data_ptr(), 4, 2, hidden.data_ptr()
+        result = _native.library().fim_mxfp8_conv2d(x.data_ptr(), exponent.data_ptr(), None, weight.data_ptr(), scales.data_ptr(), ctypes.byref(geometry),
+                                                    ctypes.byref(epilogue), out.data_ptr(), status.data_ptr(), torch.cuda.current_stream().cuda_stream)
+        torch.cuda.synchronize()
+        assert int(status) == 0
+        return result
+
+    assert [code(*c) for c in ((300, 128, 96), (300, 192, 768), (300, 160, 1024), (4000, 256, 768), (4000, 192, 512 + 32))] == [0] * 5
+    assert [code(*c) for c in ((300, 64, 128), (300, 128, 64), (4000, 192, 768), (40, 2080, 128))] == [99] * 4
