@@ -611,7 +611,7 @@ conv_kernel(const __grid_constant__ CUtensorMap act_map, const __grid_constant__
   constexpr int kAccStages = acc_stages(BN);
   constexpr int kScaleTilesB = scale_tiles_b(BN);
   constexpr int kKSteps = BK / 32;
-  constexpr bool kMayBeRagged = BK == 128 && BN <= 128;  // (256-wide tiles lose 1 % to the tests: 4x100x100x512 78 -> 79 us)
+  constexpr bool kMayBeRagged = BK == 128 && BN <= 128 && !PAIR;  // (256-wide tiles lose 1 % to the tests: 4x100x100x512 78 -> 79 us)
   constexpr uint32_t kABytes = kTileM * BK, kBBytes = (PAIR ? BN / 2 : BN) * BK;  // per CTA
   constexpr int kWeightBoxRows = BN < 128 ? BN : 128;  // rows of one weight TMA box
   constexpr uint32_t kSfbColumns = BN < 128 ? 4 : BN / 32;
@@ -1169,7 +1169,7 @@ conv_kernel(const __grid_constant__ CUtensorMap act_map, const __grid_constant__
             const uint32_t new_tile = (kb + steps - 1) >> 2;
             const bool begins = kb == 0 || new_tile != (kb - 1) >> 2;
             if (kLaneLoop || elect_one()) {
-              if constexpr (SCALED && !PAIR) {
+              if constexpr (SCALED) {
 #pragma unroll
                 for (int i = 0; i < kScaleTilesB; ++i) {
                   if (i < scale_tiles && copy_scales && fresh && begins) tc_copy_scales(sfb_resident_base + kSfbColumns * new_tile + 4 * i, sfb_from + 32 * i);
@@ -1180,23 +1180,14 @@ conv_kernel(const __grid_constant__ CUtensorMap act_map, const __grid_constant__
                 if (k < steps) {
                   const uint32_t accumulate = k > 0 ? 1u : first;
                   if (INT8) {
-                    if (PAIR) {
-                      tc_mma_i8_pair(d_tmem, a_desc + 2 * k, b_desc + 2 * k, idesc, accumulate);
-                    } else {
-                      tc_mma_i8(d_tmem, a_desc + 2 * k, b_desc + 2 * k, idesc, accumulate);
-                    }
-                  } else if constexpr (SCALED && !PAIR) {
+                    tc_mma_i8(d_tmem, a_desc + 2 * k, b_desc + 2 * k, idesc, accumulate);
+                  } else if constexpr (SCALED) {
                     tc_mma_mxf8(d_tmem, a_desc + 2 * k, b_desc + 2 * k, idesc | (static_cast<uint32_t>(k) << 29) | (((kb + k) & 3u) << 4), sfa_tmem,
                                 sfb_resident_base + kSfbColumns * ((kb + k) >> 2), accumulate);
                   }
                 }
               }
-              if (PAIR) {
-                tc_commit_pair(empty0 + 8 * s);
-                tc_commit_pair((empty0 + 8 * s) | kPeerBit);
-              } else {
-                tc_commit(&ctl.empty[s]);
-              }
+              tc_commit(&ctl.empty[s]);
             }
             kb += static_cast<uint32_t>(steps);
           } else if (kLaneLoop || elect_one()) {
@@ -2291,7 +2282,7 @@ int plan_with(const FimConvGeometry& g, int fmt, bool per_pixel, bool allow_flat
   // CTA pairs for the wide, compute-bound INT8 tiles: a pair owns two consecutive row tiles (the last one may not exist:
   // its loads are zero-filled and its stores clipped). The block-scaled form is correct too but measured slower than
   // single CTAs (its scale copies serialise the pair's tensor pipes): it only runs when asked for (tuning flag 128).
-  pl.pair = bn == 256 && row_tiles >= 2 && !(g_debug_flags & 64) && (int8 || ((g_debug_flags & 128) && !ragged)) && !convert;
+  pl.pair = bn == 256 && row_tiles >= 2 && !(g_debug_flags & 64) && (int8 || (g_debug_flags & 128)) && !convert;
   // A 128-wide block-scaled tile moves as many operand bytes through shared memory per MMA as the tensor pipe takes
   // twice as fast; a pair halves the weight bytes per CTA (64 rows each). Worth it for a spatial conv with many tiles
   // (3x3 128 -> 128 at 400 x 400: 118 -> 107 us), not for a small one, not for a flat 1x1 layer, whose short epilogue

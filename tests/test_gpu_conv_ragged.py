@@ -78,3 +78,11 @@ def test_plans_take_ragged_steps_where_they_serve():
     assert plan(192, 0, cout=256, size=200) == (256, 64) and plan(192, 0, cout=256) == (128, 128) and plan(192, 0, cout=512, size=50) == (128, 128)
     assert plan(96, 0, k=1, cout=256, size=200) == (256, 32) and plan(96, 0, k=1, cout=256) == (128, 128)
     assert plan(160, 1, cout=256, size=200) == (256, 32) and plan(160, 1, cout=256, size=20) == (64, 128)
+    # the kernel has no CTA pairs with ragged steps: none are planned, whatever is asked for
+    for cin, int8, size, k in ((96, 0, 400, 3), (160, 0, 200, 1), (96, 1, 200, 3), (160, 1, 400, 1)):
+        for flags in (0, 128, 16384, 128 | 16384):
+            for width in (0, 128, 256):
+                with conv_schedule(width, 0, flags) as c:
+                    ragged = plan(cin, int8, k, 512, size)[1] == 128
+                    assert not (ragged and c.schedule((1, size, size, cin, 512, k, k, k // 2, 1), bool(int8))["pairs"])
+                    assert ragged or width != 128
