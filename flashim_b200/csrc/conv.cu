@@ -2757,7 +2757,7 @@ int run_conv(int fmt, const void* x, const int8_t* act_exponent, const void* act
       if (rcp != kOk) return rcp;
     }
   }
-  if (fmt == kFmtMx && p.warp_panels && !pl.pair && pl.block_n >= 128 && pl.block_k == 128 && p.bias != nullptr &&
+  if (fmt == kFmtMx && pl.flat && p.warp_panels && !pl.pair && pl.block_n >= 128 && pl.block_k == 128 && p.bias != nullptr &&
       !(g_debug_flags & 1024)) {
     const bool plain = p.act == kActNone && p.out_mode == FIM_OUT_BF16;
     const bool res_ok = p.residual != nullptr && p.res_stride[3] == 1 && p.res_channels >= p.cout && p.res_stride[2] % 8 == 0 &&
