@@ -215,6 +215,10 @@ __device__ __forceinline__ int gelu_highest(const uint32_t (&r)[16]) {
   return max(static_cast<int>(high) >> 16, static_cast<int>(static_cast<int16_t>(high & 0xFFFFu)));
 }
 
+// The two forms below agree wherever the result is 2**-126 or more. Of smaller (subnormal) results the table drops bits and the arithmetic
+// rounds; exponents below -116 show them, and there a code may depend on which form the other rows of the warp ask for. (Making the choice
+// invisible, by a test for such blocks or by arithmetic for these halves behind the table, cost the layers 1 to 3 %.)
+//
 // GELU of 32 values under a static exponent: by arithmetic, unless one of the warp's lanes asks for the table. One vote decides where most
 // exponents leave it: a warp's time for its chunk is what a tile of a patch layer waits for, and a second vote on that way costs 3 to 5 %.
 __device__ __forceinline__ void gelu_chunk_static(uint32_t (&r)[16], int e, const GeluTable& table) {

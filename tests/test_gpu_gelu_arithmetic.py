@@ -25,7 +25,7 @@ def values(bits):
 
 
 def normal(bias):
-    """Results of arguments below 2**-125 are subnormal: the table gives zero or half the bits, the arithmetic torch's rounding."""
+    """Results of arguments below 2**-125 are subnormal: the table gives zero or half the bits, the arithmetic rounds."""
     magnitude = bias.view(torch.int16).to(torch.int32) & 0x7FFF
     return (magnitude == 0) | (magnitude >= 0x100)
 
