@@ -160,7 +160,10 @@ __device__ __forceinline__ Floats<N> load_floats(const float* at) {
   return r;
 }
 
-// n / d from inv = RN(1 / d): the quotient, corrected once by its exact residual
+// n / d from inv = RN(1 / d): the quotient, corrected once by its residual (Markstein, "Computation of elementary functions on the IBM RISC
+// System/6000 processor", 1990). For odd whole n below 2**22 and whole d below 2**21 it is the correctly rounded quotient: the first one is less
+// than two ulp away, so its residual is exact, and the corrected sum is off by less than 2**-22 ulp before its last rounding, while n / d lies at
+// least 1 / (2 d) ulp from every midpoint of two neighbours (d times a midpoint is a whole multiple of half an ulp that n cannot be).
 __device__ __forceinline__ float divided(float n, float d, float inv) {
   const float q = n * inv;
   return fmaf(fmaf(-q, d, n), inv, q);

@@ -105,3 +105,22 @@ def test_refiner_input_patches_inside_and_across_the_edges(ops, case):
     # a correlation, by at most 8e-6 times the difference of two neighbours, below 10 for these values.
     bad = (bf16_ulp_distance(got, want) > 1) & ((got.float() - want.float()).abs() > 1e-4)
     assert not bad.any()
+
+
+def test_quotients_of_the_pixel_grid(ops):
+    """The kernel's (2 i + 1) / size is CUDA's division to the bit: the displacement of a warp that holds each pixel's own coordinates, formed with
+    that division, is exactly zero, whatever it is scaled by."""
+    sizes = [*range(1, 130), 255, 257, 509, 511, 513, 719, 1000, 1023, 1025, 2047, 2049, 3001, 4095, 4097, 8191, 8193, 30011, 65537]
+    rest = torch.ones(1, 2, 1, 1, device="cuda"), torch.zeros(1, device="cuda"), torch.full((2,), 1e20, device="cuda")
+    for size in sizes:
+        odd = 2 * torch.arange(size, device="cuda", dtype=torch.float32) + 1
+        grid = -1 + odd / torch.full_like(odd, size)  # (by a number of the host torch multiplies with its reciprocal)
+        assert torch.equal(grid.cpu(), -1 + odd.cpu() / size)
+        for height, width in ((1, size), (size, 1)):
+            own = torch.zeros(1, height, width, 2, device="cuda")  # (of a size of one: -1 + 1 / 1)
+            own[..., 0 if height == 1 else 1] = grid.view(1, height, width)
+            f = torch.zeros(1, height, width, 32, device="cuda")
+            got = ops.romav2_refiner_input(f, f, own, *rest, 0, 0).permute(0, 2, 3, 1)
+            assert not got[..., 64].any(), (height, width)
+    wrong = torch.nextafter(grid, torch.full_like(grid, 2.0)).view(1, 1, -1)
+    assert ops.romav2_refiner_input(f.view(1, 1, -1, 32), f.view(1, 1, -1, 32), torch.stack((wrong, torch.zeros_like(wrong)), -1), *rest, 0, 0)[:, 64].all()
