@@ -139,7 +139,7 @@ struct GeluTable {
 };
 // `copies` > 1 (a power of two): entry e of copy c is word e * copies + c, and a lane reads copy lane % copies. Lanes of
 // different copies never share a bank, so the 32 scattered reads of a look-up take about 2.9 passes with eight copies
-// where one copy takes 3.4: what bounds layers with short main loops whose outputs are bf16 or have exponents per pixel (with static
+// where one copy takes 3.4 (two: 3.4, four: 3.3): what bounds layers with short main loops whose outputs are bf16 or have exponents per pixel (with static
 // exponents, before the arithmetic below: 3x3 64 -> 64 at 800x800 176 -> 154 us).
 __device__ __forceinline__ GeluTable gelu_table_at(uint32_t smem_address, uint32_t copies = 1, uint32_t lane = 0) {
   GeluTable t;
@@ -173,7 +173,7 @@ __device__ __forceinline__ uint32_t gelu_bf16x2(uint32_t r, const GeluTable& tab
 // some. Below, torch's own result is the rounding noise of 1 + erf, which no polynomial follows, but the E4M3 codes of both are the
 // same under every exponent from -9 up, except those of one value under -6 and of one under -2 (gelu_replace). Arguments in that tail under
 // smaller exponents, infinities and not-a-numbers take the table. As many issue slots as the look-up, and none of the shared-memory wavefronts that bounded these
-// epilogues (32 scattered reads take 3.3 passes, 2.9 with eight copies of the table): us, table -> arithmetic:
+// epilogues (32 scattered reads take 3.4 passes, 2.9 with eight copies of the table): us, table -> arithmetic:
 // 3x3 4x800x800x64 135 -> 122, 4x400x400x128 89 -> 74; 1x1 8x100x100x512 -> 1024 65 -> 59; residual MLP 8x400x400x128 255 -> 229 (arguments of
 // a standard deviation of 1.4, many of them in the tail: 243), 8x200x200x256 164 -> 140.
 __device__ __forceinline__ uint32_t gelu_arithmetic_bf16x2(uint32_t r) {
@@ -315,7 +315,9 @@ constexpr int kEpiGelu = 1, kEpiDynamic = 2, kEpiResidual = 4, kEpiLean = 8, kEp
 // kEpiGeluSum (with kEpiFixed | kEpiStatic): the first product of a GELU MLP, whose bias is added behind the bf16 rounding and whose
 // GELU takes the fp32 sum, so that no table serves it: bf16(erf GELU(bf16(acc) + bias)) -> E4M3, the steps of
 // gelu_quantize_mx_kernel on the same values. A lane evaluates 32 error functions per chunk, which the main loop of a short K does not
-// hide; still the hidden tensor crosses memory once and as bytes, and a launch goes (MLP of 1000 x 256 x 1024: 18.0 -> 14.2 us, 20000 x 384 x 1536: 119 -> 69).
+// hide; still the hidden tensor crosses memory once and as bytes, and a launch goes. Whatever K: us of the MLP (without its input quantiser, back to back), three launches -> two:
+// 1000 x 256 x 1024 14.6 -> 13.3, 20000 x 384 x 1536 109 -> 62, 1000 x 2048 x 2048 23.8 -> 21.2, 20000 x 2048 x 2048 318 -> 197; one row tile, 100 x 1024 x 1024,
+// 14.2 -> 14.4.
 constexpr int kEpiGeluSum = 256;
 // kEpiArithmetic (with kEpiFixed | kEpiGelu | kEpiStatic): the GELU by arithmetic. For patches and layers with a short K, whose epilogue is
 // what a tile waits for; behind a long main loop, which the power limit governs, the table is the cheaper one (4x100x100x512 3x3,
@@ -2178,7 +2180,8 @@ mlp_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constant__ CU
 // how the epilogue of a layer comes by its GELU (none: 0)
 constexpr int kGeluByTable = 1, kGeluByArithmetic = 2;
 // K steps up to which kEpiArithmetic serves tiles that come through the stage ring (1x1 4x100x100x768 -> 768, six steps: 33.8 -> 29.9 us;
-// 1024 -> 512, eight: 28.0 -> 26.4; 3x3 4x200x200x256, eighteen: 80.1 with the table, 82.6 without)
+// 1024 -> 512, eight: 28.0 -> 26.4; 3x3 4x200x200x256, eighteen: 80.1 with the table, 82.6 without). 64-wide tiles take it whatever their K, since they
+// take the same time either way (3x3 stride 2 4x200x200x192 21.2 us, 1x60x60x960 26.0; 1x1 2x100x100x1984 15.9).
 constexpr int kArithmeticSteps = 8;
 
 int g_forced_block_n = 0;

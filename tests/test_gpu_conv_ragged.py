@@ -78,6 +78,11 @@ def test_plans_take_ragged_steps_where_they_serve():
     assert plan(192, 0, cout=256, size=200) == (256, 64) and plan(192, 0, cout=256) == (128, 128) and plan(192, 0, cout=512, size=50) == (128, 128)
     assert plan(96, 0, k=1, cout=256, size=200) == (256, 32) and plan(96, 0, k=1, cout=256) == (128, 128)
     assert plan(160, 1, cout=256, size=200) == (256, 32) and plan(160, 1, cout=256, size=20) == (64, 128)
+    # patches: while a CTA has few of them to walk, up to six
+    sms = torch.cuda.get_device_properties(0).multi_processor_count if torch.cuda.is_available() else 148
+    for size in (72, 136, 200, 240, 264, 400):  # 8 x 16 pixels each
+        tiles = -(-size // 8) * -(-size // 16)
+        assert step(96, 0, cout=64, size=size) == (128 if tiles <= 6 * min(sms, tiles) else 32)
     # the kernel has no CTA pairs with ragged steps: none are planned, whatever is asked for
     for cin, int8, size, k in ((96, 0, 400, 3), (160, 0, 200, 1), (96, 1, 200, 3), (160, 1, 400, 1)):
         for flags in (0, 128, 16384, 128 | 16384):
