@@ -130,4 +130,4 @@ def test_a_wide_spread_costs_little(fused):
             end.record()
             end.synchronize()
             times[i].append(start.elapsed_time(end))
-    assert sorted(times[1])[7] < 1.22 * sorted(times[0])[7], times
+    assert min(times[1]) < 1.22 * min(times[0]), times  # (the power limit makes single ones longer, wide arguments first)
